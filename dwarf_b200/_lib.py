@@ -60,6 +60,7 @@ _SIGNATURES = {
     "dsqg_ring_prefill": (c_int, [c_void_p] * 6 + [c_int] * 6 + [c_void_p]),
     "dsqg_decode": (c_int, [c_void_p] * 3 + [c_void_p] * 2 + [c_void_p] * 2 + [c_void_p] * 3
                     + [POINTER(c_int32), c_int, c_int] + [c_void_p] + [c_int] * 4 + [c_void_p]),
+    "dsqg_ring_advance": (c_int, [c_void_p] * 4 + [c_int] * 2 + [c_void_p]),
     "dsqg_causal_mean": (c_int, [c_void_p, c_void_p] + [c_int] * 5 + [c_void_p]),
     "dsqg_decode_kv": (c_int, [c_void_p] * 3 + [c_void_p] + [c_void_p] * 2 + [c_void_p] * 3
                        + [POINTER(c_int32), c_int, c_int] + [c_void_p] + [c_int] * 4 + [c_void_p, c_int]),
@@ -99,6 +100,39 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_ext = None
+
+
+def native():
+    """The native host side of the Python operators (_dsqg_torch.so).  Raises if it is not built."""
+    global _ext
+    if _ext is None:
+        load()
+        try:
+            from . import _dsqg_torch
+        except ImportError as e:
+            raise ImportError("dwarf_b200/_dsqg_torch.so is missing or does not load. Build it with `python -m dwarf_b200.build`. "
+                              "dwarf_b200 has no fallback path.") from e
+        _ext = _dsqg_torch
+    return _ext
+
+
+_handles = {}
+
+
+def offsets_handle(offsets):
+    """The native form of an offset set (converted once per set)."""
+    if type(offsets) is tuple:
+        h = _handles.get(offsets)
+        if h is not None:
+            return h
+    key = tuple(int(o) for o in offsets)
+    h = _handles.get(key)
+    if h is None:
+        h = _handles[key] = native().offsets(list(key))
+    return h
 
 
 def check(status: int, where: str):

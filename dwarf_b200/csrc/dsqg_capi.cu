@@ -394,6 +394,13 @@ int dsqg_decode_kv(const void* q, const void* k_new, const void* v_new, void* kv
                        offsets, J, R, out, S, H, D, dtype, stream, overlapped != 0, true);
 }
 
+int dsqg_ring_advance(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R, void* stream) {
+    if (!head || !fill || !head_out || !fill_out) return DSQG_ERR_NULL_POINTER;
+    if (S < 1 || R < 1) return DSQG_ERR_BAD_SHAPE;
+    cudaError_t e = launch_ring_advance(head, fill, head_out, fill_out, S, R, static_cast<cudaStream_t>(stream));
+    return e == cudaSuccess ? DSQG_OK : cuda_fail(e);
+}
+
 int dsqg_ring_prefill_kv(const void* k, const void* v, void* kv_ring,
                          int32_t* head, int32_t* fill, int S, int H, int N, int D, int R, int dtype, void* stream) {
     if (!k || !v || !kv_ring || !head || !fill) return DSQG_ERR_NULL_POINTER;

@@ -84,6 +84,7 @@ cudaError_t launch_decode(const DecodeArgs& a, const Taps& t, int dtype, cudaStr
 cudaError_t launch_ring_prefill(const void* k, const void* v, void* k_ring, void* v_ring, int32_t* head, int32_t* fill,
                                 int S, int H, int N, int D, int R, int dtype, cudaStream_t s, bool interleaved = false);
 
+cudaError_t launch_ring_advance(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R, cudaStream_t s);
 cudaError_t launch_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, bool reverse, cudaStream_t s);
 cudaError_t launch_gate_bwd(const void* dy, const void* y, const void* gate, long long sb, long long sh, long long sn,
                             void* dout, void* dgate, float* delta, int B, int H, int N, int D, cudaStream_t s);

@@ -352,6 +352,19 @@ cudaError_t launch_ring_prefill(const void* k, const void* v, void* k_ring, void
     return cudaGetLastError();
 }
 
+__global__ void __launch_bounds__(256) ring_advance_kernel(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R) {
+    const int s = blockIdx.x * 256 + threadIdx.x;
+    if (s >= S) return;
+    const int h = (head[s] + 1) % R;
+    head_out[s] = h < 0 ? h + R : h;
+    fill_out[s] = min(fill[s] + 1, R);
+}
+
+cudaError_t launch_ring_advance(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R, cudaStream_t s) {
+    ring_advance_kernel<<<(S + 255) / 256, 256, 0, s>>>(head, fill, head_out, fill_out, S, R);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_decode(const DecodeArgs& a, const Taps& t, int dtype, cudaStream_t s, bool overlap) {
     if (dtype == DSQG_DTYPE_BF16) DSQG_DECODE_TPR(__nv_bfloat16);
     DSQG_DECODE_TPR(float);

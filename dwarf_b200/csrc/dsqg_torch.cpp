@@ -1,0 +1,424 @@
+// Host side of the Python operators: argument checks, allocation of results, the autograd nodes and the calls
+// into the C ABI, in native code.  One call costs the host a few microseconds; the same steps in Python
+// (ctypes conversions, a Python autograd.Function, tensors created one by one) cost 35-60 us per direction, more than the
+// kernels of small problems and of a decode step take.
+//
+// PyTorch supplies device memory, streams and the autograd graph only; all arithmetic is in libdsqg_b200.so.
+#include <torch/extension.h>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/Exceptions.h>
+
+#include <cmath>
+#include <map>
+#include <memory>
+#include <mutex>
+#include <optional>
+#include <sstream>
+
+#include "dsqg_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::AutogradContext;
+using torch::autograd::variable_list;
+
+namespace {
+
+// An offset set, converted once and kept for the life of the process (programs use a handful): autograd nodes and
+// the Python cache (ops._offsets) hold plain pointers to it.
+struct Offsets {
+    std::vector<int32_t> v;
+    int J() const { return (int)v.size(); }
+};
+
+const Offsets* intern_offsets(const std::vector<int32_t>& v) {
+    static std::mutex mu;
+    static std::map<std::vector<int32_t>, std::unique_ptr<Offsets>> table;
+    std::lock_guard<std::mutex> lock(mu);
+    std::unique_ptr<Offsets>& o = table[v];
+    if (!o) { o = std::make_unique<Offsets>(); o->v = v; }
+    return o.get();
+}
+
+// Raises dwarf_b200.DSQGError for a non-zero status.
+void check(int status, const char* where) {
+    if (status == DSQG_OK) return;
+    py::gil_scoped_acquire gil;
+    py::module_::import("dwarf_b200._lib").attr("check")(status, where);
+    throw std::runtime_error(std::string(where) + " failed");
+}
+
+// Runs the body of a backward node: the autograd engine's threads carry Python errors in its own exception type.
+template <typename F> auto backward_body(F f) {
+    try {
+        return f();
+    } catch (py::error_already_set& e) {
+        py::gil_scoped_acquire gil;
+        e.restore();
+        python_error err;
+        err.persist();
+        throw err;
+    }
+}
+
+int dtype_code(const Tensor& t) {
+    if (t.scalar_type() == at::kBFloat16) return DSQG_DTYPE_BF16;
+    if (t.scalar_type() == at::kFloat) return DSQG_DTYPE_F32;
+    throw py::type_error(std::string("dsqg: q/k/v must be bfloat16 or float32, got ") + toString(t.scalar_type()));
+}
+
+std::string shape_of(const Tensor& t) {
+    std::ostringstream s;
+    s << t.sizes();
+    return s.str();
+}
+
+void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
+void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+// A parameter as the kernels read it: fp32, contiguous, detached.
+Tensor f32c(const Tensor& t) {
+    if (!t.defined()) return t;
+    const Tensor d = t.requires_grad() ? t.detach() : t;
+    return (d.scalar_type() == at::kFloat ? d : d.to(at::kFloat)).contiguous();
+}
+Tensor like_param(Tensor g, at::ScalarType dt) { return g.defined() && g.scalar_type() != dt ? g.to(dt) : g; }
+Tensor opt(const std::optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); }
+at::ScalarType type_of(const Tensor& t) { return t.defined() ? t.scalar_type() : at::kFloat; }
+
+bool shape_is(const Tensor& t, std::initializer_list<int64_t> s) { return t.sizes() == at::IntArrayRef(s); }
+
+void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& pb, const Tensor& hg, const Tensor& se, int J) {
+    if (!q.is_cuda()) throw std::runtime_error("dsqg: tensors must live on a CUDA device (there is no CPU path)");
+    if (q.dim() != 4) throw py::value_error("dsqg: q must be [B,H,N,HD], got " + shape_of(q));
+    const int64_t H = q.size(1), D = q.size(3);
+    for (const Tensor* t : {&k, &v})
+        if (t->sizes() != q.sizes() || t->scalar_type() != q.scalar_type() || t->device() != q.device())
+            throw py::value_error(std::string("dsqg: ") + (t == &k ? "k" : "v") + " must match q in shape, dtype and device");
+    auto want = [](const char* n, int64_t a, int64_t b, const Tensor& t) {
+        throw py::value_error(std::string("dsqg: ") + n + " must be [" + std::to_string(a) + (b ? "," + std::to_string(b) : "") + "], got " + shape_of(t));
+    };
+    if (!shape_is(pb, {J, H})) want("pos_bias", J, H, pb);
+    if (se.defined() && !shape_is(se, {J, D})) want("scale_embed", J, D, se);
+    if (hg.defined() && !shape_is(hg, {H})) want("head_gain", H, 0, hg);
+}
+
+// Head dimension the kernels are called with (ops._padded_head_dim has the reasons).
+int64_t padded_head_dim(const Tensor& q, const Offsets& off, bool has_se) {
+    const int64_t D = q.size(3);
+    if (q.scalar_type() != at::kBFloat16 || D % 32 == 0 || D > 128 || D % 8 != 0) return D;
+    const int64_t Dp = (D + 31) / 32 * 32;
+    return dsqg_tensor_core_path(DSQG_DTYPE_BF16, (int)Dp, off.v.data(), off.J(), has_se) ? Dp : D;
+}
+
+Tensor pad_to(const Tensor& t, int64_t Dp) { return t.defined() ? at::constant_pad_nd(t, {0, Dp - t.size(-1)}) : t; }
+
+// Scratch for one backward call, returned to the caching allocator when it leaves scope.
+at::DataPtr scratch_for(size_t bytes) { return c10::cuda::CUDACachingAllocator::get()->allocate(bytes); }
+
+// ------------------------------------------------------------------------------------ dsqg_attention
+struct Forward { Tensor q, k, v, pb, hg, se, out, lse; int64_t D; };
+
+Forward attention_forward(const Tensor& q0, const Tensor& k0, const Tensor& v0, const Tensor& pos_bias, const Tensor& head_gain,
+                          const Tensor& scale_embed, const Offsets& off) {
+    check_inputs(q0, k0, v0, pos_bias, head_gain, scale_embed, off.J());
+    const int dt = dtype_code(q0);
+    const c10::cuda::CUDAGuard guard(q0.device());
+    Forward f;
+    f.pb = f32c(pos_bias); f.hg = f32c(head_gain); f.se = f32c(scale_embed);
+    f.D = q0.size(3);
+    const int64_t Dp = padded_head_dim(q0, off, scale_embed.defined());
+    f.q = q0; f.k = k0; f.v = v0;
+    if (Dp != f.D) {                                    // zero columns change no score and give zero outputs
+        f.q = pad_to(f.q, Dp); f.k = pad_to(f.k, Dp); f.v = pad_to(f.v, Dp); f.se = pad_to(f.se, Dp);
+    }
+    f.q = f.q.contiguous(); f.k = f.k.contiguous(); f.v = f.v.contiguous();
+    const int64_t B = f.q.size(0), H = f.q.size(1), N = f.q.size(2);
+    f.out = at::empty_like(f.q);
+    f.lse = at::empty({B, H, N}, f.q.options().dtype(at::kFloat));
+    check(dsqg_fwd_scaled(ptr(f.q), ptr(f.k), ptr(f.v), fptr(f.pb), fptr(f.se), fptr(f.hg), off.v.data(), off.J(), ptr(f.out), fptr(f.lse),
+                          (int)B, (int)H, (int)N, (int)Dp, dt, stream_of(f.q), (float)(1.0 / std::sqrt((double)f.D))), "dsqg_fwd");
+    return f;
+}
+
+Tensor narrow_cols(const Tensor& t, int64_t D) { return t.defined() && t.size(-1) != D ? t.narrow(-1, 0, D).contiguous() : t; }
+
+std::vector<int64_t> types_of(const Tensor& a, const Tensor& b, const Tensor& c) {
+    return {(int64_t)type_of(a), (int64_t)type_of(b), (int64_t)type_of(c)};
+}
+at::ScalarType type_at(AutogradContext* ctx, int i) { return (at::ScalarType)ctx->saved_data["types"].toIntVector()[i]; }
+const Offsets& offsets_of(AutogradContext* ctx) { return *reinterpret_cast<const Offsets*>((intptr_t)ctx->saved_data["offsets"].toInt()); }
+
+// Saves q, k, v, pos_bias, head_gain, scale_embed, out, lse like the reference (kernels/dsqg_attention_v3.py:384).
+struct AttentionNode : torch::autograd::Function<AttentionNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& pos_bias,
+                          const std::optional<Tensor>& hg, const std::optional<Tensor>& se, const Offsets* off) {
+        const Tensor head_gain = opt(hg), scale_embed = opt(se);
+        Forward f = attention_forward(q, k, v, pos_bias, head_gain, scale_embed, *off);
+        ctx->save_for_backward({f.q, f.k, f.v, f.pb, f.hg, f.se, f.out, f.lse});
+        ctx->saved_data["offsets"] = (int64_t)(intptr_t)off;
+        ctx->saved_data["D"] = f.D;
+        ctx->saved_data["types"] = types_of(pos_bias, head_gain, scale_embed);
+        return narrow_cols(f.out, f.D);
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        return backward_body([&] { return run(ctx, grads[0]); });
+    }
+
+    static variable_list run(AutogradContext* ctx, Tensor dout) {
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &q = s[0], &k = s[1], &v = s[2], &pb = s[3], &hg = s[4], &se = s[5], &out = s[6], &lse = s[7];
+        const Offsets& off = offsets_of(ctx);
+        const int64_t D = ctx->saved_data["D"].toInt(), B = q.size(0), H = q.size(1), N = q.size(2), Dp = q.size(3);
+        const c10::cuda::CUDAGuard guard(q.device());
+        if (dout.scalar_type() != q.scalar_type()) dout = dout.to(q.scalar_type());
+        if (Dp != D) dout = pad_to(dout, Dp);
+        dout = dout.contiguous();                                  // kernels/dsqg_attention_v3.py:394
+        Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), dpb = at::empty_like(pb);
+        Tensor dhg = hg.defined() ? at::empty_like(hg) : Tensor(), dse = se.defined() ? at::empty_like(se) : Tensor();
+        const size_t bytes = dsqg_bwd_scratch_bytes(off.J(), (int)B, (int)H, (int)N, (int)Dp, se.defined());
+        const at::DataPtr scratch = scratch_for(bytes);
+        check(dsqg_bwd_scaled(ptr(q), ptr(k), ptr(v), fptr(pb), fptr(se), fptr(hg), off.v.data(), off.J(), ptr(out), fptr(lse), ptr(dout),
+                              ptr(dq), ptr(dk), ptr(dv), fptr(dpb), fptr(dse), fptr(dhg), scratch.get(), bytes,
+                              (int)B, (int)H, (int)N, (int)Dp, dtype_code(q), stream_of(q), (float)(1.0 / std::sqrt((double)D))), "dsqg_bwd");
+        return {narrow_cols(dq, D), narrow_cols(dk, D), narrow_cols(dv, D), like_param(dpb, type_at(ctx, 0)),
+                like_param(dhg, type_at(ctx, 1)), like_param(narrow_cols(dse, D), type_at(ctx, 2)), Tensor()};
+    }
+};
+
+bool wants_grad(std::initializer_list<const Tensor*> ts) {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor* t : ts)
+        if (t->defined() && t->requires_grad()) return true;
+    return false;
+}
+
+Tensor attention(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& pb, const std::optional<Tensor>& hg,
+                 const std::optional<Tensor>& se, const Offsets* off) {
+    py::gil_scoped_release no_gil;
+    const Tensor h = opt(hg), e = opt(se);
+    if (wants_grad({&q, &k, &v, &pb, &h, &e})) return AttentionNode::apply(q, k, v, pb, hg, se, off);
+    const Forward f = attention_forward(q, k, v, pb, h, e, *off);
+    return narrow_cols(f.out, f.D);
+}
+
+std::tuple<Tensor, Tensor> forward_lse(const Tensor& q0, const Tensor& k0, const Tensor& v0, const Tensor& pb0, const std::optional<Tensor>& hg0,
+                                       const std::optional<Tensor>& se0, const Offsets* off) {
+    check_inputs(q0, k0, v0, pb0, opt(hg0), opt(se0), off->J());
+    const int dt = dtype_code(q0);
+    const c10::cuda::CUDAGuard guard(q0.device());
+    const Tensor q = q0.contiguous(), k = k0.contiguous(), v = v0.contiguous(), pb = f32c(pb0), hg = f32c(opt(hg0)), se = f32c(opt(se0));
+    Tensor out = at::empty_like(q, at::TensorOptions().requires_grad(false));
+    Tensor lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
+    check(dsqg_fwd(ptr(q), ptr(k), ptr(v), fptr(pb), fptr(se), fptr(hg), off->v.data(), off->J(), ptr(out), fptr(lse), (int)q.size(0),
+                   (int)q.size(1), (int)q.size(2), (int)q.size(3), dt, stream_of(q)), "dsqg_fwd");
+    return {out, lse};
+}
+
+// ------------------------------------------------------------------------------------ packed projection output
+// q, k, v read in place from qkv [B,N,3,H,HD]; y [B,N,H*HD] token-major, times sigmoid(gate).
+struct PackedStrides {
+    dsqg_strides in, out;
+    PackedStrides(int64_t N, int64_t H, int64_t D) : in{N * 3 * H * D, D, 3 * H * D}, out{N * H * D, D, H * D} {}
+};
+char* third(const Tensor& qkv, int i) { return static_cast<char*>(qkv.data_ptr()) + i * qkv.size(3) * qkv.size(4) * qkv.element_size(); }
+
+struct PackedForward { Tensor gate, pb, hg, se, y, lse; };
+
+PackedForward packed_forward(const Tensor& qkv, const Tensor& gate, const Tensor& pos_bias, const Tensor& head_gain, const Tensor& scale_embed,
+                             const Offsets& off) {
+    if (qkv.dim() != 5 || qkv.size(2) != 3 || qkv.scalar_type() != at::kBFloat16 || !qkv.is_contiguous())
+        throw py::value_error("dsqg packed: qkv must be a contiguous bf16 [B,N,3,H,HD] tensor");
+    const int64_t B = qkv.size(0), N = qkv.size(1), H = qkv.size(3), D = qkv.size(4), J = off.J();
+    if (gate.defined() && (gate.scalar_type() != at::kBFloat16 || !shape_is(gate, {B, N, H * D})))
+        throw py::value_error("dsqg packed: gate must be bf16 [B,N,H*HD]");
+    PackedForward f;
+    f.gate = gate.defined() ? gate.contiguous() : gate;
+    f.pb = f32c(pos_bias); f.hg = f32c(head_gain); f.se = f32c(scale_embed);
+    if (!shape_is(f.pb, {J, H})) throw py::value_error("dsqg: pos_bias must be [" + std::to_string(J) + "," + std::to_string(H) + "], got " + shape_of(f.pb));
+    if (f.se.defined() && !shape_is(f.se, {J, D}))
+        throw py::value_error("dsqg: scale_embed must be [" + std::to_string(J) + "," + std::to_string(D) + "], got " + shape_of(f.se));
+    if (!qkv.is_cuda()) throw std::runtime_error("dsqg: tensors must live on a CUDA device (there is no CPU path)");
+    const c10::cuda::CUDAGuard guard(qkv.device());
+    const auto opts = at::TensorOptions().device(qkv.device());
+    f.y = at::empty({B, N, H * D}, opts.dtype(at::kBFloat16));
+    f.lse = at::empty({B, H, N}, opts.dtype(at::kFloat));
+    const PackedStrides st(N, H, D);
+    if (f.se.defined())
+        check(dsqg_fwd_strided_se(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.se), fptr(f.hg), off.v.data(), off.J(),
+                                  ptr(f.y), &st.out, ptr(f.gate), fptr(f.lse), (int)B, (int)H, (int)N, (int)D, DSQG_DTYPE_BF16, stream_of(qkv), 0.f),
+              "dsqg_fwd_strided_se");
+    else
+        check(dsqg_fwd_strided(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.hg), off.v.data(), off.J(),
+                               ptr(f.y), &st.out, ptr(f.gate), fptr(f.lse), (int)B, (int)H, (int)N, (int)D, DSQG_DTYPE_BF16, stream_of(qkv), 0.f),
+              "dsqg_fwd_strided");
+    return f;
+}
+
+struct PackedGrads { Tensor dqkv, dgate, dpb, dhg, dse; };
+
+PackedGrads packed_backward(const Tensor& qkv, const PackedForward& f, const Tensor& dy0, const Offsets& off) {
+    const int64_t B = qkv.size(0), N = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
+    const c10::cuda::CUDAGuard guard(qkv.device());
+    const Tensor dy = (dy0.scalar_type() == at::kBFloat16 ? dy0 : dy0.to(at::kBFloat16)).contiguous();
+    const PackedStrides st(N, H, D);
+    void* stream = stream_of(qkv);
+    PackedGrads g;
+    g.dqkv = at::empty_like(qkv); g.dpb = at::empty_like(f.pb);
+    if (f.hg.defined()) g.dhg = at::empty_like(f.hg);
+    if (f.se.defined()) g.dse = at::empty_like(f.se);
+    const size_t bytes = dsqg_bwd_scratch_bytes(off.J(), (int)B, (int)H, (int)N, (int)D, f.se.defined());
+    const at::DataPtr scratch = scratch_for(bytes);
+    at::DataPtr dout_mem, delta_mem;
+    void* dout = ptr(dy);
+    float* delta = nullptr;
+    if (f.gate.defined()) {
+        g.dgate = at::empty_like(f.gate);
+        dout_mem = scratch_for((size_t)dy.numel() * 2);
+        delta_mem = scratch_for((size_t)B * H * N * 4);
+        dout = dout_mem.get(); delta = static_cast<float*>(delta_mem.get());
+        check(dsqg_gate_bwd(ptr(dy), ptr(f.y), ptr(f.gate), &st.out, dout, ptr(g.dgate), delta, (int)B, (int)H, (int)N, (int)D, stream), "dsqg_gate_bwd");
+    }
+    if (f.se.defined())
+        check(dsqg_bwd_strided_se(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.se), fptr(f.hg), off.v.data(), off.J(),
+                                  ptr(f.y), fptr(f.lse), dout, &st.out, delta, third(g.dqkv, 0), third(g.dqkv, 1), third(g.dqkv, 2), fptr(g.dpb),
+                                  fptr(g.dse), fptr(g.dhg), scratch.get(), bytes, (int)B, (int)H, (int)N, (int)D, DSQG_DTYPE_BF16, stream, 0.f),
+              "dsqg_bwd_strided_se");
+    else
+        check(dsqg_bwd_strided(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.hg), off.v.data(), off.J(),
+                               ptr(f.y), fptr(f.lse), dout, &st.out, delta, third(g.dqkv, 0), third(g.dqkv, 1), third(g.dqkv, 2), fptr(g.dpb),
+                               fptr(g.dhg), scratch.get(), bytes, (int)B, (int)H, (int)N, (int)D, DSQG_DTYPE_BF16, stream, 0.f), "dsqg_bwd_strided");
+    return g;
+}
+
+struct PackedNode : torch::autograd::Function<PackedNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& qkv, const std::optional<Tensor>& gate, const Tensor& pos_bias,
+                          const std::optional<Tensor>& hg, const std::optional<Tensor>& se, const Offsets* off) {
+        const Tensor head_gain = opt(hg), scale_embed = opt(se);
+        PackedForward f = packed_forward(qkv, opt(gate), pos_bias, head_gain, scale_embed, *off);
+        ctx->save_for_backward({qkv, f.gate, f.pb, f.hg, f.se, f.y, f.lse});
+        ctx->saved_data["offsets"] = (int64_t)(intptr_t)off;
+        ctx->saved_data["types"] = types_of(pos_bias, head_gain, scale_embed);
+        return f.y;
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list s = ctx->get_saved_variables();
+        const PackedForward f = {s[1], s[2], s[3], s[4], s[5], s[6]};
+        const PackedGrads g = backward_body([&] { return packed_backward(s[0], f, grads[0], offsets_of(ctx)); });
+        return {g.dqkv, g.dgate, like_param(g.dpb, type_at(ctx, 0)), like_param(g.dhg, type_at(ctx, 1)), like_param(g.dse, type_at(ctx, 2)), Tensor()};
+    }
+};
+
+Tensor attention_packed(const Tensor& qkv, const std::optional<Tensor>& gate, const Tensor& pb, const std::optional<Tensor>& hg,
+                        const std::optional<Tensor>& se, const Offsets* off) {
+    py::gil_scoped_release no_gil;
+    const Tensor g = opt(gate), h = opt(hg), e = opt(se);
+    if (wants_grad({&qkv, &g, &pb, &h, &e})) return PackedNode::apply(qkv, gate, pb, hg, se, off);
+    return packed_forward(qkv, g, pb, h, e, *off).y;
+}
+
+// ------------------------------------------------------------------------------------ causal mean
+Tensor causal_mean_run(const Tensor& x, bool reverse) {
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor out = at::empty_like(x, at::TensorOptions().requires_grad(false));
+    check(dsqg_causal_mean(ptr(x), ptr(out), (int)x.size(0), (int)x.size(1), (int)x.size(2), dtype_code(x), reverse, stream_of(x)), "dsqg_causal_mean");
+    return out;
+}
+struct CausalMeanNode : torch::autograd::Function<CausalMeanNode> {
+    static Tensor forward(AutogradContext*, const Tensor& x) { return causal_mean_run(x, false); }
+    static variable_list backward(AutogradContext*, variable_list grads) {
+        return backward_body([&] { return variable_list{causal_mean_run(grads[0].contiguous(), true)}; });
+    }
+};
+Tensor causal_mean(const Tensor& x0) {
+    py::gil_scoped_release no_gil;
+    if (!x0.is_cuda() || x0.dim() != 3 || (x0.scalar_type() != at::kBFloat16 && x0.scalar_type() != at::kFloat))
+        throw py::value_error("causal_mean: x must be a CUDA [B,N,D] tensor in bfloat16 or float32");
+    const Tensor x = x0.contiguous();
+    return wants_grad({&x}) ? CausalMeanNode::apply(x) : causal_mean_run(x, false);
+}
+
+// ------------------------------------------------------------------------------------ decode
+struct StepParams { Tensor pb, hg, se; };
+
+void check_step(const char* who, const Tensor& q, const Tensor& k, const Tensor& v, at::ScalarType dt, int64_t S, int64_t H, int64_t D,
+                const Tensor& head, const Tensor& fill, const Tensor& pb, int J) {
+    const char* names[3] = {"q", "k_new", "v_new"};
+    const Tensor* ts[3] = {&q, &k, &v};
+    for (int i = 0; i < 3; ++i)
+        if (!shape_is(*ts[i], {S, H, D}) || ts[i]->scalar_type() != dt || !ts[i]->is_contiguous())
+            throw py::value_error(std::string(who) + ": " + names[i] + " must be contiguous [" + std::to_string(S) + "," + std::to_string(H) + "," +
+                                  std::to_string(D) + "] " + toString(dt));
+    if (head.scalar_type() != at::kInt || !shape_is(head, {S})) throw py::value_error(std::string(who) + ": head must be int32 [S]");
+    if (fill.defined() && (fill.scalar_type() != at::kInt || !shape_is(fill, {S}))) throw py::value_error(std::string(who) + ": fill must be int32 [S]");
+    if (!shape_is(pb, {J, H})) throw py::value_error(std::string(who) + ": pos_bias must be [" + std::to_string(J) + "," + std::to_string(H) + "]");
+}
+
+Tensor decode_step(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& k_ring, const Tensor& v_ring, const Tensor& head,
+                   const Tensor& pos_bias, const std::optional<Tensor>& hg, const std::optional<Tensor>& se, const Offsets* off,
+                   const std::optional<Tensor>& fill0, const std::optional<Tensor>& out0, bool overlap) {
+    if (k_ring.dim() != 4) throw py::value_error("dsqg_decode: k_ring and v_ring must be contiguous [S,H,R,D]");
+    const int64_t S = k_ring.size(0), H = k_ring.size(1), R = k_ring.size(2), D = k_ring.size(3);
+    const Tensor fill = opt(fill0);
+    check_step("dsqg_decode", q, k, v, k_ring.scalar_type(), S, H, D, head, fill, pos_bias, off->J());
+    if (v_ring.sizes() != k_ring.sizes() || !k_ring.is_contiguous() || !v_ring.is_contiguous())
+        throw py::value_error("dsqg_decode: k_ring and v_ring must be contiguous [S,H,R,D]");
+    const StepParams p = {f32c(pos_bias), f32c(opt(hg)), f32c(opt(se))};
+    const c10::cuda::CUDAGuard guard(q.device());
+    Tensor out = out0.has_value() ? *out0 : at::empty_like(q, at::TensorOptions().requires_grad(false));
+    check((overlap ? dsqg_decode_overlapped : dsqg_decode)(
+              ptr(q), ptr(k), ptr(v), ptr(k_ring), ptr(v_ring), static_cast<const int32_t*>(ptr(head)), static_cast<const int32_t*>(ptr(fill)),
+              fptr(p.pb), fptr(p.se), fptr(p.hg), off->v.data(), off->J(), (int)R, ptr(out), (int)S, (int)H, (int)D, dtype_code(q), stream_of(q)),
+          "dsqg_decode");
+    return out;
+}
+
+// kv_ring [S,H,R,2,D], or the rings of all layers [L,S,H,R,2,D] and the layer to use
+Tensor decode_step_kv(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& kv, std::optional<int64_t> layer0, const Tensor& head, const Tensor& pos_bias,
+                      const std::optional<Tensor>& hg, const std::optional<Tensor>& se, const Offsets* off,
+                      const std::optional<Tensor>& fill0, const std::optional<Tensor>& out0, bool overlap) {
+    const int64_t lead = layer0.has_value() ? 1 : 0;
+    if (kv.dim() != 5 + lead || kv.size(3 + lead) != 2 || !kv.is_contiguous()) throw py::value_error("dsqg_decode_kv: kv_ring must be contiguous [S,H,R,2,D]");
+    const int64_t layer = !lead ? 0 : *layer0 < 0 ? *layer0 + kv.size(0) : *layer0;
+    if (lead && (layer < 0 || layer >= kv.size(0))) throw py::index_error("dsqg_decode_kv: no such layer");
+    const int64_t S = kv.size(lead), H = kv.size(1 + lead), R = kv.size(2 + lead), D = kv.size(4 + lead);
+    const Tensor fill = opt(fill0);
+    check_step("dsqg_decode_kv", q, k, v, kv.scalar_type(), S, H, D, head, fill, pos_bias, off->J());
+    const StepParams p = {f32c(pos_bias), f32c(opt(hg)), f32c(opt(se))};
+    const c10::cuda::CUDAGuard guard(q.device());
+    Tensor out = out0.has_value() ? *out0 : at::empty_like(q, at::TensorOptions().requires_grad(false));
+    char* ring = static_cast<char*>(kv.data_ptr()) + (lead ? layer * kv.stride(0) * kv.element_size() : 0);
+    check(dsqg_decode_kv(ptr(q), ptr(k), ptr(v), ring, static_cast<const int32_t*>(ptr(head)), static_cast<const int32_t*>(ptr(fill)),
+                         fptr(p.pb), fptr(p.se), fptr(p.hg), off->v.data(), off->J(), (int)R, ptr(out), (int)S, (int)H, (int)D, dtype_code(q),
+                         stream_of(q), overlap), "dsqg_decode_kv");
+    return out;
+}
+
+// (head + 1) mod R and min(fill + 1, R) as new tensors
+std::tuple<Tensor, Tensor> ring_advance(const Tensor& head0, const Tensor& fill0, int64_t R) {
+    const Tensor head = head0.to(at::kInt).contiguous(), fill = fill0.to(at::kInt).contiguous();
+    const c10::cuda::CUDAGuard guard(head.device());
+    Tensor h = at::empty_like(head), f = at::empty_like(fill);
+    check(dsqg_ring_advance(static_cast<const int32_t*>(ptr(head)), static_cast<const int32_t*>(ptr(fill)), static_cast<int32_t*>(ptr(h)),
+                            static_cast<int32_t*>(ptr(f)), (int)head.numel(), (int)R, stream_of(head)), "dsqg_ring_advance");
+    return {h, f};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_dsqg_torch, m) {
+    py::class_<Offsets, std::unique_ptr<Offsets, py::nodelete>>(m, "Offsets").def_property_readonly("J", &Offsets::J);
+    m.def("offsets", &intern_offsets, py::return_value_policy::reference);
+    m.def("attention", &attention);
+    m.def("forward_lse", &forward_lse);
+    m.def("attention_packed", &attention_packed);
+    m.def("causal_mean", &causal_mean);
+    m.def("decode_step", &decode_step);
+    m.def("decode_step_kv", &decode_step_kv);
+    m.def("ring_advance", &ring_advance);
+}

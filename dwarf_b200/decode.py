@@ -7,12 +7,12 @@ a write head per sequence, and one kernel launch per layer per token.
 """
 from __future__ import annotations
 
-from typing import Optional, Sequence
+from typing import Sequence
 
 import torch
 
 from . import _lib
-from .ops import OFFSETS_43, _dtype_code, _f32c, _ptr
+from .ops import OFFSETS_43, _dtype_code
 
 
 def dsqg_decode_step(q, k_new, v_new, k_ring, v_ring, head, pos_bias, head_gain=None,
@@ -27,60 +27,16 @@ def dsqg_decode_step(q, k_new, v_new, k_ring, v_ring, head, pos_bias, head_gain=
     in the stream is still finishing (`dsqg_decode_overlapped`): allowed only when that kernel
     writes none of this call's head, fill, k_ring, v_ring.
     """
-    lib = _lib.load()
-    off, J = _lib.offsets_array(offsets)
-    S, H, R, D = k_ring.shape
-    for name, t in (("q", q), ("k_new", k_new), ("v_new", v_new)):
-        if tuple(t.shape) != (S, H, D) or t.dtype != k_ring.dtype or not t.is_contiguous():
-            raise ValueError(f"dsqg_decode: {name} must be contiguous [{S},{H},{D}] {k_ring.dtype}")
-    if v_ring.shape != k_ring.shape or not (k_ring.is_contiguous() and v_ring.is_contiguous()):
-        raise ValueError("dsqg_decode: k_ring and v_ring must be contiguous [S,H,R,D]")
-    if head.dtype != torch.int32 or tuple(head.shape) != (S,):
-        raise ValueError("dsqg_decode: head must be int32 [S]")
-    if fill is not None and (fill.dtype != torch.int32 or tuple(fill.shape) != (S,)):
-        raise ValueError("dsqg_decode: fill must be int32 [S]")
-    if tuple(pos_bias.shape) != (J, H):
-        raise ValueError(f"dsqg_decode: pos_bias must be [{J},{H}]")
-    pb, hg, se = _f32c(pos_bias), _f32c(head_gain), _f32c(scale_embed)
-    if out is None:
-        out = torch.empty_like(q)
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        entry = lib.dsqg_decode_overlapped if overlap else lib.dsqg_decode
-        _lib.check(entry(q.data_ptr(), k_new.data_ptr(), v_new.data_ptr(),
-                         k_ring.data_ptr(), v_ring.data_ptr(), head.data_ptr(), _ptr(fill),
-                         pb.data_ptr(), _ptr(se), _ptr(hg), off, J, R,
-                         out.data_ptr(), S, H, D, _dtype_code(q), stream), "dsqg_decode")
-    return out
+    return _lib.native().decode_step(q, k_new, v_new, k_ring, v_ring, head, pos_bias, head_gain, scale_embed,
+                                     _lib.offsets_handle(offsets), fill, out, overlap)
 
 
 def dsqg_decode_step_kv(q, k_new, v_new, kv_ring, head, pos_bias, head_gain=None, scale_embed=None,
                         offsets: Sequence[int] = OFFSETS_43, fill=None, out=None, overlap=False):
     """dsqg_decode_step over one ring that holds key and value of a slot side by side:
     kv_ring [S,H,R,2,D] (updated in place).  A tap is one contiguous read of 2*D elements."""
-    lib = _lib.load()
-    off, J = _lib.offsets_array(offsets)
-    S, H, R, two, D = kv_ring.shape
-    if two != 2 or not kv_ring.is_contiguous():
-        raise ValueError("dsqg_decode_kv: kv_ring must be contiguous [S,H,R,2,D]")
-    for name, t in (("q", q), ("k_new", k_new), ("v_new", v_new)):
-        if tuple(t.shape) != (S, H, D) or t.dtype != kv_ring.dtype or not t.is_contiguous():
-            raise ValueError(f"dsqg_decode_kv: {name} must be contiguous [{S},{H},{D}] {kv_ring.dtype}")
-    if head.dtype != torch.int32 or tuple(head.shape) != (S,):
-        raise ValueError("dsqg_decode_kv: head must be int32 [S]")
-    if fill is not None and (fill.dtype != torch.int32 or tuple(fill.shape) != (S,)):
-        raise ValueError("dsqg_decode_kv: fill must be int32 [S]")
-    if tuple(pos_bias.shape) != (J, H):
-        raise ValueError(f"dsqg_decode_kv: pos_bias must be [{J},{H}]")
-    pb, hg, se = _f32c(pos_bias), _f32c(head_gain), _f32c(scale_embed)
-    if out is None:
-        out = torch.empty_like(q)
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        _lib.check(lib.dsqg_decode_kv(q.data_ptr(), k_new.data_ptr(), v_new.data_ptr(), kv_ring.data_ptr(),
-                                      head.data_ptr(), _ptr(fill), pb.data_ptr(), _ptr(se), _ptr(hg), off, J, R,
-                                      out.data_ptr(), S, H, D, _dtype_code(q), stream, int(overlap)), "dsqg_decode_kv")
-    return out
+    return _lib.native().decode_step_kv(q, k_new, v_new, kv_ring, None, head, pos_bias, head_gain, scale_embed,
+                                        _lib.offsets_handle(offsets), fill, out, overlap)
 
 
 class DSQGRingCache:
@@ -124,14 +80,13 @@ class DSQGRingCache:
 
     def advance(self):
         """Move every write head to the next slot; call once per token before the layers run."""
-        self.head = torch.remainder(self.head + 1, self.R).to(torch.int32)
-        self.fill = torch.clamp(self.fill + 1, max=self.R).to(torch.int32)
+        self.head, self.fill = _lib.native().ring_advance(self.head, self.fill, self.R)
 
     def step(self, layer, q, k_new, v_new, pos_bias, head_gain=None, scale_embed=None, out=None, overlap=False):
         """Decode step of `layer`.  overlap=True is safe from the second layer of a token on (the
         kernel ahead is then another layer's step or a projection, never `advance`/`prefill`)."""
         if self.interleaved:
-            return dsqg_decode_step_kv(q, k_new, v_new, self.kv[layer], self.head, pos_bias,
-                                       head_gain, scale_embed, self.offsets, self.fill, out, overlap)
+            return _lib.native().decode_step_kv(q, k_new, v_new, self.kv, layer, self.head, pos_bias, head_gain, scale_embed,
+                                                _lib.offsets_handle(self.offsets), self.fill, out, overlap)
         return dsqg_decode_step(q, k_new, v_new, self.k[layer], self.v[layer], self.head, pos_bias,
                                 head_gain, scale_embed, self.offsets, self.fill, out, overlap)

@@ -1,17 +1,17 @@
-"""DSQG attention as a torch.autograd.Function over the native C ABI.
+"""DSQG attention as a PyTorch operator over the native C ABI.
 
 Mirrors the operator layer of the DWARF reference:
 ``_DSQGFn`` / ``_DSQGFnV3`` (kernels/dsqg_attention_v2.py:337-414,
 kernels/dsqg_attention_v3.py:359-442) and their functional wrappers
 (:417-427, :445-456).  PyTorch is used for device memory and streams only; all
-arithmetic happens in libdsqg_b200.so.
+arithmetic happens in libdsqg_b200.so, and the steps around it (checks, allocation, autograd
+nodes) in _dsqg_torch.so.
 """
 from __future__ import annotations
 
-from typing import Optional, Sequence
+from typing import Sequence
 
 import torch
-import torch.nn.functional as F
 
 from . import _lib
 
@@ -32,27 +32,6 @@ def _dtype_code(t: torch.Tensor) -> int:
     raise TypeError(f"dsqg: q/k/v must be bfloat16 or float32, got {t.dtype}")
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else t.data_ptr()
-
-
-def _check_inputs(q, k, v, pos_bias, head_gain, scale_embed, J):
-    if not q.is_cuda:
-        raise RuntimeError("dsqg: tensors must live on a CUDA device (there is no CPU path)")
-    if q.dim() != 4:
-        raise ValueError(f"dsqg: q must be [B,H,N,HD], got {tuple(q.shape)}")
-    B, H, N, D = q.shape
-    for name, t in (("k", k), ("v", v)):
-        if t.shape != q.shape or t.dtype != q.dtype or t.device != q.device:
-            raise ValueError(f"dsqg: {name} must match q in shape, dtype and device")
-    if tuple(pos_bias.shape) != (J, H):
-        raise ValueError(f"dsqg: pos_bias must be [{J},{H}], got {tuple(pos_bias.shape)}")
-    if scale_embed is not None and tuple(scale_embed.shape) != (J, D):
-        raise ValueError(f"dsqg: scale_embed must be [{J},{D}], got {tuple(scale_embed.shape)}")
-    if head_gain is not None and tuple(head_gain.shape) != (H,):
-        raise ValueError(f"dsqg: head_gain must be [{H}], got {tuple(head_gain.shape)}")
-
-
 def _padded_head_dim(q, off, J, has_scale_embed):
     """Head dimension the kernels are called with.  The bf16 tensor-core kernels exist for
     D in {32, 64, 96, 128}; another bf16 head dimension (80 in the reference's 85M condM model,
@@ -69,116 +48,32 @@ def _padded_head_dim(q, off, J, has_scale_embed):
     return Dp if lib.dsqg_tensor_core_path(_lib.DSQG_DTYPE_BF16, Dp, off, J, int(has_scale_embed)) else D
 
 
-def _f32c(t):
-    return None if t is None else t.detach().to(torch.float32).contiguous()
-
-
-class DSQGFunction(torch.autograd.Function):
-    """out = DSQG(q, k, v; pos_bias, head_gain, scale_embed, offsets) with autograd.
+class DSQGFunction:
+    """out = DSQG(q, k, v; pos_bias, head_gain, scale_embed, offsets) with autograd (an autograd node in native code,
+    csrc/dsqg_torch.cpp).
 
     Saves (q, k, v, pos_bias, head_gain, scale_embed, out, lse) like the reference
     (kernels/dsqg_attention_v3.py:384) and returns gradients for the six tensors.
     """
 
     @staticmethod
-    def forward(ctx, q, k, v, pos_bias, head_gain, scale_embed, offsets):
-        lib = _lib.load()
-        off, J = _lib.offsets_array(offsets)
-        _check_inputs(q, k, v, pos_bias, head_gain, scale_embed, J)
-        pb, hg, se = _f32c(pos_bias), _f32c(head_gain), _f32c(scale_embed)
-        B, H, N, D = q.shape
-        Dp = _padded_head_dim(q, off, J, scale_embed is not None)
-        if Dp != D:                              # zero columns change no score and give zero outputs
-            q, k, v = (F.pad(t, (0, Dp - D)) for t in (q, k, v))
-            se = None if se is None else F.pad(se, (0, Dp - D))
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        out = torch.empty_like(q)
-        lse = torch.empty(B, H, N, device=q.device, dtype=torch.float32)
-        with torch.cuda.device(q.device):
-            stream = torch.cuda.current_stream(q.device).cuda_stream
-            _lib.check(lib.dsqg_fwd_scaled(q.data_ptr(), k.data_ptr(), v.data_ptr(), pb.data_ptr(), _ptr(se),
-                                           _ptr(hg), off, J, out.data_ptr(), lse.data_ptr(),
-                                           B, H, N, Dp, _dtype_code(q), stream, D ** -0.5), "dsqg_fwd")
-        ctx.save_for_backward(q, k, v, pb, hg, se, out, lse)
-        ctx.offsets = tuple(offsets)
-        ctx.head_dim = D
-        ctx.param_dtypes = (pos_bias.dtype, None if head_gain is None else head_gain.dtype,
-                            None if scale_embed is None else scale_embed.dtype)
-        return out if Dp == D else out[..., :D].contiguous()
-
-    @staticmethod
-    def backward(ctx, dout):
-        lib = _lib.load()
-        q, k, v, pb, hg, se, out, lse = ctx.saved_tensors
-        off, J = _lib.offsets_array(ctx.offsets)
-        B, H, N, Dp = q.shape
-        D = ctx.head_dim
-        if dout.dtype != q.dtype:
-            dout = dout.to(q.dtype)
-        if Dp != D:
-            dout = F.pad(dout, (0, Dp - D))
-        dout = dout.contiguous()                      # kernels/dsqg_attention_v3.py:394
-        dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        dpb = torch.empty_like(pb)
-        dse = None if se is None else torch.empty_like(se)
-        dhg = None if hg is None else torch.empty_like(hg)
-        nbytes = lib.dsqg_bwd_scratch_bytes(J, B, H, N, Dp, int(se is not None))
-        scratch = torch.empty(nbytes, device=q.device, dtype=torch.uint8)
-        with torch.cuda.device(q.device):
-            stream = torch.cuda.current_stream(q.device).cuda_stream
-            _lib.check(lib.dsqg_bwd_scaled(q.data_ptr(), k.data_ptr(), v.data_ptr(), pb.data_ptr(), _ptr(se),
-                                           _ptr(hg), off, J, out.data_ptr(), lse.data_ptr(), dout.data_ptr(),
-                                           dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                                           dpb.data_ptr(), _ptr(dse), _ptr(dhg),
-                                           scratch.data_ptr(), nbytes, B, H, N, Dp, _dtype_code(q), stream,
-                                           D ** -0.5), "dsqg_bwd")
-        if Dp != D:
-            dq, dk, dv = (t[..., :D].contiguous() for t in (dq, dk, dv))
-            dse = None if dse is None else dse[:, :D].contiguous()
-        pb_dt, hg_dt, se_dt = ctx.param_dtypes
-        return (dq, dk, dv, dpb.to(pb_dt),
-                None if dhg is None else dhg.to(hg_dt),
-                None if dse is None else dse.to(se_dt), None)
-
-
-class CausalMeanFunction(torch.autograd.Function):
-    """pool[b,n,:] = mean(x[b,0..n,:]) with autograd (the backward is the kernel's reverse mode)."""
-
-    @staticmethod
-    def forward(ctx, x):
-        if not x.is_cuda or x.dim() != 3 or x.dtype not in (torch.bfloat16, torch.float32):
-            raise ValueError("causal_mean: x must be a CUDA [B,N,D] tensor in bfloat16 or float32")
-        x = x.contiguous()
-        ctx.meta = tuple(x.shape)
-        return CausalMeanFunction._run(x, 0)
-
-    @staticmethod
-    def backward(ctx, dout):
-        return CausalMeanFunction._run(dout.contiguous(), 1)
-
-    @staticmethod
-    def _run(x, reverse):
-        lib = _lib.load()
-        B, N, D = x.shape
-        out = torch.empty_like(x)
-        with torch.cuda.device(x.device):
-            stream = torch.cuda.current_stream(x.device).cuda_stream
-            _lib.check(lib.dsqg_causal_mean(x.data_ptr(), out.data_ptr(), B, N, D, _dtype_code(x), reverse, stream),
-                       "dsqg_causal_mean")
-        return out
+    def apply(q, k, v, pos_bias, head_gain, scale_embed, offsets):
+        return _lib.native().attention(q, k, v, pos_bias, head_gain, scale_embed, _lib.offsets_handle(offsets))
 
 
 def causal_mean(x):
     """Causal running mean over the sequence dimension of x [B,N,D] (bf16 or fp32; other dtypes are
     computed in fp32 and cast back): the pooling of the reference's interference block,
-    `x.cumsum(dim=1) / counts` (train/train_2048_condU.py:289-292), as one kernel."""
+    `x.cumsum(dim=1) / counts` (train/train_2048_condU.py:289-292), as one kernel; its backward is the
+    kernel's reverse mode."""
     if x.dtype in (torch.bfloat16, torch.float32):
-        return CausalMeanFunction.apply(x)
-    return CausalMeanFunction.apply(x.float()).to(x.dtype)
+        return _lib.native().causal_mean(x)
+    return _lib.native().causal_mean(x.float()).to(x.dtype)
 
 
-class DSQGPackedFunction(torch.autograd.Function):
-    """DSQG on the un-permuted output of a fused qkv projection, with a token-major result.
+class DSQGPackedFunction:
+    """DSQG on the un-permuted output of a fused qkv projection, with a token-major result (an autograd node in
+    native code, csrc/dsqg_torch.cpp).
 
     qkv [B,N,3,H,HD] bf16 (a view of the [B,N,3*H*HD] projection output; q, k, v are read in place
     through strides), gate [B,N,H*HD] bf16 or None -> y [B,N,H*HD] = DSQG(q,k,v) (* sigmoid(gate)).
@@ -187,83 +82,8 @@ class DSQGPackedFunction(torch.autograd.Function):
     their autograd backward; the gradient comes back as one dqkv tensor in the layout of qkv."""
 
     @staticmethod
-    def forward(ctx, qkv, gate, pos_bias, head_gain, offsets, scale_embed=None):
-        lib = _lib.load()
-        off, J = _lib.offsets_array(offsets)
-        B, N, three, H, D = qkv.shape
-        if three != 3 or qkv.dtype != torch.bfloat16 or not qkv.is_contiguous():
-            raise ValueError("dsqg packed: qkv must be a contiguous bf16 [B,N,3,H,HD] tensor")
-        if gate is not None and (gate.dtype != torch.bfloat16 or tuple(gate.shape) != (B, N, H * D)):
-            raise ValueError("dsqg packed: gate must be bf16 [B,N,H*HD]")
-        gate = None if gate is None else gate.contiguous()
-        pb, hg = _f32c(pos_bias), _f32c(head_gain)
-        if tuple(pb.shape) != (J, H):
-            raise ValueError(f"dsqg: pos_bias must be [{J},{H}], got {tuple(pb.shape)}")
-        se = _f32c(scale_embed)
-        if se is not None and tuple(se.shape) != (J, D):
-            raise ValueError(f"dsqg: scale_embed must be [{J},{D}], got {tuple(se.shape)}")
-        y = torch.empty(B, N, H * D, device=qkv.device, dtype=qkv.dtype)
-        lse = torch.empty(B, H, N, device=qkv.device, dtype=torch.float32)
-        st_in = _lib.Strides(N * 3 * H * D, D, 3 * H * D)
-        st_out = _lib.Strides(N * H * D, D, H * D)
-        p0, esz = qkv.data_ptr(), qkv.element_size()
-        with torch.cuda.device(qkv.device):
-            stream = torch.cuda.current_stream(qkv.device).cuda_stream
-            if se is None:
-                _lib.check(lib.dsqg_fwd_strided(p0, p0 + H * D * esz, p0 + 2 * H * D * esz, st_in, pb.data_ptr(),
-                                                _ptr(hg), off, J, y.data_ptr(), st_out, _ptr(gate), lse.data_ptr(),
-                                                B, H, N, D, _lib.DSQG_DTYPE_BF16, stream, 0.0), "dsqg_fwd_strided")
-            else:
-                _lib.check(lib.dsqg_fwd_strided_se(p0, p0 + H * D * esz, p0 + 2 * H * D * esz, st_in, pb.data_ptr(),
-                                                   se.data_ptr(), _ptr(hg), off, J, y.data_ptr(), st_out, _ptr(gate),
-                                                   lse.data_ptr(), B, H, N, D, _lib.DSQG_DTYPE_BF16, stream, 0.0),
-                           "dsqg_fwd_strided_se")
-        ctx.save_for_backward(qkv, gate, pb, hg, y, lse, se)
-        ctx.offsets = tuple(offsets)
-        ctx.param_dtypes = (pos_bias.dtype, None if head_gain is None else head_gain.dtype,
-                            None if scale_embed is None else scale_embed.dtype)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        lib = _lib.load()
-        qkv, gate, pb, hg, y, lse, se = ctx.saved_tensors
-        off, J = _lib.offsets_array(ctx.offsets)
-        B, N, _, H, D = qkv.shape
-        dy = dy.to(qkv.dtype).contiguous()
-        st_in = _lib.Strides(N * 3 * H * D, D, 3 * H * D)
-        st_out = _lib.Strides(N * H * D, D, H * D)
-        dqkv = torch.empty_like(qkv)
-        dpb = torch.empty_like(pb)
-        dhg = None if hg is None else torch.empty_like(hg)
-        dse = None if se is None else torch.empty_like(se)
-        nbytes = lib.dsqg_bwd_scratch_bytes(J, B, H, N, D, 0 if se is None else 1)
-        scratch = torch.empty(nbytes, device=qkv.device, dtype=torch.uint8)
-        p0, g0, esz = qkv.data_ptr(), dqkv.data_ptr(), qkv.element_size()
-        with torch.cuda.device(qkv.device):
-            stream = torch.cuda.current_stream(qkv.device).cuda_stream
-            dgate, dout, delta = None, dy, None
-            if gate is not None:
-                dout, dgate = torch.empty_like(y), torch.empty_like(gate)
-                delta = torch.empty(B, H, N, device=qkv.device, dtype=torch.float32)
-                _lib.check(lib.dsqg_gate_bwd(dy.data_ptr(), y.data_ptr(), gate.data_ptr(), st_out, dout.data_ptr(),
-                                             dgate.data_ptr(), delta.data_ptr(), B, H, N, D, stream), "dsqg_gate_bwd")
-            if se is None:
-                _lib.check(lib.dsqg_bwd_strided(p0, p0 + H * D * esz, p0 + 2 * H * D * esz, st_in, pb.data_ptr(),
-                                                _ptr(hg), off, J, y.data_ptr(), lse.data_ptr(), dout.data_ptr(), st_out,
-                                                _ptr(delta), g0, g0 + H * D * esz, g0 + 2 * H * D * esz, dpb.data_ptr(),
-                                                _ptr(dhg), scratch.data_ptr(), nbytes, B, H, N, D,
-                                                _lib.DSQG_DTYPE_BF16, stream, 0.0), "dsqg_bwd_strided")
-            else:
-                _lib.check(lib.dsqg_bwd_strided_se(p0, p0 + H * D * esz, p0 + 2 * H * D * esz, st_in, pb.data_ptr(),
-                                                   se.data_ptr(), _ptr(hg), off, J, y.data_ptr(), lse.data_ptr(),
-                                                   dout.data_ptr(), st_out, _ptr(delta), g0, g0 + H * D * esz,
-                                                   g0 + 2 * H * D * esz, dpb.data_ptr(), dse.data_ptr(), _ptr(dhg),
-                                                   scratch.data_ptr(), nbytes, B, H, N, D, _lib.DSQG_DTYPE_BF16,
-                                                   stream, 0.0), "dsqg_bwd_strided_se")
-        pb_dt, hg_dt, se_dt = ctx.param_dtypes
-        return (dqkv, dgate, dpb.to(pb_dt), None if dhg is None else dhg.to(hg_dt), None,
-                None if dse is None else dse.to(se_dt))
+    def apply(qkv, gate, pos_bias, head_gain, offsets, scale_embed=None):
+        return _lib.native().attention_packed(qkv, gate, pos_bias, head_gain, scale_embed, _lib.offsets_handle(offsets))
 
 
 class InjectKVFunction(torch.autograd.Function):
@@ -306,7 +126,7 @@ def dsqg_attention_packed(qkv, pos_bias, head_gain=None, gate=None, offsets: Seq
     """DSQG straight on the fused projection output.  qkv: [B,N,3,H,HD] bf16 contiguous; gate: None
     or [B,N,H*HD] bf16 (pre-sigmoid); scale_embed: None or [J,HD] (the reference's v3 op).  Returns
     [B,N,H*HD] bf16, already multiplied by sigmoid(gate) when a gate is given."""
-    return DSQGPackedFunction.apply(qkv, gate, pos_bias, head_gain, tuple(int(o) for o in offsets), scale_embed)
+    return _lib.native().attention_packed(qkv, gate, pos_bias, head_gain, scale_embed, _lib.offsets_handle(offsets))
 
 
 def dsqg_attention(q, k, v, pos_bias, head_gain=None, scale_embed=None,
@@ -316,27 +136,14 @@ def dsqg_attention(q, k, v, pos_bias, head_gain=None, scale_embed=None,
     are computed in bf16 as the reference does (kernels/dsqg_attention_v3.py:452-456) and
     the result is returned in the caller's dtype."""
     orig_dtype = q.dtype
-    if orig_dtype not in (torch.bfloat16, torch.float32):
-        q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
-    out = DSQGFunction.apply(q, k, v, pos_bias, head_gain, scale_embed, tuple(int(o) for o in offsets))
-    return out if out.dtype == orig_dtype else out.to(orig_dtype)
+    if orig_dtype is torch.bfloat16 or orig_dtype is torch.float32:
+        return _lib.native().attention(q, k, v, pos_bias, head_gain, scale_embed, _lib.offsets_handle(offsets))
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    return _lib.native().attention(q, k, v, pos_bias, head_gain, scale_embed, _lib.offsets_handle(offsets)).to(orig_dtype)
 
 
 def dsqg_forward_lse(q, k, v, pos_bias, head_gain=None, scale_embed=None,
                      offsets: Sequence[int] = ALL_OFFSETS):
     """Forward without autograd; returns (out, lse).  lse is the natural-log softmax
     denominator per row, the tensor the reference saves for backward."""
-    lib = _lib.load()
-    off, J = _lib.offsets_array(offsets)
-    _check_inputs(q, k, v, pos_bias, head_gain, scale_embed, J)
-    q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-    pb, hg, se = _f32c(pos_bias), _f32c(head_gain), _f32c(scale_embed)
-    B, H, N, D = q.shape
-    out = torch.empty_like(q)
-    lse = torch.empty(B, H, N, device=q.device, dtype=torch.float32)
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        _lib.check(lib.dsqg_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), pb.data_ptr(), _ptr(se),
-                                _ptr(hg), off, J, out.data_ptr(), lse.data_ptr(),
-                                B, H, N, D, _dtype_code(q), stream), "dsqg_fwd")
-    return out, lse
+    return _lib.native().forward_lse(q, k, v, pos_bias, head_gain, scale_embed, _lib.offsets_handle(offsets))

@@ -269,6 +269,11 @@ int dsqg_decode(const void* q, const void* k_new, const void* v_new,
                 const int32_t* offsets, int J, int R,
                 void* out, int S, int H, int D, int dtype, void* stream);
 
+/* Moves the write heads of S sequences to the next token of a ring of R slots:
+ * head_out[s] = (head[s] + 1) mod R, fill_out[s] = min(fill[s] + 1, R).  DEVICE int32 [S] each; the
+ * outputs may be the inputs. */
+int dsqg_ring_advance(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R, void* stream);
+
 /* dsqg_decode / dsqg_ring_prefill over ONE ring per layer that holds the key and the value of a slot
  * side by side: kv_ring [S,H,R,2,D] (slot-major; element 0 of the pair is the key row, element 1 the
  * value row).  A tap is then one contiguous read of 2*D elements and a step touches half as many
