@@ -91,6 +91,7 @@ cudaError_t launch_gate_bwd(const void* dy, const void* y, const void* gate, lon
 cudaError_t launch_fwd_mma(const FwdArgs& a, const Taps& t, cudaStream_t s);
 cudaError_t launch_bwd_mma(const BwdArgs& a, const Taps& t, cudaStream_t s, int stages);
 bool mma_path_supported(int dtype, int D, const Taps& t, bool has_scale_embed);   // backward
+bool mma_tail_supported(int dtype, int D, const Taps& t, bool has_scale_embed);   // D = 48, 80 at their own width (forward and backward)
 bool mma_fwd_supported(int dtype, int D, const Taps& t, bool has_scale_embed);
 // forward with TMA-staged V (dsqg_staged.cu)
 bool staged_supported(int dtype, int D, const Taps& t, bool has_scale_embed);

@@ -1,5 +1,5 @@
 // Chooses between the tensor-core kernels (bf16; D in {32, 64} with or without scale_embed,
-// D in {96, 128} without) and the generic CUDA-core kernels (everything else: fp32 storage,
+// D in {48, 80, 96, 128} without) and the generic CUDA-core kernels (everything else: fp32 storage,
 // other head sizes, dense windows wider than the tensor-core kernels are built for).  One
 // decision per call, made on the host from the shape alone.
 #include <atomic>
@@ -27,13 +27,14 @@ cudaError_t launch_fwd(const FwdArgs& a, const Taps& t, int dtype, cudaStream_t 
     if (path == 0 && umma_pays(a, t, dtype)) return launch_fwd_umma(a, t, s);
     if (path == 4 && !a.strided && umma_supported(dtype, a.D, t, a.scale_embed != nullptr)) return launch_fwd_umma(a, t, s);
     if (path == 3 && staged_supported(dtype, a.D, t, a.scale_embed != nullptr)) return launch_fwd_staged(a, t, s);
-    if (path != 1 && mma_fwd_supported(dtype, a.D, t, a.scale_embed != nullptr)) return launch_fwd_mma(a, t, s);
+    if (path != 1 && (mma_fwd_supported(dtype, a.D, t, a.scale_embed != nullptr) || mma_tail_supported(dtype, a.D, t, a.scale_embed != nullptr)))
+        return launch_fwd_mma(a, t, s);
     return launch_fwd_generic(a, t, dtype, s);
 }
 
 cudaError_t launch_bwd(const BwdArgs& a, const Taps& t, int dtype, cudaStream_t s, int stages) {
     const int path = g_path.load();
-    if (path != 1 && mma_path_supported(dtype, a.D, t, a.scale_embed != nullptr))
+    if (path != 1 && (mma_path_supported(dtype, a.D, t, a.scale_embed != nullptr) || mma_tail_supported(dtype, a.D, t, a.scale_embed != nullptr)))
         return launch_bwd_mma(a, t, s, stages);
     return launch_bwd_generic(a, t, dtype, s, stages);
 }

@@ -1,5 +1,6 @@
 // Tensor-core DSQG kernels (bf16 storage, fp32 accumulate) for D in {32, 64} (dense windows up
-// to 64 wide) and D in {96, 128} (dense windows up to 32 wide).
+// to 64 wide) and D in {48, 80, 96, 128} (dense windows up to 32 wide; 48 and 80 contiguous tensors without
+// scale_embed only).
 //
 // One warp owns 16 consecutive rows of one (batch, head) sequence.  The dense window is a
 // banded GEMM: the 16 query rows against the WB+16 key rows [g0-WB, g0+16) with
@@ -284,7 +285,7 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float4* init_s,
 // Tuning per head dimension (measured on B200): warps per CTA, sparse taps folded together,
 // resident CTAs per SM the register budget is set for.
 template <int D> struct FwdTune {
-    static constexpr int warps = 4, group = D <= 64 ? 2 : 1, ctas = D == 32 ? 5 : (D == 64 ? 4 : (D == 96 ? 3 : 2));
+    static constexpr int warps = 4, group = D <= 80 ? 2 : 1, ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));
     static constexpr int group_se = D <= 64 ? 2 : 1, ctas_se = D == 32 ? 5 : 4;       // with scale_embed
 };
 
@@ -379,10 +380,10 @@ fwd_mma_kernel(const FwdArgs a, const Taps t) {
 // Tuning per head dimension (measured on B200): sparse taps whose loads are issued together and
 // resident CTAs per SM the register budget is set for (spills against warps in flight).
 template <int D> struct BwdTune {
-    static constexpr int dq_group = D == 32 ? 2 : 1, dq_ctas = D == 32 ? 4 : (D == 64 ? 4 : 2);   // D = 32: 105.4 us against 107.5 with group 1 / 5 CTAs
+    static constexpr int dq_group = D == 32 || D == 80 ? 2 : 1, dq_ctas = D <= 64 ? 4 : (D == 80 ? 3 : 2);   // D = 80: 69.0 us (80 with 2 CTAs); D = 32: 105.4 us against 107.5 with group 1 / 5 CTAs
     static constexpr int dq_group_se = 1, dq_ctas_se = D == 32 ? 5 : 4;      // with scale_embed: more shared memory and registers per CTA
     static constexpr int dkdv_group_se = D <= 64 ? 2 : 1, dkdv_ctas_se = D == 32 ? 4 : 3;
-    static constexpr int dkdv_group = D <= 64 ? 2 : 1, dkdv_ctas = D == 32 ? 4 : (D == 64 ? 3 : 2);
+    static constexpr int dkdv_group = D <= 80 ? 2 : 1, dkdv_ctas = D == 32 ? 4 : (D <= 64 ? 3 : 2);   // D = 80: 78.1 us (83 with group 1, 96-109 with 3 CTAs)
 };
 constexpr int kStagePitch = kRows + 4;      // 68: no bank conflicts on the scattered writes; the column sums rotate their start
 constexpr int kStagePitchSe = kRows + 4;    // 68 with scale_embed: rows are read back as 8-byte pairs by the dS MMAs
@@ -1029,13 +1030,14 @@ bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int
     __shared__ __align__(16) float2 stat_s[kStat];
     const Lane L;
     const int bh = blockIdx.y, h = bh % a.H, N = a.N;
-    // n_reduce CTAs (every reduce_stride-th one, so that no wave of CTAs is delayed as a whole)
-    // also finish the parameter gradients: one output each, from the partial sums the dQ kernel
-    // (an earlier launch on the stream) left in the scratch.
+    // Every reduce_stride-th CTA (so that no wave of CTAs is delayed as a whole) also finishes the
+    // parameter gradients: n_reduce outputs in all, from the partial sums the dQ kernel (an earlier
+    // launch on the stream) left in the scratch.
     static_assert(kWarps * 32 == kReduceThreads, "the fused reduction uses the CTA as one reduce block");
     const int cta = blockIdx.y * gridDim.x + blockIdx.x;
-    if (cta % reduce_stride == 0 && cta / reduce_stride < n_reduce)
-        reduce_one_param(a, t.J, cta / reduce_stride, reinterpret_cast<float*>(init_s));
+    if (cta % reduce_stride == 0)
+        for (int o = cta / reduce_stride; o < n_reduce; o += gridDim.x * gridDim.y / reduce_stride)
+            reduce_one_param(a, t.J, o, reinterpret_cast<float*>(init_s));
     const int m_cta = blockIdx.x * kRows;
     const int nd = t.n_dense, ndp = nd + 1, Jp = (t.J + 7) / 8 * 8;
     {
@@ -1131,7 +1133,7 @@ cudaError_t fwd_launch_mma(const FwdArgs& a, const Taps& t, cudaStream_t s) {
     constexpr int W = FwdTune<D>::warps, rows = 16 * W;
     dim3 grid((a.N + rows - 1) / rows, a.B * a.H);
     if (a.scale_embed) {
-        if constexpr (D <= 64) {
+        if constexpr (D <= 64 && !kTail<D>) {
             const size_t smem = se_tables_bytes(t.J, D, (WB + 16) / 8, W, 16);
             static int seen[64] = {0}, seen_st[64] = {0};
             cudaError_t e = a.strided ? ensure_dynamic_smem(fwd_mma_kernel<D, WB, true, true>, smem, seen_st)
@@ -1143,7 +1145,8 @@ cudaError_t fwd_launch_mma(const FwdArgs& a, const Taps& t, cudaStream_t s) {
             return cudaErrorInvalidValue;
         }
     } else if (a.strided) {
-        fwd_mma_kernel<D, WB, false, true><<<grid, W * 32, 0, s>>>(a, t);
+        if constexpr (kTail<D>) return cudaErrorInvalidValue;
+        else fwd_mma_kernel<D, WB, false, true><<<grid, W * 32, 0, s>>>(a, t);
     } else {
         fwd_mma_kernel<D, WB, false, false><<<grid, W * 32, 0, s>>>(a, t);
     }
@@ -1175,16 +1178,17 @@ cudaError_t bwd_launch_mma_se(BwdArgs a, const Taps& t, cudaStream_t s, int stag
         }
     }
     // With both stages in one call the reduction rides on CTAs of the dK/dV kernel (same code,
-    // same order of additions as the stand-alone kernel: bitwise equal results).
+    // same order of additions as the stand-alone kernel: bitwise equal results).  Up to four outputs per
+    // CTA cost less than the launch they save (about 1 us each against 2.7 us on the GPU and 4 us on the host).
     const int n_out = t.J * a.H + a.H + (SE ? t.J * a.D : 0);
     const bool fuse = (stages & DSQG_BWD_STAGE_DKDV) && (stages & DSQG_BWD_STAGE_REDUCE) &&
-                      (long long)grid.x * grid.y >= n_out;
+                      4LL * grid.x * grid.y >= n_out;
     if (stages & DSQG_BWD_STAGE_DKDV) {
         auto kern = bwd_dkdv_mma_kernel<D, WB, SE ? T::dkdv_group_se : T::dkdv_group, SE ? T::dkdv_ctas_se : T::dkdv_ctas, SE, ST>;
         const size_t smem = dkdv_smem_bytes(t.n_dense, WB, SE);
         static int seen[64] = {0};
         if ((e = ensure_dynamic_smem(kern, smem, seen)) != cudaSuccess) return e;
-        kern<<<grid, kWarps * 32, smem, s>>>(a, t, fuse ? n_out : 0, fuse ? (int)((long long)grid.x * grid.y / n_out) : 1);
+        kern<<<grid, kWarps * 32, smem, s>>>(a, t, fuse ? n_out : 0, fuse && (long long)grid.x * grid.y >= n_out ? (int)((long long)grid.x * grid.y / n_out) : 1);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if ((stages & DSQG_BWD_STAGE_REDUCE) && !fuse) e = launch_reduce_params(a, t.J, s);
@@ -1194,14 +1198,17 @@ cudaError_t bwd_launch_mma_se(BwdArgs a, const Taps& t, cudaStream_t s, int stag
 template <int D, int WB>
 cudaError_t bwd_launch_mma(const BwdArgs& a, const Taps& t, cudaStream_t s, int stages) {
     if (a.scale_embed) {
-        if constexpr (D <= 64) {
+        if constexpr (D <= 64 && !kTail<D>) {
             if (a.strided) return bwd_launch_mma_se<D, WB, true, true>(a, t, s, stages);
             return bwd_launch_mma_se<D, WB, true, false>(a, t, s, stages);
         } else {
             return cudaErrorInvalidValue;
         }
     }
-    if (a.strided) return bwd_launch_mma_se<D, WB, false, true>(a, t, s, stages);
+    if (a.strided) {
+        if constexpr (kTail<D>) return cudaErrorInvalidValue;
+        else return bwd_launch_mma_se<D, WB, false, true>(a, t, s, stages);
+    }
     return bwd_launch_mma_se<D, WB, false, false>(a, t, s, stages);
 }
 
@@ -1216,6 +1223,11 @@ static bool mma_shape_supported(int dtype, int D, const Taps& t) {
     const int wb = band_width(t);
     return dtype == DSQG_DTYPE_BF16 && t.n_sparse <= kMaxSparse &&
            (((D == 32 || D == 64) && wb != 0) || ((D == 96 || D == 128) && wb == 32));
+}
+// Widths with a 16-element tail run on their own kernels when nothing else is asked of them (contiguous tensors, no
+// scale_embed); a caller may also pad them, so mma_fwd_supported / mma_path_supported leave them out.
+bool mma_tail_supported(int dtype, int D, const Taps& t, bool has_scale_embed) {
+    return dtype == DSQG_DTYPE_BF16 && (D == 48 || D == 80) && band_width(t) == 32 && !has_scale_embed;
 }
 bool mma_fwd_supported(int dtype, int D, const Taps& t, bool has_scale_embed) {
     return mma_shape_supported(dtype, D, t) && (!has_scale_embed || D <= 64);
@@ -1232,6 +1244,8 @@ bool mma_path_supported(int dtype, int D, const Taps& t, bool has_scale_embed) {
             if (wb_ == 48) return FN<32, 48>(__VA_ARGS__);                     \
             return FN<32, 64>(__VA_ARGS__);                                    \
         }                                                                      \
+        if (a.D == 48) return FN<48, 32>(__VA_ARGS__);                         \
+        if (a.D == 80) return FN<80, 32>(__VA_ARGS__);                         \
         if (a.D == 96) return FN<96, 32>(__VA_ARGS__);                         \
         if (a.D == 128) return FN<128, 32>(__VA_ARGS__);                       \
         if (wb_ == 32) return FN<64, 32>(__VA_ARGS__);                         \

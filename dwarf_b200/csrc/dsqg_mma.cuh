@@ -4,7 +4,8 @@
 // --------------------------------------------------------
 // lane = 4*g + tig  (g = 0..7, tig = 0..3).  A warp owns a tile of 16 rows.
 // A row of D bf16 elements is split into 16-byte chunks; thread tig reads chunk tig of
-// every 64-byte group, i.e. elements  d = 32*c + 8*tig + [0,8)  for c = 0 .. D/32-1.
+// every 64-byte group, i.e. elements  d = 32*c + 8*tig + [0,8)  for c = 0 .. D/32-1.  When 16
+// elements are left over (D = 48, 80) thread tig reads the eight bytes  D-16 + 4*tig + [0,4)  of them.
 // Those 8*D/32 elements are the thread's share of the contraction dimension for BOTH
 // operands of  mma.sync.m16n8k16  (the instruction assigns k-indices {2tig,2tig+1,2tig+8,
 // 2tig+9} of every k-step to thread tig in the A and in the B fragment alike, so any fixed
@@ -27,7 +28,8 @@ constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kNeg = -1.0e30f;   // finite "minus infinity": masked scores
 constexpr float kMinM = -1.0e29f;  // floor of the running row maximum: exp2(kNeg - kMinM) == 0
 
-template <int D> struct RowFrag { uint32_t r[D / 8]; };   // D/32 chunks x 4 registers
+template <int D> struct RowFrag { uint32_t r[D / 8]; };   // D/32 chunks x 4 registers, and 2 of a 16-element tail
+template <int D> constexpr bool kTail = D % 32 == 16;
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -43,6 +45,11 @@ __device__ __forceinline__ void load_row(RowFrag<D>& f, const __nv_bfloat16* row
         uint4 u = make_uint4(0u, 0u, 0u, 0u);
         if (valid) u = __ldg(reinterpret_cast<const uint4*>(row_ptr + 32 * c + 8 * tig));
         f.r[4 * c + 0] = u.x; f.r[4 * c + 1] = u.y; f.r[4 * c + 2] = u.z; f.r[4 * c + 3] = u.w;
+    }
+    if constexpr (kTail<D>) {
+        uint2 u = make_uint2(0u, 0u);
+        if (valid) u = __ldg(reinterpret_cast<const uint2*>(row_ptr + D - 16 + 4 * tig));
+        f.r[D / 8 - 2] = u.x; f.r[D / 8 - 1] = u.y;
     }
 }
 
@@ -138,6 +145,13 @@ __device__ __forceinline__ void store_acc_rows(const float (&acc)[D / 8][4], __n
         if (ok_lo) *reinterpret_cast<uint4*>(row_lo + 32 * c + 8 * tig) = lo;
         if (ok_hi) *reinterpret_cast<uint4*>(row_hi + 32 * c + 8 * tig) = hi;
     }
+    if constexpr (kTail<D>) {
+        constexpr int J = D / 8 - 2;
+        if (ok_lo) *reinterpret_cast<uint2*>(row_lo + D - 16 + 4 * tig) =
+            make_uint2(pack_bf16x2(acc[J][0] * s_lo, acc[J][1] * s_lo), pack_bf16x2(acc[J + 1][0] * s_lo, acc[J + 1][1] * s_lo));
+        if (ok_hi) *reinterpret_cast<uint2*>(row_hi + D - 16 + 4 * tig) =
+            make_uint2(pack_bf16x2(acc[J][2] * s_hi, acc[J][3] * s_hi), pack_bf16x2(acc[J + 1][2] * s_hi, acc[J + 1][3] * s_hi));
+    }
 }
 
 // As store_acc_rows, with every element multiplied by sigmoid(gate) of the same position (gate rows
@@ -224,12 +238,17 @@ __device__ __forceinline__ void diag_fma(float (&acc)[D / 8][4], float x_lo, flo
 // (log2 units): probabilities stay below 2^kSlack, which fp32 sums and bf16 values absorb.
 constexpr float kSlack = 16.f;
 
+// p: this thread's chunk of the row (row + 8 * tig)
 template <int D>
 __device__ __forceinline__ void load_row_at(RowFrag<D>& f, const __nv_bfloat16* p) {
 #pragma unroll
     for (int c = 0; c < D / 32; ++c) {
         const uint4 u = __ldg(reinterpret_cast<const uint4*>(p + 32 * c));
         f.r[4 * c + 0] = u.x; f.r[4 * c + 1] = u.y; f.r[4 * c + 2] = u.z; f.r[4 * c + 3] = u.w;
+    }
+    if constexpr (kTail<D>) {
+        const uint2 u = __ldg(reinterpret_cast<const uint2*>(p + D - 16 - 4 * (int)(threadIdx.x & 3)));
+        f.r[D / 8 - 2] = u.x; f.r[D / 8 - 1] = u.y;
     }
 }
 

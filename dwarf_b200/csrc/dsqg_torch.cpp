@@ -7,6 +7,7 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
@@ -80,6 +81,11 @@ void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 float* fptr(const Tensor& t) { return t.defined() ? static_cast<float*>(t.data_ptr()) : nullptr; }
 void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
+// Uninitialised device tensors straight from the allocator: a dispatched at::empty costs 2.6 us on an autograd thread, this
+// one less than a third, and a backward call makes six.
+Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dt, const Tensor& on) { return at::detail::empty_cuda(sizes, dt, on.device(), std::nullopt); }
+Tensor new_like(const Tensor& t) { return t.defined() ? new_tensor(t.sizes(), t.scalar_type(), t) : t; }
+
 // A parameter as the kernels read it: fp32, contiguous, detached.
 Tensor f32c(const Tensor& t) {
     if (!t.defined()) return t;
@@ -107,11 +113,15 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
     if (hg.defined() && !shape_is(hg, {H})) want("head_gain", H, 0, hg);
 }
 
-// Head dimension the kernels are called with (ops._padded_head_dim has the reasons).
+// Head dimension the kernels are called with: ops._padded_head_dim has the reasons for padding; the widths 48 and 80 have
+// kernels of their own for the usual dense window without scale_embed (B8 H8 N2048 HD80 forward + backward: the copies into
+// 96 columns and back took 232 us of 454).
 int64_t padded_head_dim(const Tensor& q, const Offsets& off, bool has_se) {
     const int64_t D = q.size(3);
     if (q.scalar_type() != at::kBFloat16 || D % 32 == 0 || D > 128 || D % 8 != 0) return D;
     const int64_t Dp = (D + 31) / 32 * 32;
+    const bool own = (D == 48 || D == 80) && !has_se;
+    if (own && dsqg_tensor_core_path(DSQG_DTYPE_BF16, 96, off.v.data(), off.J(), 0)) return D;
     return dsqg_tensor_core_path(DSQG_DTYPE_BF16, (int)Dp, off.v.data(), off.J(), has_se) ? Dp : D;
 }
 
@@ -138,8 +148,8 @@ Forward attention_forward(const Tensor& q0, const Tensor& k0, const Tensor& v0, 
     }
     f.q = f.q.contiguous(); f.k = f.k.contiguous(); f.v = f.v.contiguous();
     const int64_t B = f.q.size(0), H = f.q.size(1), N = f.q.size(2);
-    f.out = at::empty_like(f.q);
-    f.lse = at::empty({B, H, N}, f.q.options().dtype(at::kFloat));
+    f.out = new_like(f.q);
+    f.lse = new_tensor({B, H, N}, at::kFloat, f.q);
     check(dsqg_fwd_scaled(ptr(f.q), ptr(f.k), ptr(f.v), fptr(f.pb), fptr(f.se), fptr(f.hg), off.v.data(), off.J(), ptr(f.out), fptr(f.lse),
                           (int)B, (int)H, (int)N, (int)Dp, dt, stream_of(f.q), (float)(1.0 / std::sqrt((double)f.D))), "dsqg_fwd");
     return f;
@@ -179,8 +189,8 @@ struct AttentionNode : torch::autograd::Function<AttentionNode> {
         if (dout.scalar_type() != q.scalar_type()) dout = dout.to(q.scalar_type());
         if (Dp != D) dout = pad_to(dout, Dp);
         dout = dout.contiguous();                                  // kernels/dsqg_attention_v3.py:394
-        Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v), dpb = at::empty_like(pb);
-        Tensor dhg = hg.defined() ? at::empty_like(hg) : Tensor(), dse = se.defined() ? at::empty_like(se) : Tensor();
+        Tensor dq = new_like(q), dk = new_like(k), dv = new_like(v), dpb = new_like(pb);
+        Tensor dhg = new_like(hg), dse = new_like(se);
         const size_t bytes = dsqg_bwd_scratch_bytes(off.J(), (int)B, (int)H, (int)N, (int)Dp, se.defined());
         const at::DataPtr scratch = scratch_for(bytes);
         check(dsqg_bwd_scaled(ptr(q), ptr(k), ptr(v), fptr(pb), fptr(se), fptr(hg), off.v.data(), off.J(), ptr(out), fptr(lse), ptr(dout),
@@ -213,8 +223,8 @@ std::tuple<Tensor, Tensor> forward_lse(const Tensor& q0, const Tensor& k0, const
     const int dt = dtype_code(q0);
     const c10::cuda::CUDAGuard guard(q0.device());
     const Tensor q = q0.contiguous(), k = k0.contiguous(), v = v0.contiguous(), pb = f32c(pb0), hg = f32c(opt(hg0)), se = f32c(opt(se0));
-    Tensor out = at::empty_like(q, at::TensorOptions().requires_grad(false));
-    Tensor lse = at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));
+    Tensor out = new_like(q);
+    Tensor lse = new_tensor({q.size(0), q.size(1), q.size(2)}, at::kFloat, q);
     check(dsqg_fwd(ptr(q), ptr(k), ptr(v), fptr(pb), fptr(se), fptr(hg), off->v.data(), off->J(), ptr(out), fptr(lse), (int)q.size(0),
                    (int)q.size(1), (int)q.size(2), (int)q.size(3), dt, stream_of(q)), "dsqg_fwd");
     return {out, lse};
@@ -245,9 +255,8 @@ PackedForward packed_forward(const Tensor& qkv, const Tensor& gate, const Tensor
         throw py::value_error("dsqg: scale_embed must be [" + std::to_string(J) + "," + std::to_string(D) + "], got " + shape_of(f.se));
     if (!qkv.is_cuda()) throw std::runtime_error("dsqg: tensors must live on a CUDA device (there is no CPU path)");
     const c10::cuda::CUDAGuard guard(qkv.device());
-    const auto opts = at::TensorOptions().device(qkv.device());
-    f.y = at::empty({B, N, H * D}, opts.dtype(at::kBFloat16));
-    f.lse = at::empty({B, H, N}, opts.dtype(at::kFloat));
+    f.y = new_tensor({B, N, H * D}, at::kBFloat16, qkv);
+    f.lse = new_tensor({B, H, N}, at::kFloat, qkv);
     const PackedStrides st(N, H, D);
     if (f.se.defined())
         check(dsqg_fwd_strided_se(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.se), fptr(f.hg), off.v.data(), off.J(),
@@ -269,16 +278,15 @@ PackedGrads packed_backward(const Tensor& qkv, const PackedForward& f, const Ten
     const PackedStrides st(N, H, D);
     void* stream = stream_of(qkv);
     PackedGrads g;
-    g.dqkv = at::empty_like(qkv); g.dpb = at::empty_like(f.pb);
-    if (f.hg.defined()) g.dhg = at::empty_like(f.hg);
-    if (f.se.defined()) g.dse = at::empty_like(f.se);
+    g.dqkv = new_like(qkv); g.dpb = new_like(f.pb);
+    g.dhg = new_like(f.hg); g.dse = new_like(f.se);
     const size_t bytes = dsqg_bwd_scratch_bytes(off.J(), (int)B, (int)H, (int)N, (int)D, f.se.defined());
     const at::DataPtr scratch = scratch_for(bytes);
     at::DataPtr dout_mem, delta_mem;
     void* dout = ptr(dy);
     float* delta = nullptr;
     if (f.gate.defined()) {
-        g.dgate = at::empty_like(f.gate);
+        g.dgate = new_like(f.gate);
         dout_mem = scratch_for((size_t)dy.numel() * 2);
         delta_mem = scratch_for((size_t)B * H * N * 4);
         dout = dout_mem.get(); delta = static_cast<float*>(delta_mem.get());
@@ -325,7 +333,7 @@ Tensor attention_packed(const Tensor& qkv, const std::optional<Tensor>& gate, co
 // ------------------------------------------------------------------------------------ causal mean
 Tensor causal_mean_run(const Tensor& x, bool reverse) {
     const c10::cuda::CUDAGuard guard(x.device());
-    Tensor out = at::empty_like(x, at::TensorOptions().requires_grad(false));
+    Tensor out = new_like(x);
     check(dsqg_causal_mean(ptr(x), ptr(out), (int)x.size(0), (int)x.size(1), (int)x.size(2), dtype_code(x), reverse, stream_of(x)), "dsqg_causal_mean");
     return out;
 }
@@ -370,7 +378,7 @@ Tensor decode_step(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
         throw py::value_error("dsqg_decode: k_ring and v_ring must be contiguous [S,H,R,D]");
     const StepParams p = {f32c(pos_bias), f32c(opt(hg)), f32c(opt(se))};
     const c10::cuda::CUDAGuard guard(q.device());
-    Tensor out = out0.has_value() ? *out0 : at::empty_like(q, at::TensorOptions().requires_grad(false));
+    Tensor out = out0.has_value() ? *out0 : new_like(q);
     check((overlap ? dsqg_decode_overlapped : dsqg_decode)(
               ptr(q), ptr(k), ptr(v), ptr(k_ring), ptr(v_ring), static_cast<const int32_t*>(ptr(head)), static_cast<const int32_t*>(ptr(fill)),
               fptr(p.pb), fptr(p.se), fptr(p.hg), off->v.data(), off->J(), (int)R, ptr(out), (int)S, (int)H, (int)D, dtype_code(q), stream_of(q)),
@@ -391,7 +399,7 @@ Tensor decode_step_kv(const Tensor& q, const Tensor& k, const Tensor& v, const T
     check_step("dsqg_decode_kv", q, k, v, kv.scalar_type(), S, H, D, head, fill, pos_bias, off->J());
     const StepParams p = {f32c(pos_bias), f32c(opt(hg)), f32c(opt(se))};
     const c10::cuda::CUDAGuard guard(q.device());
-    Tensor out = out0.has_value() ? *out0 : at::empty_like(q, at::TensorOptions().requires_grad(false));
+    Tensor out = out0.has_value() ? *out0 : new_like(q);
     char* ring = static_cast<char*>(kv.data_ptr()) + (lead ? layer * kv.stride(0) * kv.element_size() : 0);
     check(dsqg_decode_kv(ptr(q), ptr(k), ptr(v), ring, static_cast<const int32_t*>(ptr(head)), static_cast<const int32_t*>(ptr(fill)),
                          fptr(p.pb), fptr(p.se), fptr(p.hg), off->v.data(), off->J(), (int)R, ptr(out), (int)S, (int)H, (int)D, dtype_code(q),
@@ -403,7 +411,7 @@ Tensor decode_step_kv(const Tensor& q, const Tensor& k, const Tensor& v, const T
 std::tuple<Tensor, Tensor> ring_advance(const Tensor& head0, const Tensor& fill0, int64_t R) {
     const Tensor head = head0.to(at::kInt).contiguous(), fill = fill0.to(at::kInt).contiguous();
     const c10::cuda::CUDAGuard guard(head.device());
-    Tensor h = at::empty_like(head), f = at::empty_like(fill);
+    Tensor h = new_like(head), f = new_like(fill);
     check(dsqg_ring_advance(static_cast<const int32_t*>(ptr(head)), static_cast<const int32_t*>(ptr(fill)), static_cast<int32_t*>(ptr(h)),
                             static_cast<int32_t*>(ptr(f)), (int)head.numel(), (int)R, stream_of(head)), "dsqg_ring_advance");
     return {h, f};
