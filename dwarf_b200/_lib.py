@@ -61,6 +61,15 @@ _SIGNATURES = {
     "dsqg_decode": (c_int, [c_void_p] * 3 + [c_void_p] * 2 + [c_void_p] * 2 + [c_void_p] * 3
                     + [POINTER(c_int32), c_int, c_int] + [c_void_p] + [c_int] * 4 + [c_void_p]),
     "dsqg_ring_advance": (c_int, [c_void_p] * 4 + [c_int] * 2 + [c_void_p]),
+    "dsqg_cast_bf16": (c_int, [POINTER(c_void_p), POINTER(c_void_p), POINTER(ctypes.c_longlong), c_int, c_void_p]),
+    "dsqg_layer_norm_fwd": (c_int, [c_void_p] * 3 + [c_float] + [c_void_p] * 3 + [ctypes.c_longlong, c_int, c_void_p]),
+    "dsqg_layer_norm_bwd_scratch_bytes": (c_size_t, [ctypes.c_longlong, c_int]),
+    "dsqg_layer_norm_bwd": (c_int, [c_void_p] * 8 + [c_size_t, ctypes.c_longlong, c_int, c_void_p]),
+    "dsqg_gated_pool": (c_int, [c_void_p] * 3 + [ctypes.c_longlong, c_void_p]),
+    "dsqg_gated_pool_bwd": (c_int, [c_void_p] * 5 + [ctypes.c_longlong, c_void_p]),
+    "dsqg_inject_kv": (c_int, [c_void_p] * 3 + [ctypes.c_longlong] * 2 + [c_int, c_void_p]),
+    "dsqg_column_sums": (c_int, [POINTER(c_void_p), POINTER(ctypes.c_longlong), POINTER(c_int), POINTER(c_void_p), c_int,
+                                 ctypes.c_longlong, c_void_p]),
     "dsqg_causal_mean": (c_int, [c_void_p, c_void_p] + [c_int] * 5 + [c_void_p]),
     "dsqg_decode_kv": (c_int, [c_void_p] * 3 + [c_void_p] + [c_void_p] * 2 + [c_void_p] * 3
                        + [POINTER(c_int32), c_int, c_int] + [c_void_p] + [c_int] * 4 + [c_void_p, c_int]),

@@ -2,90 +2,172 @@
 //
 // This is the pooling of the DWARF condU "interference" block, which feeds the K/V injection of
 // its DSQG layer: `pool = xi.cumsum(dim=1) / counts` (train/train_2048_condU.py:289-292).  The
-// reference runs a cumsum in the activation dtype and a divide; here one kernel reads x twice and
+// reference runs a cumsum in the activation dtype and a divide; here one kernel reads x once and
 // writes the mean once, accumulating in fp32 whatever the storage type.
 // REVERSE is its adjoint (the backward pass): out[b,n,:] = sum_{m >= n} x[b,m,:] / (m + 1).
 //
-// One thread block takes kGroups slices of 8 contiguous channels of one batch entry over the whole
-// sequence, split into kChunks consecutive chunks of rows: every thread sums its chunk, the chunk
-// sums are combined through shared memory, then every thread walks its chunk again with the
-// running sum.  No scratch memory, no atomics, fixed order of additions.
+// Bound by memory; what there is to lose is idle SMs: a 128-byte wide slice of one batch entry is one chain
+// of additions over the sequence.  A cluster of up to eight blocks shares such a slice: every thread loads 16 bytes
+// each of `len` consecutive rows into registers and adds them up, the sums
+// are scanned over the warp (shuffles), the block (shared memory) and the cluster (each block stores its
+// total in every other block's shared memory), and the rows are written from the registers.  Only sequences
+// longer than the cluster's registers (4096 rows) read x a second time, from L2.  No scratch
+// memory, no atomics, fixed order of additions.  B8 N2048 D256 fp32: 8.4 us against 38 us with one block per 64 channels.
 #include "dsqg_common.cuh"
 
 namespace dsqg {
 namespace {
 
-constexpr int kChunks = 32, kGroups = 8;
+constexpr int kGroups = 8, kRowThreads = 32, kScanThreads = kGroups * kRowThreads, kScanCluster = 8;
+
+// One thread's 16 bytes of a row.
+template <typename T> struct Piece;
+template <> struct Piece<__nv_bfloat16> {
+    static constexpr int C = 8;
+    uint4 u;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { u = __ldg(reinterpret_cast<const uint4*>(p)); }
+    __device__ __forceinline__ void get(float (&x)[8]) const {
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { x[2 * i] = __uint_as_float(w[i] << 16); x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+    }
+    static __device__ __forceinline__ void store(__nv_bfloat16* p, const float (&x)[8]) { store8(p, x); }
+};
+template <> struct Piece<float> {
+    static constexpr int C = 4;
+    float4 a;
+    __device__ __forceinline__ void load(const float* p) { a = __ldg(reinterpret_cast<const float4*>(p)); }
+    __device__ __forceinline__ void get(float (&x)[4]) const { x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; }
+    static __device__ __forceinline__ void store(float* p, const float (&x)[4]) { *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]); }
+};
+
+// R > 0: the thread's rows (len <= R) stay in registers; R == 0: any len, read twice.
+template <typename T, bool REVERSE, int R>
+__global__ void __launch_bounds__(kScanThreads)
+causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, int len) {
+    constexpr int C = Piece<T>::C, kSlice = C * kGroups;
+    __shared__ __align__(16) float warp_sum[kScanThreads / 32][kSlice];
+    __shared__ __align__(16) float block_sum[kScanCluster][kSlice];
+    const int grp = threadIdx.x % kGroups, chunk = threadIdx.x / kGroups, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int ranks = gridDim.x, rank = blockIdx.x;                 // one cluster along x
+    if (ranks > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");     // peers may be written to once all have started
+    const int d0 = (blockIdx.y * kGroups + grp) * C;
+    const bool active = d0 < D;
+    // position along the direction of the sum: reversed sums walk the rows from the end
+    const int first = (rank * kRowThreads + chunk) * len;
+    const int mine = active ? max(0, min(len, N - first)) : 0;
+    const size_t base = (size_t)blockIdx.z * N * D + d0;
+    auto row = [&](int i) { return REVERSE ? N - 1 - first - i : first + i; };
+    float s[C] = {};
+    Piece<T> keep[R > 0 ? R : 1];
+    auto add = [&](const Piece<T>& v, int i) {
+        float f[C];
+        v.get(f);
+        const float w = REVERSE ? 1.f / (float)(row(i) + 1) : 1.f;
+#pragma unroll
+        for (int c = 0; c < C; ++c) s[c] = fmaf(f[c], w, s[c]);
+    };
+    if constexpr (R > 0) {
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (i < mine) keep[i].load(x + base + (size_t)row(i) * D);
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (i < mine) add(keep[i], i);
+    } else {
+#pragma unroll 4
+        for (int i = 0; i < mine; ++i) { keep[0].load(x + base + (size_t)row(i) * D); add(keep[0], i); }
+    }
+    // exclusive sum over the threads before this one
+    float inc[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        float v = s[c], t = __shfl_up_sync(0xffffffffu, v, kGroups);
+        if (lane >= kGroups) v += t;
+        t = __shfl_up_sync(0xffffffffu, v, 2 * kGroups);
+        if (lane >= 2 * kGroups) v += t;
+        inc[c] = v;
+        s[c] = v - s[c];
+    }
+    if (lane >= 32 - kGroups) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) warp_sum[warp][C * grp + c] = inc[c];
+    }
+    __syncthreads();
+    if (ranks > 1) {
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        if (threadIdx.x < kSlice) {
+            float t = 0.f;
+#pragma unroll
+            for (int w = 0; w < kScanThreads / 32; ++w) t += warp_sum[w][threadIdx.x];
+            const uint32_t addr = static_cast<uint32_t>(__cvta_generic_to_shared(&block_sum[rank][threadIdx.x]));
+            for (int r = 0; r < ranks; ++r) {
+                uint32_t there;
+                asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(addr), "r"(r));
+                asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(there), "f"(t) : "memory");
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        for (int r = 0; r < rank; ++r)
+#pragma unroll
+            for (int c = 0; c < C; ++c) s[c] += block_sum[r][C * grp + c];
+    }
+    for (int w = 0; w < warp; ++w)
+#pragma unroll
+        for (int c = 0; c < C; ++c) s[c] += warp_sum[w][C * grp + c];
+    auto put = [&](const Piece<T>& v, int i) {
+        float f[C], o[C];
+        v.get(f);
+        const float w = 1.f / (float)(row(i) + 1);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            s[c] = REVERSE ? fmaf(f[c], w, s[c]) : s[c] + f[c];
+            o[c] = REVERSE ? s[c] : s[c] * w;
+        }
+        Piece<T>::store(out + base + (size_t)row(i) * D, o);
+    };
+    if constexpr (R > 0) {
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (i < mine) put(keep[i], i);
+    } else {
+#pragma unroll 4
+        for (int i = 0; i < mine; ++i) { keep[0].load(x + base + (size_t)row(i) * D); put(keep[0], i); }
+    }
+}
+
+template <typename T, bool REVERSE, int R>
+cudaError_t launch_scan(const T* x, T* out, int B, int N, int D, int ranks, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(ranks, (D / Piece<T>::C + kGroups - 1) / kGroups, B); cfg.blockDim = dim3(kScanThreads); cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ranks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, causal_mean_kernel<T, REVERSE, R>, x, out, N, D, (N + ranks * kRowThreads - 1) / (ranks * kRowThreads));
+}
 
 template <typename T, bool REVERSE>
-__global__ void __launch_bounds__(kChunks * kGroups)
-causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D) {
-    __shared__ float part[kChunks][kGroups][8];
-    const int grp = threadIdx.x % kGroups, chunk = threadIdx.x / kGroups;
-    const int d0 = (blockIdx.x * kGroups + grp) * 8;
-    const bool active = d0 < D;
-    const int len = (N + kChunks - 1) / kChunks;
-    const int r0 = chunk * len, r1 = min(N, r0 + len);
-    const T* xp = x + (size_t)blockIdx.y * N * D + d0;
-    T* op = out + (size_t)blockIdx.y * N * D + d0;
-    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (active) {
-        for (int r = r0; r < r1; ++r) {
-            float v[8];
-            load8(xp + (size_t)r * D, v);
-            const float w = REVERSE ? 1.f / (float)(r + 1) : 1.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) s[i] = fmaf(v[i], w, s[i]);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) part[chunk][grp][i] = s[i];
-    __syncthreads();
-    if (!active) return;
-    // what lies before (forward) or after (reverse) this thread's chunk
-    float run[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (REVERSE) {
-        for (int c = kChunks - 1; c > chunk; --c)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) run[i] += part[c][grp][i];
-        for (int r = r1 - 1; r >= r0; --r) {
-            float v[8], o[8];
-            load8(xp + (size_t)r * D, v);
-            const float w = 1.f / (float)(r + 1);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) { run[i] = fmaf(v[i], w, run[i]); o[i] = run[i]; }
-            store8(op + (size_t)r * D, o);
-        }
-    } else {
-        for (int c = 0; c < chunk; ++c)
-#pragma unroll
-            for (int i = 0; i < 8; ++i) run[i] += part[c][grp][i];
-        for (int r = r0; r < r1; ++r) {
-            float v[8], o[8];
-            load8(xp + (size_t)r * D, v);
-            const float w = 1.f / (float)(r + 1);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) { run[i] += v[i]; o[i] = run[i] * w; }
-            store8(op + (size_t)r * D, o);
-        }
-    }
+cudaError_t launch_mean(const T* x, T* out, int B, int N, int D, cudaStream_t s) {
+    // as many blocks as give every thread two rows at least, eight at most
+    int ranks = 1;
+    while (ranks < kScanCluster && N > ranks * kRowThreads * 2) ranks *= 2;
+    const int len = (N + ranks * kRowThreads - 1) / (ranks * kRowThreads);
+    if (len <= 2) return launch_scan<T, REVERSE, 2>(x, out, B, N, D, ranks, s);
+    if (len <= 8) return launch_scan<T, REVERSE, 8>(x, out, B, N, D, ranks, s);
+    if (len <= 16) return launch_scan<T, REVERSE, 16>(x, out, B, N, D, ranks, s);
+    return launch_scan<T, REVERSE, 0>(x, out, B, N, D, ranks, s);
 }
 
 }  // namespace
 
 cudaError_t launch_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, bool reverse, cudaStream_t s) {
-    dim3 grid((D / 8 + kGroups - 1) / kGroups, B);
-    const int threads = kChunks * kGroups;
     if (dtype == DSQG_DTYPE_BF16) {
         auto xi = static_cast<const __nv_bfloat16*>(x); auto oi = static_cast<__nv_bfloat16*>(out);
-        if (reverse) causal_mean_kernel<__nv_bfloat16, true><<<grid, threads, 0, s>>>(xi, oi, N, D);
-        else causal_mean_kernel<__nv_bfloat16, false><<<grid, threads, 0, s>>>(xi, oi, N, D);
-    } else {
-        auto xi = static_cast<const float*>(x); auto oi = static_cast<float*>(out);
-        if (reverse) causal_mean_kernel<float, true><<<grid, threads, 0, s>>>(xi, oi, N, D);
-        else causal_mean_kernel<float, false><<<grid, threads, 0, s>>>(xi, oi, N, D);
+        return reverse ? launch_mean<__nv_bfloat16, true>(xi, oi, B, N, D, s) : launch_mean<__nv_bfloat16, false>(xi, oi, B, N, D, s);
     }
-    return cudaGetLastError();
+    auto xi = static_cast<const float*>(x); auto oi = static_cast<float*>(out);
+    return reverse ? launch_mean<float, true>(xi, oi, B, N, D, s) : launch_mean<float, false>(xi, oi, B, N, D, s);
 }
 
 }  // namespace dsqg

@@ -6,6 +6,7 @@
 // PyTorch supplies device memory, streams and the autograd graph only; all arithmetic is in libdsqg_b200.so.
 #include <torch/extension.h>
 
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -52,8 +53,16 @@ void check(int status, const char* where) {
     throw std::runtime_error(std::string(where) + " failed");
 }
 
-// Runs the body of a backward node: the autograd engine's threads carry Python errors in its own exception type.
-template <typename F> auto backward_body(F f) {
+// Runs the body of a backward node: the autograd engine's threads carry Python errors in its own exception type, and start
+// without a CUDA context, which cuBLAS would remark on.
+template <typename F> auto backward_body(const Tensor& on, F f) {
+    static thread_local int ready = -1;
+    if (on.defined() && on.is_cuda() && ready != on.device().index()) {
+        ready = on.device().index();
+        const int before = c10::cuda::current_device();
+        c10::cuda::SetDevice(ready, /*force=*/true);
+        c10::cuda::SetDevice(before);
+    }
     try {
         return f();
     } catch (py::error_already_set& e) {
@@ -177,7 +186,7 @@ struct AttentionNode : torch::autograd::Function<AttentionNode> {
     }
 
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
-        return backward_body([&] { return run(ctx, grads[0]); });
+        return backward_body(grads[0], [&] { return run(ctx, grads[0]); });
     }
 
     static variable_list run(AutogradContext* ctx, Tensor dout) {
@@ -317,7 +326,7 @@ struct PackedNode : torch::autograd::Function<PackedNode> {
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
         const variable_list s = ctx->get_saved_variables();
         const PackedForward f = {s[1], s[2], s[3], s[4], s[5], s[6]};
-        const PackedGrads g = backward_body([&] { return packed_backward(s[0], f, grads[0], offsets_of(ctx)); });
+        const PackedGrads g = backward_body(grads[0], [&] { return packed_backward(s[0], f, grads[0], offsets_of(ctx)); });
         return {g.dqkv, g.dgate, like_param(g.dpb, type_at(ctx, 0)), like_param(g.dhg, type_at(ctx, 1)), like_param(g.dse, type_at(ctx, 2)), Tensor()};
     }
 };
@@ -340,7 +349,7 @@ Tensor causal_mean_run(const Tensor& x, bool reverse) {
 struct CausalMeanNode : torch::autograd::Function<CausalMeanNode> {
     static Tensor forward(AutogradContext*, const Tensor& x) { return causal_mean_run(x, false); }
     static variable_list backward(AutogradContext*, variable_list grads) {
-        return backward_body([&] { return variable_list{causal_mean_run(grads[0].contiguous(), true)}; });
+        return backward_body(grads[0], [&] { return variable_list{causal_mean_run(grads[0].contiguous(), true)}; });
     }
 };
 Tensor causal_mean(const Tensor& x0) {
@@ -349,6 +358,213 @@ Tensor causal_mean(const Tensor& x0) {
         throw py::value_error("causal_mean: x must be a CUDA [B,N,D] tensor in bfloat16 or float32");
     const Tensor x = x0.contiguous();
     return wants_grad({&x}) ? CausalMeanNode::apply(x) : causal_mean_run(x, false);
+}
+
+// ------------------------------------------------------------------------------------ whole layers under bf16 autocast
+// The attention layer and the interference block as one autograd node each: what PyTorch runs as some ninety launches a
+// step (1.9 ms of host time for 0.95 ms of GPU work at B8 N2048 dim 256) is their GEMMs (cuBLAS through ATen), the operator
+// and the kernels of csrc/dsqg_layer.cu.  Weight gradients leave the GEMM in fp32 instead of being rounded to bf16 and cast.
+
+// Autocast is done by hand inside the nodes.
+struct NoAutocast {
+    c10::impl::ExcludeDispatchKeyGuard guard{c10::autocast_dispatch_keyset};
+};
+
+// bf16 copies of fp32 tensors back to back in one buffer, in one launch.
+std::vector<Tensor> cast_bf16(const std::vector<Tensor>& src0) {
+    std::vector<Tensor> src;
+    int64_t total = 0;
+    for (const Tensor& t : src0) { src.push_back(f32c(t)); total += t.numel(); }
+    const Tensor buf = new_tensor({total}, at::kBFloat16, src[0]);
+    std::vector<Tensor> out;
+    const float* sp[DSQG_CAST_MAX]; void* dp[DSQG_CAST_MAX]; long long n[DSQG_CAST_MAX];
+    int64_t o = 0;
+    for (size_t k = 0; k < src.size(); ++k) {
+        out.push_back(src[k].dim() == 2 ? at::as_strided(buf, src[k].sizes(), {src[k].size(1), 1}, o) : at::as_strided(buf, {src[k].numel()}, {1}, o));
+        sp[k] = fptr(src[k]); dp[k] = ptr(out[k]); n[k] = src[k].numel();
+        o += src[k].numel();
+    }
+    check(dsqg_cast_bf16(sp, dp, n, (int)src.size(), stream_of(buf)), "dsqg_cast_bf16");
+    return out;
+}
+
+Tensor mm_f32(const Tensor& a, const Tensor& b) { return at::mm(a, b, at::kFloat); }
+
+// Column sums of bf16 matrices, returned back to back.
+std::vector<Tensor> column_sums(const std::vector<Tensor>& ms) {
+    int64_t total = 0;
+    for (const Tensor& m : ms) total += m.size(1);
+    const Tensor buf = new_tensor({total}, at::kFloat, ms[0]);
+    std::vector<Tensor> out;
+    const void* sp[DSQG_SUM_MAX]; long long ld[DSQG_SUM_MAX]; int cols[DSQG_SUM_MAX]; float* dp[DSQG_SUM_MAX];
+    int64_t o = 0;
+    for (size_t k = 0; k < ms.size(); ++k) {
+        out.push_back(at::as_strided(buf, {ms[k].size(1)}, {1}, o));
+        sp[k] = ptr(ms[k]); ld[k] = ms[k].stride(0); cols[k] = (int)ms[k].size(1); dp[k] = fptr(out[k]);
+        o += ms[k].size(1);
+    }
+    check(dsqg_column_sums(sp, ld, cols, dp, (int)ms.size(), ms[0].size(0), stream_of(buf)), "dsqg_column_sums");
+    return out;
+}
+
+// [B,H,N,HD] view of columns [first, first + H*HD) of a row-major matrix of B*N rows, ld elements apart
+Tensor heads_view(const Tensor& m, int64_t B, int64_t H, int64_t N, int64_t HD, int64_t ld, int64_t first) {
+    return at::as_strided(m, {B, H, N, HD}, {N * ld, HD, ld, 1}, m.storage_offset() + first);
+}
+// The row stride of such a view (0: it is none).
+int64_t heads_stride(const Tensor& t) {
+    const int64_t H = t.size(1), N = t.size(2), HD = t.size(3), ld = t.stride(2);
+    const bool ok = t.stride(3) == 1 && (H == 1 || t.stride(1) == HD) && ld >= H * HD && ld % 8 == 0 && (t.size(0) == 1 || t.stride(0) == N * ld) &&
+                    (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+    return ok ? ld : 0;
+}
+Tensor rows_of(const Tensor& t) {        // [B,H,N,HD] -> [B*N, H*HD] bf16
+    return t.permute({0, 2, 1, 3}).reshape({t.size(0) * t.size(2), t.size(1) * t.size(3)}).to(at::kBFloat16);
+}
+
+// (k_delta, v_delta) of the interference block (train/train_2048_condU.py:277-295)
+struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& gamma, const Tensor& beta, const Tensor& wg, const Tensor& bg,
+                                 const Tensor& wk, const Tensor& bk, const Tensor& wv, const Tensor& bv, double eps, int64_t H) {
+        const NoAutocast no_autocast;
+        const c10::cuda::CUDAGuard guard(x.device());
+        const int64_t B = x.size(0), N = x.size(1), D = x.size(2), M = B * N;
+        const Tensor xc = f32c(x), gam = f32c(gamma);
+        const std::vector<Tensor> w = cast_bf16({wg, wk, wv, bg, bk, bv});
+        const Tensor wkv = at::as_strided(w[1], {2 * D, D}, {D, 1}, w[1].storage_offset()), bkv = at::as_strided(w[4], {2 * D}, {1}, w[4].storage_offset());
+        Tensor xi = new_tensor({B, N, D}, at::kFloat, x), xib = new_tensor({M, D}, at::kBFloat16, x), stat = new_tensor({M, 2}, at::kFloat, x);
+        check(dsqg_layer_norm_fwd(fptr(xc), fptr(gam), fptr(f32c(beta)), (float)eps, fptr(xi), ptr(xib), fptr(stat), M, (int)D, stream_of(x)), "dsqg_layer_norm_fwd");
+        const Tensor pool = causal_mean_run(xi, false), g = at::linear(xib, w[0], w[3]);
+        Tensor inter = new_like(g);
+        check(dsqg_gated_pool(ptr(g), fptr(pool), ptr(inter), M * D, stream_of(x)), "dsqg_gated_pool");
+        const Tensor kv = at::linear(inter, wkv, bkv);
+        ctx->save_for_backward({xc, gam, stat, xib, pool, g, inter, w[0], wkv});
+        ctx->saved_data["x_type"] = (int64_t)x.scalar_type();
+        return {heads_view(kv, B, H, N, D / H, 2 * D, 0), heads_view(kv, B, H, N, D / H, 2 * D, D)};
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        return backward_body(grads[0].defined() ? grads[0] : grads[1], [&] { return run(ctx, grads); });
+    }
+    static variable_list run(AutogradContext* ctx, const variable_list& grads) {
+        const NoAutocast no_autocast;
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &x = s[0], &gam = s[1], &stat = s[2], &xib = s[3], &pool = s[4], &g = s[5], &inter = s[6], &wg = s[7], &wkv = s[8];
+        const c10::cuda::CUDAGuard guard(x.device());
+        const int64_t D = x.size(2), M = x.size(0) * x.size(1);
+        Tensor dkv;                                            // [M, 2 D]: what comes from the attention layer already lies like that
+        const Tensor &dk = grads[0], &dv = grads[1];
+        if (dk.defined() && dv.defined() && dk.scalar_type() == at::kBFloat16 && dv.scalar_type() == at::kBFloat16) {
+            const int64_t ld = heads_stride(dk);
+            if (ld >= 2 * D && heads_stride(dv) == ld && static_cast<char*>(dv.data_ptr()) == static_cast<char*>(dk.data_ptr()) + 2 * D)
+                dkv = at::as_strided(dk, {M, 2 * D}, {ld, 1}, dk.storage_offset());
+        }
+        if (!dkv.defined()) {
+            const auto part = [&](const Tensor& d) { return d.defined() ? rows_of(d) : at::zeros({M, D}, xib.options()); };
+            dkv = at::cat({part(dk), part(dv)}, 1);
+        }
+        void* stream = stream_of(x);
+        const Tensor dinter = at::mm(dkv, wkv), dwkv = mm_f32(dkv.t(), inter);
+        Tensor dg = new_like(g), dpool = new_like(pool);
+        check(dsqg_gated_pool_bwd(ptr(dinter), ptr(g), fptr(pool), ptr(dg), fptr(dpool), M * D, stream), "dsqg_gated_pool_bwd");
+        const Tensor dxi = causal_mean_run(dpool, true), dxib = at::mm(dg, wg), dwg = mm_f32(dg.t(), xib);
+        const std::vector<Tensor> db = column_sums({dg, dkv});
+        Tensor dx = new_like(x), dgb = new_tensor({2, D}, at::kFloat, x);
+        const size_t bytes = dsqg_layer_norm_bwd_scratch_bytes(M, (int)D);
+        const at::DataPtr scratch = scratch_for(bytes);
+        check(dsqg_layer_norm_bwd(fptr(x), fptr(stat), fptr(gam), fptr(dxi), ptr(dxib), fptr(dx), fptr(dgb), scratch.get(), bytes, M, (int)D, stream), "dsqg_layer_norm_bwd");
+        return {like_param(dx, (at::ScalarType)ctx->saved_data["x_type"].toInt()), dgb.select(0, 0), dgb.select(0, 1), dwg, db[0],
+                dwkv.narrow(0, 0, D), db[1].narrow(0, 0, D), dwkv.narrow(0, D, D), db[1].narrow(0, D, D), Tensor(), Tensor()};
+    }
+};
+
+// qkv projection -> (K/V injection) -> operator -> gate -> output projection (train/train_2048_condU.py:171-191)
+struct LayerNode : torch::autograd::Function<LayerNode> {
+    static Tensor forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& kd, const std::optional<Tensor>& vd, const Tensor& wqkv,
+                          const Tensor& bqkv, const Tensor& wg, const Tensor& bg, const Tensor& wo, const Tensor& bo, const Tensor& pos_bias,
+                          const std::optional<Tensor>& hg, const std::optional<Tensor>& se, const Offsets* off, int64_t H) {
+        const NoAutocast no_autocast;
+        const c10::cuda::CUDAGuard guard(x.device());
+        const int64_t B = x.size(0), N = x.size(1), D = x.size(2), M = B * N;
+        std::vector<Tensor> w;
+        Tensor xb;
+        if (x.scalar_type() == at::kFloat) {
+            w = cast_bf16({wqkv, wg, wo, bqkv, bg, bo, x});
+            xb = w[6].view({M, D});
+        } else {
+            w = cast_bf16({wqkv, wg, wo, bqkv, bg, bo});
+            xb = x.reshape({M, D});
+        }
+        const Tensor qkv = at::linear(xb, w[0], w[3]);
+        if (kd.has_value()) {
+            Tensor k = *kd, v = *vd;
+            int64_t ld = k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16 ? heads_stride(k) : 0;
+            if (!ld || heads_stride(v) != ld) { k = rows_of(k).contiguous(); v = rows_of(v).contiguous(); ld = D; }
+            check(dsqg_inject_kv(ptr(qkv), ptr(k), ptr(v), ld, M, (int)D, stream_of(x)), "dsqg_inject_kv");
+        }
+        const Tensor gate = at::linear(xb, w[1], w[4]).view({B, N, D}), qkv5 = qkv.view({B, N, 3, H, D / H});
+        PackedForward f = packed_forward(qkv5, gate, pos_bias, opt(hg), opt(se), *off);
+        const Tensor out = at::linear(f.y, w[2], w[5]);
+        ctx->save_for_backward({xb, w[0], w[1], w[2], qkv5, f.gate, f.pb, f.hg, f.se, f.y, f.lse});
+        ctx->saved_data["offsets"] = (int64_t)(intptr_t)off;
+        ctx->saved_data["types"] = types_of(pos_bias, opt(hg), opt(se));
+        ctx->saved_data["x_types"] = std::vector<int64_t>{(int64_t)x.scalar_type(), (int64_t)type_of(opt(kd)), (int64_t)type_of(opt(vd))};
+        ctx->saved_data["inject"] = kd.has_value();
+        return out;
+    }
+
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        return backward_body(grads[0], [&] { return run(ctx, grads[0]); });
+    }
+    static variable_list run(AutogradContext* ctx, const Tensor& dy0) {
+        const NoAutocast no_autocast;
+        const variable_list s = ctx->get_saved_variables();
+        const Tensor &xb = s[0], &wqkv = s[1], &wg = s[2], &wo = s[3], &qkv = s[4];
+        const PackedForward f = {s[5], s[6], s[7], s[8], s[9], s[10]};
+        const int64_t B = qkv.size(0), N = qkv.size(1), H = qkv.size(3), HD = qkv.size(4), D = H * HD, M = B * N;
+        const c10::cuda::CUDAGuard guard(xb.device());
+        const Tensor dy = (dy0.scalar_type() == at::kBFloat16 ? dy0 : dy0.to(at::kBFloat16)).reshape({M, D}).contiguous();
+        const Tensor dyo = at::mm(dy, wo).view({B, N, D}), dwo = mm_f32(dy.t(), f.y.view({M, D}));
+        const PackedGrads g = packed_backward(qkv, f, dyo, offsets_of(ctx));
+        const Tensor dqkv = g.dqkv.view({M, 3 * D}), dgate = g.dgate.view({M, D});
+        const Tensor dwqkv = mm_f32(dqkv.t(), xb), dwg = mm_f32(dgate.t(), xb);
+        const std::vector<Tensor> db = column_sums({dqkv, dgate, dy});
+        const auto xt = ctx->saved_data["x_types"].toIntVector();
+        Tensor dx, dk, dv;
+        if (ctx->needs_input_grad(0)) {
+            dx = mm_f32(dqkv, wqkv);
+            at::addmm_out(dx, dx, dgate, wg, at::kFloat);       // accumulates in place
+            dx = like_param(dx.view({B, N, D}), (at::ScalarType)xt[0]);
+        }
+        if (ctx->saved_data["inject"].toBool()) {
+            dk = like_param(heads_view(dqkv, B, H, N, HD, 3 * D, D), (at::ScalarType)xt[1]);
+            dv = like_param(heads_view(dqkv, B, H, N, HD, 3 * D, 2 * D), (at::ScalarType)xt[2]);
+        }
+        return {dx, dk, dv, dwqkv, db[0], dwg, db[1], dwo, db[2], like_param(g.dpb, type_at(ctx, 0)), like_param(g.dhg, type_at(ctx, 1)),
+                like_param(g.dse, type_at(ctx, 2)), Tensor(), Tensor()};
+    }
+};
+
+// The nodes serve fp32 parameters under bf16 autocast.
+bool layer_applies(const Tensor& x, const std::vector<Tensor>& params) {
+    if (!x.is_cuda() || x.dim() != 3 || x.size(0) < 1 || x.size(1) < 1 || (x.scalar_type() != at::kFloat && x.scalar_type() != at::kBFloat16)) return false;
+    if (!at::autocast::is_autocast_enabled(at::kCUDA) || at::autocast::get_autocast_dtype(at::kCUDA) != at::kBFloat16) return false;
+    for (const Tensor& p : params)
+        if (p.scalar_type() != at::kFloat || p.device() != x.device()) return false;
+    return true;
+}
+
+std::tuple<Tensor, Tensor> interference(const Tensor& x, const Tensor& gamma, const Tensor& beta, const Tensor& wg, const Tensor& bg, const Tensor& wk,
+                                        const Tensor& bk, const Tensor& wv, const Tensor& bv, double eps, int64_t H) {
+    py::gil_scoped_release no_gil;
+    const variable_list r = InterferenceNode::apply(x, gamma, beta, wg, bg, wk, bk, wv, bv, eps, H);
+    return {r[0], r[1]};
+}
+Tensor layer(const Tensor& x, const std::optional<Tensor>& kd, const std::optional<Tensor>& vd, const Tensor& wqkv, const Tensor& bqkv, const Tensor& wg,
+             const Tensor& bg, const Tensor& wo, const Tensor& bo, const Tensor& pb, const std::optional<Tensor>& hg, const std::optional<Tensor>& se,
+             const Offsets* off, int64_t H) {
+    py::gil_scoped_release no_gil;
+    return LayerNode::apply(x, kd, vd, wqkv, bqkv, wg, bg, wo, bo, pb, hg, se, off, H);
 }
 
 // ------------------------------------------------------------------------------------ decode
@@ -425,6 +641,9 @@ PYBIND11_MODULE(_dsqg_torch, m) {
     m.def("attention", &attention);
     m.def("forward_lse", &forward_lse);
     m.def("attention_packed", &attention_packed);
+    m.def("layer_applies", &layer_applies);
+    m.def("interference", &interference);
+    m.def("layer", &layer);
     m.def("causal_mean", &causal_mean);
     m.def("decode_step", &decode_step);
     m.def("decode_step_kv", &decode_step_kv);

@@ -19,6 +19,7 @@ from typing import Optional, Sequence
 import torch
 import torch.nn as nn
 
+from . import _lib
 from .ops import (ALL_OFFSETS, InjectKVFunction, causal_mean, dsqg_attention, dsqg_attention_packed,
                   packed_path_available)
 
@@ -47,6 +48,15 @@ def _log_linear_bias(offsets, num_heads):
     alphas = torch.linspace(0.2, 2.0, num_heads)
     logs = torch.tensor([math.log(1.0 + d) for d in offsets], dtype=torch.float32)
     return -logs[:, None] * alphas[None, :]
+
+
+def _plain(*mods):
+    """True when each of the modules is the stock class with fp32-style parameters and nobody listens in on it (hooks): its
+    forward may then be part of a larger native node."""
+    for m, cls in mods:
+        if type(m) is not cls or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or m.bias is None:
+            return False
+    return True
 
 
 class _DSQGAttentionBase(nn.Module):
@@ -132,8 +142,28 @@ class _DSQGAttentionBase(nn.Module):
         flat = out.permute(0, 2, 1, 3).reshape(B, N, D)
         return self.dropout(self.out_proj(flat * torch.sigmoid(self.gate_proj(x)))), k, v
 
+    def _native_layer(self, x, kv_inject):
+        """The whole layer as one autograd node (csrc/dsqg_torch.cpp) under bf16 autocast, or None where that does not apply."""
+        qkv, gate, out = self.qkv_proj, self.gate_proj, self.out_proj
+        if not x.is_cuda or not _plain((qkv, nn.Linear), (gate, nn.Linear), (out, nn.Linear)) or x.dim() != 3 or x.shape[-1] != self.embedding_dim \
+                or self.embedding_dim % 8:
+            return None
+        n = _lib.native()
+        if not n.layer_applies(x, [qkv.weight, qkv.bias, gate.weight, gate.bias, out.weight, out.bias]):
+            return None
+        if self._packed is None:
+            self._packed = packed_path_available(self.head_dim, self._offsets, hasattr(self, "scale_embed"))
+        if not self._packed:
+            return None
+        kd, vd = (None, None) if kv_inject is None else kv_inject
+        if kd is not None and (kd.shape != (x.shape[0], self.num_heads, x.shape[1], self.head_dim) or vd.shape != kd.shape or not kd.is_cuda or not vd.is_cuda):
+            return None
+        return n.layer(x, kd, vd, qkv.weight, qkv.bias, gate.weight, gate.bias, out.weight, out.bias, self.pos_bias, getattr(self, "if_gain", None),
+                       getattr(self, "scale_embed", None), _lib.offsets_handle(self._offsets), self.num_heads)
+
     def forward(self, x, kv_inject=None):
-        return self.attend(x, kv_inject)[0]
+        y = self._native_layer(x, kv_inject)
+        return self.attend(x, kv_inject)[0] if y is None else self.dropout(y)
 
     def decode(self, x, cache, layer, overlap=False):
         """One new token per sequence: x [S,D] -> [S,D], reading the previous tokens' k, v from
@@ -207,6 +237,13 @@ class InterferenceInjection(nn.Module):
         self.inter_v_proj = nn.Linear(embedding_dim, embedding_dim)
 
     def forward(self, x):
+        norm, gate, kp, vp = self.inter_norm, self.inter_gate, self.inter_k_proj, self.inter_v_proj
+        D = x.shape[-1]
+        if x.is_cuda and D % 8 == 0 and D <= 1024 and D == self.num_heads * self.head_dim and norm.normalized_shape == (D,) and norm.weight is not None \
+                and _plain((norm, nn.LayerNorm), (gate, nn.Linear), (kp, nn.Linear), (vp, nn.Linear)):
+            n = _lib.native()
+            if n.layer_applies(x, [norm.weight, norm.bias, gate.weight, gate.bias, kp.weight, kp.bias, vp.weight, vp.bias]):
+                return n.interference(x, norm.weight, norm.bias, gate.weight, gate.bias, kp.weight, kp.bias, vp.weight, vp.bias, norm.eps, self.num_heads)
         xi = self.inter_norm(x)
         B, N, D = xi.shape
         H, HD = self.num_heads, self.head_dim

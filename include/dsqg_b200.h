@@ -254,6 +254,29 @@ int dsqg_gate_bwd(const void* dy, const void* y, const void* gate, const dsqg_st
  *   scratch memory; out may not alias x. */
 int dsqg_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, int reverse, void* stream);
 
+/* What an attention layer under bf16 autocast does between its GEMMs and the operator, one pass each (the PyTorch
+ * ops around the reference's layer, DWARF train/train_2048_condU.py:171-191 and the interference block :277-295):
+ *   dsqg_cast_bf16       fp32 -> bf16 for up to DSQG_CAST_MAX tensors (lengths multiples of 8) in one launch
+ *   dsqg_layer_norm_fwd  y = (x - mean) * rstd * gamma + beta in fp32 and bf16; stat [rows,2] = {mean, rstd}
+ *   dsqg_layer_norm_bwd  its backward for dy = dy (fp32) + dy_bf16; dgamma_dbeta [2,D]
+ *   dsqg_gated_pool      out = sigmoid(g) * pool, and dsqg_gated_pool_bwd
+ *   dsqg_inject_kv       key and value thirds of qkv [rows,3*D] += k_delta, v_delta (rows delta_stride elements apart)
+ *   dsqg_column_sums     fp32 column sums of up to DSQG_SUM_MAX bf16 matrices of the same number of rows, fixed order
+ * D a multiple of 8 (layer norm: at most 1024); all pointers 16-byte aligned; src, dst, n, row_stride, cols: HOST arrays. */
+#define DSQG_CAST_MAX 8
+#define DSQG_SUM_MAX 4
+int dsqg_cast_bf16(const float* const* src, void* const* dst, const long long* n, int count, void* stream);
+int dsqg_layer_norm_fwd(const float* x, const float* gamma, const float* beta, float eps, float* y, void* y_bf16, float* stat,
+                        long long rows, int D, void* stream);
+size_t dsqg_layer_norm_bwd_scratch_bytes(long long rows, int D);
+int dsqg_layer_norm_bwd(const float* x, const float* stat, const float* gamma, const float* dy, const void* dy_bf16, float* dx,
+                        float* dgamma_dbeta, void* scratch, size_t scratch_bytes, long long rows, int D, void* stream);
+int dsqg_gated_pool(const void* g, const float* pool, void* out, long long n, void* stream);
+int dsqg_gated_pool_bwd(const void* dout, const void* g, const float* pool, void* dg, float* dpool, long long n, void* stream);
+int dsqg_inject_kv(void* qkv, const void* k_delta, const void* v_delta, long long delta_stride, long long rows, int D, void* stream);
+int dsqg_column_sums(const void* const* src, const long long* row_stride, const int* cols, float* const* dst, int count, long long rows,
+                     void* stream);
+
 /* Single-token decode over a circular K/V ring buffer.
  * Replaces: nothing executable -- the reference only describes the O(1) cache in prose
  *   (DWARF README.md:175-179; generate() in train/train_2048_condU.py:463-487 re-runs the
