@@ -32,7 +32,7 @@ constexpr int kRows = 16 * kWarps; // rows per CTA
 // Online softmax over the dense window, then over the sparse taps, with the per-element
 // bookkeeping moved out of the tile loop:
 //   * the band mask and the position bias of the dense window are the INITIAL VALUE of the score
-//     accumulators (a per-lane table in shared memory, one 16-byte load per n-tile), so the
+//     accumulators (two 8-byte loads per n-tile from a table over the offsets, StartTable), so the
 //     scores leave the MMAs already biased and masked (in units of 1/scale);
 //   * interior tiles (all band rows inside the sequence) load with no predicates and constant
 //     offsets from one pointer; a sparse tap whose 16 key rows all exist does the same;
@@ -81,8 +81,34 @@ __device__ __forceinline__ void build_qs_tile(const SeTables& se, const RowFrag<
     __syncwarp();
 }
 
+// Start values of the score accumulators of the dense window.  Element (i, c) of a tile belongs to one offset
+// (forward, dQ: WB + i - c; dK/dV: c - i), so the tile's values are a table over x = 16 - i + c, and the two
+// columns of an accumulator pair are neighbours in it.  A second copy an odd distance away keeps the pair 8-byte
+// aligned for odd rows, 16 banks from the first so that a half warp's loads do not collide.  146 floats for WB = 32
+// against the 3 KB of a table per lane, which every 64-row block had to fill: about 100 instructions per 16-row tile
+// and most of the time before the first load of K.  B32 H8 N2048 D32: forward 67.9 -> 65.0 us; D = 64, N = 4096: dQ 299 -> 287 us
+// (with the staging of DsStage).
+template <int WB> struct StartTable {
+    static constexpr int kOdd = WB <= 48 ? 81 : 113, kSize = kOdd + WB + 33;
+    // KEYS: rows are keys (dK/dV)
+    template <bool KEYS, int THREADS>
+    static __device__ __forceinline__ void fill(float* tab, const float* pos_bias, int H, int h, int d_lo, int d_hi, float scale) {
+        const float inv_scale = 1.f / scale;
+        for (int e = threadIdx.x; e < kSize; e += THREADS) {
+            const int x = e < kOdd ? e : e - kOdd, delta = KEYS ? x - 16 : WB + 16 - x;
+            tab[e] = delta >= d_lo && delta <= d_hi ? pos_bias[(delta - d_lo) * H + h] * inv_scale : kNeg;
+        }
+    }
+    // this lane's pointer: values of (g, 8 nt + 2 tig), (g, .. + 1) at [8 nt], of row g + 8 at [8 nt - 8]
+    static __device__ __forceinline__ const float* lane(const float* tab, const Lane& L) { return tab + (L.g & 1) * kOdd + 16 - L.g + 2 * L.tig; }
+    static __device__ __forceinline__ void get(float (&s)[4], const float* lane_tab, int nt) {
+        const float2 lo = *reinterpret_cast<const float2*>(lane_tab + 8 * nt), hi = *reinterpret_cast<const float2*>(lane_tab + 8 * nt - 8);
+        s[0] = lo.x; s[1] = lo.y; s[2] = hi.x; s[3] = hi.y;
+    }
+};
+
 template <int D, int WB, bool INTERIOR, int kTapGroup, bool SE, bool ST>
-__device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float4* init_s, const int2* tap_s, int ns,
+__device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, const int2* tap_s, int ns,
                                          int bh, int h, int g0, const Lane& L, const SeTables& se) {
     constexpr int NT = (WB + 16) / 8;
     const int N = a.N, g = L.g, tig = L.tig;
@@ -111,8 +137,7 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float4* init_s,
             const int4 qo = se.off[nt * 32 + L.lane];
             S[nt][0] = se.qs[qo.x]; S[nt][1] = se.qs[qo.y]; S[nt][2] = se.qs[qo.z]; S[nt][3] = se.qs[qo.w];
         } else {
-            const float4 ini = init_s[nt * 32 + L.lane];
-            S[nt][0] = ini.x; S[nt][1] = ini.y; S[nt][2] = ini.z; S[nt][3] = ini.w;
+            StartTable<WB>::get(S[nt], start, nt);
         }
         RowFrag<D> kf;
         if (INTERIOR) {
@@ -285,7 +310,7 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float4* init_s,
 // Tuning per head dimension (measured on B200): warps per CTA, sparse taps folded together,
 // resident CTAs per SM the register budget is set for.
 template <int D> struct FwdTune {
-    static constexpr int warps = 4, group = D <= 80 ? 2 : 1, ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));
+    static constexpr int warps = 4, group = D == 64 || D > 80 ? 1 : 2, ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));   // D = 64: 104.8 us (107.8 with group 2)
     static constexpr int group_se = D <= 64 ? 2 : 1, ctas_se = D == 32 ? 5 : 4;       // with scale_embed
 };
 
@@ -345,9 +370,8 @@ template <int D, int WB, bool SE, bool ST>
 __global__ void __launch_bounds__(FwdTune<D>::warps * 32, SE ? FwdTune<D>::ctas_se : FwdTune<D>::ctas)
 fwd_mma_kernel(const FwdArgs a, const Taps t) {
     constexpr int W = FwdTune<D>::warps, G = SE ? FwdTune<D>::group_se : FwdTune<D>::group;
-    constexpr int NT = (WB + 16) / 8;
     extern __shared__ __align__(16) unsigned char se_smem[];
-    __shared__ float4 init_s[SE ? 1 : NT * 32];
+    __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
     __shared__ int2 tap_s[DSQG_MAX_TAPS];
     const Lane L;
     const int bh = blockIdx.y, h = bh % a.H, N = a.N;
@@ -355,39 +379,65 @@ fwd_mma_kernel(const FwdArgs a, const Taps t) {
     if constexpr (SE) {
         se = fill_se_tables<D, WB, W>(se_smem, a.scale_embed, a.pos_bias, t, a.H, h, a.scale, L.warp, false);
     } else {
-        const int d_lo = t.d_lo, d_hi = t.d_lo + t.n_dense - 1;
-        const float inv_scale = 1.f / a.scale;
-        for (int e = threadIdx.x; e < NT * 32; e += W * 32) {
-            const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
-            float v[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int delta = WB + gg + 8 * (r >> 1) - (8 * nt + 2 * tt + (r & 1));
-                v[r] = (delta >= d_lo && delta <= d_hi) ? a.pos_bias[(delta - d_lo) * a.H + h] * inv_scale : kNeg;
-            }
-            init_s[e] = make_float4(v[0], v[1], v[2], v[3]);
-        }
+        StartTable<WB>::template fill<false, W * 32>(start_s, a.pos_bias, a.H, h, t.d_lo, t.d_lo + t.n_dense - 1, a.scale);
     }
     for (int si = threadIdx.x; si < t.n_sparse; si += W * 32)
         tap_s[si] = make_int2(t.sparse[si], __float_as_int(a.pos_bias[(t.n_dense + si) * a.H + h] * kLog2e));
     __syncthreads();
     const int g0 = blockIdx.x * (16 * W) + L.warp * 16;
     if (g0 >= N) return;
-    if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, init_s, tap_s, t.n_sparse, bh, h, g0, L, se);
-    else fwd_tile<D, WB, false, G, SE, ST>(a, init_s, tap_s, t.n_sparse, bh, h, g0, L, se);
+    const float* start = StartTable<WB>::lane(start_s, L);
+    if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se);
+    else fwd_tile<D, WB, false, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se);
 }
 
 // Tuning per head dimension (measured on B200): sparse taps whose loads are issued together and
 // resident CTAs per SM the register budget is set for (spills against warps in flight).
 template <int D> struct BwdTune {
-    static constexpr int dq_group = D == 32 || D == 80 ? 2 : 1, dq_ctas = D <= 64 ? 4 : (D == 80 ? 3 : 2);   // D = 80: 69.0 us (80 with 2 CTAs); D = 32: 105.4 us against 107.5 with group 1 / 5 CTAs
+    static constexpr int dq_group = D <= 80 ? 2 : 1, dq_ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D == 80 ? 3 : 2));   // D = 32: 98.5 us (108.8 with 4 CTAs, 103.3 with group 1); D = 80: 69.0 us (80 with 2 CTAs)
     static constexpr int dq_group_se = 1, dq_ctas_se = D == 32 ? 5 : 4;      // with scale_embed: more shared memory and registers per CTA
     static constexpr int dkdv_group_se = D <= 64 ? 2 : 1, dkdv_ctas_se = D == 32 ? 4 : 3;
     static constexpr int dkdv_group = D <= 80 ? 2 : 1, dkdv_ctas = D == 32 ? 4 : (D <= 64 ? 3 : 2);   // D = 80: 78.1 us (83 with group 1, 96-109 with 3 CTAs)
 };
-constexpr int kStagePitch = kRows + 4;      // 68: no bank conflicts on the scattered writes; the column sums rotate their start
-constexpr int kStagePitchSe = kRows + 4;    // 68 with scale_embed: rows are read back as 8-byte pairs by the dS MMAs
-template <bool SE> struct StagePitch { static constexpr int v = SE ? kStagePitchSe : kStagePitch; };
+constexpr int kStagePitchSe = kRows + 4;    // staging tile with scale_embed, 68: rows are read back as 8-byte pairs by the dS MMAs
+
+// Where a warp of the plain dQ kernel puts its ds values for dpos_bias.  Element (g + 8 half, 8 nt + 2 tig + c) of a
+// tile belongs to offset g - 2 tig - c + 8 k with k = WB / 8 + half - nt, so elements of neighbouring n-tiles share
+// (lane, c, k) and are added in registers first: 2 (WB/8 + 3) stores per lane instead of 4 (WB/8 + 2), to [c][k + 1][lane];
+// then one lane per offset adds the eight entries of its offset in a fixed order.  The pitch of 33 makes these reads
+// (stride 4 in g, 1 in k) conflict-free.  Sparse taps: one value per row pair to [g][tap].
+template <int WB> struct DsStage {
+    static constexpr int kK = WB / 8 + 3, kDense = 2 * kK * 33;
+    static __host__ __device__ int sparse_pitch(int ns) { return ns | 1; }
+    static __host__ __device__ int floats(int ns, int J) { return kDense + 8 * sparse_pitch(ns) + J; }    // per warp, with its J sums
+    static __device__ __forceinline__ void put(float* w, int lane, int k1, float a, float b) {
+        w[k1 * 33 + lane] = a;
+        w[(kK + k1) * 33 + lane] = b;
+    }
+    static __device__ __forceinline__ void sum(float* w, const Taps& t, int lane) {
+        const float* sp = w + kDense;
+        const int pitch = sparse_pitch(t.n_sparse);
+        float* out = w + kDense + 8 * pitch;
+        __syncwarp();
+        for (int j = lane; j < t.n_dense; j += 32) {
+            float s[2] = {0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < 2; ++c)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int e = t.d_lo + j + 2 * i + c;              // = g + 8 k
+                    s[c] += w[(c * kK + (e >> 3) + 1) * 33 + 4 * (e & 7) + i];
+                }
+            out[j] = s[0] + s[1];
+        }
+        for (int j = lane; j < t.n_sparse; j += 32) {
+            float s = 0.f;
+#pragma unroll
+            for (int g = 0; g < 8; ++g) s += sp[g * pitch + j];
+            out[t.n_dense + j] = s;
+        }
+    }
+};
 
 // Extras of the dQ kernel with scale_embed.
 //   seb:  scale_embed as B fragments of dS.SE (global memory, written by se_prep_kernel)
@@ -398,11 +448,12 @@ struct SeBwd {
 };
 
 template <int D, int WB, bool INTERIOR, int G, bool SE, bool ST>
-__device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s, const int4* soff_s, const int2* tap_s,
+__device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, const int4* soff_s, const int2* tap_s,
                                          float* stage_w, int nd, int ns, int bh, int h, int g0, const Lane& L,
                                          const SeTables& se, const SeBwd& sb) {
     constexpr int NT = (WB + 16) / 8;
-    constexpr int SP = StagePitch<SE>::v;
+    constexpr int SP = kStagePitchSe;
+    using Stage = DsStage<WB>;
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = g0 + g, row_hi = row_lo + 8;
     const bool ok_lo = INTERIOR || row_lo < N, ok_hi = INTERIOR || row_hi < N;
@@ -418,6 +469,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s,
     const float gain = a.head_gain ? a.head_gain[h] : 1.f;
     const int kb0 = g0 - WB;
     float dgrow = 0.f;
+    f32x2 dgrow2 = 0ull;
 
     RowFrag<D> qa, qb, da, db;
     load_row(qa, qp + (size_t)row_lo * RS, tig, ok_lo);
@@ -456,7 +508,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s,
         if (ok_hi) rs[row_hi] = make_float2(l2_hi, delta_hi);
     }
     float dQ[D / 8][4];
-    const int stage_base = (WB + 15 + g - 2 * tig) * SP + g;      // plain kernel: see the dense loop
+    float carry[2] = {0.f, 0.f};                                   // plain kernel: row g's ds of the n-tile before
 
     // ---- dense window
 #pragma unroll
@@ -466,26 +518,16 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s,
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
             const int nt = 2 * c + hf;
-            float4 ini;
-            if constexpr (SE) {
-                const int4 qo = __ldg(se.off + nt * 32 + L.lane);      // table in global memory (se_prep_kernel)
-                ini = make_float4(se.qs[qo.x], se.qs[qo.y], se.qs[qo.z], se.qs[qo.w]);
-            } else {
-                ini = init_s[nt * 32 + L.lane];
-            }
+            float s[4], dp[4];
             int so_r[4];
             if constexpr (SE) {
+                const int4 qo = __ldg(se.off + nt * 32 + L.lane);      // table in global memory (se_prep_kernel)
+                s[0] = se.qs[qo.x]; s[1] = se.qs[qo.y]; s[2] = se.qs[qo.z]; s[3] = se.qs[qo.w];
                 const int4 so = soff_s[nt * 32 + L.lane];
                 so_r[0] = so.x; so_r[1] = so.y; so_r[2] = so.z; so_r[3] = so.w;
             } else {
-                // plain kernel: staging row = delta + 15 for every delta a tile element can have
-                // (-15 .. WB+15), so the address is a per-lane base plus a compile-time constant and
-                // entries outside the dense window (exactly zero) land in rows nobody sums
-#pragma unroll
-                for (int r = 0; r < 4; ++r)
-                    so_r[r] = stage_base + (8 * (r >> 1) - 8 * nt - (r & 1)) * SP + 8 * (r >> 1);
+                StartTable<WB>::get(s, start, nt);
             }
-            float s[4] = {ini.x, ini.y, ini.z, ini.w}, dp[4];
             RowFrag<D> vf;
             if (INTERIOR) {
                 load_row_at(kf[hf], kl + (8 * nt - WB) * RS);
@@ -504,12 +546,18 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s,
                     if (kb0 + 8 * nt + 2 * tig + (r & 1) < 0) s[r] = kNeg;
             }
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float p = ex2(fmaf(s[r], c2, r < 2 ? -l2_lo : -l2_hi));
-                dgrow = fmaf(p, dp[r], dgrow);
-                const float x = p * fmaf(gain, dp[r], r < 2 ? -delta_lo : -delta_hi);
-                ds[hf][r] = x;
-                stage_w[so_r[r]] = x;
+            for (int r = 0; r < 4; r += 2) {
+                const float l = r ? l2_hi : l2_lo, d = r ? delta_hi : delta_lo;
+                float p0, p1;
+                unpair(fma2(pair(s[r], s[r + 1]), pair(c2, c2), pair(-l, -l)), p0, p1);
+                const f32x2 pp = pair(ex2(p0), ex2(p1)), dpp = pair(dp[r], dp[r + 1]);
+                dgrow2 = fma2(pp, dpp, dgrow2);
+                unpair(mul2(pp, fma2(pair(gain, gain), dpp, pair(-d, -d))), ds[hf][r], ds[hf][r + 1]);
+                if constexpr (SE) { stage_w[so_r[r]] = ds[hf][r]; stage_w[so_r[r + 1]] = ds[hf][r + 1]; }
+            }
+            if constexpr (!SE) {
+                Stage::put(stage_w, L.lane, WB / 8 + 2 - nt, nt ? carry[0] + ds[hf][2] : ds[hf][2], nt ? carry[1] + ds[hf][3] : ds[hf][3]);
+                carry[0] = ds[hf][0]; carry[1] = ds[hf][1];
             }
         }
         RowFrag<D> kt0, kt1;
@@ -525,7 +573,8 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s,
     }
     // ---- sparse taps
     const float ls_lo = L.owner ? l2_lo : 1.0e30f, ls_hi = L.owner ? l2_hi : 1.0e30f;   // p == 0 on lanes without a diagonal entry
-    float* stage_sp = stage_w + (SE ? nd : WB + 31) * SP + g;     // plain kernel: after the WB+31 delta rows
+    if constexpr (!SE) Stage::put(stage_w, L.lane, 0, carry[0], carry[1]);
+    float* stage_sp = SE ? stage_w + nd * SP + g : stage_w + Stage::kDense + g * Stage::sparse_pitch(ns);
     auto finish = [&](int si, float sd0, float sd1, float dp0, float dp1, float pbv, bool v0, bool v1,
                       const RowFrag<D>& kf0, const RowFrag<D>& kf1) {
         float p0, p1;
@@ -538,7 +587,9 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s,
         }
         dgrow = fmaf(p0, dp0, dgrow); dgrow = fmaf(p1, dp1, dgrow);
         const float x0 = p0 * fmaf(gain, dp0, -delta_lo), x1 = p1 * fmaf(gain, dp1, -delta_hi);
-        if (L.owner) { stage_sp[si * SP] = x0; stage_sp[si * SP + 8] = x1; }
+        if (L.owner) {
+            if constexpr (SE) { stage_sp[si * SP] = x0; stage_sp[si * SP + 8] = x1; } else stage_sp[si] = x0 + x1;
+        }
         diag_fma<D>(dQ, __shfl_sync(0xffffffffu, x0, L.owner_lane), __shfl_sync(0xffffffffu, x1, L.owner_lane), kf0, kf1);
     };
     auto full_taps = [&](auto GC, int si) {
@@ -591,7 +642,9 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s,
         }
     }
     if (L.owner)                                          // taps no row of the tile reaches: zero entries
-        for (; si < ns; ++si) { stage_sp[si * SP] = 0.f; stage_sp[si * SP + 8] = 0.f; }
+        for (; si < ns; ++si) {
+            if constexpr (SE) { stage_sp[si * SP] = 0.f; stage_sp[si * SP + 8] = 0.f; } else stage_sp[si] = 0.f;
+        }
     if constexpr (SE) {
         // dQ += dS.scale_embed: the warp's ds values are complete in its 16 staging columns
         __syncwarp();
@@ -609,7 +662,9 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float4* init_s,
     }
     __nv_bfloat16* dqp = static_cast<__nv_bfloat16*>(a.dq) + base;
     store_acc_rows<D>(dQ, dqp + (size_t)row_lo * RS, dqp + (size_t)row_hi * RS, ok_lo, ok_hi, a.scale, a.scale, tig);
-    return dgrow;
+    float dg0, dg1;
+    unpair(dgrow2, dg0, dg1);
+    return dgrow + (dg0 + dg1);
 }
 
 // One block, before the dQ kernel with scale_embed.  Writes, back to back:
@@ -676,10 +731,10 @@ __global__ void se_prep_kernel(const float* __restrict__ scale_embed, const floa
 }
 
 inline size_t dq_smem_bytes(int J, int n_sparse, int D, int NT, bool se) {
-    // staging rows: with scale_embed one per tap (rounded up to the MMA shape) plus a dump row;
-    // plain kernel one per delta a tile element can have (8 NT + 15 = WB + 31) plus the sparse taps
-    const int rows = se ? (J + 15) / 16 * 16 + 1 : 8 * NT + 15 + n_sparse;
-    size_t n = sizeof(float) * ((size_t)rows * (se ? kStagePitchSe : kStagePitch) + kWarps * 32);
+    // with scale_embed a staging row per tap (rounded up to the MMA shape) and a dump row; otherwise a DsStage per warp
+    size_t n = sizeof(float) * (size_t)(se ? ((J + 15) / 16 * 16 + 1) * kStagePitchSe + kWarps * 32
+                                           : kWarps * (1 + (NT == 6 ? DsStage<32>::floats(n_sparse, J) : NT == 8 ? DsStage<48>::floats(n_sparse, J)
+                                                                                                               : DsStage<64>::floats(n_sparse, J))));
     if (se) {
         n = (n + 15) / 16 * 16;
         n += (size_t)kWarps * (16 * ((J + 7) / 8 * 8 + 2) + 4) * 4;      // one q.scale_embed tile per warp
@@ -693,35 +748,34 @@ template <int D, int WB, int G, int CT, bool SE, bool ST>
 __global__ void __launch_bounds__(kWarps * 32, CT)
 bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
     constexpr int NT = (WB + 16) / 8;
-    constexpr int SP = StagePitch<SE>::v;
-    extern __shared__ __align__(16) float stage[];     // [JS + 1][SP] ds values, then [128] dgain terms, then the scale_embed extras
-    __shared__ float4 init_s[SE ? 1 : NT * 32];
+    constexpr int SP = kStagePitchSe;
+    using Stage = DsStage<WB>;
+    // scale_embed: [JS + 1][SP] ds values, then [128] dgain terms, then the scale_embed extras; plain: [kWarps] dgain terms, a DsStage per warp
+    extern __shared__ __align__(16) float stage[];
+    __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
     __shared__ int4 soff_s[SE ? NT * 32 : 1];          // staging offsets per lane (scale_embed variant only)
     __shared__ int2 tap_s[DSQG_MAX_TAPS];
     const Lane L;
     const int bh = blockIdx.y, h = bh % a.H, N = a.N, J = t.J;
     const int JS = SE ? (J + 15) / 16 * 16 : J;         // scale_embed: staging rows (row JS is the dump for out-of-band entries)
-    constexpr int kDeltaRows = WB + 31;                 // plain kernel: one staging row per delta -15 .. WB+15
-    float* dg_s = stage + (SE ? JS + 1 : kDeltaRows + t.n_sparse) * SP;
+    float* dg_s = SE ? stage + (JS + 1) * SP : stage;
     SeTables se = {};
     SeBwd sb = {};
     {
         const int d_lo = t.d_lo, d_hi = t.d_lo + t.n_dense - 1;
-        const float inv_scale = 1.f / a.scale;
-        for (int e = threadIdx.x; e < NT * 32; e += kWarps * 32) {
-            const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
-            float v[4];
-            int o[4];
+        if constexpr (!SE) {
+            StartTable<WB>::template fill<false, kWarps * 32>(start_s, a.pos_bias, a.H, h, d_lo, d_hi, a.scale);
+        } else {
+            for (int e = threadIdx.x; e < NT * 32; e += kWarps * 32) {
+                const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
+                int o[4];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int i = gg + 8 * (r >> 1);
-                const int delta = WB + i - (8 * nt + 2 * tt + (r & 1));
-                const bool inband = delta >= d_lo && delta <= d_hi;
-                v[r] = (!SE && inband) ? a.pos_bias[(delta - d_lo) * a.H + h] * inv_scale : kNeg;
-                o[r] = (inband ? delta - d_lo : JS) * SP + i;
+                for (int r = 0; r < 4; ++r) {
+                    const int i = gg + 8 * (r >> 1), delta = WB + i - (8 * nt + 2 * tt + (r & 1));
+                    o[r] = (delta >= d_lo && delta <= d_hi ? delta - d_lo : JS) * SP + i;
+                }
+                soff_s[e] = make_int4(o[0], o[1], o[2], o[3]);
             }
-            if constexpr (!SE) init_s[e] = make_float4(v[0], v[1], v[2], v[3]);
-            if constexpr (SE) soff_s[e] = make_int4(o[0], o[1], o[2], o[3]);
         }
         for (int si = threadIdx.x; si < t.n_sparse; si += kWarps * 32)
             tap_s[si] = make_int2(t.sparse[si], __float_as_int(a.pos_bias[(t.n_dense + si) * a.H + h] * kLog2e));
@@ -748,25 +802,26 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
     }
     __syncthreads();
     const int g0 = blockIdx.x * kRows + L.warp * 16;
-    float* stage_w = stage + L.warp * 16;
+    float* stage_w = SE ? stage + L.warp * 16 : stage + kWarps + L.warp * Stage::floats(t.n_sparse, J);
+    float* sums = stage + kWarps + Stage::kDense + 8 * Stage::sparse_pitch(t.n_sparse);          // plain kernel: warp 0's J sums
+    const float* start = StartTable<WB>::lane(start_s, L);
     float dgrow = 0.f;
-    if (g0 >= N) {                                      // no rows: this warp's staging columns (and query rows) are zero
+    if (g0 >= N) {                                      // no rows: this warp's sums, or staging columns and query rows, are zero
         if constexpr (SE) {
             for (int e = L.lane; e < J * 16; e += 32) stage_w[(e >> 4) * SP + (e & 15)] = 0.f;
-        } else {                                        // the rows the column sums read: in-band deltas, then the sparse taps
-            for (int e = L.lane; e < J * 16; e += 32) {
-                const int j = e >> 4;
-                stage_w[(j < t.n_dense ? t.d_lo + j + 15 : kDeltaRows + j - t.n_dense) * SP + (e & 15)] = 0.f;
-            }
+        } else {
+            for (int j = L.lane; j < J; j += 32) sums[L.warp * Stage::floats(t.n_sparse, J) + j] = 0.f;
         }
         if constexpr (SE)
             for (int e = L.lane; e < 16 * (2 * D + 16) / 16; e += 32)
                 reinterpret_cast<uint4*>(sb.q_s + (size_t)L.warp * 16 * (2 * D + 16))[e] = make_uint4(0u, 0u, 0u, 0u);
     } else if (g0 >= WB && g0 + 16 <= N) {
-        dgrow = dq_tile<D, WB, true, G, SE, ST>(a, init_s, soff_s, tap_s, stage_w, t.n_dense, t.n_sparse, bh, h, g0, L, se, sb);
+        dgrow = dq_tile<D, WB, true, G, SE, ST>(a, start, soff_s, tap_s, stage_w, t.n_dense, t.n_sparse, bh, h, g0, L, se, sb);
     } else {
-        dgrow = dq_tile<D, WB, false, G, SE, ST>(a, init_s, soff_s, tap_s, stage_w, t.n_dense, t.n_sparse, bh, h, g0, L, se, sb);
+        dgrow = dq_tile<D, WB, false, G, SE, ST>(a, start, soff_s, tap_s, stage_w, t.n_dense, t.n_sparse, bh, h, g0, L, se, sb);
     }
+    if constexpr (!SE)
+        if (g0 < N) Stage::sum(stage_w, t, L.lane);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) dgrow += __shfl_xor_sync(0xffffffffu, dgrow, o);
     if (L.lane == 0) dg_s[L.warp] = dgrow;
@@ -800,28 +855,34 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
             }
         }
     }
-    // Column sums of the staging tile: two threads per tap (32 rows each, four independent partial
-    // sums, fixed order), so the CTA's tail is a few dozen dependent additions instead of kRows.
-    static_assert(kRows == 64 && kWarps == 4, "the column sums below split 64 rows over thread pairs");
-    for (int j0 = 0; j0 < J; j0 += kWarps * 16) {
-        const int j = j0 + (threadIdx.x >> 1), half = threadIdx.x & 1;
-        float s = 0.f;
-        if (j < J) {
-            // pitch 68 puts rows j and j+8 (and the two halves) in the same banks: start each of the
-            // four at a different column so that a warp's 32 reads fall into 32 banks
-            const int jr = SE ? j : (j < t.n_dense ? t.d_lo + j + 15 : kDeltaRows + j - t.n_dense);   // staging row of tap j
-            const float* row = stage + jr * SP + 32 * half;
-            const int rot = ((jr >> 3) & 1) + 2 * half;
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    if constexpr (!SE) {
+        static_assert(kWarps == 4, "four warps' sums");
+        const int per = Stage::floats(t.n_sparse, J);
+        for (int j = threadIdx.x; j < J; j += kWarps * 32)
+            a.dpb_part[(size_t)tile * J + j] = (sums[j] + sums[per + j]) + (sums[2 * per + j] + sums[3 * per + j]);
+    } else {
+        // Column sums of the staging tile: two threads per tap (32 rows each, four independent partial
+        // sums, fixed order), so the CTA's tail is a few dozen dependent additions instead of kRows.
+        static_assert(kRows == 64 && kWarps == 4, "the column sums below split 64 rows over thread pairs");
+        for (int j0 = 0; j0 < J; j0 += kWarps * 16) {
+            const int j = j0 + (threadIdx.x >> 1), half = threadIdx.x & 1;
+            float s = 0.f;
+            if (j < J) {
+                // pitch 68 puts rows j and j+8 (and the two halves) in the same banks: start each of the
+                // four at a different column so that a warp's 32 reads fall into 32 banks
+                const float* row = stage + j * SP + 32 * half;
+                const int rot = ((j >> 3) & 1) + 2 * half;
+                float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
-            for (int r = 0; r < 32; r += 4) {
-                s0 += row[(r + rot) & 31]; s1 += row[(r + 1 + rot) & 31];
-                s2 += row[(r + 2 + rot) & 31]; s3 += row[(r + 3 + rot) & 31];
+                for (int r = 0; r < 32; r += 4) {
+                    s0 += row[(r + rot) & 31]; s1 += row[(r + 1 + rot) & 31];
+                    s2 += row[(r + 2 + rot) & 31]; s3 += row[(r + 3 + rot) & 31];
+                }
+                s = (s0 + s1) + (s2 + s3);
             }
-            s = (s0 + s1) + (s2 + s3);
+            s += __shfl_xor_sync(0xffffffffu, s, 1);
+            if (j < J && half == 0) a.dpb_part[(size_t)tile * J + j] = s;
         }
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        if (j < J && half == 0) a.dpb_part[(size_t)tile * J + j] = s;
     }
     if (threadIdx.x == 0) a.dg_part[tile] = (dg_s[0] + dg_s[1]) + (dg_s[2] + dg_s[3]);
 }
@@ -854,10 +915,10 @@ dse_group_kernel(const float* __restrict__ tmp, float* __restrict__ part, int ti
 // dense part of qs_rows (row = query, nd + 1 columns, the last one holding the mask value), and a
 // sparse tap adds the entry of its query row read from global memory.
 template <int D, int WB, bool INTERIOR, int G, bool SE, bool ST>
-__device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float4* init_s, const int2* tap_s, const float2* stat_w,
+__device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, const int2* tap_s, const float* stat_w,
                                           int ns, int bh, int h, int m0, const Lane& L, const float* qsd_w,
                                           const int4* qoff, int nd, int Jp) {
-    constexpr int NT = (WB + 16) / 8;
+    constexpr int NT = (WB + 16) / 8, kStat = kRows + WB;
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = m0 + g, row_hi = row_lo + 8;
     const bool ok_lo = INTERIOR || row_lo < N, ok_hi = INTERIOR || row_hi < N;
@@ -893,8 +954,7 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float4* init_s
                 const int4 qo = qoff[nt * 32 + L.lane];
                 s[0] = qsd_w[qo.x]; s[1] = qsd_w[qo.y]; s[2] = qsd_w[qo.z]; s[3] = qsd_w[qo.w];
             } else {
-                const float4 ini = init_s[nt * 32 + L.lane];
-                s[0] = ini.x; s[1] = ini.y; s[2] = ini.z; s[3] = ini.w;
+                StartTable<WB>::get(s, start, nt);
             }
             if (INTERIOR) {
                 load_row_at(qf[hf], ql + 8 * nt * RS);
@@ -906,13 +966,16 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float4* init_s
             }
             mma_rows(s, ka, kb, qf[hf]);
             mma_rows_z(dp, va, vb, df[hf]);
-            // statistics of this thread's two query columns: {l2, delta} x 2
-            const float4 st = *reinterpret_cast<const float4*>(stat_w + 8 * nt + 2 * tig);
+            // statistics of this thread's two query columns: -l2 and -delta as pairs
+            const f32x2 nl2 = *reinterpret_cast<const f32x2*>(stat_w + 8 * nt + 2 * tig);
+            const f32x2 ndl = *reinterpret_cast<const f32x2*>(stat_w + kStat + 8 * nt + 2 * tig);
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const float p = ex2(fmaf(s[r], c2, (r & 1) ? -st.z : -st.x));
-                ds[hf][r] = p * fmaf(gain, dp[r], (r & 1) ? -st.w : -st.y);
-                pv[hf][r] = p * gain;
+            for (int r = 0; r < 4; r += 2) {
+                float p0, p1;
+                unpair(fma2(pair(s[r], s[r + 1]), pair(c2, c2), nl2), p0, p1);
+                p0 = ex2(p0); p1 = ex2(p1);
+                pv[hf][r] = p0; pv[hf][r + 1] = p1;
+                unpair(mul2(pair(p0, p1), fma2(pair(gain, gain), pair(dp[r], dp[r + 1]), ndl)), ds[hf][r], ds[hf][r + 1]);
             }
         }
         RowFrag<D> t0, t1;
@@ -943,9 +1006,8 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float4* init_s
                       const RowFrag<D>& qf0, const RowFrag<D>& qf1, const RowFrag<D>& df0, const RowFrag<D>& df1) {
         const float y0 = SE ? (sd0 + b0) * c2 : fmaf(sd0, c2, b0), y1 = SE ? (sd1 + b1) * c2 : fmaf(sd1, c2, b1);
         const float p0 = ex2(y0 - st0.x), p1 = ex2(y1 - st1.x);
-        const float w0 = p0 * gain, w1 = p1 * gain;
         const float x0 = p0 * fmaf(gain, dp0, -st0.y), x1 = p1 * fmaf(gain, dp1, -st1.y);
-        diag_fma<D>(dV, __shfl_sync(0xffffffffu, w0, L.owner_lane), __shfl_sync(0xffffffffu, w1, L.owner_lane), df0, df1);
+        diag_fma<D>(dV, __shfl_sync(0xffffffffu, p0, L.owner_lane), __shfl_sync(0xffffffffu, p1, L.owner_lane), df0, df1);
         diag_fma<D>(dK, __shfl_sync(0xffffffffu, x0, L.owner_lane), __shfl_sync(0xffffffffu, x1, L.owner_lane), qf0, qf1);
     };
     auto full_taps = [&](auto GC, int si) {
@@ -1012,7 +1074,7 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float4* init_s
     __nv_bfloat16* dkp = static_cast<__nv_bfloat16*>(a.dk) + base;
     __nv_bfloat16* dvp = static_cast<__nv_bfloat16*>(a.dv) + base;
     store_acc_rows<D>(dK, dkp + (size_t)row_lo * RS, dkp + (size_t)row_hi * RS, ok_lo, ok_hi, a.scale, a.scale, tig);
-    store_acc_rows<D>(dV, dvp + (size_t)row_lo * RS, dvp + (size_t)row_hi * RS, ok_lo, ok_hi, 1.f, 1.f, tig);
+    store_acc_rows<D>(dV, dvp + (size_t)row_lo * RS, dvp + (size_t)row_hi * RS, ok_lo, ok_hi, gain, gain, tig);   // dV = gain P^T.dO
 }
 
 inline size_t dkdv_smem_bytes(int n_dense, int WB, bool se) {
@@ -1025,9 +1087,11 @@ bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int
     constexpr int NT = (WB + 16) / 8;
     constexpr int kStat = kRows + WB;                  // query rows the CTA's dense windows touch
     extern __shared__ __align__(16) float qsd[];       // scale_embed: [kStat][n_dense + 1]
-    __shared__ float4 init_s[NT * 32];                 // plain: score start values; scale_embed: int4 offsets into qsd
+    __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
+    __shared__ int4 qoff_s[SE ? NT * 32 : 1];          // scale_embed: offsets into qsd
+    __shared__ float red_s[kReduceThreads];
     __shared__ int2 tap_s[DSQG_MAX_TAPS];
-    __shared__ __align__(16) float2 stat_s[kStat];
+    __shared__ __align__(16) float stat_s[2 * kStat];  // -lse * log2(e) of the rows, then -delta
     const Lane L;
     const int bh = blockIdx.y, h = bh % a.H, N = a.N;
     // Every reduce_stride-th CTA (so that no wave of CTAs is delayed as a whole) also finishes the
@@ -1037,32 +1101,32 @@ bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int
     const int cta = blockIdx.y * gridDim.x + blockIdx.x;
     if (cta % reduce_stride == 0)
         for (int o = cta / reduce_stride; o < n_reduce; o += gridDim.x * gridDim.y / reduce_stride)
-            reduce_one_param(a, t.J, o, reinterpret_cast<float*>(init_s));
+            reduce_one_param(a, t.J, o, red_s);
     const int m_cta = blockIdx.x * kRows;
     const int nd = t.n_dense, ndp = nd + 1, Jp = (t.J + 7) / 8 * 8;
     {
         const int d_lo = t.d_lo, d_hi = t.d_lo + t.n_dense - 1;
-        const float inv_scale = 1.f / a.scale;
-        for (int e = threadIdx.x; e < NT * 32; e += kWarps * 32) {
-            const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
-            float v[4];
-            int o[4];
+        if constexpr (!SE) {
+            StartTable<WB>::template fill<true, kWarps * 32>(start_s, a.pos_bias, a.H, h, d_lo, d_hi, a.scale);
+        } else {
+            for (int e = threadIdx.x; e < NT * 32; e += kWarps * 32) {
+                const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
+                int o[4];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int cc = 8 * nt + 2 * tt + (r & 1);
-                const int delta = cc - (gg + 8 * (r >> 1));
-                const bool inband = delta >= d_lo && delta <= d_hi;
-                v[r] = (!SE && inband) ? a.pos_bias[(delta - d_lo) * a.H + h] * inv_scale : kNeg;
-                o[r] = cc * ndp + (inband ? delta - d_lo : nd);       // column nd of every row holds the mask value
+                for (int r = 0; r < 4; ++r) {
+                    const int cc = 8 * nt + 2 * tt + (r & 1), delta = cc - (gg + 8 * (r >> 1));
+                    o[r] = cc * ndp + (delta >= d_lo && delta <= d_hi ? delta - d_lo : nd);   // column nd of every row holds the mask value
+                }
+                qoff_s[e] = make_int4(o[0], o[1], o[2], o[3]);
             }
-            if constexpr (SE) reinterpret_cast<int4*>(init_s)[e] = make_int4(o[0], o[1], o[2], o[3]);
-            else init_s[e] = make_float4(v[0], v[1], v[2], v[3]);
         }
         for (int si = threadIdx.x; si < t.n_sparse; si += kWarps * 32)
             tap_s[si] = make_int2(t.sparse[si], __float_as_int(a.pos_bias[(t.n_dense + si) * a.H + h] * kLog2e));
         const float2* rs = reinterpret_cast<const float2*>(a.delta) + (size_t)bh * N;
-        for (int i = threadIdx.x; i < kStat; i += kWarps * 32)
-            stat_s[i] = m_cta + i < N ? rs[m_cta + i] : make_float2(0.f, 0.f);
+        for (int i = threadIdx.x; i < kStat; i += kWarps * 32) {
+            const float2 x = m_cta + i < N ? rs[m_cta + i] : make_float2(0.f, 0.f);
+            stat_s[i] = -x.x; stat_s[kStat + i] = -x.y;
+        }
         if constexpr (SE) {
             const float* src = a.qs_rows + ((size_t)bh * N + m_cta) * Jp;
             for (int r = threadIdx.x; r < kStat; r += kWarps * 32) qsd[r * ndp + nd] = kNeg;      // the mask column
@@ -1104,11 +1168,11 @@ bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int
     const int m0 = m_cta + L.warp * 16;
     if (m0 >= N) return;
     const float* qsd_w = qsd + L.warp * 16 * ndp;
-    const int4* qoff = reinterpret_cast<const int4*>(init_s);
+    const float* start = StartTable<WB>::lane(start_s, L);
     if (m0 + 16 + WB <= N)
-        dkdv_tile<D, WB, true, G, SE, ST>(a, init_s, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, qsd_w, qoff, nd, Jp);
+        dkdv_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, qsd_w, qoff_s, nd, Jp);
     else
-        dkdv_tile<D, WB, false, G, SE, ST>(a, init_s, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, qsd_w, qoff, nd, Jp);
+        dkdv_tile<D, WB, false, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, qsd_w, qoff_s, nd, Jp);
 }
 
 // Raises a kernel's dynamic shared-memory limit to what this launch needs.  The attribute is set
