@@ -18,6 +18,7 @@
 // produces dscale_embed partials per 64-row tile (dS^T.Q, MMA; dse_group_kernel adds groups of
 // eight tiles) and leaves the per-row tile in global memory for the dK/dV kernel.
 #include "dsqg_mma.cuh"
+#include <initializer_list>
 #include <mutex>
 #include <type_traits>
 
@@ -27,6 +28,11 @@ namespace {
 constexpr int kMaxSparse = DSQG_MAX_TAPS;   // any number of sparse taps (they are processed in a loop)
 constexpr int kWarps = 4;
 constexpr int kRows = 16 * kWarps; // rows per CTA
+
+// How q, k, v, out, ... are addressed: contiguous [B,H,N,D]; through the element strides in FwdArgs / BwdArgs (rows of D
+// contiguous elements; any batch / head / row strides), e.g. the un-permuted output of a fused qkv projection and a token-major
+// result; the same with pieces that are aligned to 16 bytes only where a piece is 32 (D a multiple of 64).
+constexpr int kContiguous = 0, kStrided = 1, kStridedAny = 2;
 
 // ------------------------------------------------------------------------------ forward
 // Online softmax over the dense window, then over the sparse taps, with the per-element
@@ -65,10 +71,11 @@ __device__ __forceinline__ void build_qs_tile(const SeTables& se, const RowFrag<
         RowFrag<D> sf;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            const uint4* src = reinterpret_cast<const uint4*>((half ? se.se_lo : se.se_hi) + (8 * m + g) * D + 8 * tig);
+            const uint4* src = reinterpret_cast<const uint4*>((half ? se.se_lo : se.se_hi) + (8 * m + g) * D + kLane<D> * tig);
 #pragma unroll
             for (int cc = 0; cc < D / 32; ++cc) {
-                const uint4 u = GL ? __ldg(src + 4 * cc) : src[4 * cc];
+                const int o = kLane<D> == 16 ? 8 * (cc >> 1) + (cc & 1) : 4 * cc;
+                const uint4 u = GL ? __ldg(src + o) : src[o];
                 sf.r[4 * cc + 0] = u.x; sf.r[4 * cc + 1] = u.y; sf.r[4 * cc + 2] = u.z; sf.r[4 * cc + 3] = u.w;
             }
             mma_rows(c, qa, qb, sf);
@@ -107,26 +114,27 @@ template <int WB> struct StartTable {
     }
 };
 
-template <int D, int WB, bool INTERIOR, int kTapGroup, bool SE, bool ST>
+template <int D, int WB, bool INTERIOR, int kTapGroup, bool SE, int ST>
 __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, const int2* tap_s, int ns,
                                          int bh, int h, int g0, const Lane& L, const SeTables& se) {
     constexpr int NT = (WB + 16) / 8;
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = g0 + g, row_hi = row_lo + 8;
     const bool ok_lo = INTERIOR || row_lo < N, ok_hi = INTERIOR || row_hi < N;
+    constexpr bool AL = ST != kStridedAny;
     const ptrdiff_t RS = ST ? (ptrdiff_t)a.in_sn : D, OS = ST ? (ptrdiff_t)a.out_sn : D;   // row strides of q/k/v and of out
     const size_t base = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : (size_t)bh * N * D;
     const size_t obase = ST ? (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh : base;
     const __nv_bfloat16* qp = static_cast<const __nv_bfloat16*>(a.q) + base;
     // per-thread pointers to this thread's chunk of row row_lo of K and V
-    const __nv_bfloat16* kl = static_cast<const __nv_bfloat16*>(a.k) + base + (ptrdiff_t)row_lo * RS + 8 * tig;
-    const __nv_bfloat16* vl = static_cast<const __nv_bfloat16*>(a.v) + base + (ptrdiff_t)row_lo * RS + 8 * tig;
+    const __nv_bfloat16* kl = static_cast<const __nv_bfloat16*>(a.k) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
+    const __nv_bfloat16* vl = static_cast<const __nv_bfloat16*>(a.v) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
     const float c2 = a.scale * kLog2e;
     const int kb0 = g0 - WB;
 
     RowFrag<D> qa, qb;
-    load_row(qa, qp + (size_t)row_lo * RS, tig, ok_lo);
-    load_row(qb, qp + (size_t)row_hi * RS, tig, ok_hi);
+    load_row<D, AL>(qa, qp + (size_t)row_lo * RS, tig, ok_lo);
+    load_row<D, AL>(qb, qp + (size_t)row_hi * RS, tig, ok_hi);
     if constexpr (SE) build_qs_tile<D, false>(se, qa, qb, g, tig);
 
     // ---- dense window: key row of n-tile nt for this thread is kb0 + 8 nt + g = row_lo - WB + 8 nt
@@ -141,10 +149,10 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
         }
         RowFrag<D> kf;
         if (INTERIOR) {
-            load_row_at(kf, kl + (8 * nt - WB) * RS);
+            load_row_at<D, AL>(kf, kl + (8 * nt - WB) * RS);
         } else {
             const int kr = kb0 + 8 * nt + g;
-            load_row(kf, kl + (ptrdiff_t)(8 * nt - WB) * RS - 8 * tig, tig, kr >= 0 && kr < N);
+            load_row<D, AL>(kf, kl + (ptrdiff_t)(8 * nt - WB) * RS - kLane<D> * tig, tig, kr >= 0 && kr < N);
         }
         mma_rows(S[nt], qa, qb, kf);
     }
@@ -174,12 +182,12 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
     for (int c = 0; c < NT / 2; ++c) {
         RowFrag<D> vf0, vf1, vt0, vt1;
         if (INTERIOR) {
-            load_row_at(vf0, vl + (16 * c - WB) * RS);
-            load_row_at(vf1, vl + (16 * c + 8 - WB) * RS);
+            load_row_at<D, AL>(vf0, vl + (16 * c - WB) * RS);
+            load_row_at<D, AL>(vf1, vl + (16 * c + 8 - WB) * RS);
         } else {
             const int kr = kb0 + 16 * c + g;
-            load_row(vf0, vl + (ptrdiff_t)(16 * c - WB) * RS - 8 * tig, tig, kr >= 0 && kr < N);
-            load_row(vf1, vl + (ptrdiff_t)(16 * c + 8 - WB) * RS - 8 * tig, tig, kr + 8 >= 0 && kr + 8 < N);
+            load_row<D, AL>(vf0, vl + (ptrdiff_t)(16 * c - WB) * RS - kLane<D> * tig, tig, kr >= 0 && kr < N);
+            load_row<D, AL>(vf1, vl + (ptrdiff_t)(16 * c + 8 - WB) * RS - kLane<D> * tig, tig, kr + 8 >= 0 && kr + 8 < N);
         }
         transpose_frag(vt0, vf0); transpose_frag(vt1, vf1);
         const uint32_t a0 = pack_bf16x2(S[2 * c][0], S[2 * c][1]), a1 = pack_bf16x2(S[2 * c][2], S[2 * c][3]);
@@ -230,10 +238,10 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             const int2 tp = tap_s[si + i];
             const ptrdiff_t off = (ptrdiff_t)tp.x * RS;
             pbv[i] = __int_as_float(tp.y);
-            load_row_at(kf0[i], kl - off);
-            load_row_at(kf1[i], kl - off + 8 * RS);
-            load_row_at(vf0[i], vl - off);
-            load_row_at(vf1[i], vl - off + 8 * RS);
+            load_row_at<D, AL>(kf0[i], kl - off);
+            load_row_at<D, AL>(kf1[i], kl - off + 8 * RS);
+            load_row_at<D, AL>(vf0[i], vl - off);
+            load_row_at<D, AL>(vf1[i], vl - off + 8 * RS);
         }
         float x0[G], x1[G];
 #pragma unroll
@@ -273,12 +281,12 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             const float pbv = __int_as_float(tap_s[si].y);
             const int kr0 = row_lo - delta, kr1 = row_hi - delta;
             const bool v0 = kr0 >= 0 && kr0 < N, v1 = kr1 >= 0 && kr1 < N;
-            const ptrdiff_t off = (ptrdiff_t)delta * RS + 8 * tig;
+            const ptrdiff_t off = (ptrdiff_t)delta * RS + kLane<D> * tig;
             RowFrag<D> kf0, kf1, vf0[1], vf1[1];
-            load_row(kf0, kl - off, tig, v0);
-            load_row(kf1, kl - off + 8 * RS, tig, v1);
-            load_row(vf0[0], vl - off, tig, v0);
-            load_row(vf1[0], vl - off + 8 * RS, tig, v1);
+            load_row<D, AL>(kf0, kl - off, tig, v0);
+            load_row<D, AL>(kf1, kl - off + 8 * RS, tig, v1);
+            load_row<D, AL>(vf0[0], vl - off, tig, v0);
+            load_row<D, AL>(vf1[0], vl - off + 8 * RS, tig, v1);
             float s0[4], s1[4];
             mma_rows_z(s0, qa, qb, kf0);
             mma_rows_z(s1, qa, qb, kf1);
@@ -296,10 +304,10 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
     const float sc_lo = l_lo > 0.f ? __fdividef(gain, l_lo) : 0.f, sc_hi = l_hi > 0.f ? __fdividef(gain, l_hi) : 0.f;
     if (ST && a.gate) {
         const __nv_bfloat16* gp = static_cast<const __nv_bfloat16*>(a.gate) + obase;
-        store_acc_rows_gated<D>(O, op + (size_t)row_lo * OS, op + (size_t)row_hi * OS, gp + (size_t)row_lo * OS,
+        store_acc_rows_gated<D, AL>(O, op + (size_t)row_lo * OS, op + (size_t)row_hi * OS, gp + (size_t)row_lo * OS,
                                 gp + (size_t)row_hi * OS, ok_lo, ok_hi, sc_lo, sc_hi, tig);
     } else {
-        store_acc_rows<D>(O, op + (size_t)row_lo * OS, op + (size_t)row_hi * OS, ok_lo, ok_hi, sc_lo, sc_hi, tig);
+        store_acc_rows<D, AL>(O, op + (size_t)row_lo * OS, op + (size_t)row_hi * OS, ok_lo, ok_hi, sc_lo, sc_hi, tig);
     }
     if (tig == 0) {
         if (ok_lo) a.lse[(size_t)bh * N + row_lo] = l_lo > 0.f ? (m_lo + __log2f(l_lo)) * kLn2 : -INFINITY;
@@ -363,10 +371,8 @@ __host__ __device__ inline size_t se_tables_bytes(int J, int D, int NT, int warp
     return (size_t)2 * Jp * D * 2 + (size_t)Jp * 4 + (size_t)NT * 32 * 16 + (size_t)warps * (tile_rows * (Jp + 2) + 4) * 4;
 }
 
-// ST: q, k, v and out are addressed through the element strides in FwdArgs (rows of D contiguous
-// elements; any batch / head / row strides), e.g. the un-permuted output of a fused qkv projection
-// and a token-major result; with a gate tensor the epilogue multiplies by sigmoid(gate).
-template <int D, int WB, bool SE, bool ST>
+// ST: addressing (kContiguous ...); with strides and a gate tensor the epilogue multiplies by sigmoid(gate).
+template <int D, int WB, bool SE, int ST>
 __global__ void __launch_bounds__(FwdTune<D>::warps * 32, SE ? FwdTune<D>::ctas_se : FwdTune<D>::ctas)
 fwd_mma_kernel(const FwdArgs a, const Taps t) {
     constexpr int W = FwdTune<D>::warps, G = SE ? FwdTune<D>::group_se : FwdTune<D>::group;
@@ -447,7 +453,7 @@ struct SeBwd {
     int JS;            // J rounded up to 16
 };
 
-template <int D, int WB, bool INTERIOR, int G, bool SE, bool ST>
+template <int D, int WB, bool INTERIOR, int G, bool SE, int ST>
 __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, const int4* soff_s, const int2* tap_s,
                                          float* stage_w, int nd, int ns, int bh, int h, int g0, const Lane& L,
                                          const SeTables& se, const SeBwd& sb) {
@@ -457,14 +463,15 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = g0 + g, row_hi = row_lo + 8;
     const bool ok_lo = INTERIOR || row_lo < N, ok_hi = INTERIOR || row_hi < N;
+    constexpr bool AL = ST != kStridedAny;
     const ptrdiff_t RS = ST ? (ptrdiff_t)a.in_sn : D, OS = ST ? (ptrdiff_t)a.out_sn : D;   // row strides of q/k/v/dq and of out/dout
     const size_t base = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : (size_t)bh * N * D;
     const size_t obase = ST ? (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh : base;
     const __nv_bfloat16* qp = static_cast<const __nv_bfloat16*>(a.q) + base;
     const __nv_bfloat16* op = static_cast<const __nv_bfloat16*>(a.out) + obase;
     const __nv_bfloat16* dop = static_cast<const __nv_bfloat16*>(a.dout) + obase;
-    const __nv_bfloat16* kl = static_cast<const __nv_bfloat16*>(a.k) + base + (ptrdiff_t)row_lo * RS + 8 * tig;
-    const __nv_bfloat16* vl = static_cast<const __nv_bfloat16*>(a.v) + base + (ptrdiff_t)row_lo * RS + 8 * tig;
+    const __nv_bfloat16* kl = static_cast<const __nv_bfloat16*>(a.k) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
+    const __nv_bfloat16* vl = static_cast<const __nv_bfloat16*>(a.v) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
     const float c2 = a.scale * kLog2e;
     const float gain = a.head_gain ? a.head_gain[h] : 1.f;
     const int kb0 = g0 - WB;
@@ -472,20 +479,21 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     f32x2 dgrow2 = 0ull;
 
     RowFrag<D> qa, qb, da, db;
-    load_row(qa, qp + (size_t)row_lo * RS, tig, ok_lo);
-    load_row(qb, qp + (size_t)row_hi * RS, tig, ok_hi);
-    load_row(da, dop + (size_t)row_lo * OS, tig, ok_lo);
-    load_row(db, dop + (size_t)row_hi * OS, tig, ok_hi);
+    load_row<D, AL>(qa, qp + (size_t)row_lo * RS, tig, ok_lo);
+    load_row<D, AL>(qb, qp + (size_t)row_hi * RS, tig, ok_hi);
+    load_row<D, AL>(da, dop + (size_t)row_lo * OS, tig, ok_lo);
+    load_row<D, AL>(db, dop + (size_t)row_hi * OS, tig, ok_hi);
     if constexpr (SE) {
         // the tile also goes to global memory for the dK/dV kernel (rows of this warp, Jp floats each)
         float* rows = a.qs_rows + ((size_t)bh * N + row_lo) * se.Jp;
         build_qs_tile<D, true>(se, qa, qb, g, tig, ok_lo ? rows : nullptr, ok_hi ? rows + 8 * se.Jp : nullptr);
         // and the query rows to shared memory for the CTA's dscale_embed partial
-        unsigned char* qrow = sb.q_s + (size_t)(L.warp * 16 + g) * (2 * D + 16) + 16 * tig;
+        unsigned char* qrow = sb.q_s + (size_t)(L.warp * 16 + g) * (2 * D + 16) + 2 * kLane<D> * tig;
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) {
-            *reinterpret_cast<uint4*>(qrow + 64 * c) = make_uint4(qa.r[4 * c], qa.r[4 * c + 1], qa.r[4 * c + 2], qa.r[4 * c + 3]);
-            *reinterpret_cast<uint4*>(qrow + 8 * (2 * D + 16) + 64 * c) = make_uint4(qb.r[4 * c], qb.r[4 * c + 1], qb.r[4 * c + 2], qb.r[4 * c + 3]);
+            const int o = kLane<D> == 16 ? 128 * (c >> 1) + 16 * (c & 1) : 64 * c;
+            *reinterpret_cast<uint4*>(qrow + o) = make_uint4(qa.r[4 * c], qa.r[4 * c + 1], qa.r[4 * c + 2], qa.r[4 * c + 3]);
+            *reinterpret_cast<uint4*>(qrow + 8 * (2 * D + 16) + o) = make_uint4(qb.r[4 * c], qb.r[4 * c + 1], qb.r[4 * c + 2], qb.r[4 * c + 3]);
         }
     }
     float delta_lo, delta_hi;
@@ -494,8 +502,8 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
         delta_hi = ok_hi ? a.delta_pre[(size_t)bh * N + row_hi] : 0.f;
     } else {
         RowFrag<D> oa, ob;
-        load_row(oa, op + (size_t)row_lo * OS, tig, ok_lo);
-        load_row(ob, op + (size_t)row_hi * OS, tig, ok_hi);
+        load_row<D, AL>(oa, op + (size_t)row_lo * OS, tig, ok_lo);
+        load_row<D, AL>(ob, op + (size_t)row_hi * OS, tig, ok_hi);
         delta_lo = quad_sum(frag_dot(da, oa));
         delta_hi = quad_sum(frag_dot(db, ob));
     }
@@ -530,13 +538,13 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
             }
             RowFrag<D> vf;
             if (INTERIOR) {
-                load_row_at(kf[hf], kl + (8 * nt - WB) * RS);
-                load_row_at(vf, vl + (8 * nt - WB) * RS);
+                load_row_at<D, AL>(kf[hf], kl + (8 * nt - WB) * RS);
+                load_row_at<D, AL>(vf, vl + (8 * nt - WB) * RS);
             } else {
                 const int kr = kb0 + 8 * nt + g;
                 const bool kv = kr >= 0 && kr < N;
-                load_row(kf[hf], kl + (ptrdiff_t)(8 * nt - WB) * RS - 8 * tig, tig, kv);
-                load_row(vf, vl + (ptrdiff_t)(8 * nt - WB) * RS - 8 * tig, tig, kv);
+                load_row<D, AL>(kf[hf], kl + (ptrdiff_t)(8 * nt - WB) * RS - kLane<D> * tig, tig, kv);
+                load_row<D, AL>(vf, vl + (ptrdiff_t)(8 * nt - WB) * RS - kLane<D> * tig, tig, kv);
             }
             mma_rows(s, qa, qb, kf[hf]);
             mma_rows_z(dp, da, db, vf);
@@ -601,10 +609,10 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
             const int2 tp = tap_s[si + i];
             const ptrdiff_t off = (ptrdiff_t)tp.x * RS;
             pbv[i] = __int_as_float(tp.y);
-            load_row_at(kf0[i], kl - off);
-            load_row_at(kf1[i], kl - off + 8 * RS);
-            load_row_at(vf0[i], vl - off);
-            load_row_at(vf1[i], vl - off + 8 * RS);
+            load_row_at<D, AL>(kf0[i], kl - off);
+            load_row_at<D, AL>(kf1[i], kl - off + 8 * RS);
+            load_row_at<D, AL>(vf0[i], vl - off);
+            load_row_at<D, AL>(vf1[i], vl - off + 8 * RS);
         }
 #pragma unroll
         for (int i = 0; i < GG; ++i) {
@@ -628,12 +636,12 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
         } else {
             const float pbv = __int_as_float(tap_s[si].y);
             const bool v0 = row_lo >= delta && row_lo - delta < N, v1 = row_hi >= delta && row_hi - delta < N;
-            const ptrdiff_t off = (ptrdiff_t)delta * RS + 8 * tig;
+            const ptrdiff_t off = (ptrdiff_t)delta * RS + kLane<D> * tig;
             RowFrag<D> kf0, kf1, vf0, vf1;
-            load_row(kf0, kl - off, tig, v0);
-            load_row(kf1, kl - off + 8 * RS, tig, v1);
-            load_row(vf0, vl - off, tig, v0);
-            load_row(vf1, vl - off + 8 * RS, tig, v1);
+            load_row<D, AL>(kf0, kl - off, tig, v0);
+            load_row<D, AL>(kf1, kl - off + 8 * RS, tig, v1);
+            load_row<D, AL>(vf0, vl - off, tig, v0);
+            load_row<D, AL>(vf1, vl - off + 8 * RS, tig, v1);
             float s0[4], s1[4], e0[4], e1[4];
             mma_rows_z(s0, qa, qb, kf0); mma_rows_z(s1, qa, qb, kf1);
             mma_rows_z(e0, da, db, vf0); mma_rows_z(e1, da, db, vf1);
@@ -661,7 +669,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
         }
     }
     __nv_bfloat16* dqp = static_cast<__nv_bfloat16*>(a.dq) + base;
-    store_acc_rows<D>(dQ, dqp + (size_t)row_lo * RS, dqp + (size_t)row_hi * RS, ok_lo, ok_hi, a.scale, a.scale, tig);
+    store_acc_rows<D, AL>(dQ, dqp + (size_t)row_lo * RS, dqp + (size_t)row_hi * RS, ok_lo, ok_hi, a.scale, a.scale, tig);
     float dg0, dg1;
     unpair(dgrow2, dg0, dg1);
     return dgrow + (dg0 + dg1);
@@ -670,7 +678,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
 // One block, before the dQ kernel with scale_embed.  Writes, back to back:
 //   scale_embed split into bf16 halves [2][Jp][D];
 //   its B fragments for dQ += dS.scale_embed, [JS/16][D/8][32] x uint2, in the element order of the
-//     dQ accumulators (n-tile jn, column g <-> d = 32 (jn/4) + 8 (g>>1) + 2 (jn%4) + (g&1)), rows j >= J zero;
+//     dQ accumulators (row fragment register jn of lane tig = g>>1, element g&1), rows j >= J zero;
 //   pos_bias[j,h] / scale for every head, [H][Jp];
 //   the offset table of the dense window into a per-warp tile of the given pitch, [NT*32] x int4
 //     (16 * pitch = the dump entry that holds the mask value).
@@ -706,7 +714,8 @@ __global__ void se_prep_kernel(const float* __restrict__ scale_embed, const floa
     for (int e = threadIdx.x; e < (JS / 16) * (D / 8) * 32; e += blockDim.x) {
         const int ln = e & 31, jn = (e >> 5) % (D / 8), kk = (e >> 5) / (D / 8);
         const int gg = ln >> 2, tt = ln & 3;
-        const int d = 32 * (jn / 4) + 8 * (gg >> 1) + 2 * (jn % 4) + (gg & 1);
+        constexpr int kPer = kLane<D> / 2;                       // n-tiles per piece
+        const int d = 4 * kLane<D> * (jn / kPer) + kLane<D> * (gg >> 1) + 2 * (jn % kPer) + (gg & 1);
         const int j0 = 16 * kk + 2 * tt;
         auto sev = [&](int j) { return j < J ? scale_embed[j * D + d] : 0.f; };
         seb[e] = make_uint2(pack_bf16x2(sev(j0), sev(j0 + 1)), pack_bf16x2(sev(j0 + 8), sev(j0 + 9)));
@@ -744,7 +753,7 @@ inline size_t dq_smem_bytes(int J, int n_sparse, int D, int NT, bool se) {
     return n;
 }
 
-template <int D, int WB, int G, int CT, bool SE, bool ST>
+template <int D, int WB, int G, int CT, bool SE, int ST>
 __global__ void __launch_bounds__(kWarps * 32, CT)
 bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
     constexpr int NT = (WB + 16) / 8;
@@ -914,7 +923,7 @@ dse_group_kernel(const float* __restrict__ tmp, float* __restrict__ part, int ti
 // With scale_embed the score accumulators of the dense window start from qsd, the CTA's copy of the
 // dense part of qs_rows (row = query, nd + 1 columns, the last one holding the mask value), and a
 // sparse tap adds the entry of its query row read from global memory.
-template <int D, int WB, bool INTERIOR, int G, bool SE, bool ST>
+template <int D, int WB, bool INTERIOR, int G, bool SE, int ST>
 __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, const int2* tap_s, const float* stat_w,
                                           int ns, int bh, int h, int m0, const Lane& L, const float* qsd_w,
                                           const int4* qoff, int nd, int Jp) {
@@ -922,22 +931,23 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = m0 + g, row_hi = row_lo + 8;
     const bool ok_lo = INTERIOR || row_lo < N, ok_hi = INTERIOR || row_hi < N;
+    constexpr bool AL = ST != kStridedAny;
     const ptrdiff_t RS = ST ? (ptrdiff_t)a.in_sn : D, OS = ST ? (ptrdiff_t)a.out_sn : D;   // row strides of q/k/v/dk/dv and of dout
     const size_t base = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : (size_t)bh * N * D;
     const size_t obase = ST ? (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh : base;
     const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(a.k) + base;
     const __nv_bfloat16* vp = static_cast<const __nv_bfloat16*>(a.v) + base;
-    const __nv_bfloat16* ql = static_cast<const __nv_bfloat16*>(a.q) + base + (ptrdiff_t)row_lo * RS + 8 * tig;
-    const __nv_bfloat16* dl = static_cast<const __nv_bfloat16*>(a.dout) + obase + (ptrdiff_t)row_lo * OS + 8 * tig;
+    const __nv_bfloat16* ql = static_cast<const __nv_bfloat16*>(a.q) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
+    const __nv_bfloat16* dl = static_cast<const __nv_bfloat16*>(a.dout) + obase + (ptrdiff_t)row_lo * OS + kLane<D> * tig;
     const float2* rs = reinterpret_cast<const float2*>(a.delta) + (size_t)bh * N + row_lo;
     const float c2 = a.scale * kLog2e;
     const float gain = a.head_gain ? a.head_gain[h] : 1.f;
 
     RowFrag<D> ka, kb, va, vb;
-    load_row(ka, kp + (size_t)row_lo * RS, tig, ok_lo);
-    load_row(kb, kp + (size_t)row_hi * RS, tig, ok_hi);
-    load_row(va, vp + (size_t)row_lo * RS, tig, ok_lo);
-    load_row(vb, vp + (size_t)row_hi * RS, tig, ok_hi);
+    load_row<D, AL>(ka, kp + (size_t)row_lo * RS, tig, ok_lo);
+    load_row<D, AL>(kb, kp + (size_t)row_hi * RS, tig, ok_hi);
+    load_row<D, AL>(va, vp + (size_t)row_lo * RS, tig, ok_lo);
+    load_row<D, AL>(vb, vp + (size_t)row_hi * RS, tig, ok_hi);
     float dK[D / 8][4], dV[D / 8][4];
 
     // ---- dense window: query row of n-tile nt for this thread is m0 + 8 nt + g
@@ -957,12 +967,12 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
                 StartTable<WB>::get(s, start, nt);
             }
             if (INTERIOR) {
-                load_row_at(qf[hf], ql + 8 * nt * RS);
-                load_row_at(df[hf], dl + 8 * nt * OS);
+                load_row_at<D, AL>(qf[hf], ql + 8 * nt * RS);
+                load_row_at<D, AL>(df[hf], dl + 8 * nt * OS);
             } else {
                 const bool qv = m0 + 8 * nt + g < N;
-                load_row(qf[hf], ql + (ptrdiff_t)8 * nt * RS - 8 * tig, tig, qv);
-                load_row(df[hf], dl + (ptrdiff_t)8 * nt * OS - 8 * tig, tig, qv);
+                load_row<D, AL>(qf[hf], ql + (ptrdiff_t)8 * nt * RS - kLane<D> * tig, tig, qv);
+                load_row<D, AL>(df[hf], dl + (ptrdiff_t)8 * nt * OS - kLane<D> * tig, tig, qv);
             }
             mma_rows(s, ka, kb, qf[hf]);
             mma_rows_z(dp, va, vb, df[hf]);
@@ -1025,10 +1035,10 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
             } else {
                 b0[i] = b1[i] = __int_as_float(tp.y);
             }
-            load_row_at(qf0[i], ql + off);
-            load_row_at(qf1[i], ql + off + 8 * RS);
-            load_row_at(df0[i], dl + offd);
-            load_row_at(df1[i], dl + offd + 8 * OS);
+            load_row_at<D, AL>(qf0[i], ql + off);
+            load_row_at<D, AL>(qf1[i], ql + off + 8 * RS);
+            load_row_at<D, AL>(df0[i], dl + offd);
+            load_row_at<D, AL>(df1[i], dl + offd + 8 * OS);
             st0[i] = __ldg(rs + tp.x);
             st1[i] = __ldg(rs + tp.x + 8);
         }
@@ -1056,12 +1066,12 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
                 b0 = v0 ? __ldg(qs_r + (size_t)delta * Jp + si) : 0.f;
                 b1 = v1 ? __ldg(qs_r + (size_t)(delta + 8) * Jp + si) : 0.f;
             }
-            const ptrdiff_t off = (ptrdiff_t)delta * RS - 8 * tig, offd = (ptrdiff_t)delta * OS - 8 * tig;
+            const ptrdiff_t off = (ptrdiff_t)delta * RS - kLane<D> * tig, offd = (ptrdiff_t)delta * OS - kLane<D> * tig;
             RowFrag<D> qf0, qf1, df0, df1;
-            load_row(qf0, ql + off, tig, v0);
-            load_row(qf1, ql + off + 8 * RS, tig, v1);
-            load_row(df0, dl + offd, tig, v0);
-            load_row(df1, dl + offd + 8 * OS, tig, v1);
+            load_row<D, AL>(qf0, ql + off, tig, v0);
+            load_row<D, AL>(qf1, ql + off + 8 * RS, tig, v1);
+            load_row<D, AL>(df0, dl + offd, tig, v0);
+            load_row<D, AL>(df1, dl + offd + 8 * OS, tig, v1);
             const float2 st0 = v0 ? __ldg(rs + delta) : make_float2(0.f, 0.f);
             const float2 st1 = v1 ? __ldg(rs + delta + 8) : make_float2(0.f, 0.f);
             float s0[4], s1[4], e0[4], e1[4];
@@ -1073,15 +1083,15 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
     }
     __nv_bfloat16* dkp = static_cast<__nv_bfloat16*>(a.dk) + base;
     __nv_bfloat16* dvp = static_cast<__nv_bfloat16*>(a.dv) + base;
-    store_acc_rows<D>(dK, dkp + (size_t)row_lo * RS, dkp + (size_t)row_hi * RS, ok_lo, ok_hi, a.scale, a.scale, tig);
-    store_acc_rows<D>(dV, dvp + (size_t)row_lo * RS, dvp + (size_t)row_hi * RS, ok_lo, ok_hi, gain, gain, tig);   // dV = gain P^T.dO
+    store_acc_rows<D, AL>(dK, dkp + (size_t)row_lo * RS, dkp + (size_t)row_hi * RS, ok_lo, ok_hi, a.scale, a.scale, tig);
+    store_acc_rows<D, AL>(dV, dvp + (size_t)row_lo * RS, dvp + (size_t)row_hi * RS, ok_lo, ok_hi, gain, gain, tig);   // dV = gain P^T.dO
 }
 
 inline size_t dkdv_smem_bytes(int n_dense, int WB, bool se) {
     return se ? (size_t)(kRows + WB) * (n_dense + 1) * 4 : 0;
 }
 
-template <int D, int WB, int G, int CT, bool SE, bool ST>
+template <int D, int WB, int G, int CT, bool SE, int ST>
 __global__ void __launch_bounds__(kWarps * 32, CT)
 bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int reduce_stride) {
     constexpr int NT = (WB + 16) / 8;
@@ -1192,33 +1202,52 @@ cudaError_t ensure_dynamic_smem(K kernel, size_t bytes, int (&seen)[64]) {
     return e;
 }
 
-template <int D, int WB>
-cudaError_t fwd_launch_mma(const FwdArgs& a, const Taps& t, cudaStream_t s) {
+// Whether every piece of every row starts on a multiple of `bytes`.
+inline bool aligned_to(size_t bytes, std::initializer_list<const void*> ptrs, std::initializer_list<long long> strides) {
+    for (const void* p : ptrs) if (reinterpret_cast<uintptr_t>(p) % bytes) return false;
+    for (long long x : strides) if ((size_t)x * 2 % bytes) return false;
+    return true;
+}
+
+template <int D, int WB, bool SE, int ST>
+cudaError_t fwd_launch_mode(const FwdArgs& a, const Taps& t, cudaStream_t s) {
     constexpr int W = FwdTune<D>::warps, rows = 16 * W;
     dim3 grid((a.N + rows - 1) / rows, a.B * a.H);
-    if (a.scale_embed) {
-        if constexpr (D <= 64 && !kTail<D>) {
-            const size_t smem = se_tables_bytes(t.J, D, (WB + 16) / 8, W, 16);
-            static int seen[64] = {0}, seen_st[64] = {0};
-            cudaError_t e = a.strided ? ensure_dynamic_smem(fwd_mma_kernel<D, WB, true, true>, smem, seen_st)
-                                      : ensure_dynamic_smem(fwd_mma_kernel<D, WB, true, false>, smem, seen);
-            if (e != cudaSuccess) return e;
-            if (a.strided) fwd_mma_kernel<D, WB, true, true><<<grid, W * 32, smem, s>>>(a, t);
-            else fwd_mma_kernel<D, WB, true, false><<<grid, W * 32, smem, s>>>(a, t);
-        } else {
-            return cudaErrorInvalidValue;
-        }
-    } else if (a.strided) {
-        if constexpr (kTail<D>) return cudaErrorInvalidValue;
-        else fwd_mma_kernel<D, WB, false, true><<<grid, W * 32, 0, s>>>(a, t);
-    } else {
-        fwd_mma_kernel<D, WB, false, false><<<grid, W * 32, 0, s>>>(a, t);
+    size_t smem = 0;
+    if constexpr (SE) {
+        static int seen[64] = {0};
+        smem = se_tables_bytes(t.J, D, (WB + 16) / 8, W, 16);
+        const cudaError_t e = ensure_dynamic_smem(fwd_mma_kernel<D, WB, SE, ST>, smem, seen);
+        if (e != cudaSuccess) return e;
     }
+    fwd_mma_kernel<D, WB, SE, ST><<<grid, W * 32, smem, s>>>(a, t);
     return cudaGetLastError();
 }
 
-template <int D, int WB, bool SE, bool ST>
-cudaError_t bwd_launch_mma_se(BwdArgs a, const Taps& t, cudaStream_t s, int stages) {
+template <int D, int WB, bool SE>
+cudaError_t fwd_launch_se(FwdArgs a, const Taps& t, cudaStream_t s) {
+    if constexpr (kLane<D> == 16) {
+        if (!aligned_to(32, {a.q, a.k, a.v, a.out, a.gate}, {a.in_sb, a.in_sh, a.in_sn, a.out_sb, a.out_sh, a.out_sn})) {
+            if (!a.strided) {
+                a.in_sn = a.out_sn = D; a.in_sh = a.out_sh = (long long)a.N * D; a.in_sb = a.out_sb = (long long)a.H * a.N * D;
+            }
+            return fwd_launch_mode<D, WB, SE, kStridedAny>(a, t, s);
+        }
+    }
+    if (!a.strided) return fwd_launch_mode<D, WB, SE, kContiguous>(a, t, s);
+    if constexpr (kTail<D>) return cudaErrorInvalidValue;
+    else return fwd_launch_mode<D, WB, SE, kStrided>(a, t, s);
+}
+
+template <int D, int WB>
+cudaError_t fwd_launch_mma(const FwdArgs& a, const Taps& t, cudaStream_t s) {
+    if (!a.scale_embed) return fwd_launch_se<D, WB, false>(a, t, s);
+    if constexpr (D <= 64 && !kTail<D>) return fwd_launch_se<D, WB, true>(a, t, s);
+    else return cudaErrorInvalidValue;
+}
+
+template <int D, int WB, bool SE, int ST>
+cudaError_t bwd_launch_mode(BwdArgs a, const Taps& t, cudaStream_t s, int stages) {
     using T = BwdTune<D>;
     constexpr int NT = (WB + 16) / 8;
     if constexpr (SE) carve_bwd_scratch_mma_se(a, t.J); else carve_bwd_scratch(a, kRows, t.J, false);
@@ -1259,21 +1288,26 @@ cudaError_t bwd_launch_mma_se(BwdArgs a, const Taps& t, cudaStream_t s, int stag
     return e;
 }
 
-template <int D, int WB>
-cudaError_t bwd_launch_mma(const BwdArgs& a, const Taps& t, cudaStream_t s, int stages) {
-    if (a.scale_embed) {
-        if constexpr (D <= 64 && !kTail<D>) {
-            if (a.strided) return bwd_launch_mma_se<D, WB, true, true>(a, t, s, stages);
-            return bwd_launch_mma_se<D, WB, true, false>(a, t, s, stages);
-        } else {
-            return cudaErrorInvalidValue;
+template <int D, int WB, bool SE>
+cudaError_t bwd_launch_se(BwdArgs a, const Taps& t, cudaStream_t s, int stages) {
+    if constexpr (kLane<D> == 16) {
+        if (!aligned_to(32, {a.q, a.k, a.v, a.out, a.dout, a.dq, a.dk, a.dv}, {a.in_sb, a.in_sh, a.in_sn, a.out_sb, a.out_sh, a.out_sn})) {
+            if (!a.strided) {
+                a.in_sn = a.out_sn = D; a.in_sh = a.out_sh = (long long)a.N * D; a.in_sb = a.out_sb = (long long)a.H * a.N * D;
+            }
+            return bwd_launch_mode<D, WB, SE, kStridedAny>(a, t, s, stages);
         }
     }
-    if (a.strided) {
-        if constexpr (kTail<D>) return cudaErrorInvalidValue;
-        else return bwd_launch_mma_se<D, WB, false, true>(a, t, s, stages);
-    }
-    return bwd_launch_mma_se<D, WB, false, false>(a, t, s, stages);
+    if (!a.strided) return bwd_launch_mode<D, WB, SE, kContiguous>(a, t, s, stages);
+    if constexpr (kTail<D>) return cudaErrorInvalidValue;
+    else return bwd_launch_mode<D, WB, SE, kStrided>(a, t, s, stages);
+}
+
+template <int D, int WB>
+cudaError_t bwd_launch_mma(const BwdArgs& a, const Taps& t, cudaStream_t s, int stages) {
+    if (!a.scale_embed) return bwd_launch_se<D, WB, false>(a, t, s, stages);
+    if constexpr (D <= 64 && !kTail<D>) return bwd_launch_se<D, WB, true>(a, t, s, stages);
+    else return cudaErrorInvalidValue;
 }
 
 int band_width(const Taps& t) {

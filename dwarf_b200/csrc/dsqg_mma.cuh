@@ -4,7 +4,8 @@
 // --------------------------------------------------------
 // lane = 4*g + tig  (g = 0..7, tig = 0..3).  A warp owns a tile of 16 rows.
 // A row of D bf16 elements is split into 16-byte chunks; thread tig reads chunk tig of
-// every 64-byte group, i.e. elements  d = 32*c + 8*tig + [0,8)  for c = 0 .. D/32-1.  When 16
+// every 64-byte group, i.e. elements  d = 32*c + 8*tig + [0,8)  for c = 0 .. D/32-1 (D a multiple of 64:
+// 32-byte pieces of 128-byte groups, d = 64*c + 16*tig + [0,16)).  When 16
 // elements are left over (D = 48, 80) thread tig reads the eight bytes  D-16 + 4*tig + [0,4)  of them.
 // Those 8*D/32 elements are the thread's share of the contraction dimension for BOTH
 // operands of  mma.sync.m16n8k16  (the instruction assigns k-indices {2tig,2tig+1,2tig+8,
@@ -19,6 +20,8 @@
 //     d = 32*c + 8*tig + [0,8) of rows g and g+8: one 16-byte store per chunk.
 #pragma once
 
+#include <type_traits>
+
 #include "dsqg_common.cuh"
 
 namespace dsqg {
@@ -30,6 +33,7 @@ constexpr float kMinM = -1.0e29f;  // floor of the running row maximum: exp2(kNe
 
 template <int D> struct RowFrag { uint32_t r[D / 8]; };   // D/32 chunks x 4 registers, and 2 of a 16-element tail
 template <int D> constexpr bool kTail = D % 32 == 16;
+template <int D> constexpr int kLane = D % 64 == 0 ? 16 : 8;   // consecutive elements of a row a thread holds
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -37,20 +41,37 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// 16-byte chunks of one row; zero-filled when !valid (the pointer is not dereferenced then).
-template <int D>
-__device__ __forceinline__ void load_row(RowFrag<D>& f, const __nv_bfloat16* row_ptr, int tig, bool valid) {
+// p: this thread's piece of the row (row + kLane<D> * tig).  With D a multiple of 64 a piece is 32 bytes, one load, and the four
+// lanes of a row cover a whole 128-byte line: the L1 takes a line per cycle whatever part of it is wanted, so 16-byte pieces
+// (half a line per row and load) cost twice the passes.  B16 H12 N2048 D64: forward 104.8 -> 91.0, dQ 135.5 -> 122.0,
+// dK/dV 157.5 -> 137.3 us.  A32 = false: pieces aligned to 16 bytes only.
+template <int D, bool A32 = true>
+__device__ __forceinline__ void load_row_at(RowFrag<D>& f, const __nv_bfloat16* p) {
+    if constexpr (kLane<D> == 16 && A32) {
 #pragma unroll
-    for (int c = 0; c < D / 32; ++c) {
-        uint4 u = make_uint4(0u, 0u, 0u, 0u);
-        if (valid) u = __ldg(reinterpret_cast<const uint4*>(row_ptr + 32 * c + 8 * tig));
-        f.r[4 * c + 0] = u.x; f.r[4 * c + 1] = u.y; f.r[4 * c + 2] = u.z; f.r[4 * c + 3] = u.w;
+        for (int c = 0; c < D / 64; ++c)
+            asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                : "=r"(f.r[8 * c]), "=r"(f.r[8 * c + 1]), "=r"(f.r[8 * c + 2]), "=r"(f.r[8 * c + 3]), "=r"(f.r[8 * c + 4]),
+                  "=r"(f.r[8 * c + 5]), "=r"(f.r[8 * c + 6]), "=r"(f.r[8 * c + 7]) : "l"(p + 64 * c));
+    } else {
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) {
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(p + (kLane<D> == 16 ? 64 * (c >> 1) + 8 * (c & 1) : 32 * c)));
+            f.r[4 * c + 0] = u.x; f.r[4 * c + 1] = u.y; f.r[4 * c + 2] = u.z; f.r[4 * c + 3] = u.w;
+        }
     }
     if constexpr (kTail<D>) {
-        uint2 u = make_uint2(0u, 0u);
-        if (valid) u = __ldg(reinterpret_cast<const uint2*>(row_ptr + D - 16 + 4 * tig));
+        const uint2 u = __ldg(reinterpret_cast<const uint2*>(p + D - 16 - 4 * (int)(threadIdx.x & 3)));
         f.r[D / 8 - 2] = u.x; f.r[D / 8 - 1] = u.y;
     }
+}
+
+// One row; zero-filled when !valid (the pointer is not dereferenced then).
+template <int D, bool A32 = true>
+__device__ __forceinline__ void load_row(RowFrag<D>& f, const __nv_bfloat16* row_ptr, int tig, bool valid) {
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j) f.r[j] = 0u;
+    if (valid) load_row_at<D, A32>(f, row_ptr + kLane<D> * tig);
 }
 
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
@@ -127,37 +148,37 @@ __device__ __forceinline__ void diag_frag(float x_lo, float x_hi, bool owner, in
     a3 = hi << sh;
 }
 
-// Store rows g and g+8 of an accumulator tile (contiguous-d layout) as bf16, scaled per row.
-template <int D>
+// Store rows g and g+8 of an accumulator tile (the elements of load_row_at) as bf16, scaled per row.
+template <int D, bool A32>
+__device__ __forceinline__ void store_row_at(const uint32_t (&w)[D / 8], __nv_bfloat16* p) {
+    if constexpr (kLane<D> == 16 && A32) {
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c)
+            asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" :: "l"(p + 64 * c), "r"(w[8 * c]), "r"(w[8 * c + 1]), "r"(w[8 * c + 2]),
+                         "r"(w[8 * c + 3]), "r"(w[8 * c + 4]), "r"(w[8 * c + 5]), "r"(w[8 * c + 6]), "r"(w[8 * c + 7]) : "memory");
+    } else {
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c)
+            *reinterpret_cast<uint4*>(p + (kLane<D> == 16 ? 64 * (c >> 1) + 8 * (c & 1) : 32 * c)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+    }
+    if constexpr (kTail<D>) *reinterpret_cast<uint2*>(p + D - 16 - 4 * (int)(threadIdx.x & 3)) = make_uint2(w[D / 8 - 2], w[D / 8 - 1]);
+}
+template <int D, bool A32 = true>
 __device__ __forceinline__ void store_acc_rows(const float (&acc)[D / 8][4], __nv_bfloat16* row_lo, __nv_bfloat16* row_hi,
                                                bool ok_lo, bool ok_hi, float s_lo, float s_hi, int tig) {
+    uint32_t w[D / 8];
 #pragma unroll
-    for (int c = 0; c < D / 32; ++c) {
-        uint4 lo, hi;
-        lo.x = pack_bf16x2(acc[4 * c + 0][0] * s_lo, acc[4 * c + 0][1] * s_lo);
-        lo.y = pack_bf16x2(acc[4 * c + 1][0] * s_lo, acc[4 * c + 1][1] * s_lo);
-        lo.z = pack_bf16x2(acc[4 * c + 2][0] * s_lo, acc[4 * c + 2][1] * s_lo);
-        lo.w = pack_bf16x2(acc[4 * c + 3][0] * s_lo, acc[4 * c + 3][1] * s_lo);
-        hi.x = pack_bf16x2(acc[4 * c + 0][2] * s_hi, acc[4 * c + 0][3] * s_hi);
-        hi.y = pack_bf16x2(acc[4 * c + 1][2] * s_hi, acc[4 * c + 1][3] * s_hi);
-        hi.z = pack_bf16x2(acc[4 * c + 2][2] * s_hi, acc[4 * c + 2][3] * s_hi);
-        hi.w = pack_bf16x2(acc[4 * c + 3][2] * s_hi, acc[4 * c + 3][3] * s_hi);
-        if (ok_lo) *reinterpret_cast<uint4*>(row_lo + 32 * c + 8 * tig) = lo;
-        if (ok_hi) *reinterpret_cast<uint4*>(row_hi + 32 * c + 8 * tig) = hi;
-    }
-    if constexpr (kTail<D>) {
-        constexpr int J = D / 8 - 2;
-        if (ok_lo) *reinterpret_cast<uint2*>(row_lo + D - 16 + 4 * tig) =
-            make_uint2(pack_bf16x2(acc[J][0] * s_lo, acc[J][1] * s_lo), pack_bf16x2(acc[J + 1][0] * s_lo, acc[J + 1][1] * s_lo));
-        if (ok_hi) *reinterpret_cast<uint2*>(row_hi + D - 16 + 4 * tig) =
-            make_uint2(pack_bf16x2(acc[J][2] * s_hi, acc[J][3] * s_hi), pack_bf16x2(acc[J + 1][2] * s_hi, acc[J + 1][3] * s_hi));
-    }
+    for (int j = 0; j < D / 8; ++j) w[j] = pack_bf16x2(acc[j][0] * s_lo, acc[j][1] * s_lo);
+    if (ok_lo) store_row_at<D, A32>(w, row_lo + kLane<D> * tig);
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j) w[j] = pack_bf16x2(acc[j][2] * s_hi, acc[j][3] * s_hi);
+    if (ok_hi) store_row_at<D, A32>(w, row_hi + kLane<D> * tig);
 }
 
 // As store_acc_rows, with every element multiplied by sigmoid(gate) of the same position (gate rows
 // are bf16 in the layout of the output rows): the sigmoid gate of the attention block folded into
 // the epilogue (DWARF train/train_2048_condU.py:190-191).
-template <int D>
+template <int D, bool A32 = true>
 __device__ __forceinline__ void store_acc_rows_gated(const float (&acc)[D / 8][4], __nv_bfloat16* row_lo, __nv_bfloat16* row_hi,
                                                      const __nv_bfloat16* gate_lo, const __nv_bfloat16* gate_hi,
                                                      bool ok_lo, bool ok_hi, float s_lo, float s_hi, int tig) {
@@ -165,23 +186,21 @@ __device__ __forceinline__ void store_acc_rows_gated(const float (&acc)[D / 8][4
         a = __fdividef(1.f, 1.f + __expf(-__uint_as_float(u << 16)));
         b = __fdividef(1.f, 1.f + __expf(-__uint_as_float(u & 0xffff0000u)));
     };
+    auto half = [&](auto HC, const __nv_bfloat16* gate, __nv_bfloat16* row, float s) {
+        constexpr int H = decltype(HC)::value;
+        RowFrag<D> gf;
+        load_row_at<D, A32>(gf, gate + kLane<D> * tig);
+        uint32_t w[D / 8];
 #pragma unroll
-    for (int c = 0; c < D / 32; ++c) {
-        uint4 gl = make_uint4(0u, 0u, 0u, 0u), gh = gl;
-        if (ok_lo) gl = __ldg(reinterpret_cast<const uint4*>(gate_lo + 32 * c + 8 * tig));
-        if (ok_hi) gh = __ldg(reinterpret_cast<const uint4*>(gate_hi + 32 * c + 8 * tig));
-        const uint32_t gls[4] = {gl.x, gl.y, gl.z, gl.w}, ghs[4] = {gh.x, gh.y, gh.z, gh.w};
-        uint32_t lo[4], hi[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float a0, a1, b0, b1;
-            sig2(gls[j], a0, a1); sig2(ghs[j], b0, b1);
-            lo[j] = pack_bf16x2(acc[4 * c + j][0] * s_lo * a0, acc[4 * c + j][1] * s_lo * a1);
-            hi[j] = pack_bf16x2(acc[4 * c + j][2] * s_hi * b0, acc[4 * c + j][3] * s_hi * b1);
+        for (int j = 0; j < D / 8; ++j) {
+            float a, b;
+            sig2(gf.r[j], a, b);
+            w[j] = pack_bf16x2(acc[j][2 * H] * s * a, acc[j][2 * H + 1] * s * b);
         }
-        if (ok_lo) *reinterpret_cast<uint4*>(row_lo + 32 * c + 8 * tig) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        if (ok_hi) *reinterpret_cast<uint4*>(row_hi + 32 * c + 8 * tig) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-    }
+        store_row_at<D, A32>(w, row + kLane<D> * tig);
+    };
+    if (ok_lo) half(std::integral_constant<int, 0>(), gate_lo, row_lo, s_lo);
+    if (ok_hi) half(std::integral_constant<int, 1>(), gate_hi, row_hi, s_hi);
 }
 
 // Partial dot product of two row fragments over this thread's elements (fp32).
@@ -244,19 +263,5 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f
 // The running maximum of the online softmax only moves when a score exceeds it by more than this
 // (log2 units): probabilities stay below 2^kSlack, which fp32 sums and bf16 values absorb.
 constexpr float kSlack = 16.f;
-
-// p: this thread's chunk of the row (row + 8 * tig)
-template <int D>
-__device__ __forceinline__ void load_row_at(RowFrag<D>& f, const __nv_bfloat16* p) {
-#pragma unroll
-    for (int c = 0; c < D / 32; ++c) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(p + 32 * c));
-        f.r[4 * c + 0] = u.x; f.r[4 * c + 1] = u.y; f.r[4 * c + 2] = u.z; f.r[4 * c + 3] = u.w;
-    }
-    if constexpr (kTail<D>) {
-        const uint2 u = __ldg(reinterpret_cast<const uint2*>(p + D - 16 - 4 * (int)(threadIdx.x & 3)));
-        f.r[D / 8 - 2] = u.x; f.r[D / 8 - 1] = u.y;
-    }
-}
 
 }  // namespace dsqg

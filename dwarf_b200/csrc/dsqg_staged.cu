@@ -128,17 +128,17 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const FwdCtx& cx, con
     const size_t base = (size_t)bh * N * D;
     const __nv_bfloat16* qp = static_cast<const __nv_bfloat16*>(a.q) + base;
     // this thread's 16-byte chunk of row row_lo of K
-    const __nv_bfloat16* kl = static_cast<const __nv_bfloat16*>(a.k) + base + (ptrdiff_t)row_lo * D + 8 * tig;
+    const __nv_bfloat16* kl = static_cast<const __nv_bfloat16*>(a.k) + base + (ptrdiff_t)row_lo * D + kLane<D> * tig;
     const int2 nv = cx.tb->tile_nv[L.warp];
     const int n_valid = nv.x, n_full = nv.y;
 
     RowFrag<D> qa, qb;
     if (INTERIOR) {
-        load_row_at(qa, qp + (size_t)row_lo * D + 8 * tig);
-        load_row_at(qb, qp + (size_t)row_hi * D + 8 * tig);
+        load_row_at<D, false>(qa, qp + (size_t)row_lo * D + kLane<D> * tig);
+        load_row_at<D, false>(qb, qp + (size_t)row_hi * D + kLane<D> * tig);
     } else {
-        load_row(qa, qp + (size_t)row_lo * D, tig, row_lo < N);
-        load_row(qb, qp + (size_t)row_hi * D, tig, row_hi < N);
+        load_row<D, false>(qa, qp + (size_t)row_lo * D, tig, row_lo < N);
+        load_row<D, false>(qb, qp + (size_t)row_hi * D, tig, row_hi < N);
     }
 
     // ---- scores of the dense window: key row of n-tile nt for this thread is g0 - 32 + 8 nt + g
@@ -150,10 +150,10 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const FwdCtx& cx, con
             S[nt][0] = pb[-8 * nt]; S[nt][1] = pb[-8 * nt - 1]; S[nt][2] = pb[8 - 8 * nt]; S[nt][3] = pb[7 - 8 * nt];
             RowFrag<D> kf;
             if (INTERIOR) {
-                load_row_at(kf, kl + (8 * nt - kWB) * D);
+                load_row_at<D, false>(kf, kl + (8 * nt - kWB) * D);
             } else {
                 const int kr = row_lo - kWB + 8 * nt;
-                load_row(kf, kl + (ptrdiff_t)(8 * nt - kWB) * D - 8 * tig, tig, kr >= 0 && kr < N);
+                load_row<D, false>(kf, kl + (ptrdiff_t)(8 * nt - kWB) * D - kLane<D> * tig, tig, kr >= 0 && kr < N);
             }
             mma_rows(S[nt], qa, qb, kf);
         }
@@ -179,12 +179,12 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const FwdCtx& cx, con
         const int dl = cx.tb->taps[tp].x;
         RowFrag<D> k0, k1;
         if (full) {
-            load_row_at(k0, kl - (ptrdiff_t)dl * D);
-            load_row_at(k1, kl - (ptrdiff_t)dl * D + 8 * D);
+            load_row_at<D, false>(k0, kl - (ptrdiff_t)dl * D);
+            load_row_at<D, false>(k1, kl - (ptrdiff_t)dl * D + 8 * D);
         } else {
             const int kr0 = row_lo - dl, kr1 = row_hi - dl;
-            load_row(k0, kl - (ptrdiff_t)dl * D - 8 * tig, tig, kr0 >= 0 && kr0 < N);
-            load_row(k1, kl - (ptrdiff_t)dl * D + 8 * D - 8 * tig, tig, kr1 >= 0 && kr1 < N);
+            load_row<D, false>(k0, kl - (ptrdiff_t)dl * D - kLane<D> * tig, tig, kr0 >= 0 && kr0 < N);
+            load_row<D, false>(k1, kl - (ptrdiff_t)dl * D + 8 * D - kLane<D> * tig, tig, kr1 >= 0 && kr1 < N);
         }
         const uint32_t sel = g == c ? kOnes : 0u;
 #pragma unroll

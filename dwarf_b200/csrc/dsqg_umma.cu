@@ -390,15 +390,15 @@ fwd_umma_kernel(const FwdArgs a, const Taps t, int tiles_per_seq, int n_tiles,
                 const Lane L;
                 const size_t seq = (size_t)bh * N * D;
                 const __nv_bfloat16* qg = static_cast<const __nv_bfloat16*>(a.q) + seq;
-                const __nv_bfloat16* kg = static_cast<const __nv_bfloat16*>(a.k) + seq + 8 * L.tig;
-                const __nv_bfloat16* vg = static_cast<const __nv_bfloat16*>(a.v) + seq + 8 * L.tig;
+                const __nv_bfloat16* kg = static_cast<const __nv_bfloat16*>(a.k) + seq + kLane<D> * L.tig;
+                const __nv_bfloat16* vg = static_cast<const __nv_bfloat16*>(a.v) + seq + kLane<D> * L.tig;
                 const int gw = n0 + 32 * wq;                  // first row of the warp
                 Half<D> hs[2];
 #pragma unroll
                 for (int hh = 0; hh < 2; ++hh) {
                     const int row_lo = gw + 16 * hh + L.g, row_hi = row_lo + 8;
-                    load_row(hs[hh].qa, qg + (size_t)row_lo * D, L.tig, row_lo < N);
-                    load_row(hs[hh].qb, qg + (size_t)row_hi * D, L.tig, row_hi < N);
+                    load_row<D, false>(hs[hh].qa, qg + (size_t)row_lo * D, L.tig, row_lo < N);
+                    load_row<D, false>(hs[hh].qb, qg + (size_t)row_hi * D, L.tig, row_hi < N);
                     hs[hh].m_lo = fmaxf(__shfl_sync(0xffffffffu, m_raw, 16 * hh + L.g), kMinM);
                     hs[hh].m_hi = fmaxf(__shfl_sync(0xffffffffu, m_raw, 16 * hh + L.g + 8), kMinM);
                     hs[hh].ms_lo = L.owner ? hs[hh].m_lo : 1.0e30f; hs[hh].ms_hi = L.owner ? hs[hh].m_hi : 1.0e30f;
@@ -419,7 +419,7 @@ fwd_umma_kernel(const FwdArgs a, const Taps t, int tiles_per_seq, int n_tiles,
                         const __nv_bfloat16* vp = vg + (ptrdiff_t)(gw + L.g - delta) * D;
                         RowFrag<D> kf[4], vf[4];
 #pragma unroll
-                        for (int q4 = 0; q4 < 4; ++q4) { load_row_at(kf[q4], kp + 8 * q4 * D); load_row_at(vf[q4], vp + 8 * q4 * D); }
+                        for (int q4 = 0; q4 < 4; ++q4) { load_row_at<D, false>(kf[q4], kp + 8 * q4 * D); load_row_at<D, false>(vf[q4], vp + 8 * q4 * D); }
 #pragma unroll
                         for (int hh = 0; hh < 2; ++hh) {
                             float s0[4], s1[4];
@@ -436,10 +436,10 @@ fwd_umma_kernel(const FwdArgs a, const Taps t, int tiles_per_seq, int n_tiles,
                             const int kr0 = g0 + L.g - delta, kr1 = kr0 + 8;
                             const bool v0 = kr0 >= 0 && kr0 < N, v1 = kr1 >= 0 && kr1 < N;
                             RowFrag<D> kf0, kf1, vf0, vf1;
-                            load_row(kf0, kg + (ptrdiff_t)kr0 * D - 8 * L.tig, L.tig, v0);
-                            load_row(kf1, kg + (ptrdiff_t)kr1 * D - 8 * L.tig, L.tig, v1);
-                            load_row(vf0, vg + (ptrdiff_t)kr0 * D - 8 * L.tig, L.tig, v0);
-                            load_row(vf1, vg + (ptrdiff_t)kr1 * D - 8 * L.tig, L.tig, v1);
+                            load_row<D, false>(kf0, kg + (ptrdiff_t)kr0 * D - kLane<D> * L.tig, L.tig, v0);
+                            load_row<D, false>(kf1, kg + (ptrdiff_t)kr1 * D - kLane<D> * L.tig, L.tig, v1);
+                            load_row<D, false>(vf0, vg + (ptrdiff_t)kr0 * D - kLane<D> * L.tig, L.tig, v0);
+                            load_row<D, false>(vf1, vg + (ptrdiff_t)kr1 * D - kLane<D> * L.tig, L.tig, v1);
                             float s0[4], s1[4];
                             mma_rows_z(s0, hs[hh].qa, hs[hh].qb, kf0);
                             mma_rows_z(s1, hs[hh].qa, hs[hh].qb, kf1);
