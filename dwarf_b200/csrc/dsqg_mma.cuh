@@ -3,21 +3,20 @@
 // Fragment convention used by every kernel in dsqg_mma*.cu
 // --------------------------------------------------------
 // lane = 4*g + tig  (g = 0..7, tig = 0..3).  A warp owns a tile of 16 rows.
-// A row of D bf16 elements is split into 16-byte chunks; thread tig reads chunk tig of
-// every 64-byte group, i.e. elements  d = 32*c + 8*tig + [0,8)  for c = 0 .. D/32-1 (D a multiple of 64:
-// 32-byte pieces of 128-byte groups, d = 64*c + 16*tig + [0,16)).  When 16
-// elements are left over (D = 48, 80) thread tig reads the eight bytes  D-16 + 4*tig + [0,4)  of them.
-// Those 8*D/32 elements are the thread's share of the contraction dimension for BOTH
+// A row of D bf16 elements is split into groups of 64, 32 and 16 elements (as many of each as fit, in this order); thread tig reads
+// a quarter of every group: elements 64*c + 16*tig + [0,16), then 8*tig + [0,8) of a 32-element group, then 4*tig + [0,4) of
+// a 16-element tail.
+// Those D/4 elements are the thread's share of the contraction dimension for BOTH
 // operands of  mma.sync.m16n8k16  (the instruction assigns k-indices {2tig,2tig+1,2tig+8,
 // 2tig+9} of every k-step to thread tig in the A and in the B fragment alike, so any fixed
 // assignment of physical d to k-index is legal as long as A and B agree).  Hence
-//   * a "row fragment" (RowFrag) is loaded with one 16-byte load per 32 elements of D,
+//   * a "row fragment" (RowFrag) is loaded with one load per group,
 //   * the same RowFrag serves as A operand (rows g, g+8 of the warp tile) or as B operand
 //     (row g of an 8-row n-tile) of a product that contracts over d,
 //   * movmatrix(.trans) turns a RowFrag into the B operand of a product that contracts over
-//     ROWS (P.V, dS.K, ...); the accumulator column n of such a product maps to
-//     d = 32*c + 8*(n>>1) + 2*j + (n&1), so thread tig ends up owning the contiguous elements
-//     d = 32*c + 8*tig + [0,8) of rows g and g+8: one 16-byte store per chunk.
+//     ROWS (P.V, dS.K, ...); column n of n-tile j of such a product is element n&1 of register j of
+//     thread n>>1, so thread tig ends up owning the elements of rows g and g+8 that it would load of
+//     them: one store per group.
 #pragma once
 
 #include <type_traits>
@@ -31,9 +30,10 @@ constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kNeg = -1.0e30f;   // finite "minus infinity": masked scores
 constexpr float kMinM = -1.0e29f;  // floor of the running row maximum: exp2(kNeg - kMinM) == 0
 
-template <int D> struct RowFrag { uint32_t r[D / 8]; };   // D/32 chunks x 4 registers, and 2 of a 16-element tail
-template <int D> constexpr bool kTail = D % 32 == 16;
-template <int D> constexpr int kLane = D % 64 == 0 ? 16 : 8;   // consecutive elements of a row a thread holds
+template <int D> struct RowFrag { uint32_t r[D / 8]; };
+template <int D> constexpr bool kTail = D % 32 == 16;      // 8 bytes per thread
+template <int D> constexpr bool kMid = D % 64 >= 32;       // 16 bytes per thread
+template <int D> constexpr int kLane = D >= 64 ? 16 : 8;   // consecutive elements of a row a thread holds (of the first piece)
 
 __device__ __forceinline__ float ex2(float x) {
     float y;
@@ -41,27 +41,37 @@ __device__ __forceinline__ float ex2(float x) {
     return y;
 }
 
-// p: this thread's piece of the row (row + kLane<D> * tig).  With D a multiple of 64 a piece is 32 bytes, one load, and the four
-// lanes of a row cover a whole 128-byte line: the L1 takes a line per cycle whatever part of it is wanted, so 16-byte pieces
+// Where the 16-byte and 8-byte pieces of a row lie from the thread's first piece on (row + kLane<D> * tig).
+template <int D> __device__ __forceinline__ int mid_at() { return D >= 64 ? D / 64 * 64 - 8 * (int)(threadIdx.x & 3) : 0; }
+template <int D> __device__ __forceinline__ int tail_at() { return D - 16 - (kLane<D> - 4) * (int)(threadIdx.x & 3); }
+
+// p: this thread's first piece of the row (row + kLane<D> * tig).  64 elements are one load of 32 bytes per thread, so that the
+// four lanes of a row cover a whole 128-byte line: the L1 takes a line per cycle whatever part of it is wanted, so 16-byte pieces
 // (half a line per row and load) cost twice the passes.  B16 H12 N2048 D64: forward 104.8 -> 91.0, dQ 135.5 -> 122.0,
 // dK/dV 157.5 -> 137.3 us.  A32 = false: pieces aligned to 16 bytes only.
 template <int D, bool A32 = true>
 __device__ __forceinline__ void load_row_at(RowFrag<D>& f, const __nv_bfloat16* p) {
-    if constexpr (kLane<D> == 16 && A32) {
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c)
+    for (int c = 0; c < D / 64; ++c) {
+        if constexpr (A32) {
             asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                 : "=r"(f.r[8 * c]), "=r"(f.r[8 * c + 1]), "=r"(f.r[8 * c + 2]), "=r"(f.r[8 * c + 3]), "=r"(f.r[8 * c + 4]),
                   "=r"(f.r[8 * c + 5]), "=r"(f.r[8 * c + 6]), "=r"(f.r[8 * c + 7]) : "l"(p + 64 * c));
-    } else {
+        } else {
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) {
-            const uint4 u = __ldg(reinterpret_cast<const uint4*>(p + (kLane<D> == 16 ? 64 * (c >> 1) + 8 * (c & 1) : 32 * c)));
-            f.r[4 * c + 0] = u.x; f.r[4 * c + 1] = u.y; f.r[4 * c + 2] = u.z; f.r[4 * c + 3] = u.w;
+            for (int h = 0; h < 2; ++h) {
+                const uint4 u = __ldg(reinterpret_cast<const uint4*>(p + 64 * c) + h);
+                f.r[8 * c + 4 * h] = u.x; f.r[8 * c + 4 * h + 1] = u.y; f.r[8 * c + 4 * h + 2] = u.z; f.r[8 * c + 4 * h + 3] = u.w;
+            }
         }
     }
+    if constexpr (kMid<D>) {
+        constexpr int J = D / 64 * 8;
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(p + mid_at<D>()));
+        f.r[J] = u.x; f.r[J + 1] = u.y; f.r[J + 2] = u.z; f.r[J + 3] = u.w;
+    }
     if constexpr (kTail<D>) {
-        const uint2 u = __ldg(reinterpret_cast<const uint2*>(p + D - 16 - 4 * (int)(threadIdx.x & 3)));
+        const uint2 u = __ldg(reinterpret_cast<const uint2*>(p + tail_at<D>()));
         f.r[D / 8 - 2] = u.x; f.r[D / 8 - 1] = u.y;
     }
 }
@@ -151,17 +161,22 @@ __device__ __forceinline__ void diag_frag(float x_lo, float x_hi, bool owner, in
 // Store rows g and g+8 of an accumulator tile (the elements of load_row_at) as bf16, scaled per row.
 template <int D, bool A32>
 __device__ __forceinline__ void store_row_at(const uint32_t (&w)[D / 8], __nv_bfloat16* p) {
-    if constexpr (kLane<D> == 16 && A32) {
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c)
+    for (int c = 0; c < D / 64; ++c) {
+        if constexpr (A32) {
             asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" :: "l"(p + 64 * c), "r"(w[8 * c]), "r"(w[8 * c + 1]), "r"(w[8 * c + 2]),
                          "r"(w[8 * c + 3]), "r"(w[8 * c + 4]), "r"(w[8 * c + 5]), "r"(w[8 * c + 6]), "r"(w[8 * c + 7]) : "memory");
-    } else {
+        } else {
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c)
-            *reinterpret_cast<uint4*>(p + (kLane<D> == 16 ? 64 * (c >> 1) + 8 * (c & 1) : 32 * c)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
+            for (int h = 0; h < 2; ++h)
+                *(reinterpret_cast<uint4*>(p + 64 * c) + h) = make_uint4(w[8 * c + 4 * h], w[8 * c + 4 * h + 1], w[8 * c + 4 * h + 2], w[8 * c + 4 * h + 3]);
+        }
     }
-    if constexpr (kTail<D>) *reinterpret_cast<uint2*>(p + D - 16 - 4 * (int)(threadIdx.x & 3)) = make_uint2(w[D / 8 - 2], w[D / 8 - 1]);
+    if constexpr (kMid<D>) {
+        constexpr int J = D / 64 * 8;
+        *reinterpret_cast<uint4*>(p + mid_at<D>()) = make_uint4(w[J], w[J + 1], w[J + 2], w[J + 3]);
+    }
+    if constexpr (kTail<D>) *reinterpret_cast<uint2*>(p + tail_at<D>()) = make_uint2(w[D / 8 - 2], w[D / 8 - 1]);
 }
 template <int D, bool A32 = true>
 __device__ __forceinline__ void store_acc_rows(const float (&acc)[D / 8][4], __nv_bfloat16* row_lo, __nv_bfloat16* row_hi,
