@@ -34,7 +34,8 @@ def _torch_flags():
     comp = ["-I", inc, "-I", os.path.join(inc, "torch", "csrc", "api", "include"), "-I", os.path.join(cuda, "include"),
             "-I", sysconfig.get_paths()["include"], "-DTORCH_EXTENSION_NAME=_dsqg_torch",
             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
-    return comp, ["-L", lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", f"-Wl,-rpath,{lib}"]
+    return comp, ["-L", lib, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", f"-Wl,-rpath,{lib}",
+                  "-L", os.path.join(cuda, "lib64"), "-lcublasLt", "-lcublas"]
 
 
 def _stale() -> bool:

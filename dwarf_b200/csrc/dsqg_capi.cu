@@ -103,7 +103,8 @@ static int fwd_impl(const void* q, const void* k, const void* v,
                     const float* pos_bias, const float* scale_embed, const float* head_gain,
                     const int32_t* offsets, int J, void* out, float* lse,
                     int B, int H, int N, int D, int dtype, void* stream, float scale,
-                    const dsqg_strides* in_st = nullptr, const dsqg_strides* out_st = nullptr, const void* gate = nullptr) {
+                    const dsqg_strides* in_st = nullptr, const dsqg_strides* out_st = nullptr, const void* gate = nullptr,
+                    const dsqg_strides* gate_st = nullptr, void* keep = nullptr) {
     if (!q || !k || !v || !pos_bias || !out || !lse) return DSQG_ERR_NULL_POINTER;
     int rc = check_op_shape(B, H, N, D, dtype);
     if (rc) return rc;
@@ -118,15 +119,18 @@ static int fwd_impl(const void* q, const void* k, const void* v,
     a.head_gain = head_gain; a.out = out; a.lse = lse;
     a.B = B; a.H = H; a.N = N; a.D = D;
     a.scale = scale > 0.f ? scale : 1.0f / sqrtf((float)D);
-    a.strided = 0; a.gate = nullptr;
-    a.in_sb = a.in_sh = a.in_sn = a.out_sb = a.out_sh = a.out_sn = 0;
+    a.strided = 0; a.gate = nullptr; a.keep = nullptr;
+    a.in_sb = a.in_sh = a.in_sn = a.out_sb = a.out_sh = a.out_sn = a.gate_sb = a.gate_sh = a.gate_sn = 0;
     NvtxRange range(in_st ? "dsqg_fwd_strided" : "dsqg_fwd");
     if (in_st) {
         // strided tensors exist for the tensor-core kernels only
         if (!out_st) return DSQG_ERR_NULL_POINTER;
-        if (bad_strides(in_st) || bad_strides(out_st) || (gate && misaligned16(gate))) return DSQG_ERR_MISALIGNED;
+        if (!gate_st) gate_st = out_st;
+        if (bad_strides(in_st) || bad_strides(out_st) || (gate && (misaligned16(gate) || bad_strides(gate_st))) || misaligned16(keep))
+            return DSQG_ERR_MISALIGNED;
         if (!mma_fwd_supported(dtype, D, t, scale_embed != nullptr)) return DSQG_ERR_UNSUPPORTED;
-        a.strided = 1; a.gate = gate;
+        a.strided = 1; a.gate = gate; a.keep = keep;
+        a.gate_sb = gate_st->batch; a.gate_sh = gate_st->head; a.gate_sn = gate_st->row;
         a.in_sb = in_st->batch; a.in_sh = in_st->head; a.in_sn = in_st->row;
         a.out_sb = out_st->batch; a.out_sh = out_st->head; a.out_sn = out_st->row;
         cudaError_t e = launch_fwd_mma(a, t, static_cast<cudaStream_t>(stream));
@@ -195,7 +199,7 @@ static int bwd_impl(const void* q, const void* k, const void* v,
                     void* scratch, size_t scratch_bytes,
                     int B, int H, int N, int D, int dtype, void* stream, int stages, float scale,
                     const dsqg_strides* in_st = nullptr, const dsqg_strides* out_st = nullptr,
-                    const float* delta_pre = nullptr);
+                    const float* delta_pre = nullptr, bool kept = false);
 
 int dsqg_bwd_stages(const void* q, const void* k, const void* v,
                     const float* pos_bias, const float* scale_embed, const float* head_gain,
@@ -231,7 +235,7 @@ static int bwd_impl(const void* q, const void* k, const void* v,
                     float* dpos_bias, float* dscale_embed, float* dhead_gain,
                     void* scratch, size_t scratch_bytes,
                     int B, int H, int N, int D, int dtype, void* stream, int stages, float scale,
-                    const dsqg_strides* in_st, const dsqg_strides* out_st, const float* delta_pre) {
+                    const dsqg_strides* in_st, const dsqg_strides* out_st, const float* delta_pre, bool kept) {
     if (stages < 1 || stages > DSQG_BWD_STAGE_ALL) return DSQG_ERR_UNSUPPORTED;
     if (!q || !k || !v || !pos_bias || !out || !lse || !dout || !dq || !dk || !dv || !dpos_bias || !scratch)
         return DSQG_ERR_NULL_POINTER;
@@ -258,14 +262,15 @@ static int bwd_impl(const void* q, const void* k, const void* v,
     a.n_tiles = a.tiles_per_bh = a.n_dse_blocks = 0;
     a.B = B; a.H = H; a.N = N; a.D = D;
     a.scale = scale > 0.f ? scale : 1.0f / sqrtf((float)D);
-    a.strided = 0; a.delta_pre = nullptr;
+    a.strided = 0; a.delta_pre = nullptr; a.kept = 0;
     a.in_sb = a.in_sh = a.in_sn = a.out_sb = a.out_sh = a.out_sn = 0;
     NvtxRange range(in_st ? "dsqg_bwd_strided" : "dsqg_bwd");
     if (in_st) {
         if (!out_st) return DSQG_ERR_NULL_POINTER;
         if (bad_strides(in_st) || bad_strides(out_st)) return DSQG_ERR_MISALIGNED;
         if (!mma_path_supported(dtype, D, t, scale_embed != nullptr)) return DSQG_ERR_UNSUPPORTED;
-        a.strided = 1; a.delta_pre = delta_pre;
+        if (kept && (!kept_pays(D) || !delta_pre)) return DSQG_ERR_UNSUPPORTED;
+        a.strided = 1; a.delta_pre = delta_pre; a.kept = kept;
         a.in_sb = in_st->batch; a.in_sh = in_st->head; a.in_sn = in_st->row;
         a.out_sb = out_st->batch; a.out_sh = out_st->head; a.out_sn = out_st->row;
         cudaError_t e = launch_bwd_mma(a, t, static_cast<cudaStream_t>(stream), stages);
@@ -315,6 +320,55 @@ int dsqg_bwd_strided_se(const void* q, const void* k, const void* v, const dsqg_
                     DSQG_BWD_STAGE_ALL, scale, qkv_strides, out_strides, delta_pre);
 }
 
+size_t dsqg_packed_keep_bytes(int B, int H, int N, int D) {
+    return kept_pays(D) && !check_op_shape(B, H, N, D, DSQG_DTYPE_BF16) ? (size_t)3 * B * H * N * D * 2 : 0;
+}
+
+int dsqg_packed_fwd(const dsqg_packed* p, void* stream) {
+    if (!p) return DSQG_ERR_NULL_POINTER;
+    return fwd_impl(p->q, p->k, p->v, p->pos_bias, p->scale_embed, p->head_gain, p->offsets, p->J, p->out, p->lse, p->B, p->H, p->N, p->D,
+                    DSQG_DTYPE_BF16, stream, 0.f, &p->qkv_strides, &p->out_strides, p->gate, &p->gate_strides, p->keep);
+}
+
+size_t dsqg_packed_bwd_scratch_bytes(const dsqg_packed* p) {
+    if (!p) return 0;
+    const size_t need = dsqg_bwd_scratch_bytes(p->J, p->B, p->H, p->N, p->D, p->scale_embed != nullptr);
+    if (!need || !p->gate) return need;
+    const size_t rows = (size_t)p->B * p->H * p->N;
+    return round256(need) + round256(rows * 4) + rows * p->D * 2;          // delta and dout of the gate's backward
+}
+
+int dsqg_packed_bwd(const dsqg_packed* p, const dsqg_packed_grads* g, void* scratch, size_t scratch_bytes, void* stream) {
+    if (!p || !g || !scratch) return DSQG_ERR_NULL_POINTER;
+    const int B = p->B, H = p->H, N = p->N, D = p->D;
+    int rc = check_op_shape(B, H, N, D, DSQG_DTYPE_BF16);
+    if (rc) return rc;
+    if (scratch_bytes < dsqg_packed_bwd_scratch_bytes(p)) return DSQG_ERR_SCRATCH_TOO_SMALL;
+    const size_t need = dsqg_bwd_scratch_bytes(p->J, B, H, N, D, p->scale_embed != nullptr);
+    const void* dout = g->dy;
+    dsqg_strides dout_st = p->out_strides;
+    const float* delta = nullptr;
+    if (p->gate) {
+        if (!g->dy || !p->out || !g->dgate) return DSQG_ERR_NULL_POINTER;
+        if (bad_strides(&p->out_strides) || bad_strides(&p->gate_strides) || misaligned16(g->dy) || misaligned16(p->out) || misaligned16(p->gate) ||
+            misaligned16(g->dgate) || misaligned16(scratch))
+            return DSQG_ERR_MISALIGNED;
+        char* mem = static_cast<char*>(scratch) + round256(need);
+        float* dl = reinterpret_cast<float*>(mem);
+        void* buf = mem + round256((size_t)B * H * N * 4);
+        dout_st.batch = (long long)H * N * D; dout_st.head = (long long)N * D; dout_st.row = D;   // head-major: the operator's backward reads whole lines
+        const cudaError_t e = launch_gate_bwd(g->dy, p->out, p->out_strides, p->gate, g->dgate, p->gate_strides, buf, dout_st, dl,
+                                              B, H, N, D, static_cast<cudaStream_t>(stream));
+        if (e != cudaSuccess) return cuda_fail(e);
+        dout = buf; delta = dl;
+    }
+    const size_t part = (size_t)B * H * N * D;
+    const __nv_bfloat16* kept = static_cast<const __nv_bfloat16*>(p->keep);
+    return bwd_impl(kept ? kept : p->q, kept ? kept + part : p->k, kept ? kept + 2 * part : p->v, p->pos_bias, p->scale_embed, p->head_gain,
+                    p->offsets, p->J, p->out, p->lse, dout, g->dq, g->dk, g->dv, g->dpos_bias, g->dscale_embed, g->dhead_gain, scratch, need,
+                    B, H, N, D, DSQG_DTYPE_BF16, stream, DSQG_BWD_STAGE_ALL, 0.f, &p->qkv_strides, &dout_st, delta, kept != nullptr);
+}
+
 int dsqg_gate_bwd(const void* dy, const void* y, const void* gate, const dsqg_strides* strides,
                   void* dout, void* dgate, float* delta, int B, int H, int N, int D, void* stream) {
     if (!dy || !y || !gate || !strides || !dout || !dgate || !delta) return DSQG_ERR_NULL_POINTER;
@@ -323,8 +377,7 @@ int dsqg_gate_bwd(const void* dy, const void* y, const void* gate, const dsqg_st
     if (bad_strides(strides) || misaligned16(dy) || misaligned16(y) || misaligned16(gate) || misaligned16(dout) ||
         misaligned16(dgate))
         return DSQG_ERR_MISALIGNED;
-    cudaError_t e = launch_gate_bwd(dy, y, gate, strides->batch, strides->head, strides->row, dout, dgate, delta,
-                                    B, H, N, D, static_cast<cudaStream_t>(stream));
+    cudaError_t e = launch_gate_bwd(dy, y, *strides, gate, dgate, *strides, dout, *strides, delta, B, H, N, D, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? DSQG_OK : cuda_fail(e);
 }
 

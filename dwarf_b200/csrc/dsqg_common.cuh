@@ -36,6 +36,9 @@ struct FwdArgs {
     int strided;
     long long in_sb, in_sh, in_sn, out_sb, out_sh, out_sn;
     const void* gate;
+    long long gate_sb, gate_sh, gate_sn;      // element strides of gate
+    // Strided only, nullable: [3][B,H,N,D], receives copies of q, k and v for a backward that reads them contiguous (BwdArgs::kept).
+    void* keep;
 };
 
 struct BwdArgs {
@@ -61,6 +64,8 @@ struct BwdArgs {
     int strided;
     long long in_sb, in_sh, in_sn, out_sb, out_sh, out_sn;
     const float* delta_pre;
+    // Strided only: q, k, v and dout are contiguous [B,H,N,D] all the same (in_* then addresses dq, dk, dv only; needs delta_pre).
+    int kept;
 };
 
 struct DecodeArgs {
@@ -86,8 +91,9 @@ cudaError_t launch_ring_prefill(const void* k, const void* v, void* k_ring, void
 
 cudaError_t launch_ring_advance(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R, cudaStream_t s);
 cudaError_t launch_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, bool reverse, cudaStream_t s);
-cudaError_t launch_gate_bwd(const void* dy, const void* y, const void* gate, long long sb, long long sh, long long sn,
-                            void* dout, void* dgate, float* delta, int B, int H, int N, int D, cudaStream_t s);
+// y and dy, gate and dgate, and dout have strides of their own
+cudaError_t launch_gate_bwd(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, void* dgate, const dsqg_strides& gs,
+                            void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s);
 cudaError_t launch_fwd_mma(const FwdArgs& a, const Taps& t, cudaStream_t s);
 cudaError_t launch_bwd_mma(const BwdArgs& a, const Taps& t, cudaStream_t s, int stages);
 bool mma_path_supported(int dtype, int D, const Taps& t, bool has_scale_embed);   // backward
@@ -102,6 +108,11 @@ cudaError_t launch_wait_timeout(long long limit_cycles, int site, cudaStream_t s
 bool umma_supported(int dtype, int D, const Taps& t, bool has_scale_embed);
 cudaError_t launch_fwd_umma(const FwdArgs& a, const Taps& t, cudaStream_t s);
 cudaError_t read_umma_error(int* value, bool reset);
+
+// Whether the backward of strided tensors gains from contiguous copies of q, k, v that the forward leaves (FwdArgs::keep): rows shorter
+// than a 128-byte line cost as much L1 time as whole lines unless the next row follows (B32 H8 N2048 D32: dQ 126 -> 104, dK/dV
+// 125 -> 102 us for copies that cost the forward 13 us).  Whole rows are read at the same rate wherever they lie.
+constexpr bool kept_pays(int D) { return D == 32; }
 
 // Backward scratch layout: row statistics (8 bytes per row) | dpos_bias partials | dhead_gain partials | dscale_embed
 // partials, each block rounded up to 256 bytes.  A "tile" is the set of rows whose partial

@@ -167,15 +167,15 @@ __global__ void __launch_bounds__(kT) gated_pool_bwd_kernel(const __nv_bfloat16*
     store8(dg + i, o); store8(dpool + i, q);
 }
 
-// ---- k += k_delta, v += v_delta on the key and value thirds of qkv [rows][3 D]; delta rows ld elements apart
-__global__ void __launch_bounds__(kT) inject_kernel(__nv_bfloat16* __restrict__ qkv, const __nv_bfloat16* __restrict__ kd,
+// ---- k += k_delta, v += v_delta on columns D .. 3 D of qkv; rows lq / ld elements apart
+__global__ void __launch_bounds__(kT) inject_kernel(__nv_bfloat16* __restrict__ qkv, long long lq, const __nv_bfloat16* __restrict__ kd,
                                                     const __nv_bfloat16* __restrict__ vd, long long ld, long long rows, int D) {
     const long long i = (long long)blockIdx.x * kT + threadIdx.x;
     const int per = D / 8;                                     // 16-byte pieces of a delta row
     if (i >= rows * 2 * per) return;
     const long long row = i / (2 * per);
     const int c = (int)(i - row * 2 * per);
-    __nv_bfloat16* dst = qkv + row * 3 * D + D + 8 * c;
+    __nv_bfloat16* dst = qkv + row * lq + D + 8 * c;
     float x[8], y[8];
     load8(dst, x); load8((c < per ? kd + 8 * c : vd + 8 * (c - per)) + row * ld, y);
 #pragma unroll
@@ -318,12 +318,12 @@ int dsqg_gated_pool_bwd(const void* dout, const void* g, const float* pool, void
     return status();
 }
 
-int dsqg_inject_kv(void* qkv, const void* k_delta, const void* v_delta, long long delta_stride, long long rows, int D, void* stream) {
+int dsqg_inject_kv(void* qkv, long long qkv_stride, const void* k_delta, const void* v_delta, long long delta_stride, long long rows, int D, void* stream) {
     if (!qkv || !k_delta || !v_delta) return DSQG_ERR_NULL_POINTER;
     if (rows < 1 || D < 8 || D % 8) return DSQG_ERR_BAD_SHAPE;
-    if (bad(qkv) || bad(k_delta) || bad(v_delta) || delta_stride < D || delta_stride % 8) return DSQG_ERR_MISALIGNED;
+    if (bad(qkv) || bad(k_delta) || bad(v_delta) || delta_stride < D || delta_stride % 8 || qkv_stride < 3 * D || qkv_stride % 8) return DSQG_ERR_MISALIGNED;
     inject_kernel<<<blocks_for(rows * (D / 4)), kT, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(k_delta), static_cast<const __nv_bfloat16*>(v_delta), delta_stride, rows, D);
+        static_cast<__nv_bfloat16*>(qkv), qkv_stride, static_cast<const __nv_bfloat16*>(k_delta), static_cast<const __nv_bfloat16*>(v_delta), delta_stride, rows, D);
     return status();
 }
 

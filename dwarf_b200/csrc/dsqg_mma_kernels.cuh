@@ -32,8 +32,9 @@ constexpr int kRows = 16 * kWarps; // rows per CTA
 
 // How q, k, v, out, ... are addressed: contiguous [B,H,N,D]; through the element strides in FwdArgs / BwdArgs (rows of D
 // contiguous elements; any batch / head / row strides), e.g. the un-permuted output of a fused qkv projection and a token-major
-// result; the same with pieces that are aligned to 16 bytes only where a piece is 32 (D a multiple of 64).
-constexpr int kContiguous = 0, kStrided = 1, kStridedAny = 2;
+// result; the same with pieces that are aligned to 16 bytes only where a piece is 32 (D >= 64); backward only: strides for the
+// gradients, everything that is read contiguous.
+constexpr int kContiguous = 0, kStrided = 1, kStridedAny = 2, kKept = 3;
 
 // ------------------------------------------------------------------------------ forward
 // Online softmax over the dense window, then over the sparse taps, with the per-element
@@ -136,6 +137,12 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
     RowFrag<D> qa, qb;
     load_row<D, AL>(qa, qp + (size_t)row_lo * RS, tig, ok_lo);
     load_row<D, AL>(qb, qp + (size_t)row_hi * RS, tig, ok_hi);
+    // Copies for the backward: tensor x (0: q, 1: k, 2: v), rows g / g + 8
+    auto keep = [&](int x, const RowFrag<D>& f, int row, bool ok) {
+        if (ST && a.keep && ok)
+            store_row_at<D, true>(f.r, static_cast<__nv_bfloat16*>(a.keep) + (((size_t)x * a.B * a.H + bh) * N + row) * D + kLane<D> * tig);
+    };
+    keep(0, qa, row_lo, ok_lo); keep(0, qb, row_hi, ok_hi);
     if constexpr (SE) build_qs_tile<D, false>(se, qa, qb, g, tig);
 
     // ---- dense window: key row of n-tile nt for this thread is kb0 + 8 nt + g = row_lo - WB + 8 nt
@@ -155,6 +162,7 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             const int kr = kb0 + 8 * nt + g;
             load_row<D, AL>(kf, kl + (ptrdiff_t)(8 * nt - WB) * RS - kLane<D> * tig, tig, kr >= 0 && kr < N);
         }
+        if (nt >= WB / 8) keep(1, kf, nt == WB / 8 ? row_lo : row_hi, nt == WB / 8 ? ok_lo : ok_hi);
         mma_rows(S[nt], qa, qb, kf);
     }
     if (!INTERIOR && kb0 < 0) {
@@ -190,6 +198,7 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             load_row<D, AL>(vf0, vl + (ptrdiff_t)(16 * c - WB) * RS - kLane<D> * tig, tig, kr >= 0 && kr < N);
             load_row<D, AL>(vf1, vl + (ptrdiff_t)(16 * c + 8 - WB) * RS - kLane<D> * tig, tig, kr + 8 >= 0 && kr + 8 < N);
         }
+        if (c == WB / 16) { keep(2, vf0, row_lo, ok_lo); keep(2, vf1, row_hi, ok_hi); }
         transpose_frag(vt0, vf0); transpose_frag(vt1, vf1);
         const uint32_t a0 = pack_bf16x2(S[2 * c][0], S[2 * c][1]), a1 = pack_bf16x2(S[2 * c][2], S[2 * c][3]);
         const uint32_t a2 = pack_bf16x2(S[2 * c + 1][0], S[2 * c + 1][1]), a3 = pack_bf16x2(S[2 * c + 1][2], S[2 * c + 1][3]);
@@ -304,9 +313,9 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
     __nv_bfloat16* op = static_cast<__nv_bfloat16*>(a.out) + obase;
     const float sc_lo = l_lo > 0.f ? __fdividef(gain, l_lo) : 0.f, sc_hi = l_hi > 0.f ? __fdividef(gain, l_hi) : 0.f;
     if (ST && a.gate) {
-        const __nv_bfloat16* gp = static_cast<const __nv_bfloat16*>(a.gate) + obase;
-        store_acc_rows_gated<D, AL>(O, op + (size_t)row_lo * OS, op + (size_t)row_hi * OS, gp + (size_t)row_lo * OS,
-                                gp + (size_t)row_hi * OS, ok_lo, ok_hi, sc_lo, sc_hi, tig);
+        const __nv_bfloat16* gp = static_cast<const __nv_bfloat16*>(a.gate) + (size_t)(bh / a.H) * a.gate_sb + (size_t)h * a.gate_sh;
+        store_acc_rows_gated<D, AL>(O, op + (size_t)row_lo * OS, op + (size_t)row_hi * OS, gp + (size_t)row_lo * a.gate_sn,
+                                    gp + (size_t)row_hi * a.gate_sn, ok_lo, ok_hi, sc_lo, sc_hi, tig);
     } else {
         store_acc_rows<D, AL>(O, op + (size_t)row_lo * OS, op + (size_t)row_hi * OS, ok_lo, ok_hi, sc_lo, sc_hi, tig);
     }
@@ -464,10 +473,10 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = g0 + g, row_hi = row_lo + 8;
     const bool ok_lo = INTERIOR || row_lo < N, ok_hi = INTERIOR || row_hi < N;
-    constexpr bool AL = ST != kStridedAny;
-    const ptrdiff_t RS = ST ? (ptrdiff_t)a.in_sn : D, OS = ST ? (ptrdiff_t)a.out_sn : D;   // row strides of q/k/v/dq and of out/dout
-    const size_t base = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : (size_t)bh * N * D;
-    const size_t obase = ST ? (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh : base;
+    constexpr bool AL = ST != kStridedAny, CI = ST == kContiguous || ST == kKept;          // CI: what is read is contiguous
+    const ptrdiff_t GS = ST ? (ptrdiff_t)a.in_sn : D, RS = CI ? D : GS, OS = CI ? D : (ptrdiff_t)a.out_sn;   // row strides of dq, q/k/v, out/dout
+    const size_t cbase = (size_t)bh * N * D, gbase = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : cbase, base = CI ? cbase : gbase;
+    const size_t obase = CI ? cbase : (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh;
     const __nv_bfloat16* qp = static_cast<const __nv_bfloat16*>(a.q) + base;
     const __nv_bfloat16* op = static_cast<const __nv_bfloat16*>(a.out) + obase;
     const __nv_bfloat16* dop = static_cast<const __nv_bfloat16*>(a.dout) + obase;
@@ -669,8 +678,8 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
             }
         }
     }
-    __nv_bfloat16* dqp = static_cast<__nv_bfloat16*>(a.dq) + base;
-    store_acc_rows<D, AL>(dQ, dqp + (size_t)row_lo * RS, dqp + (size_t)row_hi * RS, ok_lo, ok_hi, a.scale, a.scale, tig);
+    __nv_bfloat16* dqp = static_cast<__nv_bfloat16*>(a.dq) + gbase;
+    store_acc_rows<D, AL>(dQ, dqp + (size_t)row_lo * GS, dqp + (size_t)row_hi * GS, ok_lo, ok_hi, a.scale, a.scale, tig);
     float dg0, dg1;
     unpair(dgrow2, dg0, dg1);
     return dgrow + (dg0 + dg1);
@@ -932,10 +941,10 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = m0 + g, row_hi = row_lo + 8;
     const bool ok_lo = INTERIOR || row_lo < N, ok_hi = INTERIOR || row_hi < N;
-    constexpr bool AL = ST != kStridedAny;
-    const ptrdiff_t RS = ST ? (ptrdiff_t)a.in_sn : D, OS = ST ? (ptrdiff_t)a.out_sn : D;   // row strides of q/k/v/dk/dv and of dout
-    const size_t base = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : (size_t)bh * N * D;
-    const size_t obase = ST ? (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh : base;
+    constexpr bool AL = ST != kStridedAny, CI = ST == kContiguous || ST == kKept;          // CI: what is read is contiguous
+    const ptrdiff_t GS = ST ? (ptrdiff_t)a.in_sn : D, RS = CI ? D : GS, OS = CI ? D : (ptrdiff_t)a.out_sn;   // row strides of dk/dv, q/k/v, dout
+    const size_t cbase = (size_t)bh * N * D, gbase = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : cbase, base = CI ? cbase : gbase;
+    const size_t obase = CI ? cbase : (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh;
     const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(a.k) + base;
     const __nv_bfloat16* vp = static_cast<const __nv_bfloat16*>(a.v) + base;
     const __nv_bfloat16* ql = static_cast<const __nv_bfloat16*>(a.q) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
@@ -1082,10 +1091,10 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
                    b0, b1, st0, st1, qf0, qf1, df0, df1);
         }
     }
-    __nv_bfloat16* dkp = static_cast<__nv_bfloat16*>(a.dk) + base;
-    __nv_bfloat16* dvp = static_cast<__nv_bfloat16*>(a.dv) + base;
-    store_acc_rows<D, AL>(dK, dkp + (size_t)row_lo * RS, dkp + (size_t)row_hi * RS, ok_lo, ok_hi, a.scale, a.scale, tig);
-    store_acc_rows<D, AL>(dV, dvp + (size_t)row_lo * RS, dvp + (size_t)row_hi * RS, ok_lo, ok_hi, gain, gain, tig);   // dV = gain P^T.dO
+    __nv_bfloat16* dkp = static_cast<__nv_bfloat16*>(a.dk) + gbase;
+    __nv_bfloat16* dvp = static_cast<__nv_bfloat16*>(a.dv) + gbase;
+    store_acc_rows<D, AL>(dK, dkp + (size_t)row_lo * GS, dkp + (size_t)row_hi * GS, ok_lo, ok_hi, a.scale, a.scale, tig);
+    store_acc_rows<D, AL>(dV, dvp + (size_t)row_lo * GS, dvp + (size_t)row_hi * GS, ok_lo, ok_hi, gain, gain, tig);   // dV = gain P^T.dO
 }
 
 inline size_t dkdv_smem_bytes(int n_dense, int WB, bool se) {
@@ -1228,7 +1237,7 @@ cudaError_t fwd_launch_mode(const FwdArgs& a, const Taps& t, cudaStream_t s) {
 template <int D, int WB, bool SE>
 cudaError_t fwd_launch_se(FwdArgs a, const Taps& t, cudaStream_t s) {
     if constexpr (kLane<D> == 16) {       // 32-byte pieces
-        if (!aligned_to(32, {a.q, a.k, a.v, a.out, a.gate}, {a.in_sb, a.in_sh, a.in_sn, a.out_sb, a.out_sh, a.out_sn})) {
+        if (!aligned_to(32, {a.q, a.k, a.v, a.out, a.gate, a.keep}, {a.in_sb, a.in_sh, a.in_sn, a.out_sb, a.out_sh, a.out_sn, a.gate_sb, a.gate_sh, a.gate_sn})) {
             if (!a.strided) {
                 a.in_sn = a.out_sn = D; a.in_sh = a.out_sh = (long long)a.N * D; a.in_sb = a.out_sb = (long long)a.H * a.N * D;
             }
@@ -1300,6 +1309,10 @@ cudaError_t bwd_launch_se(BwdArgs a, const Taps& t, cudaStream_t s, int stages) 
         }
     }
     if (!a.strided) return bwd_launch_mode<D, WB, SE, kContiguous>(a, t, s, stages);
+    if (a.kept) {
+        if constexpr (kept_pays(D)) return bwd_launch_mode<D, WB, SE, kKept>(a, t, s, stages);
+        else return cudaErrorInvalidValue;
+    }
     if constexpr (kTail<D>) return cudaErrorInvalidValue;
     else return bwd_launch_mode<D, WB, SE, kStrided>(a, t, s, stages);
 }

@@ -13,6 +13,10 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/Exceptions.h>
 
+#include <cublasLt.h>
+#include <cublas_v2.h>
+
+#include <array>
 #include <cmath>
 #include <map>
 #include <memory>
@@ -240,94 +244,104 @@ std::tuple<Tensor, Tensor> forward_lse(const Tensor& q0, const Tensor& k0, const
 }
 
 // ------------------------------------------------------------------------------------ packed projection output
-// q, k, v read in place from qkv [B,N,3,H,HD]; y [B,N,H*HD] token-major, times sigmoid(gate).
-struct PackedStrides {
-    dsqg_strides in, out;
-    PackedStrides(int64_t N, int64_t H, int64_t D) : in{N * 3 * H * D, D, 3 * H * D}, out{N * H * D, D, H * D} {}
-};
-char* third(const Tensor& qkv, int i) { return static_cast<char*>(qkv.data_ptr()) + i * qkv.size(3) * qkv.size(4) * qkv.element_size(); }
+// What a packed forward leaves for its backward.  proj: the projection output [B*N, cols] (row-major) that q, k, v and, in a layer,
+// the gate are read from in place; keep: the copies of q, k, v that stand in for it (dsqg_packed_keep_bytes).
+struct PackedForward { Tensor proj, gate, pb, hg, se, y, lse, keep; };
 
-struct PackedForward { Tensor gate, pb, hg, se, y, lse; };
+// q, k, v at columns 0, H*D, 2*H*D of rows of `cols` elements; the gate at column 3*H*D of the same rows or in a tensor laid out like y.
+dsqg_packed describe(const PackedForward& f, void* proj, int64_t cols, const Offsets& off) {
+    const int64_t B = f.lse.size(0), H = f.lse.size(1), N = f.lse.size(2), D = f.y.size(2) / H;
+    dsqg_packed p = {};
+    char* at = static_cast<char*>(proj);
+    p.q = at; p.k = at + H * D * 2; p.v = at + 2 * H * D * 2;
+    p.qkv_strides = {N * cols, D, cols};
+    p.out_strides = {N * H * D, D, H * D};
+    p.gate = f.gate.defined() ? ptr(f.gate) : cols == 4 * H * D ? at + 3 * H * D * 2 : nullptr;
+    p.gate_strides = f.gate.defined() ? p.out_strides : p.qkv_strides;
+    p.pos_bias = fptr(f.pb); p.scale_embed = fptr(f.se); p.head_gain = fptr(f.hg);
+    p.offsets = off.v.data(); p.J = off.J();
+    p.B = (int)B; p.H = (int)H; p.N = (int)N; p.D = (int)D;
+    p.out = ptr(f.y); p.lse = fptr(f.lse); p.keep = ptr(f.keep);
+    return p;
+}
 
-PackedForward packed_forward(const Tensor& qkv, const Tensor& gate, const Tensor& pos_bias, const Tensor& head_gain, const Tensor& scale_embed,
-                             const Offsets& off) {
-    if (qkv.dim() != 5 || qkv.size(2) != 3 || qkv.scalar_type() != at::kBFloat16 || !qkv.is_contiguous())
-        throw py::value_error("dsqg packed: qkv must be a contiguous bf16 [B,N,3,H,HD] tensor");
-    const int64_t B = qkv.size(0), N = qkv.size(1), H = qkv.size(3), D = qkv.size(4), J = off.J();
-    if (gate.defined() && (gate.scalar_type() != at::kBFloat16 || !shape_is(gate, {B, N, H * D})))
-        throw py::value_error("dsqg packed: gate must be bf16 [B,N,H*HD]");
+// proj [.., cols]; with_grad: whether a backward will follow.
+PackedForward packed_forward(const Tensor& proj, int64_t B, int64_t N, int64_t H, int64_t D, int64_t cols, const Tensor& gate, const Tensor& pos_bias,
+                             const Tensor& head_gain, const Tensor& scale_embed, const Offsets& off, bool with_grad) {
+    const int64_t J = off.J();
     PackedForward f;
+    f.proj = proj;
     f.gate = gate.defined() ? gate.contiguous() : gate;
     f.pb = f32c(pos_bias); f.hg = f32c(head_gain); f.se = f32c(scale_embed);
     if (!shape_is(f.pb, {J, H})) throw py::value_error("dsqg: pos_bias must be [" + std::to_string(J) + "," + std::to_string(H) + "], got " + shape_of(f.pb));
     if (f.se.defined() && !shape_is(f.se, {J, D}))
         throw py::value_error("dsqg: scale_embed must be [" + std::to_string(J) + "," + std::to_string(D) + "], got " + shape_of(f.se));
-    if (!qkv.is_cuda()) throw std::runtime_error("dsqg: tensors must live on a CUDA device (there is no CPU path)");
-    const c10::cuda::CUDAGuard guard(qkv.device());
-    f.y = new_tensor({B, N, H * D}, at::kBFloat16, qkv);
-    f.lse = new_tensor({B, H, N}, at::kFloat, qkv);
-    const PackedStrides st(N, H, D);
-    if (f.se.defined())
-        check(dsqg_fwd_strided_se(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.se), fptr(f.hg), off.v.data(), off.J(),
-                                  ptr(f.y), &st.out, ptr(f.gate), fptr(f.lse), (int)B, (int)H, (int)N, (int)D, DSQG_DTYPE_BF16, stream_of(qkv), 0.f),
-              "dsqg_fwd_strided_se");
-    else
-        check(dsqg_fwd_strided(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.hg), off.v.data(), off.J(),
-                               ptr(f.y), &st.out, ptr(f.gate), fptr(f.lse), (int)B, (int)H, (int)N, (int)D, DSQG_DTYPE_BF16, stream_of(qkv), 0.f),
-              "dsqg_fwd_strided");
+    f.y = new_tensor({B, N, H * D}, at::kBFloat16, proj);
+    f.lse = new_tensor({B, H, N}, at::kFloat, proj);
+    // a gated backward has dout in contiguous rows of its own; without a gate dy stays where it is and the copies would gain less than they cost
+    const bool gated = f.gate.defined() || cols == 4 * H * D;
+    if (with_grad && gated && dsqg_packed_keep_bytes((int)B, (int)H, (int)N, (int)D)) f.keep = new_tensor({3, B, H, N, D}, at::kBFloat16, proj);
+    const dsqg_packed p = describe(f, ptr(proj), cols, off);
+    check(dsqg_packed_fwd(&p, stream_of(proj)), "dsqg_packed_fwd");
     return f;
 }
 
-struct PackedGrads { Tensor dqkv, dgate, dpb, dhg, dse; };
+struct PackedGrads { Tensor dproj, dgate, dpb, dhg, dse; };
 
-PackedGrads packed_backward(const Tensor& qkv, const PackedForward& f, const Tensor& dy0, const Offsets& off) {
-    const int64_t B = qkv.size(0), N = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
-    const c10::cuda::CUDAGuard guard(qkv.device());
-    const Tensor dy = (dy0.scalar_type() == at::kBFloat16 ? dy0 : dy0.to(at::kBFloat16)).contiguous();
-    const PackedStrides st(N, H, D);
-    void* stream = stream_of(qkv);
+// dproj [B*N, cols]; proj may be undefined where keep stands in for it and the gate has a tensor of its own.
+PackedGrads packed_backward(const PackedForward& f, const Tensor& dy, int64_t cols, const Offsets& off) {
+    const int64_t B = f.lse.size(0), N = f.lse.size(2);
     PackedGrads g;
-    g.dqkv = new_like(qkv); g.dpb = new_like(f.pb);
-    g.dhg = new_like(f.hg); g.dse = new_like(f.se);
-    const size_t bytes = dsqg_bwd_scratch_bytes(off.J(), (int)B, (int)H, (int)N, (int)D, f.se.defined());
+    g.dproj = new_tensor({B * N, cols}, at::kBFloat16, dy);
+    g.dgate = new_like(f.gate); g.dpb = new_like(f.pb); g.dhg = new_like(f.hg); g.dse = new_like(f.se);
+    const dsqg_packed p = describe(f, f.proj.defined() ? ptr(f.proj) : ptr(f.keep), cols, off);
+    const int64_t third = (int64_t)p.H * p.D * 2;
+    char* at = static_cast<char*>(ptr(g.dproj));
+    dsqg_packed_grads d = {};
+    d.dy = ptr(dy); d.dq = at; d.dk = at + third; d.dv = at + 2 * third;
+    d.dgate = g.dgate.defined() ? ptr(g.dgate) : at + 3 * third;
+    d.dpos_bias = fptr(g.dpb); d.dscale_embed = fptr(g.dse); d.dhead_gain = fptr(g.dhg);
+    const size_t bytes = dsqg_packed_bwd_scratch_bytes(&p);
     const at::DataPtr scratch = scratch_for(bytes);
-    at::DataPtr dout_mem, delta_mem;
-    void* dout = ptr(dy);
-    float* delta = nullptr;
-    if (f.gate.defined()) {
-        g.dgate = new_like(f.gate);
-        dout_mem = scratch_for((size_t)dy.numel() * 2);
-        delta_mem = scratch_for((size_t)B * H * N * 4);
-        dout = dout_mem.get(); delta = static_cast<float*>(delta_mem.get());
-        check(dsqg_gate_bwd(ptr(dy), ptr(f.y), ptr(f.gate), &st.out, dout, ptr(g.dgate), delta, (int)B, (int)H, (int)N, (int)D, stream), "dsqg_gate_bwd");
-    }
-    if (f.se.defined())
-        check(dsqg_bwd_strided_se(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.se), fptr(f.hg), off.v.data(), off.J(),
-                                  ptr(f.y), fptr(f.lse), dout, &st.out, delta, third(g.dqkv, 0), third(g.dqkv, 1), third(g.dqkv, 2), fptr(g.dpb),
-                                  fptr(g.dse), fptr(g.dhg), scratch.get(), bytes, (int)B, (int)H, (int)N, (int)D, DSQG_DTYPE_BF16, stream, 0.f),
-              "dsqg_bwd_strided_se");
-    else
-        check(dsqg_bwd_strided(third(qkv, 0), third(qkv, 1), third(qkv, 2), &st.in, fptr(f.pb), fptr(f.hg), off.v.data(), off.J(),
-                               ptr(f.y), fptr(f.lse), dout, &st.out, delta, third(g.dqkv, 0), third(g.dqkv, 1), third(g.dqkv, 2), fptr(g.dpb),
-                               fptr(g.dhg), scratch.get(), bytes, (int)B, (int)H, (int)N, (int)D, DSQG_DTYPE_BF16, stream, 0.f), "dsqg_bwd_strided");
+    check(dsqg_packed_bwd(&p, &d, scratch.get(), bytes, stream_of(dy)), "dsqg_packed_bwd");
     return g;
 }
+
+PackedForward packed_op(const Tensor& qkv, const Tensor& gate, const Tensor& pos_bias, const Tensor& head_gain, const Tensor& scale_embed,
+                        const Offsets& off, bool with_grad) {
+    if (qkv.dim() != 5 || qkv.size(2) != 3 || qkv.scalar_type() != at::kBFloat16 || !qkv.is_contiguous())
+        throw py::value_error("dsqg packed: qkv must be a contiguous bf16 [B,N,3,H,HD] tensor");
+    const int64_t B = qkv.size(0), N = qkv.size(1), H = qkv.size(3), D = qkv.size(4);
+    if (gate.defined() && (gate.scalar_type() != at::kBFloat16 || !shape_is(gate, {B, N, H * D})))
+        throw py::value_error("dsqg packed: gate must be bf16 [B,N,H*HD]");
+    if (!qkv.is_cuda()) throw std::runtime_error("dsqg: tensors must live on a CUDA device (there is no CPU path)");
+    const c10::cuda::CUDAGuard guard(qkv.device());
+    return packed_forward(qkv, B, N, H, D, 3 * H * D, gate, pos_bias, head_gain, scale_embed, off, with_grad);
+}
+
+Tensor bf16c(const Tensor& t) { return (t.scalar_type() == at::kBFloat16 ? t : t.to(at::kBFloat16)).contiguous(); }
 
 struct PackedNode : torch::autograd::Function<PackedNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& qkv, const std::optional<Tensor>& gate, const Tensor& pos_bias,
                           const std::optional<Tensor>& hg, const std::optional<Tensor>& se, const Offsets* off) {
         const Tensor head_gain = opt(hg), scale_embed = opt(se);
-        PackedForward f = packed_forward(qkv, opt(gate), pos_bias, head_gain, scale_embed, *off);
-        ctx->save_for_backward({qkv, f.gate, f.pb, f.hg, f.se, f.y, f.lse});
+        PackedForward f = packed_op(qkv, opt(gate), pos_bias, head_gain, scale_embed, *off, true);
+        ctx->save_for_backward({f.keep.defined() ? Tensor() : qkv, f.gate, f.pb, f.hg, f.se, f.y, f.lse, f.keep});
         ctx->saved_data["offsets"] = (int64_t)(intptr_t)off;
         ctx->saved_data["types"] = types_of(pos_bias, head_gain, scale_embed);
         return f.y;
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        return backward_body(grads[0], [&] { return run(ctx, grads[0]); });
+    }
+    static variable_list run(AutogradContext* ctx, const Tensor& dy) {
         const variable_list s = ctx->get_saved_variables();
-        const PackedForward f = {s[1], s[2], s[3], s[4], s[5], s[6]};
-        const PackedGrads g = backward_body(grads[0], [&] { return packed_backward(s[0], f, grads[0], offsets_of(ctx)); });
-        return {g.dqkv, g.dgate, like_param(g.dpb, type_at(ctx, 0)), like_param(g.dhg, type_at(ctx, 1)), like_param(g.dse, type_at(ctx, 2)), Tensor()};
+        const PackedForward f = {s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7]};
+        const c10::cuda::CUDAGuard guard(dy.device());
+        const int64_t B = f.lse.size(0), H = f.lse.size(1), N = f.lse.size(2), D = f.y.size(2) / H;
+        const PackedGrads g = packed_backward(f, bf16c(dy), 3 * H * D, offsets_of(ctx));
+        return {g.dproj.view({B, N, 3, H, D}), g.dgate, like_param(g.dpb, type_at(ctx, 0)), like_param(g.dhg, type_at(ctx, 1)),
+                like_param(g.dse, type_at(ctx, 2)), Tensor()};
     }
 };
 
@@ -336,7 +350,7 @@ Tensor attention_packed(const Tensor& qkv, const std::optional<Tensor>& gate, co
     py::gil_scoped_release no_gil;
     const Tensor g = opt(gate), h = opt(hg), e = opt(se);
     if (wants_grad({&qkv, &g, &pb, &h, &e})) return PackedNode::apply(qkv, gate, pb, hg, se, off);
-    return packed_forward(qkv, g, pb, h, e, *off).y;
+    return packed_op(qkv, g, pb, h, e, *off, false).y;
 }
 
 // ------------------------------------------------------------------------------------ causal mean
@@ -370,41 +384,131 @@ struct NoAutocast {
     c10::impl::ExcludeDispatchKeyGuard guard{c10::autocast_dispatch_keyset};
 };
 
-// bf16 copies of fp32 tensors back to back in one buffer, in one launch.
-std::vector<Tensor> cast_bf16(const std::vector<Tensor>& src0) {
-    std::vector<Tensor> src;
-    int64_t total = 0;
-    for (const Tensor& t : src0) { src.push_back(f32c(t)); total += t.numel(); }
-    const Tensor buf = new_tensor({total}, at::kBFloat16, src[0]);
-    std::vector<Tensor> out;
-    const float* sp[DSQG_CAST_MAX]; void* dp[DSQG_CAST_MAX]; long long n[DSQG_CAST_MAX];
-    int64_t o = 0;
-    for (size_t k = 0; k < src.size(); ++k) {
-        out.push_back(src[k].dim() == 2 ? at::as_strided(buf, src[k].sizes(), {src[k].size(1), 1}, o) : at::as_strided(buf, {src[k].numel()}, {1}, o));
-        sp[k] = fptr(src[k]); dp[k] = ptr(out[k]); n[k] = src[k].numel();
-        o += src[k].numel();
+// Row-major C[M,N] = op(A) . op(B) (+ bias[N]) on bf16 operands, C in bf16 or fp32, through cuBLASLt with plans kept per thread and
+// problem: a call costs the host 4 us where at::linear and at::mm (dispatch, checks, a heuristic query each time) take 16-22, and
+// a layer's step makes eleven.
+struct GemmPlan {
+    cublasLtMatmulDesc_t op = nullptr;
+    cublasLtMatrixLayout_t a = nullptr, b = nullptr, c = nullptr;
+    cublasLtMatmulAlgo_t algo;
+    size_t workspace = 0;
+    GemmPlan() = default;
+    GemmPlan(const GemmPlan&) = delete;
+    ~GemmPlan() {
+        if (a) cublasLtMatrixLayoutDestroy(a);
+        if (b) cublasLtMatrixLayoutDestroy(b);
+        if (c) cublasLtMatrixLayoutDestroy(c);
+        if (op) cublasLtMatmulDescDestroy(op);
     }
-    check(dsqg_cast_bf16(sp, dp, n, (int)src.size(), stream_of(buf)), "dsqg_cast_bf16");
-    return out;
+};
+void lt_check(cublasStatus_t s, const char* what) {
+    if (s != CUBLAS_STATUS_SUCCESS) throw std::runtime_error(std::string("dsqg: ") + what + ": " + cublasGetStatusString(s));
+}
+using GemmKey = std::array<int64_t, 8>;       // device, M, N, K, transposes and bias, output type, workspace, lda
+
+// ta: A is stored [K,M]; tb: B is stored [N,K]; lda: elements between A's rows (0: none skipped)
+void gemm(void* C, bool f32_out, const void* A, bool ta, const void* B, bool tb, const void* bias, int64_t M, int64_t N, int64_t K, const Tensor& on,
+          int64_t lda = 0) {
+    static thread_local std::map<GemmKey, std::unique_ptr<GemmPlan>> plans;
+    constexpr size_t kMostPlans = 128;
+    cublasLtHandle_t lt = at::cuda::getCurrentCUDABlasLtHandle();
+    size_t space = at::cuda::getCUDABlasLtWorkspaceSize();
+    const GemmKey key = {on.device().index(), M, N, K, (ta ? 1 : 0) | (tb ? 2 : 0) | (bias ? 4 : 0), f32_out, (int64_t)space, lda};
+    if (plans.size() >= kMostPlans && !plans.count(key)) plans.clear();
+    std::unique_ptr<GemmPlan>& slot = plans[key];
+    if (!slot) {
+        // cuBLAS is column-major: C^T[N,M] = op(B)^T . op(A)^T
+        auto p = std::make_unique<GemmPlan>();
+        lt_check(cublasLtMatmulDescCreate(&p->op, CUBLAS_COMPUTE_32F, CUDA_R_32F), "cublasLtMatmulDescCreate");
+        const cublasOperation_t opb = tb ? CUBLAS_OP_T : CUBLAS_OP_N, opa = ta ? CUBLAS_OP_T : CUBLAS_OP_N;
+        lt_check(cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_TRANSA, &opb, sizeof opb), "cublasLtMatmulDescSetAttribute");
+        lt_check(cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_TRANSB, &opa, sizeof opa), "cublasLtMatmulDescSetAttribute");
+        if (bias) {
+            const cublasLtEpilogue_t e = CUBLASLT_EPILOGUE_BIAS;
+            lt_check(cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_EPILOGUE, &e, sizeof e), "cublasLtMatmulDescSetAttribute");
+            lt_check(cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof bias), "cublasLtMatmulDescSetAttribute");
+        }
+        lt_check(cublasLtMatrixLayoutCreate(&p->b, CUDA_R_16BF, tb ? K : N, tb ? N : K, tb ? K : N), "cublasLtMatrixLayoutCreate");
+        lt_check(cublasLtMatrixLayoutCreate(&p->a, CUDA_R_16BF, ta ? M : K, ta ? K : M, lda ? lda : ta ? M : K), "cublasLtMatrixLayoutCreate");
+        lt_check(cublasLtMatrixLayoutCreate(&p->c, f32_out ? CUDA_R_32F : CUDA_R_16BF, N, M, N), "cublasLtMatrixLayoutCreate");
+        cublasLtMatmulPreference_t pref;
+        lt_check(cublasLtMatmulPreferenceCreate(&pref), "cublasLtMatmulPreferenceCreate");
+        const uint32_t align = 16;
+        cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &space, sizeof space);
+        for (auto attr : {CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES,
+                          CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_D_BYTES})
+            cublasLtMatmulPreferenceSetAttribute(pref, attr, &align, sizeof align);
+        cublasLtMatmulHeuristicResult_t best;
+        int found = 0;
+        const cublasStatus_t st = cublasLtMatmulAlgoGetHeuristic(lt, p->op, p->b, p->a, p->c, p->c, pref, 1, &best, &found);
+        cublasLtMatmulPreferenceDestroy(pref);
+        lt_check(st == CUBLAS_STATUS_SUCCESS && !found ? CUBLAS_STATUS_NOT_SUPPORTED : st, "cublasLtMatmulAlgoGetHeuristic");
+        p->algo = best.algo; p->workspace = best.workspaceSize;
+        slot = std::move(p);
+    }
+    GemmPlan& p = *slot;
+    if (bias) lt_check(cublasLtMatmulDescSetAttribute(p.op, CUBLASLT_MATMUL_DESC_BIAS_POINTER, &bias, sizeof bias), "cublasLtMatmulDescSetAttribute");
+    const float one = 1.f, zero = 0.f;
+    lt_check(cublasLtMatmul(lt, p.op, &one, B, p.b, A, p.a, &zero, C, p.c, C, p.c, &p.algo, p.workspace ? at::cuda::getCUDABlasLtWorkspace() : nullptr,
+                            p.workspace, static_cast<cudaStream_t>(stream_of(on))), "cublasLtMatmul");
+}
+// X[M,K] . W[N,K]^T + bias -> bf16 [M,N]
+Tensor linear(const Tensor& X, const void* W, const void* bias, int64_t M, int64_t N, int64_t K) {
+    Tensor C = new_tensor({M, N}, at::kBFloat16, X);
+    gemm(ptr(C), false, ptr(X), false, W, true, bias, M, N, K, X);
+    return C;
+}
+// dY[M,N] . W[N,K] -> [M,K]
+Tensor grad_input(const Tensor& dY, const void* W, int64_t M, int64_t N, int64_t K, bool f32_out) {
+    Tensor C = new_tensor({M, K}, f32_out ? at::kFloat : at::kBFloat16, dY);
+    gemm(ptr(C), f32_out, ptr(dY), false, W, false, nullptr, M, K, N, dY);
+    return C;
+}
+// dY[M,N]^T . X[M,K] -> fp32 [N,K]
+Tensor grad_weight(const Tensor& dY, const Tensor& X, int64_t M, int64_t N, int64_t K) {
+    Tensor C = new_tensor({N, K}, at::kFloat, dY);
+    gemm(ptr(C), true, ptr(dY), true, ptr(X), false, nullptr, N, K, M, dY);
+    return C;
 }
 
-Tensor mm_f32(const Tensor& a, const Tensor& b) { return at::mm(a, b, at::kFloat); }
-
-// Column sums of bf16 matrices, returned back to back.
-std::vector<Tensor> column_sums(const std::vector<Tensor>& ms) {
+// fp32 tensors as bf16 back to back in one buffer, in one launch; at[k]: where the k-th begins (elements).
+struct Bf16Pack {
+    Tensor buf;
+    std::vector<int64_t> at;
+    const char* operator[](int k) const { return static_cast<const char*>(buf.data_ptr()) + 2 * at[k]; }
+};
+Bf16Pack cast_bf16(std::initializer_list<Tensor> src0) {
+    Bf16Pack p;
+    std::vector<Tensor> src;
     int64_t total = 0;
-    for (const Tensor& m : ms) total += m.size(1);
-    const Tensor buf = new_tensor({total}, at::kFloat, ms[0]);
-    std::vector<Tensor> out;
+    for (const Tensor& t : src0) { src.push_back(f32c(t)); p.at.push_back(total); total += t.numel(); }
+    p.buf = new_tensor({total}, at::kBFloat16, src[0]);
+    const float* sp[DSQG_CAST_MAX]; void* dp[DSQG_CAST_MAX]; long long n[DSQG_CAST_MAX];
+    for (size_t k = 0; k < src.size(); ++k) { sp[k] = fptr(src[k]); dp[k] = const_cast<char*>(p[(int)k]); n[k] = src[k].numel(); }
+    check(dsqg_cast_bf16(sp, dp, n, (int)src.size(), stream_of(p.buf)), "dsqg_cast_bf16");
+    return p;
+}
+
+// A vector or row-major matrix inside a flat buffer
+Tensor part(const Tensor& buf, at::IntArrayRef sizes, int64_t first) {
+    return sizes.size() == 1 ? at::as_strided(buf, sizes, {1}, first) : at::as_strided(buf, sizes, {sizes[1], 1}, first);
+}
+
+struct Columns { const void* p; int64_t ld; int cols; };
+// Column sums of bf16 matrices of `rows` rows, back to back.
+Tensor column_sums(std::initializer_list<Columns> ms, int64_t rows, const Tensor& on) {
+    int64_t total = 0;
+    for (const Columns& m : ms) total += m.cols;
+    Tensor buf = new_tensor({total}, at::kFloat, on);
     const void* sp[DSQG_SUM_MAX]; long long ld[DSQG_SUM_MAX]; int cols[DSQG_SUM_MAX]; float* dp[DSQG_SUM_MAX];
+    int k = 0;
     int64_t o = 0;
-    for (size_t k = 0; k < ms.size(); ++k) {
-        out.push_back(at::as_strided(buf, {ms[k].size(1)}, {1}, o));
-        sp[k] = ptr(ms[k]); ld[k] = ms[k].stride(0); cols[k] = (int)ms[k].size(1); dp[k] = fptr(out[k]);
-        o += ms[k].size(1);
+    for (const Columns& m : ms) {
+        sp[k] = m.p; ld[k] = m.ld; cols[k] = m.cols; dp[k] = fptr(buf) + o;
+        o += m.cols; ++k;
     }
-    check(dsqg_column_sums(sp, ld, cols, dp, (int)ms.size(), ms[0].size(0), stream_of(buf)), "dsqg_column_sums");
-    return out;
+    check(dsqg_column_sums(sp, ld, cols, dp, k, rows, stream_of(on)), "dsqg_column_sums");
+    return buf;
 }
 
 // [B,H,N,HD] view of columns [first, first + H*HD) of a row-major matrix of B*N rows, ld elements apart
@@ -419,7 +523,7 @@ int64_t heads_stride(const Tensor& t) {
     return ok ? ld : 0;
 }
 Tensor rows_of(const Tensor& t) {        // [B,H,N,HD] -> [B*N, H*HD] bf16
-    return t.permute({0, 2, 1, 3}).reshape({t.size(0) * t.size(2), t.size(1) * t.size(3)}).to(at::kBFloat16);
+    return t.permute({0, 2, 1, 3}).reshape({t.size(0) * t.size(2), t.size(1) * t.size(3)}).to(at::kBFloat16).contiguous();
 }
 
 // (k_delta, v_delta) of the interference block (train/train_2048_condU.py:277-295)
@@ -430,15 +534,14 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         const c10::cuda::CUDAGuard guard(x.device());
         const int64_t B = x.size(0), N = x.size(1), D = x.size(2), M = B * N;
         const Tensor xc = f32c(x), gam = f32c(gamma);
-        const std::vector<Tensor> w = cast_bf16({wg, wk, wv, bg, bk, bv});
-        const Tensor wkv = at::as_strided(w[1], {2 * D, D}, {D, 1}, w[1].storage_offset()), bkv = at::as_strided(w[4], {2 * D}, {1}, w[4].storage_offset());
+        const Bf16Pack w = cast_bf16({wg, wk, wv, bg, bk, bv});                   // wk, wv and bk, bv are one matrix and one vector
         Tensor xi = new_tensor({B, N, D}, at::kFloat, x), xib = new_tensor({M, D}, at::kBFloat16, x), stat = new_tensor({M, 2}, at::kFloat, x);
         check(dsqg_layer_norm_fwd(fptr(xc), fptr(gam), fptr(f32c(beta)), (float)eps, fptr(xi), ptr(xib), fptr(stat), M, (int)D, stream_of(x)), "dsqg_layer_norm_fwd");
-        const Tensor pool = causal_mean_run(xi, false), g = at::linear(xib, w[0], w[3]);
+        const Tensor pool = causal_mean_run(xi, false), g = linear(xib, w[0], w[3], M, D, D);
         Tensor inter = new_like(g);
         check(dsqg_gated_pool(ptr(g), fptr(pool), ptr(inter), M * D, stream_of(x)), "dsqg_gated_pool");
-        const Tensor kv = at::linear(inter, wkv, bkv);
-        ctx->save_for_backward({xc, gam, stat, xib, pool, g, inter, w[0], wkv});
+        const Tensor kv = linear(inter, w[1], w[4], M, 2 * D, D);
+        ctx->save_for_backward({xc, gam, stat, xib, pool, g, inter, w.buf});
         ctx->saved_data["x_type"] = (int64_t)x.scalar_type();
         return {heads_view(kv, B, H, N, D / H, 2 * D, 0), heads_view(kv, B, H, N, D / H, 2 * D, D)};
     }
@@ -449,63 +552,63 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
     static variable_list run(AutogradContext* ctx, const variable_list& grads) {
         const NoAutocast no_autocast;
         const variable_list s = ctx->get_saved_variables();
-        const Tensor &x = s[0], &gam = s[1], &stat = s[2], &xib = s[3], &pool = s[4], &g = s[5], &inter = s[6], &wg = s[7], &wkv = s[8];
+        const Tensor &x = s[0], &gam = s[1], &stat = s[2], &xib = s[3], &pool = s[4], &g = s[5], &inter = s[6], &w = s[7];
         const c10::cuda::CUDAGuard guard(x.device());
         const int64_t D = x.size(2), M = x.size(0) * x.size(1);
-        Tensor dkv;                                            // [M, 2 D]: what comes from the attention layer already lies like that
+        // [M, 2 D]: the gradients of an attention layer lie like that already
+        Tensor dkv;
+        const void* dp = nullptr;
+        int64_t ld = 0;
         const Tensor &dk = grads[0], &dv = grads[1];
         if (dk.defined() && dv.defined() && dk.scalar_type() == at::kBFloat16 && dv.scalar_type() == at::kBFloat16) {
-            const int64_t ld = heads_stride(dk);
-            if (ld >= 2 * D && heads_stride(dv) == ld && static_cast<char*>(dv.data_ptr()) == static_cast<char*>(dk.data_ptr()) + 2 * D)
-                dkv = at::as_strided(dk, {M, 2 * D}, {ld, 1}, dk.storage_offset());
+            ld = heads_stride(dk);
+            if (ld >= 2 * D && heads_stride(dv) == ld && static_cast<char*>(ptr(dv)) == static_cast<char*>(ptr(dk)) + 2 * D) dp = ptr(dk);
         }
-        if (!dkv.defined()) {
-            const auto part = [&](const Tensor& d) { return d.defined() ? rows_of(d) : at::zeros({M, D}, xib.options()); };
-            dkv = at::cat({part(dk), part(dv)}, 1);
+        if (!dp) {
+            const auto half = [&](const Tensor& d) { return d.defined() ? rows_of(d) : at::zeros({M, D}, xib.options()); };
+            dkv = at::cat({half(dk), half(dv)}, 1);
+            dp = ptr(dkv); ld = 2 * D;
         }
         void* stream = stream_of(x);
-        const Tensor dinter = at::mm(dkv, wkv), dwkv = mm_f32(dkv.t(), inter);
+        const char* wb = static_cast<const char*>(ptr(w));
+        Tensor dinter = new_like(inter), dwkv = new_tensor({2 * D, D}, at::kFloat, x);
+        gemm(ptr(dinter), false, dp, false, wb + 2 * D * D, false, nullptr, M, D, 2 * D, x, ld);
+        gemm(ptr(dwkv), true, dp, true, ptr(inter), false, nullptr, 2 * D, D, M, x, ld);
         Tensor dg = new_like(g), dpool = new_like(pool);
         check(dsqg_gated_pool_bwd(ptr(dinter), ptr(g), fptr(pool), ptr(dg), fptr(dpool), M * D, stream), "dsqg_gated_pool_bwd");
-        const Tensor dxi = causal_mean_run(dpool, true), dxib = at::mm(dg, wg), dwg = mm_f32(dg.t(), xib);
-        const std::vector<Tensor> db = column_sums({dg, dkv});
-        Tensor dx = new_like(x), dgb = new_tensor({2, D}, at::kFloat, x);
+        const Tensor dxi = causal_mean_run(dpool, true), dxib = grad_input(dg, wb, M, D, D, false), dwg = grad_weight(dg, xib, M, D, D);
+        const Tensor db = column_sums({{ptr(dg), D, (int)D}, {dp, ld, (int)(2 * D)}}, M, x);
+        Tensor dx = new_like(x), dgb = new_tensor({2 * D}, at::kFloat, x);
         const size_t bytes = dsqg_layer_norm_bwd_scratch_bytes(M, (int)D);
         const at::DataPtr scratch = scratch_for(bytes);
         check(dsqg_layer_norm_bwd(fptr(x), fptr(stat), fptr(gam), fptr(dxi), ptr(dxib), fptr(dx), fptr(dgb), scratch.get(), bytes, M, (int)D, stream), "dsqg_layer_norm_bwd");
-        return {like_param(dx, (at::ScalarType)ctx->saved_data["x_type"].toInt()), dgb.select(0, 0), dgb.select(0, 1), dwg, db[0],
-                dwkv.narrow(0, 0, D), db[1].narrow(0, 0, D), dwkv.narrow(0, D, D), db[1].narrow(0, D, D), Tensor(), Tensor()};
+        return {like_param(dx, (at::ScalarType)ctx->saved_data["x_type"].toInt()), part(dgb, {D}, 0), part(dgb, {D}, D), dwg, part(db, {D}, 0),
+                part(dwkv, {D, D}, 0), part(db, {D}, D), part(dwkv, {D, D}, D * D), part(db, {D}, 2 * D), Tensor(), Tensor()};
     }
 };
 
-// qkv projection -> (K/V injection) -> operator -> gate -> output projection (train/train_2048_condU.py:171-191)
+// qkv projection -> (K/V injection) -> operator -> gate -> output projection (train/train_2048_condU.py:171-191).  The gate's
+// projection is part of the qkv product (one GEMM over [q | k | v | gate] columns, one weight gradient, one input gradient).
 struct LayerNode : torch::autograd::Function<LayerNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& kd, const std::optional<Tensor>& vd, const Tensor& wqkv,
                           const Tensor& bqkv, const Tensor& wg, const Tensor& bg, const Tensor& wo, const Tensor& bo, const Tensor& pos_bias,
-                          const std::optional<Tensor>& hg, const std::optional<Tensor>& se, const Offsets* off, int64_t H) {
+                          const std::optional<Tensor>& hg, const std::optional<Tensor>& se, const Offsets* off, int64_t H, bool with_grad) {
         const NoAutocast no_autocast;
         const c10::cuda::CUDAGuard guard(x.device());
         const int64_t B = x.size(0), N = x.size(1), D = x.size(2), M = B * N;
-        std::vector<Tensor> w;
-        Tensor xb;
-        if (x.scalar_type() == at::kFloat) {
-            w = cast_bf16({wqkv, wg, wo, bqkv, bg, bo, x});
-            xb = w[6].view({M, D});
-        } else {
-            w = cast_bf16({wqkv, wg, wo, bqkv, bg, bo});
-            xb = x.reshape({M, D});
-        }
-        const Tensor qkv = at::linear(xb, w[0], w[3]);
+        const bool cast_x = x.scalar_type() == at::kFloat;
+        const Bf16Pack w = cast_x ? cast_bf16({wqkv, wg, wo, bqkv, bg, bo, x}) : cast_bf16({wqkv, wg, wo, bqkv, bg, bo});
+        const Tensor xb = cast_x ? part(w.buf, {M, D}, w.at[6]) : x.contiguous();
+        const Tensor proj = linear(xb, w[0], w[3], M, 4 * D, D);
         if (kd.has_value()) {
             Tensor k = *kd, v = *vd;
             int64_t ld = k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16 ? heads_stride(k) : 0;
-            if (!ld || heads_stride(v) != ld) { k = rows_of(k).contiguous(); v = rows_of(v).contiguous(); ld = D; }
-            check(dsqg_inject_kv(ptr(qkv), ptr(k), ptr(v), ld, M, (int)D, stream_of(x)), "dsqg_inject_kv");
+            if (!ld || heads_stride(v) != ld) { k = rows_of(k); v = rows_of(v); ld = D; }
+            check(dsqg_inject_kv(ptr(proj), 4 * D, ptr(k), ptr(v), ld, M, (int)D, stream_of(x)), "dsqg_inject_kv");
         }
-        const Tensor gate = at::linear(xb, w[1], w[4]).view({B, N, D}), qkv5 = qkv.view({B, N, 3, H, D / H});
-        PackedForward f = packed_forward(qkv5, gate, pos_bias, opt(hg), opt(se), *off);
-        const Tensor out = at::linear(f.y, w[2], w[5]);
-        ctx->save_for_backward({xb, w[0], w[1], w[2], qkv5, f.gate, f.pb, f.hg, f.se, f.y, f.lse});
+        const PackedForward f = packed_forward(proj, B, N, H, D / H, 4 * D, Tensor(), pos_bias, opt(hg), opt(se), *off, with_grad);
+        const Tensor out = linear(f.y, w[2], w[5], M, D, D).view({B, N, D});
+        ctx->save_for_backward({xb, w.buf, proj, f.pb, f.hg, f.se, f.y, f.lse, f.keep});
         ctx->saved_data["offsets"] = (int64_t)(intptr_t)off;
         ctx->saved_data["types"] = types_of(pos_bias, opt(hg), opt(se));
         ctx->saved_data["x_types"] = std::vector<int64_t>{(int64_t)x.scalar_type(), (int64_t)type_of(opt(kd)), (int64_t)type_of(opt(vd))};
@@ -519,29 +622,28 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
     static variable_list run(AutogradContext* ctx, const Tensor& dy0) {
         const NoAutocast no_autocast;
         const variable_list s = ctx->get_saved_variables();
-        const Tensor &xb = s[0], &wqkv = s[1], &wg = s[2], &wo = s[3], &qkv = s[4];
-        const PackedForward f = {s[5], s[6], s[7], s[8], s[9], s[10]};
-        const int64_t B = qkv.size(0), N = qkv.size(1), H = qkv.size(3), HD = qkv.size(4), D = H * HD, M = B * N;
+        const Tensor &xb = s[0], &w = s[1];
+        const PackedForward f = {s[2], Tensor(), s[3], s[4], s[5], s[6], s[7], s[8]};
+        const int64_t B = f.lse.size(0), H = f.lse.size(1), N = f.lse.size(2), D = f.y.size(2), M = B * N, HD = D / H;
         const c10::cuda::CUDAGuard guard(xb.device());
-        const Tensor dy = (dy0.scalar_type() == at::kBFloat16 ? dy0 : dy0.to(at::kBFloat16)).reshape({M, D}).contiguous();
-        const Tensor dyo = at::mm(dy, wo).view({B, N, D}), dwo = mm_f32(dy.t(), f.y.view({M, D}));
-        const PackedGrads g = packed_backward(qkv, f, dyo, offsets_of(ctx));
-        const Tensor dqkv = g.dqkv.view({M, 3 * D}), dgate = g.dgate.view({M, D});
-        const Tensor dwqkv = mm_f32(dqkv.t(), xb), dwg = mm_f32(dgate.t(), xb);
-        const std::vector<Tensor> db = column_sums({dqkv, dgate, dy});
+        const Tensor dy = bf16c(dy0);
+        const char* wb = static_cast<const char*>(ptr(w));
+        const Tensor dyo = grad_input(dy, wb + 2 * 4 * D * D, M, D, D, false), dwo = grad_weight(dy, f.y, M, D, D);
+        const PackedGrads g = packed_backward(f, dyo, 4 * D, offsets_of(ctx));
+        const Tensor dw = grad_weight(g.dproj, xb, M, 4 * D, D);
+        const Tensor db = column_sums({{ptr(g.dproj), 4 * D, (int)(4 * D)}, {ptr(dy), D, (int)D}}, M, xb);
         const auto xt = ctx->saved_data["x_types"].toIntVector();
         Tensor dx, dk, dv;
         if (ctx->needs_input_grad(0)) {
-            dx = mm_f32(dqkv, wqkv);
-            at::addmm_out(dx, dx, dgate, wg, at::kFloat);       // accumulates in place
-            dx = like_param(dx.view({B, N, D}), (at::ScalarType)xt[0]);
+            const auto t = (at::ScalarType)xt[0];
+            dx = like_param(grad_input(g.dproj, wb, M, 4 * D, D, t == at::kFloat).view({B, N, D}), t);
         }
         if (ctx->saved_data["inject"].toBool()) {
-            dk = like_param(heads_view(dqkv, B, H, N, HD, 3 * D, D), (at::ScalarType)xt[1]);
-            dv = like_param(heads_view(dqkv, B, H, N, HD, 3 * D, 2 * D), (at::ScalarType)xt[2]);
+            dk = like_param(heads_view(g.dproj, B, H, N, HD, 4 * D, D), (at::ScalarType)xt[1]);
+            dv = like_param(heads_view(g.dproj, B, H, N, HD, 4 * D, 2 * D), (at::ScalarType)xt[2]);
         }
-        return {dx, dk, dv, dwqkv, db[0], dwg, db[1], dwo, db[2], like_param(g.dpb, type_at(ctx, 0)), like_param(g.dhg, type_at(ctx, 1)),
-                like_param(g.dse, type_at(ctx, 2)), Tensor(), Tensor()};
+        return {dx, dk, dv, part(dw, {3 * D, D}, 0), part(db, {3 * D}, 0), part(dw, {D, D}, 3 * D * D), part(db, {D}, 3 * D), dwo, part(db, {D}, 4 * D),
+                like_param(g.dpb, type_at(ctx, 0)), like_param(g.dhg, type_at(ctx, 1)), like_param(g.dse, type_at(ctx, 2)), Tensor(), Tensor(), Tensor()};
     }
 };
 
@@ -564,7 +666,7 @@ Tensor layer(const Tensor& x, const std::optional<Tensor>& kd, const std::option
              const Tensor& bg, const Tensor& wo, const Tensor& bo, const Tensor& pb, const std::optional<Tensor>& hg, const std::optional<Tensor>& se,
              const Offsets* off, int64_t H) {
     py::gil_scoped_release no_gil;
-    return LayerNode::apply(x, kd, vd, wqkv, bqkv, wg, bg, wo, bo, pb, hg, se, off, H);
+    return LayerNode::apply(x, kd, vd, wqkv, bqkv, wg, bg, wo, bo, pb, hg, se, off, H, at::GradMode::is_enabled());
 }
 
 // ------------------------------------------------------------------------------------ decode

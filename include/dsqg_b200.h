@@ -254,13 +254,38 @@ int dsqg_gate_bwd(const void* dy, const void* y, const void* gate, const dsqg_st
  *   scratch memory; out may not alias x. */
 int dsqg_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, int reverse, void* stream);
 
+/* dsqg_fwd_strided(_se) and its backward, the gate included, as one call each with one description of the problem
+ * (the attention layer of the reference between its projections, DWARF train/train_2048_condU.py:171-191).
+ * bf16; every pointer is a DEVICE pointer except offsets.  gate has strides of its own, so that it may lie in the output
+ * of the same projection as q, k, v; the gradients are laid out like what they belong to.
+ * keep (nullable, with a gate only; dsqg_packed_keep_bytes, which is 0 where it would not pay): the forward leaves copies of
+ * q, k and v there that the backward reads faster than the strided rows; a backward given keep does not read q, k, v.  The same
+ * keep (or none) has to be given to both.  scratch: dsqg_packed_bwd_scratch_bytes. */
+typedef struct dsqg_packed {
+    const void* q; const void* k; const void* v; dsqg_strides qkv_strides;
+    const void* gate; dsqg_strides gate_strides;                              /* nullable */
+    const float* pos_bias; const float* scale_embed; const float* head_gain;  /* the last two nullable */
+    const int32_t* offsets; int J; int B; int H; int N; int D;
+    void* out; dsqg_strides out_strides; float* lse;
+    void* keep;
+} dsqg_packed;
+typedef struct dsqg_packed_grads {
+    const void* dy;                                     /* laid out like out */
+    void* dq; void* dk; void* dv; void* dgate;          /* dgate with a gate */
+    float* dpos_bias; float* dscale_embed; float* dhead_gain;
+} dsqg_packed_grads;
+size_t dsqg_packed_keep_bytes(int B, int H, int N, int D);
+int dsqg_packed_fwd(const dsqg_packed* p, void* stream);
+size_t dsqg_packed_bwd_scratch_bytes(const dsqg_packed* p);
+int dsqg_packed_bwd(const dsqg_packed* p, const dsqg_packed_grads* g, void* scratch, size_t scratch_bytes, void* stream);
+
 /* What an attention layer under bf16 autocast does between its GEMMs and the operator, one pass each (the PyTorch
  * ops around the reference's layer, DWARF train/train_2048_condU.py:171-191 and the interference block :277-295):
  *   dsqg_cast_bf16       fp32 -> bf16 for up to DSQG_CAST_MAX tensors (lengths multiples of 8) in one launch
  *   dsqg_layer_norm_fwd  y = (x - mean) * rstd * gamma + beta in fp32 and bf16; stat [rows,2] = {mean, rstd}
  *   dsqg_layer_norm_bwd  its backward for dy = dy (fp32) + dy_bf16; dgamma_dbeta [2,D]
  *   dsqg_gated_pool      out = sigmoid(g) * pool, and dsqg_gated_pool_bwd
- *   dsqg_inject_kv       key and value thirds of qkv [rows,3*D] += k_delta, v_delta (rows delta_stride elements apart)
+ *   dsqg_inject_kv       columns [D,2D) and [2D,3D) of qkv += k_delta, v_delta (rows qkv_stride / delta_stride elements apart)
  *   dsqg_column_sums     fp32 column sums of up to DSQG_SUM_MAX bf16 matrices of the same number of rows, fixed order
  * D a multiple of 8 (layer norm: at most 1024); all pointers 16-byte aligned; src, dst, n, row_stride, cols: HOST arrays. */
 #define DSQG_CAST_MAX 8
@@ -273,7 +298,7 @@ int dsqg_layer_norm_bwd(const float* x, const float* stat, const float* gamma, c
                         float* dgamma_dbeta, void* scratch, size_t scratch_bytes, long long rows, int D, void* stream);
 int dsqg_gated_pool(const void* g, const float* pool, void* out, long long n, void* stream);
 int dsqg_gated_pool_bwd(const void* dout, const void* g, const float* pool, void* dg, float* dpool, long long n, void* stream);
-int dsqg_inject_kv(void* qkv, const void* k_delta, const void* v_delta, long long delta_stride, long long rows, int D, void* stream);
+int dsqg_inject_kv(void* qkv, long long qkv_stride, const void* k_delta, const void* v_delta, long long delta_stride, long long rows, int D, void* stream);
 int dsqg_column_sums(const void* const* src, const long long* row_stride, const int* cols, float* const* dst, int count, long long rows,
                      void* stream);
 
