@@ -90,6 +90,8 @@ cudaError_t launch_ring_prefill(const void* k, const void* v, void* k_ring, void
                                 int S, int H, int N, int D, int R, int dtype, cudaStream_t s, bool interleaved = false);
 
 cudaError_t launch_ring_advance(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R, cudaStream_t s);
+cudaError_t launch_gated_mean(const float* x, const void* g, float* pool, void* inter, int B, int N, int D, cudaStream_t s);
+cudaError_t launch_gated_mean_bwd(const void* dinter, const void* g, const float* pool, void* dg, float* dx, int B, int N, int D, cudaStream_t s);
 cudaError_t launch_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, bool reverse, cudaStream_t s);
 // y and dy, gate and dgate, and dout have strides of their own
 cudaError_t launch_gate_bwd(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, void* dgate, const dsqg_strides& gs,

@@ -11,8 +11,6 @@ namespace {
 
 constexpr int kT = 256;
 
-__device__ __forceinline__ float sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-
 // ---- fp32 -> bf16 for up to kCastMax tensors in one launch
 struct CastArgs { const float* src[DSQG_CAST_MAX]; __nv_bfloat16* dst[DSQG_CAST_MAX]; long long end[DSQG_CAST_MAX]; int count; };   // end: running sum of the lengths
 
@@ -140,33 +138,6 @@ __global__ void __launch_bounds__(kT) sum_rows_kernel(const float* __restrict__ 
     }
 }
 
-// ---- inter = sigmoid(g) * pool, and its backward
-__global__ void __launch_bounds__(kT) gated_pool_kernel(const __nv_bfloat16* __restrict__ g, const float* __restrict__ pool,
-                                                        __nv_bfloat16* __restrict__ out, long long n) {
-    const long long i = ((long long)blockIdx.x * kT + threadIdx.x) * 8;
-    if (i >= n) return;
-    float x[8], p[8], o[8];
-    load8(g + i, x); load8(pool + i, p);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) o[c] = sigmoid(x[c]) * p[c];
-    store8(out + i, o);
-}
-__global__ void __launch_bounds__(kT) gated_pool_bwd_kernel(const __nv_bfloat16* __restrict__ d, const __nv_bfloat16* __restrict__ g,
-                                                            const float* __restrict__ pool, __nv_bfloat16* __restrict__ dg,
-                                                            float* __restrict__ dpool, long long n) {
-    const long long i = ((long long)blockIdx.x * kT + threadIdx.x) * 8;
-    if (i >= n) return;
-    float x[8], p[8], e[8], o[8], q[8];
-    load8(d + i, e); load8(g + i, x); load8(pool + i, p);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const float s = sigmoid(x[c]);
-        o[c] = e[c] * p[c] * s * (1.f - s);
-        q[c] = e[c] * s;
-    }
-    store8(dg + i, o); store8(dpool + i, q);
-}
-
 // ---- k += k_delta, v += v_delta on columns D .. 3 D of qkv; rows lq / ld elements apart
 __global__ void __launch_bounds__(kT) inject_kernel(__nv_bfloat16* __restrict__ qkv, long long lq, const __nv_bfloat16* __restrict__ kd,
                                                     const __nv_bfloat16* __restrict__ vd, long long ld, long long rows, int D) {
@@ -184,22 +155,23 @@ __global__ void __launch_bounds__(kT) inject_kernel(__nv_bfloat16* __restrict__ 
 }
 
 // ---- column sums of up to DSQG_SUM_MAX bf16 matrices [rows][cols] in one launch (bias gradients).  A cluster of eight blocks
-// takes 32 columns; each block adds an eighth of the rows, block 0 adds the eight results.
+// takes 64 columns (a 128-byte line of every row); each block adds an eighth of the rows, block 0 adds the eight results.
 struct SumArgs { const __nv_bfloat16* src[DSQG_SUM_MAX]; float* dst[DSQG_SUM_MAX]; long long ld[DSQG_SUM_MAX]; int slice_end[DSQG_SUM_MAX], cols[DSQG_SUM_MAX]; int count; long long rows; };
+constexpr int kSumThreads = 512, kSumCols = 64, kSumRows = kSumThreads / (kSumCols / 8);
 
-__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kT) column_sum_kernel(const SumArgs a) {
-    __shared__ float red[kT / 4][33];
-    __shared__ float total[8][32];
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSumThreads) column_sum_kernel(const SumArgs a) {
+    __shared__ float red[kSumRows][kSumCols + 1];
+    __shared__ float total[8][kSumCols];
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");      // block 0 may be written to once it has started
     int k = 0;
     while ((int)blockIdx.y >= a.slice_end[k]) ++k;
-    const int c0 = ((int)blockIdx.y - (k ? a.slice_end[k - 1] : 0)) * 32, c = threadIdx.x % 4 * 8, r = threadIdx.x / 4;
+    const int c0 = ((int)blockIdx.y - (k ? a.slice_end[k - 1] : 0)) * kSumCols, c = threadIdx.x % (kSumCols / 8) * 8, r = threadIdx.x / (kSumCols / 8);
     const long long per = (a.rows + 7) / 8, first = blockIdx.x * per, last = min(a.rows, first + per);
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (c0 + c < a.cols[k]) {
         const __nv_bfloat16* p = a.src[k] + c0 + c;
-#pragma unroll 4
-        for (long long i = first + r; i < last; i += kT / 4) {
+#pragma unroll 8
+        for (long long i = first + r; i < last; i += kSumRows) {
             float x[8];
             load8(p + i * a.ld[k], x);
 #pragma unroll
@@ -209,15 +181,15 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kT) column_sum_kerne
 #pragma unroll
     for (int e = 0; e < 8; ++e) red[r][c + e] = s[e];
     __syncthreads();
-    const int col = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int col = threadIdx.x % kSumCols, part = threadIdx.x / kSumCols;          // eight parts of eight rows
     float t = 0.f;
 #pragma unroll
-    for (int i = 0; i < kT / 4 / 8; ++i) t += red[w * (kT / 4 / 8) + i][col];
+    for (int i = 0; i < 8; ++i) t += red[part * 8 + i][col];
     __syncthreads();
-    red[w][col] = t;
+    red[part][col] = t;
     __syncthreads();
     asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-    if (w == 0) {
+    if (part == 0) {
         t = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) t += red[i][col];
@@ -227,7 +199,7 @@ __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kT) column_sum_kerne
         asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(there), "f"(t) : "memory");
     }
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (blockIdx.x == 0 && w == 0 && c0 + col < a.cols[k]) {
+    if (blockIdx.x == 0 && part == 0 && c0 + col < a.cols[k]) {
         t = 0.f;
 #pragma unroll
         for (int i = 0; i < 8; ++i) t += total[i][col];
@@ -300,22 +272,18 @@ int dsqg_layer_norm_bwd(const float* x, const float* stat, const float* gamma, c
     return status();
 }
 
-int dsqg_gated_pool(const void* g, const float* pool, void* out, long long n, void* stream) {
-    if (!g || !pool || !out) return DSQG_ERR_NULL_POINTER;
-    if (n < 8 || n % 8) return DSQG_ERR_BAD_SHAPE;
-    if (bad(g) || bad(pool) || bad(out)) return DSQG_ERR_MISALIGNED;
-    gated_pool_kernel<<<blocks_for(n / 8), kT, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(g), pool, static_cast<__nv_bfloat16*>(out), n);
-    return status();
+int dsqg_gated_mean(const float* x, const void* g, float* pool, void* inter, int B, int N, int D, void* stream) {
+    if (!x || !g || !pool || !inter) return DSQG_ERR_NULL_POINTER;
+    if (B < 1 || B > 65535 || N < 1 || D < 8 || D % 8) return DSQG_ERR_BAD_SHAPE;
+    if (bad(x) || bad(g) || bad(pool) || bad(inter)) return DSQG_ERR_MISALIGNED;
+    return launch_gated_mean(x, g, pool, inter, B, N, D, static_cast<cudaStream_t>(stream)) == cudaSuccess ? DSQG_OK : DSQG_ERR_CUDA;
 }
 
-int dsqg_gated_pool_bwd(const void* dout, const void* g, const float* pool, void* dg, float* dpool, long long n, void* stream) {
-    if (!dout || !g || !pool || !dg || !dpool) return DSQG_ERR_NULL_POINTER;
-    if (n < 8 || n % 8) return DSQG_ERR_BAD_SHAPE;
-    if (bad(dout) || bad(g) || bad(pool) || bad(dg) || bad(dpool)) return DSQG_ERR_MISALIGNED;
-    gated_pool_bwd_kernel<<<blocks_for(n / 8), kT, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(dout), static_cast<const __nv_bfloat16*>(g), pool, static_cast<__nv_bfloat16*>(dg), dpool, n);
-    return status();
+int dsqg_gated_mean_bwd(const void* dinter, const void* g, const float* pool, void* dg, float* dx, int B, int N, int D, void* stream) {
+    if (!dinter || !g || !pool || !dg || !dx) return DSQG_ERR_NULL_POINTER;
+    if (B < 1 || B > 65535 || N < 1 || D < 8 || D % 8) return DSQG_ERR_BAD_SHAPE;
+    if (bad(dinter) || bad(g) || bad(pool) || bad(dg) || bad(dx)) return DSQG_ERR_MISALIGNED;
+    return launch_gated_mean_bwd(dinter, g, pool, dg, dx, B, N, D, static_cast<cudaStream_t>(stream)) == cudaSuccess ? DSQG_OK : DSQG_ERR_CUDA;
 }
 
 int dsqg_inject_kv(void* qkv, long long qkv_stride, const void* k_delta, const void* v_delta, long long delta_stride, long long rows, int D, void* stream) {
@@ -338,10 +306,10 @@ int dsqg_column_sums(const void* const* src, const long long* row_stride, const 
         if (cols[k] < 8 || cols[k] % 8) return DSQG_ERR_BAD_SHAPE;
         if (bad(src[k]) || row_stride[k] < cols[k] || row_stride[k] % 8) return DSQG_ERR_MISALIGNED;
         a.src[k] = static_cast<const __nv_bfloat16*>(src[k]); a.dst[k] = dst[k]; a.ld[k] = row_stride[k]; a.cols[k] = cols[k];
-        a.slice_end[k] = slices += (cols[k] + 31) / 32;
+        a.slice_end[k] = slices += (cols[k] + kSumCols - 1) / kSumCols;
     }
     if (slices > 65535) return DSQG_ERR_BAD_SHAPE;
-    column_sum_kernel<<<dim3(8, slices), kT, 0, static_cast<cudaStream_t>(stream)>>>(a);
+    column_sum_kernel<<<dim3(8, slices), kSumThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
     return status();
 }
 

@@ -41,10 +41,26 @@ template <> struct Piece<float> {
     static __device__ __forceinline__ void store(float* p, const float (&x)[4]) { *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]); }
 };
 
+// The gate of the interference block around the mean (train/train_2048_condU.py:289-293, fp32 mean of bf16-gated channels), so
+// that its products cost no pass of their own.  Forward: inter = sigmoid(g) * mean.  Backward (REVERSE): the summands are
+// dpool = d * sigmoid(g), and dg = d * pool * s (1 - s) is written on the way (d: gradient of inter).
+struct PoolGate {
+    const __nv_bfloat16* g; const __nv_bfloat16* d; const float* pool; __nv_bfloat16* out;       // out: inter / dg
+};
+__device__ __forceinline__ float pool_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+__device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&x)[4]) {
+    const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+    x[0] = __uint_as_float(u.x << 16); x[1] = __uint_as_float(u.x & 0xffff0000u);
+    x[2] = __uint_as_float(u.y << 16); x[3] = __uint_as_float(u.y & 0xffff0000u);
+}
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&x)[4]) {
+    *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(x[0], x[1]), pack_bf16x2(x[2], x[3]));
+}
+
 // R > 0: the thread's rows (len <= R) stay in registers; R == 0: any len, read twice.
-template <typename T, bool REVERSE, int R>
+template <typename T, bool REVERSE, int R, bool GATED = false>
 __global__ void __launch_bounds__(kScanThreads)
-causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, int len) {
+causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, int len, const PoolGate gate) {
     constexpr int C = Piece<T>::C, kSlice = C * kGroups;
     __shared__ __align__(16) float warp_sum[kScanThreads / 32][kSlice];
     __shared__ __align__(16) float block_sum[kScanCluster][kSlice];
@@ -60,6 +76,25 @@ causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, i
     auto row = [&](int i) { return REVERSE ? N - 1 - first - i : first + i; };
     float s[C] = {};
     Piece<T> keep[R > 0 ? R : 1];
+    auto load = [&](Piece<T>& v, int i, bool first_pass) {
+        const size_t o = base + (size_t)row(i) * D;
+        if constexpr (GATED && REVERSE) {
+            float g[4], d[4], p[4], w[4];
+            load4(gate.g + o, g); load4(gate.d + o, d);
+            const float4 pl = __ldg(reinterpret_cast<const float4*>(gate.pool + o));
+            p[0] = pl.x; p[1] = pl.y; p[2] = pl.z; p[3] = pl.w;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float sg = pool_sigmoid(g[c]);
+                w[c] = d[c] * p[c] * sg * (1.f - sg);
+                d[c] *= sg;
+            }
+            if (first_pass) store4(gate.out + o, w);
+            v.a = make_float4(d[0], d[1], d[2], d[3]);
+        } else {
+            v.load(x + o);
+        }
+    };
     auto add = [&](const Piece<T>& v, int i) {
         float f[C];
         v.get(f);
@@ -70,13 +105,13 @@ causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, i
     if constexpr (R > 0) {
 #pragma unroll
         for (int i = 0; i < R; ++i)
-            if (i < mine) keep[i].load(x + base + (size_t)row(i) * D);
+            if (i < mine) load(keep[i], i, true);
 #pragma unroll
         for (int i = 0; i < R; ++i)
             if (i < mine) add(keep[i], i);
     } else {
 #pragma unroll 4
-        for (int i = 0; i < mine; ++i) { keep[0].load(x + base + (size_t)row(i) * D); add(keep[0], i); }
+        for (int i = 0; i < mine; ++i) { load(keep[0], i, true); add(keep[0], i); }
     }
     // exclusive sum over the threads before this one
     float inc[C];
@@ -125,6 +160,13 @@ causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, i
             o[c] = REVERSE ? s[c] : s[c] * w;
         }
         Piece<T>::store(out + base + (size_t)row(i) * D, o);
+        if constexpr (GATED && !REVERSE) {
+            float g[4];
+            load4(gate.g + base + (size_t)row(i) * D, g);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) g[c] = pool_sigmoid(g[c]) * o[c];
+            store4(gate.out + base + (size_t)row(i) * D, g);
+        }
     };
     if constexpr (R > 0) {
 #pragma unroll
@@ -132,34 +174,42 @@ causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, i
             if (i < mine) put(keep[i], i);
     } else {
 #pragma unroll 4
-        for (int i = 0; i < mine; ++i) { keep[0].load(x + base + (size_t)row(i) * D); put(keep[0], i); }
+        for (int i = 0; i < mine; ++i) { load(keep[0], i, false); put(keep[0], i); }
     }
 }
 
-template <typename T, bool REVERSE, int R>
-cudaError_t launch_scan(const T* x, T* out, int B, int N, int D, int ranks, cudaStream_t s) {
+template <typename T, bool REVERSE, bool GATED, int R>
+cudaError_t launch_scan(const T* x, T* out, int B, int N, int D, int ranks, const PoolGate& gate, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ranks, (D / Piece<T>::C + kGroups - 1) / kGroups, B); cfg.blockDim = dim3(kScanThreads); cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = ranks; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, causal_mean_kernel<T, REVERSE, R>, x, out, N, D, (N + ranks * kRowThreads - 1) / (ranks * kRowThreads));
+    return cudaLaunchKernelEx(&cfg, causal_mean_kernel<T, REVERSE, R, GATED>, x, out, N, D, (N + ranks * kRowThreads - 1) / (ranks * kRowThreads), gate);
 }
 
-template <typename T, bool REVERSE>
-cudaError_t launch_mean(const T* x, T* out, int B, int N, int D, cudaStream_t s) {
+template <typename T, bool REVERSE, bool GATED = false>
+cudaError_t launch_mean(const T* x, T* out, int B, int N, int D, cudaStream_t s, const PoolGate& gate = {}) {
     // as many blocks as give every thread two rows at least, eight at most
     int ranks = 1;
     while (ranks < kScanCluster && N > ranks * kRowThreads * 2) ranks *= 2;
     const int len = (N + ranks * kRowThreads - 1) / (ranks * kRowThreads);
-    if (len <= 2) return launch_scan<T, REVERSE, 2>(x, out, B, N, D, ranks, s);
-    if (len <= 8) return launch_scan<T, REVERSE, 8>(x, out, B, N, D, ranks, s);
-    if (len <= 16) return launch_scan<T, REVERSE, 16>(x, out, B, N, D, ranks, s);
-    return launch_scan<T, REVERSE, 0>(x, out, B, N, D, ranks, s);
+    if (len <= 2) return launch_scan<T, REVERSE, GATED, 2>(x, out, B, N, D, ranks, gate, s);
+    if (len <= 8) return launch_scan<T, REVERSE, GATED, 8>(x, out, B, N, D, ranks, gate, s);
+    if (len <= 16) return launch_scan<T, REVERSE, GATED, 16>(x, out, B, N, D, ranks, gate, s);
+    return launch_scan<T, REVERSE, GATED, 0>(x, out, B, N, D, ranks, gate, s);
 }
 
 }  // namespace
+
+cudaError_t launch_gated_mean(const float* x, const void* g, float* pool, void* inter, int B, int N, int D, cudaStream_t s) {
+    return launch_mean<float, false, true>(x, pool, B, N, D, s, {static_cast<const __nv_bfloat16*>(g), nullptr, nullptr, static_cast<__nv_bfloat16*>(inter)});
+}
+cudaError_t launch_gated_mean_bwd(const void* dinter, const void* g, const float* pool, void* dg, float* dx, int B, int N, int D, cudaStream_t s) {
+    return launch_mean<float, true, true>(nullptr, dx, B, N, D, s, {static_cast<const __nv_bfloat16*>(g), static_cast<const __nv_bfloat16*>(dinter), pool,
+                                                                    static_cast<__nv_bfloat16*>(dg)});
+}
 
 cudaError_t launch_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, bool reverse, cudaStream_t s) {
     if (dtype == DSQG_DTYPE_BF16) {

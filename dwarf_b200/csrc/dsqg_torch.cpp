@@ -99,11 +99,10 @@ void* stream_of(const Tensor& t) { return at::cuda::getCurrentCUDAStream(t.devic
 Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType dt, const Tensor& on) { return at::detail::empty_cuda(sizes, dt, on.device(), std::nullopt); }
 Tensor new_like(const Tensor& t) { return t.defined() ? new_tensor(t.sizes(), t.scalar_type(), t) : t; }
 
-// A parameter as the kernels read it: fp32, contiguous, detached.
+// A parameter as the kernels read it: fp32 and contiguous (no copy where it is so already; it may be the caller's own tensor).
 Tensor f32c(const Tensor& t) {
-    if (!t.defined()) return t;
-    const Tensor d = t.requires_grad() ? t.detach() : t;
-    return (d.scalar_type() == at::kFloat ? d : d.to(at::kFloat)).contiguous();
+    if (!t.defined() || (t.scalar_type() == at::kFloat && t.is_contiguous())) return t;
+    return t.detach().to(at::kFloat).contiguous();
 }
 Tensor like_param(Tensor g, at::ScalarType dt) { return g.defined() && g.scalar_type() != dt ? g.to(dt) : g; }
 Tensor opt(const std::optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); }
@@ -489,9 +488,12 @@ Bf16Pack cast_bf16(std::initializer_list<Tensor> src0) {
     return p;
 }
 
-// A vector or row-major matrix inside a flat buffer
+// A vector or row-major matrix inside a flat buffer (a tensor on the same storage; a dispatched at::as_strided costs three times as much)
 Tensor part(const Tensor& buf, at::IntArrayRef sizes, int64_t first) {
-    return sizes.size() == 1 ? at::as_strided(buf, sizes, {1}, first) : at::as_strided(buf, sizes, {sizes[1], 1}, first);
+    Tensor t = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(buf.storage()), buf.key_set(), buf.dtype());
+    t.unsafeGetTensorImpl()->set_storage_offset(buf.storage_offset() + first);
+    t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+    return t;
 }
 
 struct Columns { const void* p; int64_t ld; int cols; };
@@ -537,9 +539,9 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         const Bf16Pack w = cast_bf16({wg, wk, wv, bg, bk, bv});                   // wk, wv and bk, bv are one matrix and one vector
         Tensor xi = new_tensor({B, N, D}, at::kFloat, x), xib = new_tensor({M, D}, at::kBFloat16, x), stat = new_tensor({M, 2}, at::kFloat, x);
         check(dsqg_layer_norm_fwd(fptr(xc), fptr(gam), fptr(f32c(beta)), (float)eps, fptr(xi), ptr(xib), fptr(stat), M, (int)D, stream_of(x)), "dsqg_layer_norm_fwd");
-        const Tensor pool = causal_mean_run(xi, false), g = linear(xib, w[0], w[3], M, D, D);
-        Tensor inter = new_like(g);
-        check(dsqg_gated_pool(ptr(g), fptr(pool), ptr(inter), M * D, stream_of(x)), "dsqg_gated_pool");
+        const Tensor g = linear(xib, w[0], w[3], M, D, D);
+        Tensor pool = new_like(xi), inter = new_like(g);
+        check(dsqg_gated_mean(fptr(xi), ptr(g), fptr(pool), ptr(inter), (int)B, (int)N, (int)D, stream_of(x)), "dsqg_gated_mean");
         const Tensor kv = linear(inter, w[1], w[4], M, 2 * D, D);
         ctx->save_for_backward({xc, gam, stat, xib, pool, g, inter, w.buf});
         ctx->saved_data["x_type"] = (int64_t)x.scalar_type();
@@ -574,9 +576,9 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         Tensor dinter = new_like(inter), dwkv = new_tensor({2 * D, D}, at::kFloat, x);
         gemm(ptr(dinter), false, dp, false, wb + 2 * D * D, false, nullptr, M, D, 2 * D, x, ld);
         gemm(ptr(dwkv), true, dp, true, ptr(inter), false, nullptr, 2 * D, D, M, x, ld);
-        Tensor dg = new_like(g), dpool = new_like(pool);
-        check(dsqg_gated_pool_bwd(ptr(dinter), ptr(g), fptr(pool), ptr(dg), fptr(dpool), M * D, stream), "dsqg_gated_pool_bwd");
-        const Tensor dxi = causal_mean_run(dpool, true), dxib = grad_input(dg, wb, M, D, D, false), dwg = grad_weight(dg, xib, M, D, D);
+        Tensor dg = new_like(g), dxi = new_like(pool);
+        check(dsqg_gated_mean_bwd(ptr(dinter), ptr(g), fptr(pool), ptr(dg), fptr(dxi), (int)x.size(0), (int)x.size(1), (int)D, stream), "dsqg_gated_mean_bwd");
+        const Tensor dxib = grad_input(dg, wb, M, D, D, false), dwg = grad_weight(dg, xib, M, D, D);
         const Tensor db = column_sums({{ptr(dg), D, (int)D}, {dp, ld, (int)(2 * D)}}, M, x);
         Tensor dx = new_like(x), dgb = new_tensor({2 * D}, at::kFloat, x);
         const size_t bytes = dsqg_layer_norm_bwd_scratch_bytes(M, (int)D);
