@@ -208,13 +208,15 @@ decode_1pass_kernel(const DecodeArgs a, const Taps t) {
     // ---- request every row of the step
     Raw8<T> vraw[VREG > 0 ? VREG : 1];
     const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
+    unsigned exists = 0;              // bit r: this lane group's tap of round r exists
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
         const int j = r * GROUPS + g;
         const int delta = j < t.J ? t.delta(j) : 0;
         int slot = head - delta;
         if (slot < 0) slot += a.R;
-        const bool on = j < t.J && delta < fill && active;
+        if (j < t.J && delta < fill) exists |= 1u << r;
+        const bool on = (exists >> r & 1) && active;
         if (PDL && j == 0 && delta == 0) continue;       // the new token itself: after the wait
         // the tap with delta == 0 reads k_new / v_new, so nothing waits for the ring store below
         const T* ksrc = delta == 0 ? kn + d0 : kr + (size_t)slot * RS + d0;
@@ -242,25 +244,68 @@ decode_1pass_kernel(const DecodeArgs a, const Taps t) {
     }
     float qx[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (active) load8(static_cast<const T*>(a.q) + (size_t)sh * D + d0, qx);
+    float sc[ROUNDS];                 // position bias of this lane group's taps, -inf where there is none; then the scores
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+        sc[r] = exists >> r & 1 ? __ldg(a.pos_bias + (r * GROUPS + g) * a.H + h) : -INFINITY;
+    }
     if (g == 0 && active) {          // store the new token in the ring
         *reinterpret_cast<uint4*>(kr + (size_t)head * RS + d0) = *reinterpret_cast<const uint4*>(kn + d0);
         *reinterpret_cast<uint4*>(vr + (size_t)head * RS + d0) = *reinterpret_cast<const uint4*>(vn + d0);
     }
     cp_async_wait_all();
 
-    // ---- scores and online softmax over this lane group's taps
-    TapState st;
+    // ---- softmax over all taps at once.  Everything from here on is the serial part of a step that no other block of the launch
+    // hides (one wave), so the scores of all rounds advance together: one dependent chain of shuffles and one exponential
+    // per step instead of one per tap, and the lane groups agree on the maximum first, so that sums and outputs only add up.
+    float dot[ROUNDS];
 #pragma unroll
     for (int r = 0; r < ROUNDS; ++r) {
-        const int j = r * GROUPS + g;
-        const bool valid = j < t.J && t.delta(j < t.J ? j : 0) < fill;
-        float kx[8], vx[8];
+        float kx[8];
         Raw8<T> kk; kk.u = k_sm[warp][r][lane]; kk.get(kx);
+        if (a.scale_embed != nullptr && r * GROUPS + g < t.J && active) {
+            float se[8];
+            load8(a.scale_embed + (size_t)(r * GROUPS + g) * D + d0, se);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) kx[i] += se[i];
+        }
+        dot[r] = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dot[r] = fmaf(qx[i], kx[i], dot[r]);
+    }
+#pragma unroll
+    for (int o = TPR / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < ROUNDS; ++r) dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], o);
+    float m = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) { sc[r] = fmaf(dot[r], a.scale, sc[r]); m = fmaxf(m, sc[r]); }
+#pragma unroll
+    for (int o = TPR; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float ms = m == -INFINITY ? 0.f : m;
+    float l = 0.f, acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+        const float p = __expf(sc[r] - ms);
+        float vx[8];
         if (r < VSM) { Raw8<T> vv; vv.u = v_sm[warp][r][lane]; vv.get(vx); }
         else vraw[r - VSM].get(vx);
-        fold_tap<TPR>(st, a, j, h, d0, valid, active, qx, kx, vx);
+        l += p;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = fmaf(p, vx[i], acc[i]);
     }
-    merge_and_store<T, TPR>(st, a, sh, h, d0, g == 0 && active);
+#pragma unroll
+    for (int o = TPR; o < 32; o <<= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+    }
+    if (g == 0 && active) {
+        const float inv = l > 0.f ? (a.head_gain ? a.head_gain[h] : 1.f) / l : 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] *= inv;
+        store8(static_cast<T*>(a.out) + (size_t)sh * D + d0, acc);
+    }
 }
 
 template <int TPR, int ROUNDS, int VSM, int CTAS>
@@ -291,12 +336,13 @@ template <typename T, int TPR>
 cudaError_t decode_launch(const DecodeArgs& a, const Taps& t, cudaStream_t s, bool overlap) {
     const int rounds = (t.J + 32 / TPR - 1) / (32 / TPR);
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-        // bf16 rings, up to 12 rounds: single-pass kernel.  K rows plus four rounds of V rows in
-        // shared memory leave 80 registers (6 CTAs per SM); measured 9.95 us per launch on the
-        // benchmark shape against 14.4 us for two register passes, 15.1 us with all of V in
-        // registers (5 CTAs per SM) and 15.7 us with all of V in shared memory (4 CTAs per SM).
+        // bf16 rings, up to 12 rounds: single-pass kernel.  K rows and seven rounds of V rows in shared memory leave 80
+        // registers, six CTAs per SM: every warp of the benchmark shape (256 sequences, 12 heads of 64, 43 taps) is resident at once.
+        // Ten overlapped layers of it: 86 us (88 with five rounds of V, 97 with one round more than 43 taps need; 116 with
+        // five CTAs; 115 with the online softmax, one tap after the other, that this kernel had before).
         if (rounds <= 6) return decode_launch_1pass<TPR, 6, 0, 24 / kWarpsPerBlock>(a, t, s, overlap);
-        if (rounds <= 12) return decode_launch_1pass<TPR, 12, 4, 24 / kWarpsPerBlock>(a, t, s, overlap);
+        if (rounds <= 11) return decode_launch_1pass<TPR, 11, 7, 24 / kWarpsPerBlock>(a, t, s, overlap);
+        if (rounds <= 12) return decode_launch_1pass<TPR, 12, 6, 24 / kWarpsPerBlock>(a, t, s, overlap);
     }
     // Other cases (fp32 rings, more than 12 rounds): register passes of 6 rounds (96 registers),
     // launched as an ordinary kernel (the overlapped form is a hint, not a requirement).
