@@ -90,6 +90,110 @@ __device__ __forceinline__ void build_qs_tile(const SeTables& se, const RowFrag<
     __syncwarp();
 }
 
+// Scale embedding: s_j += q.scale_embed[j] / sqrt(D) (reference: kernels/dsqg_attention_v3.py:112-118).  q.scale_embed is formed
+// per 16-row tile with MMAs, in the order the scores need it: column x = WB + 16 - delta for the dense offsets (as StartTable), then
+// the sparse taps.  Row i of a tile reads its start values at x = 16 - i + c, pairs of them 8-byte aligned (the row
+// pitch is odd and 9 mod 32: no bank conflicts), at compile-time distances from one address per lane.  The earlier tiles in tap
+// order were gathered through a table of offsets: an index load, four address computations and four loads per n-tile.
+//   hi + lo: bf16 halves of the table rows (their sum carries 16 mantissa bits), kDense rows for x = 16 .. WB + 23, then
+//   the sparse taps rounded up to eight; pb: pos_bias / scale per row, the mask value where the row is no tap.
+template <int WB> struct SeGeo {
+    static constexpr int kC = WB + 16, kTiles = WB / 8 + 1, kDense = 8 * kTiles, kPitch = WB == 32 ? 73 : 105;
+    static __host__ __device__ int rows(int ns) { return kDense + (ns + 7) / 8 * 8; }
+    static __host__ __device__ int sparse_pitch(int ns) { return (ns + 7) / 8 * 8 + 1; }
+    // tap of table row r, -1: none
+    static __device__ __forceinline__ int tap(const Taps& t, int r) {
+        const int j = r < kDense ? WB - r - t.d_lo : t.n_dense + r - kDense;
+        return r < kDense ? (j >= 0 && j < t.n_dense ? j : -1) : (j < t.J ? j : -1);
+    }
+};
+struct SeRows { const __nv_bfloat16* hi; const __nv_bfloat16* lo; const float* pb; };
+
+// The tile of 16 query rows (A fragments qa: rows g, qb: rows g + 8): dense part to dense[row * pitch + x], sparse part to
+// sparse[row * sp + tap], and to rows_lo / rows_hi (nullable, global memory).  GL: the table is in global memory.
+template <int D, int WB, bool GL>
+__device__ __forceinline__ void build_se_tile(const SeRows& tab, int ns, const RowFrag<D>& qa, const RowFrag<D>& qb, int g, int tig, float* dense,
+                                              int pitch, float* sparse, int sp, float* rows_lo = nullptr, float* rows_hi = nullptr) {
+    using G = SeGeo<WB>;
+    auto product = [&](int m, float (&c)[4]) {
+        const float2* pbp = reinterpret_cast<const float2*>(tab.pb + 8 * m + 2 * tig);
+        const float2 pb = GL ? __ldg(pbp) : *pbp;
+        c[0] = c[2] = pb.x; c[1] = c[3] = pb.y;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            RowFrag<D> sf;
+            const uint4* src = reinterpret_cast<const uint4*>((half ? tab.lo : tab.hi) + (8 * m + g) * D + kLane<D> * tig);
+#pragma unroll
+            for (int cc = 0; cc < D / 32; ++cc) {
+                const int o = kLane<D> == 16 ? 8 * (cc >> 1) + (cc & 1) : 4 * cc;
+                const uint4 u = GL ? __ldg(src + o) : src[o];
+                sf.r[4 * cc + 0] = u.x; sf.r[4 * cc + 1] = u.y; sf.r[4 * cc + 2] = u.z; sf.r[4 * cc + 3] = u.w;
+            }
+            mma_rows(c, qa, qb, sf);
+        }
+    };
+    float* at = dense + g * pitch + 16 + 2 * tig;
+#pragma unroll
+    for (int m = 0; m < G::kTiles; ++m) {
+        float c[4];
+        product(m, c);
+        at[8 * m] = c[0]; at[8 * m + 1] = c[1];
+        at[8 * pitch + 8 * m] = c[2]; at[8 * pitch + 8 * m + 1] = c[3];
+    }
+    at = sparse + g * sp + 2 * tig;
+#pragma unroll 1
+    for (int m = 0; 8 * m < ns; ++m) {
+        float c[4];
+        product(G::kTiles + m, c);
+        at[8 * m] = c[0]; at[8 * m + 1] = c[1];
+        at[8 * sp + 8 * m] = c[2]; at[8 * sp + 8 * m + 1] = c[3];
+        if (rows_lo) *reinterpret_cast<float2*>(rows_lo + 8 * m + 2 * tig) = make_float2(c[0], c[1]);
+        if (rows_hi) *reinterpret_cast<float2*>(rows_hi + 8 * m + 2 * tig) = make_float2(c[2], c[3]);
+    }
+    __syncwarp();
+}
+// Start values of n-tile nt; lane: dense + g * pitch + 16 - g + 2 tig.  Columns below x = 16 and from WB + 24 on are not in the tile:
+// they belong to no offset.
+template <int WB>
+__device__ __forceinline__ void se_start(float (&s)[4], const float* lane, int pitch, int nt, int g, int tig) {
+    const int c = 2 * tig;
+    const float2 lo = *reinterpret_cast<const float2*>(lane + 8 * nt);
+    s[0] = lo.x; s[1] = lo.y; s[2] = s[3] = kNeg;
+    if (nt > 0) {
+        const float2 hi = *reinterpret_cast<const float2*>(lane + 8 * (pitch - 1) + 8 * nt);
+        s[2] = hi.x; s[3] = hi.y;
+    }
+    if (nt == 0) { if (c < g) s[0] = kNeg; if (c + 1 < g) s[1] = kNeg; }
+    if (nt == 1) { if (c < g) s[2] = kNeg; if (c + 1 < g) s[3] = kNeg; }
+    if (nt == WB / 8 + 1) { if (c >= g) s[0] = kNeg; if (c + 1 >= g) s[1] = kNeg; }
+}
+
+// The table in shared memory (all threads of the CTA; the caller syncs): hi | lo | pb, then what follows it.
+template <int D, int WB, int THREADS>
+__device__ __forceinline__ SeRows fill_se_rows(float* smem, const float* scale_embed, const float* pos_bias, const Taps& t, int H, int h, float scale) {
+    const int R = SeGeo<WB>::rows(t.n_sparse);
+    __nv_bfloat16* hi = reinterpret_cast<__nv_bfloat16*>(smem);
+    __nv_bfloat16* lo = hi + R * D;
+    float* pb = reinterpret_cast<float*>(lo + R * D);
+    for (int e = threadIdx.x; e < R * (D / 4); e += THREADS) {
+        const int j = SeGeo<WB>::tap(t, e / (D / 4));
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j >= 0) x = __ldg(reinterpret_cast<const float4*>(scale_embed + j * D) + e % (D / 4));
+        const __nv_bfloat162 a = __floats2bfloat162_rn(x.x, x.y), b = __floats2bfloat162_rn(x.z, x.w);
+        reinterpret_cast<uint2*>(hi)[e] = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        reinterpret_cast<uint2*>(lo)[e] = make_uint2(pack_bf16x2(x.x - __low2float(a), x.y - __high2float(a)),
+                                                     pack_bf16x2(x.z - __low2float(b), x.w - __high2float(b)));
+    }
+    const float inv_scale = 1.f / scale;
+    for (int r = threadIdx.x; r < R; r += THREADS) {
+        const int j = SeGeo<WB>::tap(t, r);
+        pb[r] = j >= 0 ? pos_bias[j * H + h] * inv_scale : kNeg;
+    }
+    return {hi, lo, pb};
+}
+template <int WB> __host__ __device__ inline size_t se_rows_bytes(int ns, int D) { return (size_t)SeGeo<WB>::rows(ns) * (4 * D + 4); }
+template <int WB> __host__ __device__ inline size_t se_tile_floats(int ns) { return (size_t)16 * (SeGeo<WB>::kPitch + SeGeo<WB>::sparse_pitch(ns)); }
+
 // Start values of the score accumulators of the dense window.  Element (i, c) of a tile belongs to one offset
 // (forward, dQ: WB + i - c; dK/dV: c - i), so the tile's values are a table over x = 16 - i + c, and the two
 // columns of an accumulator pair are neighbours in it.  A second copy an odd distance away keeps the pair 8-byte
@@ -118,7 +222,12 @@ template <int WB> struct StartTable {
 
 template <int D, int WB, bool INTERIOR, int kTapGroup, bool SE, int ST>
 __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, const int2* tap_s, int ns,
-                                         int bh, int h, int g0, const Lane& L, const SeTables& se) {
+                                         int bh, int h, int g0, const Lane& L, const SeRows& se, float* se_tile) {
+    // scale_embed: the warp's tile, dense part first; qs0 / qs1: sparse entries of rows g / g + 8
+    const int sp = SE ? SeGeo<WB>::sparse_pitch(ns) : 0;
+    float* se_sparse = se_tile + 16 * SeGeo<WB>::kPitch;
+    const float* qs0 = se_sparse + L.g * sp;
+    const float* qs1 = qs0 + 8 * sp;
     constexpr int NT = (WB + 16) / 8;
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = g0 + g, row_hi = row_lo + 8;
@@ -143,15 +252,15 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             store_row_at<D, true>(f.r, static_cast<__nv_bfloat16*>(a.keep) + (((size_t)x * a.B * a.H + bh) * N + row) * D + kLane<D> * tig);
     };
     keep(0, qa, row_lo, ok_lo); keep(0, qb, row_hi, ok_hi);
-    if constexpr (SE) build_qs_tile<D, false>(se, qa, qb, g, tig);
+    if constexpr (SE) build_se_tile<D, WB, false>(se, ns, qa, qb, g, tig, se_tile, SeGeo<WB>::kPitch, se_sparse, sp);
+    const float* se_lane = se_tile + g * (SeGeo<WB>::kPitch - 1) + 16 + 2 * tig;
 
     // ---- dense window: key row of n-tile nt for this thread is kb0 + 8 nt + g = row_lo - WB + 8 nt
     float S[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
         if constexpr (SE) {
-            const int4 qo = se.off[nt * 32 + L.lane];
-            S[nt][0] = se.qs[qo.x]; S[nt][1] = se.qs[qo.y]; S[nt][2] = se.qs[qo.z]; S[nt][3] = se.qs[qo.w];
+            se_start<WB>(S[nt], se_lane, SeGeo<WB>::kPitch, nt, g, tig);
         } else {
             StartTable<WB>::get(S[nt], start, nt);
         }
@@ -261,8 +370,8 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             mma_rows_z(s1, qa, qb, kf1[i]);
             const float d0 = (g & 1) ? s0[1] : s0[0], d1 = (g & 1) ? s1[3] : s1[2];
             if constexpr (SE) {
-                x0[i] = (d0 + se.qs[g * se.pitch + se.nd + si + i]) * c2;
-                x1[i] = (d1 + se.qs[(g + 8) * se.pitch + se.nd + si + i]) * c2;
+                x0[i] = (d0 + qs0[si + i]) * c2;
+                x1[i] = (d1 + qs1[si + i]) * c2;
             } else {
                 x0[i] = fmaf(d0, c2, pbv[i]);
                 x1[i] = fmaf(d1, c2, pbv[i]);
@@ -301,8 +410,8 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             mma_rows_z(s0, qa, qb, kf0);
             mma_rows_z(s1, qa, qb, kf1);
             const float d0 = (g & 1) ? s0[1] : s0[0], d1 = (g & 1) ? s1[3] : s1[2];
-            const float y0 = SE ? (d0 + se.qs[g * se.pitch + se.nd + si]) * c2 : fmaf(d0, c2, pbv);
-            const float y1 = SE ? (d1 + se.qs[(g + 8) * se.pitch + se.nd + si]) * c2 : fmaf(d1, c2, pbv);
+            const float y0 = SE ? (d0 + qs0[si]) * c2 : fmaf(d0, c2, pbv);
+            const float y1 = SE ? (d1 + qs1[si]) * c2 : fmaf(d1, c2, pbv);
             const float x0[1] = {v0 ? y0 : kNeg};
             const float x1[1] = {v1 ? y1 : kNeg};
             fold(std::integral_constant<int, 1>(), x0, x1, vf0, vf1);
@@ -332,68 +441,19 @@ template <int D> struct FwdTune {
     static constexpr int group_se = D <= 64 ? 2 : 1, ctas_se = D == 32 ? 5 : 4;       // with scale_embed
 };
 
-// Fills the shared tables of the scale_embed variants (all threads of the CTA; the caller syncs).
-// smem layout: se_hi [Jp][D] bf16 | se_lo [Jp][D] bf16 | pbs [Jp] f32 | off [NT*32] int4 | qs [warps][16*pitch+4] f32
-template <int D, int WB, int W>
-__device__ __forceinline__ SeTables fill_se_tables(unsigned char* smem, const float* scale_embed, const float* pos_bias,
-                                                   const Taps& t, int H, int h, float scale, int warp, bool transposed) {
-    constexpr int NT = (WB + 16) / 8;
-    const int J = t.J, Jp = (J + 7) / 8 * 8, pitch = Jp + 2;
-    __nv_bfloat16* se_hi = reinterpret_cast<__nv_bfloat16*>(smem);
-    __nv_bfloat16* se_lo = se_hi + Jp * D;
-    float* pbs = reinterpret_cast<float*>(se_lo + Jp * D);
-    int4* off = reinterpret_cast<int4*>(pbs + Jp);
-    float* qs = reinterpret_cast<float*>(off + NT * 32);
-    for (int e = threadIdx.x; e < Jp * D / 2; e += W * 32) {
-        const int j = (2 * e) / D;
-        float2 x = make_float2(0.f, 0.f);
-        if (j < J) x = *reinterpret_cast<const float2*>(scale_embed + 2 * e);
-        const __nv_bfloat162 hi = __floats2bfloat162_rn(x.x, x.y);
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(x.x - __low2float(hi), x.y - __high2float(hi));
-        reinterpret_cast<__nv_bfloat162*>(se_hi)[e] = hi;
-        reinterpret_cast<__nv_bfloat162*>(se_lo)[e] = lo;
-    }
-    const float inv_scale = 1.f / scale;
-    for (int j = threadIdx.x; j < Jp; j += W * 32) pbs[j] = j < J ? pos_bias[j * H + h] * inv_scale : 0.f;
-    const int d_lo = t.d_lo, d_hi = t.d_lo + t.n_dense - 1;
-    for (int e = threadIdx.x; e < NT * 32; e += W * 32) {
-        const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
-        int o[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int i = gg + 8 * (r >> 1), cc = 8 * nt + 2 * tt + (r & 1);
-            // forward / dQ: rows are queries, columns keys (delta = WB + i - cc); dK/dV: rows keys, columns queries
-            const int delta = transposed ? cc - i : WB + i - cc;
-            const int row = transposed ? cc : i;          // tile row = query index inside the tile
-            o[r] = (delta >= d_lo && delta <= d_hi) ? row * pitch + (delta - d_lo) : 16 * pitch;
-        }
-        off[e] = make_int4(o[0], o[1], o[2], o[3]);
-    }
-    float* qs_w = qs + warp * (16 * pitch + 4);
-    if ((threadIdx.x & 31) == 0) qs_w[16 * pitch] = kNeg;      // the dump entry: masked
-    SeTables s;
-    s.se_hi = se_hi; s.se_lo = se_lo; s.pbs = pbs; s.off = off; s.qs = qs_w;
-    s.Jp = Jp; s.pitch = pitch; s.nd = t.n_dense;
-    return s;
-}
-__host__ __device__ inline size_t se_tables_bytes(int J, int D, int NT, int warps, int tile_rows) {
-    const int Jp = (J + 7) / 8 * 8;
-    return (size_t)2 * Jp * D * 2 + (size_t)Jp * 4 + (size_t)NT * 32 * 16 + (size_t)warps * (tile_rows * (Jp + 2) + 4) * 4;
-}
-
 // ST: addressing (kContiguous ...); with strides and a gate tensor the epilogue multiplies by sigmoid(gate).
 template <int D, int WB, bool SE, int ST>
 __global__ void __launch_bounds__(FwdTune<D>::warps * 32, SE ? FwdTune<D>::ctas_se : FwdTune<D>::ctas)
 fwd_mma_kernel(const FwdArgs a, const Taps t) {
     constexpr int W = FwdTune<D>::warps, G = SE ? FwdTune<D>::group_se : FwdTune<D>::group;
-    extern __shared__ __align__(16) unsigned char se_smem[];
+    extern __shared__ __align__(16) float se_smem[];      // scale_embed: the table, then a tile per warp
     __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
     __shared__ int2 tap_s[DSQG_MAX_TAPS];
     const Lane L;
     const int bh = blockIdx.y, h = bh % a.H, N = a.N;
-    SeTables se = {};
+    SeRows se = {};
     if constexpr (SE) {
-        se = fill_se_tables<D, WB, W>(se_smem, a.scale_embed, a.pos_bias, t, a.H, h, a.scale, L.warp, false);
+        se = fill_se_rows<D, WB, W * 32>(se_smem, a.scale_embed, a.pos_bias, t, a.H, h, a.scale);
     } else {
         StartTable<WB>::template fill<false, W * 32>(start_s, a.pos_bias, a.H, h, t.d_lo, t.d_lo + t.n_dense - 1, a.scale);
     }
@@ -403,8 +463,9 @@ fwd_mma_kernel(const FwdArgs a, const Taps t) {
     const int g0 = blockIdx.x * (16 * W) + L.warp * 16;
     if (g0 >= N) return;
     const float* start = StartTable<WB>::lane(start_s, L);
-    if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se);
-    else fwd_tile<D, WB, false, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se);
+    float* se_tile = SE ? se_smem + se_rows_bytes<WB>(t.n_sparse, D) / 4 + L.warp * se_tile_floats<WB>(t.n_sparse) : se_smem;
+    if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
+    else fwd_tile<D, WB, false, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
 }
 
 // Tuning per head dimension (measured on B200): sparse taps whose loads are issued together and
@@ -1226,7 +1287,7 @@ cudaError_t fwd_launch_mode(const FwdArgs& a, const Taps& t, cudaStream_t s) {
     size_t smem = 0;
     if constexpr (SE) {
         static int seen[64] = {0};
-        smem = se_tables_bytes(t.J, D, (WB + 16) / 8, W, 16);
+        smem = se_rows_bytes<WB>(t.n_sparse, D) + W * se_tile_floats<WB>(t.n_sparse) * 4;
         const cudaError_t e = ensure_dynamic_smem(fwd_mma_kernel<D, WB, SE, ST>, smem, seen);
         if (e != cudaSuccess) return e;
     }
