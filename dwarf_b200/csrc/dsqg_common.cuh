@@ -53,8 +53,8 @@ struct BwdArgs {
     float* dpb_part;   // [n_tiles, J]
     float* dg_part;    // [n_tiles]
     float* dse_part;   // [n_dse_blocks, J, D] (only with scale_embed)
-    float* qs_rows;    // [B*H*N, Jp] q.scale_embed[j] + pos_bias[j]/scale per row (tensor-core kernels with scale_embed)
-    void* se_pre;      // tables of se_prep_kernel: split scale_embed, its dS.SE fragments, pos_bias/scale, offsets (same kernels)
+    float* qs_rows;    // [B*H*N, n_sparse up to 8] q.scale_embed + pos_bias/scale of the sparse taps per row (tensor-core kernels with scale_embed)
+    void* se_pre;      // tables of se_prep_kernel: split scale_embed, its dS.SE fragments, pos_bias/scale (same kernels)
     float* dse_tmp;    // [n_tiles, J, D] dscale_embed partial of every 64-row tile (same kernels)
     int n_tiles, tiles_per_bh, n_dse_blocks;
     int B, H, N, D;
@@ -128,12 +128,12 @@ inline size_t bwd_scratch_need(int rows_per_tile, int J, int B, int H, int N, in
            (has_se ? round256(tiles * J * D * 4) : 0);
 }
 // Tensor-core kernels with scale_embed: 64-row tiles, dscale_embed partials per group of
-// kSeGroup consecutive tiles of a sequence, and the per-row table qs_rows[B*H*N][Jp], Jp = J rounded up to 8.
+// kSeGroup consecutive tiles of a sequence, and the per-row table qs_rows (room for every tap to be sparse).
 constexpr int kSeGroup = 8;
-// split scale_embed | dS.SE fragments | pos_bias/scale per head [H][Jp] | dense-window offset table (<= 10 n-tiles)
+// scale_embed halves | dS.SE fragments | pos_bias/scale per head, for the widest dense window (72 table rows, 65 columns of dS)
 inline size_t se_pre_bytes(int J, int D, int H) {
-    const size_t Jp = (J + 7) / 8 * 8, JS = (J + 15) / 16 * 16;
-    return 2 * Jp * D * 2 + (JS / 16) * (D / 8) * 32 * 8 + (size_t)H * Jp * 4 + 10 * 32 * 16;
+    const size_t rows = 72 + (J + 7) / 8 * 8, steps = (65 + J + 15) / 16;
+    return 2 * rows * D * 2 + steps * (D / 8) * 32 * 8 + (size_t)H * rows * 4;
 }
 inline size_t bwd_scratch_need_mma_se(int J, int B, int H, int N, int D) {
     const size_t tiles_bh = (N + kMinRowsPerBwdTile - 1) / kMinRowsPerBwdTile;

@@ -48,48 +48,6 @@ constexpr int kContiguous = 0, kStrided = 1, kStridedAny = 2, kKept = 3;
 //     (log2 units): p stays below 2^kSlack, which fp32 sums and bf16 probabilities absorb;
 //   * lanes that do not own a diagonal entry subtract +1e30 instead of the maximum, so their
 //     probability is exactly zero without a select.
-// Shared-memory tables of the scale_embed variants (reference: kernels/dsqg_attention_v3.py:112-118,
-// s_j += q.scale_embed[j] / sqrt(D)).  se_hi + se_lo are the bf16 halves of scale_embed (their sum
-// carries 16 mantissa bits), pbs[j] = pos_bias[j,h] / scale, and qs (one tile per warp,
-// [16][pitch] floats + one dump word holding the mask value) receives q.scale_embed[j] + pbs[j]
-// for the warp's rows.  off[] maps dense-window accumulator slots to tile entries (or the dump).
-struct SeTables {
-    const __nv_bfloat16* se_hi; const __nv_bfloat16* se_lo;
-    const float* pbs; const int4* off; float* qs;
-    int Jp, pitch, nd;
-};
-
-// qs[row][j] = q[row].scale_embed[j] + pbs[j] for the 16 rows held as A fragments qa (rows g) / qb (rows g+8)
-// GL: the tables (se_hi, se_lo, pbs) are in global memory (read-only path) instead of shared memory
-// rows_lo / rows_hi (optional): global-memory rows (Jp floats each) that receive a copy of rows g / g+8
-template <int D, bool GL>
-__device__ __forceinline__ void build_qs_tile(const SeTables& se, const RowFrag<D>& qa, const RowFrag<D>& qb, int g, int tig,
-                                              float* rows_lo = nullptr, float* rows_hi = nullptr) {
-#pragma unroll 2
-    for (int m = 0; m < se.Jp / 8; ++m) {
-        const float2* pbp = reinterpret_cast<const float2*>(se.pbs + 8 * m + 2 * tig);
-        const float2 pb2 = GL ? __ldg(pbp) : *pbp;
-        float c[4] = {pb2.x, pb2.y, pb2.x, pb2.y};
-        RowFrag<D> sf;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const uint4* src = reinterpret_cast<const uint4*>((half ? se.se_lo : se.se_hi) + (8 * m + g) * D + kLane<D> * tig);
-#pragma unroll
-            for (int cc = 0; cc < D / 32; ++cc) {
-                const int o = kLane<D> == 16 ? 8 * (cc >> 1) + (cc & 1) : 4 * cc;
-                const uint4 u = GL ? __ldg(src + o) : src[o];
-                sf.r[4 * cc + 0] = u.x; sf.r[4 * cc + 1] = u.y; sf.r[4 * cc + 2] = u.z; sf.r[4 * cc + 3] = u.w;
-            }
-            mma_rows(c, qa, qb, sf);
-        }
-        *reinterpret_cast<float2*>(se.qs + g * se.pitch + 8 * m + 2 * tig) = make_float2(c[0], c[1]);
-        *reinterpret_cast<float2*>(se.qs + (g + 8) * se.pitch + 8 * m + 2 * tig) = make_float2(c[2], c[3]);
-        if (rows_lo) *reinterpret_cast<float2*>(rows_lo + 8 * m + 2 * tig) = make_float2(c[0], c[1]);
-        if (rows_hi) *reinterpret_cast<float2*>(rows_hi + 8 * m + 2 * tig) = make_float2(c[2], c[3]);
-    }
-    __syncwarp();
-}
-
 // Scale embedding: s_j += q.scale_embed[j] / sqrt(D) (reference: kernels/dsqg_attention_v3.py:112-118).  q.scale_embed is formed
 // per 16-row tile with MMAs, in the order the scores need it: column x = WB + 16 - delta for the dense offsets (as StartTable), then
 // the sparse taps.  Row i of a tile reads its start values at x = 16 - i + c, pairs of them 8-byte aligned (the row
@@ -191,6 +149,21 @@ __device__ __forceinline__ SeRows fill_se_rows(float* smem, const float* scale_e
     }
     return {hi, lo, pb};
 }
+// The same for the backward, where rows are keys (dK/dV) and the tile holds the query rows of the whole CTA: element (key i, query c)
+// of a warp's tile belongs to row c, column WB + 16 - c + i.  lane: tile of the warp's first query + 2 tig (pitch - 1) + WB + 16 + g; the
+// pitch is 5 mod 32, so that the eight keys of four queries hit different banks.
+template <int WB> constexpr int kSeKeyPitch = WB == 32 ? 69 : 101;
+template <int WB>
+__device__ __forceinline__ void se_start_keys(float (&s)[4], const float* lane, int nt, int g, int tig) {
+    constexpr int Q = kSeKeyPitch<WB> - 1, last = WB / 8 + 1;
+    const float* p = lane + 8 * nt * Q;
+    const int c = 2 * tig;
+    s[0] = p[0]; s[1] = p[Q]; s[2] = p[8]; s[3] = p[Q + 8];
+    if (nt == last) { s[0] = s[1] = kNeg; if (g < c) s[2] = kNeg; if (g < c + 1) s[3] = kNeg; }
+    if (nt == last - 1) { if (g < c) s[0] = kNeg; if (g < c + 1) s[1] = kNeg; }
+    if (nt == 0) { if (g >= c) s[2] = kNeg; if (g >= c + 1) s[3] = kNeg; }
+}
+
 template <int WB> __host__ __device__ inline size_t se_rows_bytes(int ns, int D) { return (size_t)SeGeo<WB>::rows(ns) * (4 * D + 4); }
 template <int WB> __host__ __device__ inline size_t se_tile_floats(int ns) { return (size_t)16 * (SeGeo<WB>::kPitch + SeGeo<WB>::sparse_pitch(ns)); }
 
@@ -438,7 +411,8 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
 // resident CTAs per SM the register budget is set for.
 template <int D> struct FwdTune {
     static constexpr int warps = 4, group = D == 64 || D > 80 ? 1 : 2, ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));   // D = 64: 104.8 us (107.8 with group 2)
-    static constexpr int group_se = D <= 64 ? 2 : 1, ctas_se = D == 32 ? 5 : 4;       // with scale_embed
+    // with scale_embed; two tiles per warp share the table: 96.0 us (98.6 with one, 97.6 with four), D = 64 126.7 (133.1, 130.8)
+    static constexpr int group_se = 2, ctas_se = D == 32 ? 5 : 4, tiles_se = 2;
 };
 
 // ST: addressing (kContiguous ...); with strides and a gate tensor the epilogue multiplies by sigmoid(gate).
@@ -460,12 +434,17 @@ fwd_mma_kernel(const FwdArgs a, const Taps t) {
     for (int si = threadIdx.x; si < t.n_sparse; si += W * 32)
         tap_s[si] = make_int2(t.sparse[si], __float_as_int(a.pos_bias[(t.n_dense + si) * a.H + h] * kLog2e));
     __syncthreads();
-    const int g0 = blockIdx.x * (16 * W) + L.warp * 16;
-    if (g0 >= N) return;
     const float* start = StartTable<WB>::lane(start_s, L);
     float* se_tile = SE ? se_smem + se_rows_bytes<WB>(t.n_sparse, D) / 4 + L.warp * se_tile_floats<WB>(t.n_sparse) : se_smem;
-    if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
-    else fwd_tile<D, WB, false, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
+    constexpr int kTiles = SE ? FwdTune<D>::tiles_se : 1;
+#pragma unroll 1
+    for (int i = 0; i < kTiles; ++i) {
+        const int g0 = (blockIdx.x * kTiles + i) * (16 * W) + L.warp * 16;
+        if (g0 >= N) return;
+        if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
+        else fwd_tile<D, WB, false, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
+        if (kTiles > 1) __syncwarp();
+    }
 }
 
 // Tuning per head dimension (measured on B200): sparse taps whose loads are issued together and
@@ -476,8 +455,6 @@ template <int D> struct BwdTune {
     static constexpr int dkdv_group_se = D <= 64 ? 2 : 1, dkdv_ctas_se = D == 32 ? 4 : 3;
     static constexpr int dkdv_group = D <= 80 ? 2 : 1, dkdv_ctas = D == 32 ? 4 : (D <= 64 ? 3 : 2);   // D = 80: 78.1 us (83 with group 1, 96-109 with 3 CTAs)
 };
-constexpr int kStagePitchSe = kRows + 4;    // staging tile with scale_embed, 68: rows are read back as 8-byte pairs by the dS MMAs
-
 // Where a warp of the plain dQ kernel puts its ds values for dpos_bias.  Element (g + 8 half, 8 nt + 2 tig + c) of a
 // tile belongs to offset g - 2 tig - c + 8 k with k = WB / 8 + half - nt, so elements of neighbouring n-tiles share
 // (lane, c, k) and are added in registers first: 2 (WB/8 + 3) stores per lane instead of 4 (WB/8 + 2), to [c][k + 1][lane];
@@ -516,20 +493,34 @@ template <int WB> struct DsStage {
     }
 };
 
-// Extras of the dQ kernel with scale_embed.
-//   seb:  scale_embed as B fragments of dS.SE (global memory, written by se_prep_kernel)
-//   q_s:  the CTA's 64 query rows as bf16 in shared memory, row pitch 2D+16 bytes (conflict-free ldmatrix)
-struct SeBwd {
-    const uint2* seb; unsigned char* q_s;
-    int JS;            // J rounded up to 16
+// Extras of the dQ kernel with scale_embed.  A warp's tile of start values (build_se_tile) becomes its tile of ds values: every
+// element is read and then overwritten by the lane that owns it, and the sparse taps follow the dense ones at column
+// WB + 17, so that columns 16 .. 16 (steps + 1) are dS in the order of the table rows and the products dS.SE and dS^T.Q read it in place.
+template <int WB> struct SeBwd {
+    SeRows rows;
+    const uint2* seb;            // table as B fragments of dS.SE (global memory, written by se_prep_kernel)
+    unsigned char* q_s;          // the CTA's 64 query rows as bf16 in shared memory, row pitch 2D+16 bytes (conflict-free ldmatrix)
+    float* tile; float* sparse;  // this warp's
+    int pitch, sp;
+    static constexpr int kSparse = WB + 17;                                                              // column of the first sparse tap
+    static __host__ __device__ int steps(int ns) { return (WB + 1 + ns + 15) / 16; }                      // 16-column steps of dS
+    static __host__ __device__ int pitch_for(int ns) {                                                    // 9 mod 32
+        const int need = steps(ns) * 16 + 16 > WB + 32 ? steps(ns) * 16 + 16 : WB + 32;
+        return (need - 9 + 31) / 32 * 32 + 9;
+    }
+    // floats per warp; the odd multiple of 8 puts the tiles two warps apart 16 banks apart (column sums)
+    static __host__ __device__ int floats(int ns) { return 16 * (pitch_for(ns) + SeGeo<WB>::sparse_pitch(ns)) + 8; }
+    // tap of column 16 + p of dS, -1: none
+    static __device__ __forceinline__ int tap(const Taps& t, int p) {
+        const int j = p <= WB ? WB - p - t.d_lo : t.n_dense + p - WB - 1;
+        return p <= WB ? (j >= 0 && j < t.n_dense ? j : -1) : (j < t.J ? j : -1);
+    }
 };
 
 template <int D, int WB, bool INTERIOR, int G, bool SE, int ST>
-__device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, const int4* soff_s, const int2* tap_s,
-                                         float* stage_w, int nd, int ns, int bh, int h, int g0, const Lane& L,
-                                         const SeTables& se, const SeBwd& sb) {
+__device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, const int2* tap_s,
+                                         float* stage_w, int ns, int bh, int h, int g0, const Lane& L, const SeBwd<WB>& sb) {
     constexpr int NT = (WB + 16) / 8;
-    constexpr int SP = kStagePitchSe;
     using Stage = DsStage<WB>;
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = g0 + g, row_hi = row_lo + 8;
@@ -555,9 +546,11 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     load_row<D, AL>(da, dop + (size_t)row_lo * OS, tig, ok_lo);
     load_row<D, AL>(db, dop + (size_t)row_hi * OS, tig, ok_hi);
     if constexpr (SE) {
-        // the tile also goes to global memory for the dK/dV kernel (rows of this warp, Jp floats each)
-        float* rows = a.qs_rows + ((size_t)bh * N + row_lo) * se.Jp;
-        build_qs_tile<D, true>(se, qa, qb, g, tig, ok_lo ? rows : nullptr, ok_hi ? rows + 8 * se.Jp : nullptr);
+        // the sparse part also goes to global memory for the dK/dV kernel (a row of ns8 floats per query)
+        const int ns8 = (ns + 7) / 8 * 8;
+        float* rows = a.qs_rows + ((size_t)bh * N + row_lo) * ns8;
+        build_se_tile<D, WB, true>(sb.rows, ns, qa, qb, g, tig, sb.tile, sb.pitch, sb.sparse, sb.sp, ok_lo ? rows : nullptr,
+                                   ok_hi ? rows + 8 * ns8 : nullptr);
         // and the query rows to shared memory for the CTA's dscale_embed partial
         unsigned char* qrow = sb.q_s + (size_t)(L.warp * 16 + g) * (2 * D + 16) + 2 * kLane<D> * tig;
 #pragma unroll
@@ -588,6 +581,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     }
     float dQ[D / 8][4];
     float carry[2] = {0.f, 0.f};                                   // plain kernel: row g's ds of the n-tile before
+    float* se_lane = SE ? sb.tile + g * (sb.pitch - 1) + 16 + 2 * tig : nullptr;
 
     // ---- dense window
 #pragma unroll
@@ -598,12 +592,8 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
         for (int hf = 0; hf < 2; ++hf) {
             const int nt = 2 * c + hf;
             float s[4], dp[4];
-            int so_r[4];
             if constexpr (SE) {
-                const int4 qo = __ldg(se.off + nt * 32 + L.lane);      // table in global memory (se_prep_kernel)
-                s[0] = se.qs[qo.x]; s[1] = se.qs[qo.y]; s[2] = se.qs[qo.z]; s[3] = se.qs[qo.w];
-                const int4 so = soff_s[nt * 32 + L.lane];
-                so_r[0] = so.x; so_r[1] = so.y; so_r[2] = so.z; so_r[3] = so.w;
+                se_start<WB>(s, se_lane, sb.pitch, nt, g, tig);
             } else {
                 StartTable<WB>::get(s, start, nt);
             }
@@ -632,7 +622,10 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
                 const f32x2 pp = pair(ex2(p0), ex2(p1)), dpp = pair(dp[r], dp[r + 1]);
                 dgrow2 = fma2(pp, dpp, dgrow2);
                 unpair(mul2(pp, fma2(pair(gain, gain), dpp, pair(-d, -d))), ds[hf][r], ds[hf][r + 1]);
-                if constexpr (SE) { stage_w[so_r[r]] = ds[hf][r]; stage_w[so_r[r + 1]] = ds[hf][r + 1]; }
+            }
+            if constexpr (SE) {
+                *reinterpret_cast<float2*>(se_lane + 8 * nt) = make_float2(ds[hf][0], ds[hf][1]);
+                if (nt > 0) *reinterpret_cast<float2*>(se_lane + 8 * (sb.pitch - 1) + 8 * nt) = make_float2(ds[hf][2], ds[hf][3]);
             }
             if constexpr (!SE) {
                 Stage::put(stage_w, L.lane, WB / 8 + 2 - nt, nt ? carry[0] + ds[hf][2] : ds[hf][2], nt ? carry[1] + ds[hf][3] : ds[hf][3]);
@@ -653,13 +646,22 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     // ---- sparse taps
     const float ls_lo = L.owner ? l2_lo : 1.0e30f, ls_hi = L.owner ? l2_hi : 1.0e30f;   // p == 0 on lanes without a diagonal entry
     if constexpr (!SE) Stage::put(stage_w, L.lane, 0, carry[0], carry[1]);
-    float* stage_sp = SE ? stage_w + nd * SP + g : stage_w + Stage::kDense + g * Stage::sparse_pitch(ns);
+    // one value per sparse tap: row pairs' sums in the plain kernel, rows g and g + 8 with scale_embed
+    float* stage_sp = SE ? sb.tile + g * sb.pitch + SeBwd<WB>::kSparse : stage_w + Stage::kDense + g * Stage::sparse_pitch(ns);
+    const int stage_hi = SE ? 8 * sb.pitch : 0;
+    const float* qs0 = SE ? sb.sparse + g * sb.sp : nullptr;
+    const float* qs1 = qs0 + 8 * sb.sp;
+    if constexpr (SE) {
+        __syncwarp();                                     // the dense columns' owners have written what lies under the sparse ones
+        const int first = SeBwd<WB>::kSparse + ns, pad = 16 * SeBwd<WB>::steps(ns) + 16 - first;
+        for (int e = L.lane; e < 16 * pad; e += 32) sb.tile[(e & 15) * sb.pitch + first + (e >> 4)] = 0.f;
+    }
     auto finish = [&](int si, float sd0, float sd1, float dp0, float dp1, float pbv, bool v0, bool v1,
                       const RowFrag<D>& kf0, const RowFrag<D>& kf1) {
         float p0, p1;
         if constexpr (SE) {
-            p0 = v0 ? ex2((sd0 + se.qs[g * se.pitch + nd + si]) * c2 - ls_lo) : 0.f;
-            p1 = v1 ? ex2((sd1 + se.qs[(g + 8) * se.pitch + nd + si]) * c2 - ls_hi) : 0.f;
+            p0 = v0 ? ex2((sd0 + qs0[si]) * c2 - ls_lo) : 0.f;
+            p1 = v1 ? ex2((sd1 + qs1[si]) * c2 - ls_hi) : 0.f;
         } else {
             p0 = v0 ? ex2(fmaf(sd0, c2, pbv) - ls_lo) : 0.f;
             p1 = v1 ? ex2(fmaf(sd1, c2, pbv) - ls_hi) : 0.f;
@@ -667,7 +669,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
         dgrow = fmaf(p0, dp0, dgrow); dgrow = fmaf(p1, dp1, dgrow);
         const float x0 = p0 * fmaf(gain, dp0, -delta_lo), x1 = p1 * fmaf(gain, dp1, -delta_hi);
         if (L.owner) {
-            if constexpr (SE) { stage_sp[si * SP] = x0; stage_sp[si * SP + 8] = x1; } else stage_sp[si] = x0 + x1;
+            if constexpr (SE) { stage_sp[si] = x0; stage_sp[stage_hi + si] = x1; } else stage_sp[si] = x0 + x1;
         }
         diag_fma<D>(dQ, __shfl_sync(0xffffffffu, x0, L.owner_lane), __shfl_sync(0xffffffffu, x1, L.owner_lane), kf0, kf1);
     };
@@ -722,16 +724,18 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     }
     if (L.owner)                                          // taps no row of the tile reaches: zero entries
         for (; si < ns; ++si) {
-            if constexpr (SE) { stage_sp[si * SP] = 0.f; stage_sp[si * SP + 8] = 0.f; } else stage_sp[si] = 0.f;
+            stage_sp[si] = 0.f;
+            if constexpr (SE) stage_sp[stage_hi + si] = 0.f;
         }
     if constexpr (SE) {
-        // dQ += dS.scale_embed: the warp's ds values are complete in its 16 staging columns
+        // dQ += dS.scale_embed: the warp's ds values are complete in its tile
         __syncwarp();
 #pragma unroll 1
-        for (int kk = 0; kk < sb.JS / 16; ++kk) {
-            const float* col = stage_w + (16 * kk + 2 * tig) * SP + g;
-            const uint32_t a0 = pack_bf16x2(col[0], col[SP]), a1 = pack_bf16x2(col[8], col[SP + 8]);
-            const uint32_t a2 = pack_bf16x2(col[8 * SP], col[9 * SP]), a3 = pack_bf16x2(col[8 * SP + 8], col[9 * SP + 8]);
+        for (int kk = 0; kk < SeBwd<WB>::steps(ns); ++kk) {
+            const float* lo = sb.tile + g * sb.pitch + 16 + 16 * kk + 2 * tig;
+            const float* hi = lo + 8 * sb.pitch;
+            const uint32_t a0 = pack_bf16x2(lo[0], lo[1]), a1 = pack_bf16x2(hi[0], hi[1]);
+            const uint32_t a2 = pack_bf16x2(lo[8], lo[9]), a3 = pack_bf16x2(hi[8], hi[9]);
 #pragma unroll
             for (int jn = 0; jn < D / 8; ++jn) {
                 const uint2 b = __ldg(sb.seb + (kk * (D / 8) + jn) * 32 + L.lane);
@@ -746,149 +750,93 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     return dgrow + (dg0 + dg1);
 }
 
-// One block, before the dQ kernel with scale_embed.  Writes, back to back:
-//   scale_embed split into bf16 halves [2][Jp][D];
-//   its B fragments for dQ += dS.scale_embed, [JS/16][D/8][32] x uint2, in the element order of the
-//     dQ accumulators (row fragment register jn of lane tig = g>>1, element g&1), rows j >= J zero;
-//   pos_bias[j,h] / scale for every head, [H][Jp];
-//   the offset table of the dense window into a per-warp tile of the given pitch, [NT*32] x int4
-//     (16 * pitch = the dump entry that holds the mask value).
+// One block, before the dQ kernel with scale_embed.  Writes, back to back: the table (SeRows) as bf16 halves [2][R][D]; its B fragments for
+// dQ += dS.scale_embed, [steps][D/8][32] x uint2, in the element order of the dQ accumulators (row fragment register jn of lane
+// tig = g>>1, element g&1); pos_bias / scale or the mask value for every head, [H][R].
 struct SePre {
-    const __nv_bfloat16* se_hi; const __nv_bfloat16* se_lo; const uint2* seb; const float* pbs; const int4* off;
+    const __nv_bfloat16* hi; const __nv_bfloat16* lo; const uint2* seb; const float* pb;
 };
-__host__ __device__ inline SePre se_pre_layout(const void* base, int J, int D, int H) {
-    const int Jp = (J + 7) / 8 * 8, JS = (J + 15) / 16 * 16;
+template <int WB>
+__host__ __device__ inline SePre se_pre_layout(const void* base, int ns, int D) {
+    const int R = SeGeo<WB>::rows(ns);
     SePre p;
-    p.se_hi = static_cast<const __nv_bfloat16*>(base);
-    p.se_lo = p.se_hi + Jp * D;
-    p.seb = reinterpret_cast<const uint2*>(p.se_lo + Jp * D);
-    p.pbs = reinterpret_cast<const float*>(p.seb + (JS / 16) * (D / 8) * 32);
-    p.off = reinterpret_cast<const int4*>(p.pbs + H * Jp);
+    p.hi = static_cast<const __nv_bfloat16*>(base);
+    p.lo = p.hi + R * D;
+    p.seb = reinterpret_cast<const uint2*>(p.lo + R * D);
+    p.pb = reinterpret_cast<const float*>(p.seb + SeBwd<WB>::steps(ns) * (D / 8) * 32);
     return p;
 }
-template <int D>
-__global__ void se_prep_kernel(const float* __restrict__ scale_embed, const float* __restrict__ pos_bias, float scale,
-                               int J, int H, int d_lo, int n_dense, int WB, void* out) {
-    const int Jp = (J + 7) / 8 * 8, JS = (J + 15) / 16 * 16;
-    const SePre P = se_pre_layout(out, J, D, H);
-    __nv_bfloat162* hi = reinterpret_cast<__nv_bfloat162*>(const_cast<__nv_bfloat16*>(P.se_hi));
-    __nv_bfloat162* lo = reinterpret_cast<__nv_bfloat162*>(const_cast<__nv_bfloat16*>(P.se_lo));
-    for (int e = threadIdx.x; e < Jp * D / 2; e += blockDim.x) {
-        const int j = (2 * e) / D;
+template <int D, int WB>
+__global__ void se_prep_kernel(const float* __restrict__ scale_embed, const float* __restrict__ pos_bias, float scale, const Taps t, int H, void* out) {
+    const SePre P = se_pre_layout<WB>(out, t.n_sparse, D);
+    const int R = SeGeo<WB>::rows(t.n_sparse);
+    __nv_bfloat162* hi = reinterpret_cast<__nv_bfloat162*>(const_cast<__nv_bfloat16*>(P.hi));
+    __nv_bfloat162* lo = reinterpret_cast<__nv_bfloat162*>(const_cast<__nv_bfloat16*>(P.lo));
+    for (int e = threadIdx.x; e < R * D / 2; e += blockDim.x) {
+        const int j = SeGeo<WB>::tap(t, 2 * e / D);
         float2 x = make_float2(0.f, 0.f);
-        if (j < J) x = *reinterpret_cast<const float2*>(scale_embed + 2 * e);
+        if (j >= 0) x = *reinterpret_cast<const float2*>(scale_embed + j * D + 2 * e % D);
         const __nv_bfloat162 h2 = __floats2bfloat162_rn(x.x, x.y);
         hi[e] = h2;
         lo[e] = __floats2bfloat162_rn(x.x - __low2float(h2), x.y - __high2float(h2));
     }
     uint2* seb = const_cast<uint2*>(P.seb);
-    for (int e = threadIdx.x; e < (JS / 16) * (D / 8) * 32; e += blockDim.x) {
+    for (int e = threadIdx.x; e < SeBwd<WB>::steps(t.n_sparse) * (D / 8) * 32; e += blockDim.x) {
         const int ln = e & 31, jn = (e >> 5) % (D / 8), kk = (e >> 5) / (D / 8);
         const int gg = ln >> 2, tt = ln & 3;
         constexpr int kPer = kLane<D> / 2;                       // n-tiles per piece
         const int d = 4 * kLane<D> * (jn / kPer) + kLane<D> * (gg >> 1) + 2 * (jn % kPer) + (gg & 1);
-        const int j0 = 16 * kk + 2 * tt;
-        auto sev = [&](int j) { return j < J ? scale_embed[j * D + d] : 0.f; };
-        seb[e] = make_uint2(pack_bf16x2(sev(j0), sev(j0 + 1)), pack_bf16x2(sev(j0 + 8), sev(j0 + 9)));
+        auto sev = [&](int p) { const int j = SeBwd<WB>::tap(t, p); return j >= 0 ? scale_embed[j * D + d] : 0.f; };
+        const int p0 = 16 * kk + 2 * tt;
+        seb[e] = make_uint2(pack_bf16x2(sev(p0), sev(p0 + 1)), pack_bf16x2(sev(p0 + 8), sev(p0 + 9)));
     }
-    float* pbs = const_cast<float*>(P.pbs);
+    float* pb = const_cast<float*>(P.pb);
     const float inv_scale = 1.f / scale;
-    for (int e = threadIdx.x; e < H * Jp; e += blockDim.x) {
-        const int h = e / Jp, j = e - h * Jp;
-        pbs[e] = j < J ? pos_bias[j * H + h] * inv_scale : 0.f;
-    }
-    int4* off = const_cast<int4*>(P.off);
-    const int NT = (WB + 16) / 8, pitch = Jp + 2, d_hi = d_lo + n_dense - 1;
-    for (int e = threadIdx.x; e < NT * 32; e += blockDim.x) {
-        const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
-        int o[4];
-        for (int r = 0; r < 4; ++r) {
-            const int i = gg + 8 * (r >> 1), delta = WB + i - (8 * nt + 2 * tt + (r & 1));
-            o[r] = (delta >= d_lo && delta <= d_hi) ? i * pitch + (delta - d_lo) : 16 * pitch;
-        }
-        off[e] = make_int4(o[0], o[1], o[2], o[3]);
+    for (int e = threadIdx.x; e < H * R; e += blockDim.x) {
+        const int h = e / R, j = SeGeo<WB>::tap(t, e - h * R);
+        pb[e] = j >= 0 ? pos_bias[j * H + h] * inv_scale : kNeg;
     }
 }
 
-inline size_t dq_smem_bytes(int J, int n_sparse, int D, int NT, bool se) {
-    // with scale_embed a staging row per tap (rounded up to the MMA shape) and a dump row; otherwise a DsStage per warp
-    size_t n = sizeof(float) * (size_t)(se ? ((J + 15) / 16 * 16 + 1) * kStagePitchSe + kWarps * 32
-                                           : kWarps * (1 + (NT == 6 ? DsStage<32>::floats(n_sparse, J) : NT == 8 ? DsStage<48>::floats(n_sparse, J)
-                                                                                                               : DsStage<64>::floats(n_sparse, J))));
-    if (se) {
-        n = (n + 15) / 16 * 16;
-        n += (size_t)kWarps * (16 * ((J + 7) / 8 * 8 + 2) + 4) * 4;      // one q.scale_embed tile per warp
-        n = (n + 15) / 16 * 16;
-        n += (size_t)kRows * (2 * D + 16);
-    }
-    return n;
+// [kWarps] dgain terms, then per warp a DsStage or, with scale_embed, a SeBwd tile; then the query rows
+template <int D, int WB>
+inline size_t dq_smem_bytes(int J, int ns, bool se) {
+    return sizeof(float) * kWarps * (size_t)(1 + (se ? SeBwd<WB>::floats(ns) : DsStage<WB>::floats(ns, J))) + (se ? (size_t)kRows * (2 * D + 16) : 0);
 }
 
 template <int D, int WB, int G, int CT, bool SE, int ST>
 __global__ void __launch_bounds__(kWarps * 32, CT)
 bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
-    constexpr int NT = (WB + 16) / 8;
-    constexpr int SP = kStagePitchSe;
     using Stage = DsStage<WB>;
-    // scale_embed: [JS + 1][SP] ds values, then [128] dgain terms, then the scale_embed extras; plain: [kWarps] dgain terms, a DsStage per warp
-    extern __shared__ __align__(16) float stage[];
+    extern __shared__ __align__(16) float stage[];     // see dq_smem_bytes
     __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
-    __shared__ int4 soff_s[SE ? NT * 32 : 1];          // staging offsets per lane (scale_embed variant only)
     __shared__ int2 tap_s[DSQG_MAX_TAPS];
     const Lane L;
     const int bh = blockIdx.y, h = bh % a.H, N = a.N, J = t.J;
-    const int JS = SE ? (J + 15) / 16 * 16 : J;         // scale_embed: staging rows (row JS is the dump for out-of-band entries)
-    float* dg_s = SE ? stage + (JS + 1) * SP : stage;
-    SeTables se = {};
-    SeBwd sb = {};
-    {
-        const int d_lo = t.d_lo, d_hi = t.d_lo + t.n_dense - 1;
-        if constexpr (!SE) {
-            StartTable<WB>::template fill<false, kWarps * 32>(start_s, a.pos_bias, a.H, h, d_lo, d_hi, a.scale);
-        } else {
-            for (int e = threadIdx.x; e < NT * 32; e += kWarps * 32) {
-                const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
-                int o[4];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int i = gg + 8 * (r >> 1), delta = WB + i - (8 * nt + 2 * tt + (r & 1));
-                    o[r] = (delta >= d_lo && delta <= d_hi ? delta - d_lo : JS) * SP + i;
-                }
-                soff_s[e] = make_int4(o[0], o[1], o[2], o[3]);
-            }
-        }
-        for (int si = threadIdx.x; si < t.n_sparse; si += kWarps * 32)
-            tap_s[si] = make_int2(t.sparse[si], __float_as_int(a.pos_bias[(t.n_dense + si) * a.H + h] * kLog2e));
-        if constexpr (SE) {
-            // tables come from global memory (se_prep_kernel); shared memory only holds the per-warp
-            // q.scale_embed tiles and the CTA's query rows
-            const SePre P = se_pre_layout(a.se_pre, J, D, a.H);
-            const int Jp = (J + 7) / 8 * 8, pitch = Jp + 2;
-            unsigned char* p = reinterpret_cast<unsigned char*>(dg_s + kWarps * 32);
-            p = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
-            float* qs_w = reinterpret_cast<float*>(p) + L.warp * (16 * pitch + 4);
-            if (L.lane == 0) qs_w[16 * pitch] = kNeg;          // the dump entry: masked
-            se.se_hi = P.se_hi; se.se_lo = P.se_lo; se.pbs = P.pbs + h * Jp; se.off = P.off; se.qs = qs_w;
-            se.Jp = Jp; se.pitch = pitch; se.nd = t.n_dense;
-            p += (size_t)kWarps * (16 * pitch + 4) * 4;
-            p = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
-            sb.JS = JS;
-            sb.seb = P.seb;
-            sb.q_s = p;
-            // staging rows J .. JS-1 take part in the dS MMAs: zero
-            for (int e = threadIdx.x; e < (JS - J) * kRows; e += kWarps * 32)
-                stage[(J + e / kRows) * SP + e % kRows] = 0.f;
-        }
+    float* dg_s = stage;
+    SeBwd<WB> sb = {};
+    if constexpr (!SE) StartTable<WB>::template fill<false, kWarps * 32>(start_s, a.pos_bias, a.H, h, t.d_lo, t.d_lo + t.n_dense - 1, a.scale);
+    for (int si = threadIdx.x; si < t.n_sparse; si += kWarps * 32)
+        tap_s[si] = make_int2(t.sparse[si], __float_as_int(a.pos_bias[(t.n_dense + si) * a.H + h] * kLog2e));
+    const int per_se = SE ? SeBwd<WB>::floats(t.n_sparse) : 0;
+    if constexpr (SE) {
+        const SePre P = se_pre_layout<WB>(a.se_pre, t.n_sparse, D);
+        sb.rows = {P.hi, P.lo, P.pb + h * SeGeo<WB>::rows(t.n_sparse)};
+        sb.seb = P.seb;
+        sb.pitch = SeBwd<WB>::pitch_for(t.n_sparse); sb.sp = SeGeo<WB>::sparse_pitch(t.n_sparse);
+        sb.tile = stage + kWarps + L.warp * per_se;
+        sb.sparse = sb.tile + 16 * sb.pitch;
+        sb.q_s = reinterpret_cast<unsigned char*>(stage + kWarps + kWarps * per_se);
     }
     __syncthreads();
     const int g0 = blockIdx.x * kRows + L.warp * 16;
-    float* stage_w = SE ? stage + L.warp * 16 : stage + kWarps + L.warp * Stage::floats(t.n_sparse, J);
+    float* stage_w = stage + kWarps + L.warp * Stage::floats(t.n_sparse, J);                     // plain kernel
     float* sums = stage + kWarps + Stage::kDense + 8 * Stage::sparse_pitch(t.n_sparse);          // plain kernel: warp 0's J sums
     const float* start = StartTable<WB>::lane(start_s, L);
     float dgrow = 0.f;
-    if (g0 >= N) {                                      // no rows: this warp's sums, or staging columns and query rows, are zero
+    if (g0 >= N) {                                      // no rows: this warp's sums, or ds tile and query rows, are zero
         if constexpr (SE) {
-            for (int e = L.lane; e < J * 16; e += 32) stage_w[(e >> 4) * SP + (e & 15)] = 0.f;
+            for (int e = L.lane; e < 16 * sb.pitch; e += 32) sb.tile[e] = 0.f;
         } else {
             for (int j = L.lane; j < J; j += 32) sums[L.warp * Stage::floats(t.n_sparse, J) + j] = 0.f;
         }
@@ -896,9 +844,9 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
             for (int e = L.lane; e < 16 * (2 * D + 16) / 16; e += 32)
                 reinterpret_cast<uint4*>(sb.q_s + (size_t)L.warp * 16 * (2 * D + 16))[e] = make_uint4(0u, 0u, 0u, 0u);
     } else if (g0 >= WB && g0 + 16 <= N) {
-        dgrow = dq_tile<D, WB, true, G, SE, ST>(a, start, soff_s, tap_s, stage_w, t.n_dense, t.n_sparse, bh, h, g0, L, se, sb);
+        dgrow = dq_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stage_w, t.n_sparse, bh, h, g0, L, sb);
     } else {
-        dgrow = dq_tile<D, WB, false, G, SE, ST>(a, start, soff_s, tap_s, stage_w, t.n_dense, t.n_sparse, bh, h, g0, L, se, sb);
+        dgrow = dq_tile<D, WB, false, G, SE, ST>(a, start, tap_s, stage_w, t.n_sparse, bh, h, g0, L, sb);
     }
     if constexpr (!SE)
         if (g0 < N) Stage::sum(stage_w, t, L.lane);
@@ -908,30 +856,30 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
     __syncthreads();
     const int tile = bh * a.tiles_per_bh + blockIdx.x;
     if constexpr (SE) {
-        // CTA partial of dscale_embed = scale * dS^T[JS x 64] . Q[64 x D]; warp w takes n-tiles w, w+4, ...
+        // CTA partial of dscale_embed = scale * dS^T . Q[64 x D]; warp w takes n-tiles w, w+4, ...
         constexpr int QP = 2 * D + 16;
         const uint32_t q_base = static_cast<uint32_t>(__cvta_generic_to_shared(sb.q_s));
 #pragma unroll 1
         for (int jn = L.warp; jn < D / 8; jn += kWarps) {
 #pragma unroll 1
-            for (int mt = 0; mt < JS / 16; ++mt) {
+            for (int mt = 0; mt < SeBwd<WB>::steps(t.n_sparse); ++mt) {
                 float c[4];
 #pragma unroll
                 for (int kk = 0; kk < kRows / 16; ++kk) {
-                    const float* r0 = stage + (16 * mt + L.g) * SP + 16 * kk + 2 * L.tig;
-                    const float2 u0 = *reinterpret_cast<const float2*>(r0), u1 = *reinterpret_cast<const float2*>(r0 + 8 * SP);
-                    const float2 u2 = *reinterpret_cast<const float2*>(r0 + 8), u3 = *reinterpret_cast<const float2*>(r0 + 8 * SP + 8);
+                    const float* r0 = stage + kWarps + kk * per_se + 2 * L.tig * sb.pitch + 16 + 16 * mt + L.g;
+                    const float* r8 = r0 + 8 * sb.pitch;
                     uint32_t b0, b1;
                     const uint32_t addr = q_base + (16 * kk + (L.lane & 15)) * QP + 16 * jn;
                     asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
-                    const uint32_t a0 = pack_bf16x2(u0.x, u0.y), a1 = pack_bf16x2(u1.x, u1.y);
-                    const uint32_t a2 = pack_bf16x2(u2.x, u2.y), a3 = pack_bf16x2(u3.x, u3.y);
+                    const uint32_t a0 = pack_bf16x2(r0[0], r0[sb.pitch]), a1 = pack_bf16x2(r0[8], r0[sb.pitch + 8]);
+                    const uint32_t a2 = pack_bf16x2(r8[0], r8[sb.pitch]), a3 = pack_bf16x2(r8[8], r8[sb.pitch + 8]);
                     if (kk == 0) mma16816_z(c, a0, a1, a2, a3, b0, b1); else mma16816(c, a0, a1, a2, a3, b0, b1);
                 }
                 // the tile's partial goes to global memory; dse_group_kernel adds the tiles of a group
-                float* dst = a.dse_tmp + (size_t)tile * J * D + (16 * mt + L.g) * D + 8 * jn + 2 * L.tig;
-                if (16 * mt + L.g < J) *reinterpret_cast<float2*>(dst) = make_float2(c[0] * a.scale, c[1] * a.scale);
-                if (16 * mt + L.g + 8 < J) *reinterpret_cast<float2*>(dst + 8 * D) = make_float2(c[2] * a.scale, c[3] * a.scale);
+                const int j0 = SeBwd<WB>::tap(t, 16 * mt + L.g), j1 = SeBwd<WB>::tap(t, 16 * mt + L.g + 8);
+                float* dst = a.dse_tmp + (size_t)tile * J * D + 8 * jn + 2 * L.tig;
+                if (j0 >= 0) *reinterpret_cast<float2*>(dst + j0 * D) = make_float2(c[0] * a.scale, c[1] * a.scale);
+                if (j1 >= 0) *reinterpret_cast<float2*>(dst + j1 * D) = make_float2(c[2] * a.scale, c[3] * a.scale);
             }
         }
     }
@@ -941,27 +889,24 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
         for (int j = threadIdx.x; j < J; j += kWarps * 32)
             a.dpb_part[(size_t)tile * J + j] = (sums[j] + sums[per + j]) + (sums[2 * per + j] + sums[3 * per + j]);
     } else {
-        // Column sums of the staging tile: two threads per tap (32 rows each, four independent partial
-        // sums, fixed order), so the CTA's tail is a few dozen dependent additions instead of kRows.
-        static_assert(kRows == 64 && kWarps == 4, "the column sums below split 64 rows over thread pairs");
-        for (int j0 = 0; j0 < J; j0 += kWarps * 16) {
-            const int j = j0 + (threadIdx.x >> 1), half = threadIdx.x & 1;
+        // Column sums of the ds tiles: two threads per tap (two tiles each, fixed order); half 1's tiles lie 16 banks from half 0's
+        static_assert(kWarps == 4, "two tiles per thread");
+        for (int p0 = 0; p0 < 16 * SeBwd<WB>::steps(t.n_sparse); p0 += kWarps * 16) {
+            const int p = p0 + (threadIdx.x >> 1), half = threadIdx.x & 1;
+            const int j = p < 16 * SeBwd<WB>::steps(t.n_sparse) ? SeBwd<WB>::tap(t, p) : -1;
             float s = 0.f;
-            if (j < J) {
-                // pitch 68 puts rows j and j+8 (and the two halves) in the same banks: start each of the
-                // four at a different column so that a warp's 32 reads fall into 32 banks
-                const float* row = stage + j * SP + 32 * half;
-                const int rot = ((j >> 3) & 1) + 2 * half;
+            if (j >= 0) {
+                const float* u = stage + kWarps + 2 * half * per_se + 16 + p;
                 float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
 #pragma unroll
-                for (int r = 0; r < 32; r += 4) {
-                    s0 += row[(r + rot) & 31]; s1 += row[(r + 1 + rot) & 31];
-                    s2 += row[(r + 2 + rot) & 31]; s3 += row[(r + 3 + rot) & 31];
+                for (int r = 0; r < 16; r += 2) {
+                    s0 += u[r * sb.pitch]; s1 += u[(r + 1) * sb.pitch];
+                    s2 += u[per_se + r * sb.pitch]; s3 += u[per_se + (r + 1) * sb.pitch];
                 }
                 s = (s0 + s1) + (s2 + s3);
             }
             s += __shfl_xor_sync(0xffffffffu, s, 1);
-            if (j < J && half == 0) a.dpb_part[(size_t)tile * J + j] = s;
+            if (j >= 0 && half == 0) a.dpb_part[(size_t)tile * J + j] = s;
         }
     }
     if (threadIdx.x == 0) a.dg_part[tile] = (dg_s[0] + dg_s[1]) + (dg_s[2] + dg_s[3]);
@@ -991,13 +936,12 @@ dse_group_kernel(const float* __restrict__ tmp, float* __restrict__ part, int ti
 // query rows [m0, m0+16+WB) for the dense window and the diagonal of the tile at m0+delta for
 // every sparse tap.  Key rows are owned by exactly one warp: no atomics.  The per-query
 // statistics {lse*log2(e), delta} of the CTA's dense query range sit in shared memory.
-// With scale_embed the score accumulators of the dense window start from qsd, the CTA's copy of the
-// dense part of qs_rows (row = query, nd + 1 columns, the last one holding the mask value), and a
-// sparse tap adds the entry of its query row read from global memory.
+// With scale_embed the CTA forms q.scale_embed of its dense query range once more (build_se_tile, 16 rows per warp and step) instead of
+// reading a per-row table of it from global memory; the score accumulators of the dense window start from that tile, and a
+// sparse tap adds the entry of its query row, which the dQ kernel left in qs_rows.
 template <int D, int WB, bool INTERIOR, int G, bool SE, int ST>
 __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, const int2* tap_s, const float* stat_w,
-                                          int ns, int bh, int h, int m0, const Lane& L, const float* qsd_w,
-                                          const int4* qoff, int nd, int Jp) {
+                                          int ns, int bh, int h, int m0, const Lane& L, const float* se_tile) {
     constexpr int NT = (WB + 16) / 8, kStat = kRows + WB;
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = m0 + g, row_hi = row_lo + 8;
@@ -1020,6 +964,7 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
     load_row<D, AL>(va, vp + (size_t)row_lo * RS, tig, ok_lo);
     load_row<D, AL>(vb, vp + (size_t)row_hi * RS, tig, ok_hi);
     float dK[D / 8][4], dV[D / 8][4];
+    const float* se_lane = SE ? se_tile + 2 * tig * (kSeKeyPitch<WB> - 1) + WB + 16 + g : nullptr;
 
     // ---- dense window: query row of n-tile nt for this thread is m0 + 8 nt + g
 #pragma unroll
@@ -1032,8 +977,7 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
             const int nt = 2 * c + hf;
             float s[4], dp[4];
             if constexpr (SE) {
-                const int4 qo = qoff[nt * 32 + L.lane];
-                s[0] = qsd_w[qo.x]; s[1] = qsd_w[qo.y]; s[2] = qsd_w[qo.z]; s[3] = qsd_w[qo.w];
+                se_start_keys<WB>(s, se_lane, nt, g, tig);
             } else {
                 StartTable<WB>::get(s, start, nt);
             }
@@ -1080,7 +1024,8 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
         }
     }
     // ---- sparse taps
-    const float* qs_r = SE ? a.qs_rows + ((size_t)bh * N + row_lo) * Jp + nd : nullptr;   // entry of tap si of query row row_lo + delta: qs_r[delta * Jp + si]
+    const int ns8 = (ns + 7) / 8 * 8;
+    const float* qs_r = SE ? a.qs_rows + ((size_t)bh * N + row_lo) * ns8 : nullptr;   // entry of tap si of query row row_lo + delta: qs_r[delta * ns8 + si]
     // b0/b1: what is added to the raw score: the bias in log2 units (plain) or the qs_rows entry of
     // the query row, in units of 1/scale (scale_embed)
     auto finish = [&](float sd0, float sd1, float dp0, float dp1, float b0, float b1, float2 st0, float2 st1,
@@ -1101,8 +1046,8 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
             const int2 tp = tap_s[si + i];
             const ptrdiff_t off = (ptrdiff_t)tp.x * RS, offd = (ptrdiff_t)tp.x * OS;
             if constexpr (SE) {
-                b0[i] = __ldg(qs_r + (size_t)tp.x * Jp + si + i);
-                b1[i] = __ldg(qs_r + (size_t)(tp.x + 8) * Jp + si + i);
+                b0[i] = __ldg(qs_r + (size_t)tp.x * ns8 + si + i);
+                b1[i] = __ldg(qs_r + (size_t)(tp.x + 8) * ns8 + si + i);
             } else {
                 b0[i] = b1[i] = __int_as_float(tp.y);
             }
@@ -1134,8 +1079,8 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
             const bool v0 = row_lo + delta < N, v1 = row_hi + delta < N;
             float b0 = __int_as_float(tap_s[si].y), b1 = b0;
             if constexpr (SE) {
-                b0 = v0 ? __ldg(qs_r + (size_t)delta * Jp + si) : 0.f;
-                b1 = v1 ? __ldg(qs_r + (size_t)(delta + 8) * Jp + si) : 0.f;
+                b0 = v0 ? __ldg(qs_r + (size_t)delta * ns8 + si) : 0.f;
+                b1 = v1 ? __ldg(qs_r + (size_t)(delta + 8) * ns8 + si) : 0.f;
             }
             const ptrdiff_t off = (ptrdiff_t)delta * RS - kLane<D> * tig, offd = (ptrdiff_t)delta * OS - kLane<D> * tig;
             RowFrag<D> qf0, qf1, df0, df1;
@@ -1158,18 +1103,14 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
     store_acc_rows<D, AL>(dV, dvp + (size_t)row_lo * GS, dvp + (size_t)row_hi * GS, ok_lo, ok_hi, gain, gain, tig);   // dV = gain P^T.dO
 }
 
-inline size_t dkdv_smem_bytes(int n_dense, int WB, bool se) {
-    return se ? (size_t)(kRows + WB) * (n_dense + 1) * 4 : 0;
-}
+template <int WB> inline size_t dkdv_smem_bytes(bool se) { return se ? (size_t)(kRows + WB) * kSeKeyPitch<WB> * 4 : 0; }
 
 template <int D, int WB, int G, int CT, bool SE, int ST>
 __global__ void __launch_bounds__(kWarps * 32, CT)
 bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int reduce_stride) {
-    constexpr int NT = (WB + 16) / 8;
     constexpr int kStat = kRows + WB;                  // query rows the CTA's dense windows touch
-    extern __shared__ __align__(16) float qsd[];       // scale_embed: [kStat][n_dense + 1]
+    extern __shared__ __align__(16) float se_tile[];   // scale_embed: [kStat][kSeKeyPitch]
     __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
-    __shared__ int4 qoff_s[SE ? NT * 32 : 1];          // scale_embed: offsets into qsd
     __shared__ float red_s[kReduceThreads];
     __shared__ int2 tap_s[DSQG_MAX_TAPS];
     __shared__ __align__(16) float stat_s[2 * kStat];  // -lse * log2(e) of the rows, then -delta
@@ -1184,23 +1125,8 @@ bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int
         for (int o = cta / reduce_stride; o < n_reduce; o += gridDim.x * gridDim.y / reduce_stride)
             reduce_one_param(a, t.J, o, red_s);
     const int m_cta = blockIdx.x * kRows;
-    const int nd = t.n_dense, ndp = nd + 1, Jp = (t.J + 7) / 8 * 8;
     {
-        const int d_lo = t.d_lo, d_hi = t.d_lo + t.n_dense - 1;
-        if constexpr (!SE) {
-            StartTable<WB>::template fill<true, kWarps * 32>(start_s, a.pos_bias, a.H, h, d_lo, d_hi, a.scale);
-        } else {
-            for (int e = threadIdx.x; e < NT * 32; e += kWarps * 32) {
-                const int nt = e >> 5, gg = (e & 31) >> 2, tt = e & 3;
-                int o[4];
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const int cc = 8 * nt + 2 * tt + (r & 1), delta = cc - (gg + 8 * (r >> 1));
-                    o[r] = cc * ndp + (delta >= d_lo && delta <= d_hi ? delta - d_lo : nd);   // column nd of every row holds the mask value
-                }
-                qoff_s[e] = make_int4(o[0], o[1], o[2], o[3]);
-            }
-        }
+        if constexpr (!SE) StartTable<WB>::template fill<true, kWarps * 32>(start_s, a.pos_bias, a.H, h, t.d_lo, t.d_lo + t.n_dense - 1, a.scale);
         for (int si = threadIdx.x; si < t.n_sparse; si += kWarps * 32)
             tap_s[si] = make_int2(t.sparse[si], __float_as_int(a.pos_bias[(t.n_dense + si) * a.H + h] * kLog2e));
         const float2* rs = reinterpret_cast<const float2*>(a.delta) + (size_t)bh * N;
@@ -1209,51 +1135,30 @@ bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int
             stat_s[i] = -x.x; stat_s[kStat + i] = -x.y;
         }
         if constexpr (SE) {
-            const float* src = a.qs_rows + ((size_t)bh * N + m_cta) * Jp;
-            for (int r = threadIdx.x; r < kStat; r += kWarps * 32) qsd[r * ndp + nd] = kNeg;      // the mask column
-            {
-                // 16-byte loads for the first nd/4*4 columns: lane c4 < nd/4 of warp w takes rows w, w+4, ...;
-                // eight rows per batch in flight
-                const int per_row = nd / 4;
-                constexpr int kBatch = 8;
-                for (int c4 = L.lane; c4 < per_row; c4 += 32) {
+            const SePre P = se_pre_layout<WB>(a.se_pre, t.n_sparse, D);
+            const SeRows rows = {P.hi, P.lo, P.pb + h * SeGeo<WB>::rows(t.n_sparse)};
+            constexpr bool AL = ST != kStridedAny, CI = ST == kContiguous || ST == kKept;
+            const ptrdiff_t RS = CI ? D : (ptrdiff_t)a.in_sn;
+            const __nv_bfloat16* q = static_cast<const __nv_bfloat16*>(a.q) + (CI ? (size_t)bh * N * D : (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh);
 #pragma unroll 1
-                    for (int r0 = L.warp; r0 < kStat; r0 += kWarps * kBatch) {
-                        float4 x[kBatch];
-#pragma unroll
-                        for (int u = 0; u < kBatch; ++u) {
-                            const int r = r0 + kWarps * u;
-                            x[u] = (r < kStat && m_cta + r < N) ? __ldg(reinterpret_cast<const float4*>(src + (size_t)r * Jp) + c4)
-                                                                : make_float4(0.f, 0.f, 0.f, 0.f);
-                        }
-#pragma unroll
-                        for (int u = 0; u < kBatch; ++u) {
-                            const int r = r0 + kWarps * u;
-                            if (r < kStat) {
-                                float* dst = qsd + r * ndp + 4 * c4;
-                                dst[0] = x[u].x; dst[1] = x[u].y; dst[2] = x[u].z; dst[3] = x[u].w;
-                            }
-                        }
-                    }
-                }
-            }
-            // the last nd % 4 columns, one element per thread
-            const int rem = nd & 3, c_first = nd - rem;
-            for (int e = threadIdx.x; e < kStat * rem; e += kWarps * 32) {
-                const int r = e / rem, c = c_first + e - r * rem;
-                qsd[r * ndp + c] = m_cta + r < N ? __ldg(src + (size_t)r * Jp + c) : 0.f;
+            for (int b = L.warp; b < kStat / 16; b += kWarps) {
+                const int r = m_cta + 16 * b + L.g;
+                RowFrag<D> qa, qb;
+                load_row<D, AL>(qa, q + (ptrdiff_t)r * RS, L.tig, r < N);
+                load_row<D, AL>(qb, q + (ptrdiff_t)(r + 8) * RS, L.tig, r + 8 < N);
+                build_se_tile<D, WB, true>(rows, 0, qa, qb, L.g, L.tig, se_tile + 16 * b * kSeKeyPitch<WB>, kSeKeyPitch<WB>, nullptr, 0);
             }
         }
     }
     __syncthreads();
     const int m0 = m_cta + L.warp * 16;
     if (m0 >= N) return;
-    const float* qsd_w = qsd + L.warp * 16 * ndp;
+    const float* se_w = SE ? se_tile + L.warp * 16 * kSeKeyPitch<WB> : nullptr;
     const float* start = StartTable<WB>::lane(start_s, L);
     if (m0 + 16 + WB <= N)
-        dkdv_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, qsd_w, qoff_s, nd, Jp);
+        dkdv_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, se_w);
     else
-        dkdv_tile<D, WB, false, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, qsd_w, qoff_s, nd, Jp);
+        dkdv_tile<D, WB, false, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, se_w);
 }
 
 // Raises a kernel's dynamic shared-memory limit to what this launch needs.  The attribute is set
@@ -1282,7 +1187,7 @@ inline bool aligned_to(size_t bytes, std::initializer_list<const void*> ptrs, st
 
 template <int D, int WB, bool SE, int ST>
 cudaError_t fwd_launch_mode(const FwdArgs& a, const Taps& t, cudaStream_t s) {
-    constexpr int W = FwdTune<D>::warps, rows = 16 * W;
+    constexpr int W = FwdTune<D>::warps, rows = 16 * W * (SE ? FwdTune<D>::tiles_se : 1);
     dim3 grid((a.N + rows - 1) / rows, a.B * a.H);
     size_t smem = 0;
     if constexpr (SE) {
@@ -1326,11 +1231,11 @@ cudaError_t bwd_launch_mode(BwdArgs a, const Taps& t, cudaStream_t s, int stages
     cudaError_t e = cudaSuccess;
     if (stages & DSQG_BWD_STAGE_DQ) {
         if constexpr (SE) {
-            se_prep_kernel<D><<<1, 1024, 0, s>>>(a.scale_embed, a.pos_bias, a.scale, t.J, a.H, t.d_lo, t.n_dense, WB, a.se_pre);
+            se_prep_kernel<D, WB><<<1, 1024, 0, s>>>(a.scale_embed, a.pos_bias, a.scale, t, a.H, a.se_pre);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
         auto kern = bwd_dq_mma_kernel<D, WB, SE ? T::dq_group_se : T::dq_group, SE ? T::dq_ctas_se : T::dq_ctas, SE, ST>;
-        const size_t smem = dq_smem_bytes(t.J, t.n_sparse, D, NT, SE);
+        const size_t smem = dq_smem_bytes<D, WB>(t.J, t.n_sparse, SE);
         static int seen[64] = {0};
         if ((e = ensure_dynamic_smem(kern, smem, seen)) != cudaSuccess) return e;
         kern<<<grid, kWarps * 32, smem, s>>>(a, t);
@@ -1349,7 +1254,7 @@ cudaError_t bwd_launch_mode(BwdArgs a, const Taps& t, cudaStream_t s, int stages
                       4LL * grid.x * grid.y >= n_out;
     if (stages & DSQG_BWD_STAGE_DKDV) {
         auto kern = bwd_dkdv_mma_kernel<D, WB, SE ? T::dkdv_group_se : T::dkdv_group, SE ? T::dkdv_ctas_se : T::dkdv_ctas, SE, ST>;
-        const size_t smem = dkdv_smem_bytes(t.n_dense, WB, SE);
+        const size_t smem = dkdv_smem_bytes<WB>(SE);
         static int seen[64] = {0};
         if ((e = ensure_dynamic_smem(kern, smem, seen)) != cudaSuccess) return e;
         kern<<<grid, kWarps * 32, smem, s>>>(a, t, fuse ? n_out : 0, fuse && (long long)grid.x * grid.y >= n_out ? (int)((long long)grid.x * grid.y / n_out) : 1);
