@@ -451,7 +451,7 @@ fwd_mma_kernel(const FwdArgs a, const Taps t) {
 // resident CTAs per SM the register budget is set for (spills against warps in flight).
 template <int D> struct BwdTune {
     static constexpr int dq_group = D <= 80 ? 2 : 1, dq_ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D == 80 ? 3 : 2));   // D = 32: 98.5 us (108.8 with 4 CTAs, 103.3 with group 1); D = 80: 69.0 us (80 with 2 CTAs)
-    static constexpr int dq_group_se = 1, dq_ctas_se = D == 32 ? 5 : 4;      // with scale_embed: more shared memory and registers per CTA
+    static constexpr int dq_group_se = D == 32 ? 2 : 1, dq_ctas_se = 4;    // with scale_embed: D = 32 172 us (180 with group 1 and 5 CTAs), D = 64 231 us (242 with group 2)
     static constexpr int dkdv_group_se = D <= 64 ? 2 : 1, dkdv_ctas_se = D == 32 ? 4 : 3;
     static constexpr int dkdv_group = D <= 80 ? 2 : 1, dkdv_ctas = D == 32 ? 4 : (D <= 64 ? 3 : 2);   // D = 80: 78.1 us (83 with group 1, 96-109 with 3 CTAs)
 };
