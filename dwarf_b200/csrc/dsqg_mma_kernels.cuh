@@ -411,14 +411,26 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
 // resident CTAs per SM the register budget is set for.
 template <int D> struct FwdTune {
     static constexpr int warps = 4, group = D == 64 || D > 80 ? 1 : 2, ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));   // D = 64: 104.8 us (107.8 with group 2)
-    // with scale_embed; two tiles per warp share the table: 96.0 us (98.6 with one, 97.6 with four), D = 64 126.7 (133.1, 130.8)
-    static constexpr int group_se = 2, ctas_se = D == 32 ? 5 : 4, tiles_se = 2;
+    // With scale_embed a CTA first lays out the table, about a quarter of a tile's time, so a warp does up to three tiles with it.
+    // The count is the one for which (waves of CTAs) x (tiles + 1/4) is least: one where the grid is a single wave (2x8x777x32 11.6 us,
+    // 12.5 with two), two or three where that saves a wave or its table (4x8x2048x32 19.5 -> 18.7, 32x8x2048x32 101.4 -> 97.3,
+    // 8x12x2048x64 73.9 -> 69.1; a fixed two would take 8x8x2048x32 from 30.0 to 33.1, three gives 28.9).
+    static int tiles_se(int N, int BH) {
+        int best = 1;
+        long long least = 0;
+        for (int t = 1; t <= 3; ++t) {
+            const long long n = (long long)((N + 16 * warps * t - 1) / (16 * warps * t)) * BH, cost = (n + 148 * ctas_se - 1) / (148 * ctas_se) * (4 * t + 1);
+            if (t == 1 || cost < least) { least = cost; best = t; }
+        }
+        return best;
+    }
+    static constexpr int group_se = 2, ctas_se = D == 32 ? 5 : 4;
 };
 
 // ST: addressing (kContiguous ...); with strides and a gate tensor the epilogue multiplies by sigmoid(gate).
 template <int D, int WB, bool SE, int ST>
 __global__ void __launch_bounds__(FwdTune<D>::warps * 32, SE ? FwdTune<D>::ctas_se : FwdTune<D>::ctas)
-fwd_mma_kernel(const FwdArgs a, const Taps t) {
+fwd_mma_kernel(const FwdArgs a, const Taps t, const int tiles_se) {
     constexpr int W = FwdTune<D>::warps, G = SE ? FwdTune<D>::group_se : FwdTune<D>::group;
     extern __shared__ __align__(16) float se_smem[];      // scale_embed: the table, then a tile per warp
     __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
@@ -436,14 +448,14 @@ fwd_mma_kernel(const FwdArgs a, const Taps t) {
     __syncthreads();
     const float* start = StartTable<WB>::lane(start_s, L);
     float* se_tile = SE ? se_smem + se_rows_bytes<WB>(t.n_sparse, D) / 4 + L.warp * se_tile_floats<WB>(t.n_sparse) : se_smem;
-    constexpr int kTiles = SE ? FwdTune<D>::tiles_se : 1;
+    const int tiles = SE ? tiles_se : 1;
 #pragma unroll 1
-    for (int i = 0; i < kTiles; ++i) {
-        const int g0 = (blockIdx.x * kTiles + i) * (16 * W) + L.warp * 16;
+    for (int i = 0; i < tiles; ++i) {
+        const int g0 = (blockIdx.x * tiles + i) * (16 * W) + L.warp * 16;
         if (g0 >= N) return;
         if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
         else fwd_tile<D, WB, false, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
-        if (kTiles > 1) __syncwarp();
+        if (SE) __syncwarp();
     }
 }
 
@@ -1187,7 +1199,8 @@ inline bool aligned_to(size_t bytes, std::initializer_list<const void*> ptrs, st
 
 template <int D, int WB, bool SE, int ST>
 cudaError_t fwd_launch_mode(const FwdArgs& a, const Taps& t, cudaStream_t s) {
-    constexpr int W = FwdTune<D>::warps, rows = 16 * W * (SE ? FwdTune<D>::tiles_se : 1);
+    constexpr int W = FwdTune<D>::warps;
+    const int tiles_se = SE ? FwdTune<D>::tiles_se(a.N, a.B * a.H) : 1, rows = 16 * W * tiles_se;
     dim3 grid((a.N + rows - 1) / rows, a.B * a.H);
     size_t smem = 0;
     if constexpr (SE) {
@@ -1196,7 +1209,7 @@ cudaError_t fwd_launch_mode(const FwdArgs& a, const Taps& t, cudaStream_t s) {
         const cudaError_t e = ensure_dynamic_smem(fwd_mma_kernel<D, WB, SE, ST>, smem, seen);
         if (e != cudaSuccess) return e;
     }
-    fwd_mma_kernel<D, WB, SE, ST><<<grid, W * 32, smem, s>>>(a, t);
+    fwd_mma_kernel<D, WB, SE, ST><<<grid, W * 32, smem, s>>>(a, t, tiles_se);
     return cudaGetLastError();
 }
 
