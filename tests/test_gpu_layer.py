@@ -1,0 +1,92 @@
+"""The layer around the operator in native code: its elementwise and reduction kernels against fp32 PyTorch, and the two autograd
+nodes (attention layer, interference block) against the same modules in fp32."""
+import ctypes
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+import dwarf_b200
+from dwarf_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _stream():
+    return torch.cuda.current_stream().cuda_stream
+
+
+def _close(x, ref, rel, name):
+    x, ref = x.double(), ref.double()
+    assert torch.isfinite(x).all() and (x - ref).norm() <= rel * ref.norm() + 1e-6, (name, (x - ref).norm().item(), ref.norm().item())
+
+
+@pytest.mark.parametrize("rows,D", [(1, 8), (3, 40), (8, 256), (301, 264), (2400, 512), (33, 1024)])
+def test_layer_norm_and_column_sums(rows, D):
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, w, b, dy, dyb = rnd(rows, D) * 2 + 0.5, rnd(D), rnd(D), rnd(rows, D), rnd(rows, D).bfloat16()
+    y, yb, stat = torch.empty_like(x), torch.empty_like(dyb), torch.empty(rows, 2, device="cuda")
+    _lib.check(lib.dsqg_layer_norm_fwd(x.data_ptr(), w.data_ptr(), b.data_ptr(), 1e-5, y.data_ptr(), yb.data_ptr(), stat.data_ptr(), rows, D, _stream()), "fwd")
+    xr, wr, br = (t.double().requires_grad_(True) for t in (x, w, b))
+    ref = F.layer_norm(xr, (D,), wr, br, 1e-5)
+    _close(y, ref.detach(), 1e-5, "y")
+    assert torch.equal(yb, y.bfloat16())
+    dx, dwb = torch.empty_like(x), torch.empty(2, D, device="cuda")
+    n = lib.dsqg_layer_norm_bwd_scratch_bytes(rows, D)
+    sc = torch.empty(n, dtype=torch.uint8, device="cuda")
+    _lib.check(lib.dsqg_layer_norm_bwd(x.data_ptr(), stat.data_ptr(), w.data_ptr(), dy.data_ptr(), dyb.data_ptr(), dx.data_ptr(), dwb.data_ptr(),
+                                       sc.data_ptr(), n, rows, D, _stream()), "bwd")
+    grads = torch.autograd.grad(ref, [xr, wr, br], dy.double() + dyb.double())
+    for got, want, nm in zip((dx, dwb[0], dwb[1]), grads, ("dx", "dgamma", "dbeta")):
+        _close(got, want, 1e-5, nm)
+    # two matrices at once, the second a block of columns of a wider one
+    wide = rnd(rows, D + 72).bfloat16()
+    out = torch.empty(D + 64, device="cuda")
+    arr = lambda t, v: (t * 2)(*v)  # noqa: E731
+    _lib.check(lib.dsqg_column_sums(arr(ctypes.c_void_p, [dyb.data_ptr(), wide.data_ptr() + 16]), arr(ctypes.c_longlong, [D, D + 72]), arr(ctypes.c_int, [D, 64]),
+                                    arr(ctypes.c_void_p, [out.data_ptr(), out.data_ptr() + 4 * D]), 2, rows, _stream()), "sums")
+    _close(out, torch.cat([dyb.double().sum(0), wide[:, 8:72].double().sum(0)]), 1e-5, "sums")
+
+
+@pytest.mark.parametrize("B,N,D", [(1, 1, 8), (2, 31, 72), (1, 33, 64), (3, 257, 40), (1, 1025, 256), (1, 5000, 64)])
+def test_gated_mean(B, N, D):
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(N)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    x, gate, dinter = rnd(B, N, D), rnd(B, N, D).bfloat16(), rnd(B, N, D).bfloat16()
+    pool, inter = torch.empty_like(x), torch.empty_like(gate)
+    _lib.check(lib.dsqg_gated_mean(x.data_ptr(), gate.data_ptr(), pool.data_ptr(), inter.data_ptr(), B, N, D, _stream()), "fwd")
+    xr, gr = x.double().requires_grad_(True), gate.double().requires_grad_(True)
+    pr = xr.cumsum(1) / torch.arange(1, N + 1, device="cuda")[None, :, None]
+    ref = torch.sigmoid(gr) * pr
+    _close(pool, pr.detach(), 1e-5, "pool")
+    _close(inter, ref.detach(), 4e-3, "inter")
+    dg, dx = torch.empty_like(gate), torch.empty_like(x)
+    _lib.check(lib.dsqg_gated_mean_bwd(dinter.data_ptr(), gate.data_ptr(), pool.data_ptr(), dg.data_ptr(), dx.data_ptr(), B, N, D, _stream()), "bwd")
+    want = torch.autograd.grad(ref, [xr, gr], dinter.double())
+    _close(dx, want[0], 1e-2, "dx")
+    _close(dg, want[1], 1e-2, "dg")
+
+
+@pytest.mark.parametrize("B,N,dim,H", [(1, 1, 64, 2), (2, 33, 256, 8), (1, 300, 128, 2), (3, 129, 96, 3)])
+@pytest.mark.parametrize("inject", [False, True])
+def test_layer_under_autocast_vs_fp32(B, N, dim, H, inject):
+    torch.manual_seed(N)
+    attn = dwarf_b200.DSQGAttentionQW(dim, H, dropout=0.0).cuda()
+    block = dwarf_b200.InterferenceInjection(dim, H).cuda()
+    torch.nn.init.normal_(attn.scale_embed, 0, 0.1)
+    x = torch.randn(B, N, dim, device="cuda", requires_grad=True)
+    dy = torch.randn(B, N, dim, device="cuda").bfloat16()
+    # a bias on every key moves all scores of a query alike, so that its gradient is zero but for rounding
+    named = [("x", x), *attn.named_parameters()] + ([(k, p) for k, p in block.named_parameters() if k != "inter_k_proj.bias"] if inject else [])
+
+    def run(autocast):
+        with torch.autocast("cuda", dtype=torch.bfloat16, enabled=autocast):
+            y = attn(x, kv_inject=block(x) if inject else None)
+        return [y.detach()] + list(torch.autograd.grad(y, [p for _, p in named], dy.to(y.dtype)))
+    for (name, _), got, want in zip([("y", None)] + named, run(True), run(False)):
+        assert got.shape == want.shape
+        got, want = got.double(), want.double()
+        assert (got - want).norm() <= 3e-2 * want.norm() + 1e-2 * got.numel() ** 0.5, (name, (got - want).norm().item(), want.norm().item())
