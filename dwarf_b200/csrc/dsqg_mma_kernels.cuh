@@ -507,13 +507,16 @@ template <int WB> struct DsStage {
 
 // Extras of the dQ kernel with scale_embed.  A warp's tile of start values (build_se_tile) becomes its tile of ds values: every
 // element is read and then overwritten by the lane that owns it, and the sparse taps follow the dense ones at column
-// WB + 17, so that columns 16 .. 16 (steps + 1) are dS in the order of the table rows and the products dS.SE and dS^T.Q read it in place.
+// WB + 17, so that columns 16 .. 16 (steps + 1) are dS in the order of the table rows.  The products dS.SE take their operand from there; its
+// bf16 fragments are also stored row by row (ds16), from where ldmatrix.trans hands them to the products dS^T.Q of the whole CTA
+// (four words of the fp32 tile per fragment register instead: dQ stage at 32x8x2048x32 172 us, now 162 us; 16x12x2048x64 231 and 216 us).
 template <int WB> struct SeBwd {
     SeRows rows;
     const uint2* seb;            // table as B fragments of dS.SE (global memory, written by se_prep_kernel)
     unsigned char* q_s;          // the CTA's 64 query rows as bf16 in shared memory, row pitch 2D+16 bytes (conflict-free ldmatrix)
     float* tile; float* sparse;  // this warp's
-    int pitch, sp;
+    unsigned char* ds16;         // this warp's 16 rows of dS as bf16, row pitch pitch16 bytes (an odd multiple of 16: conflict-free)
+    int pitch, sp, pitch16;
     static constexpr int kSparse = WB + 17;                                                              // column of the first sparse tap
     static __host__ __device__ int steps(int ns) { return (WB + 1 + ns + 15) / 16; }                      // 16-column steps of dS
     static __host__ __device__ int pitch_for(int ns) {                                                    // 9 mod 32
@@ -522,6 +525,7 @@ template <int WB> struct SeBwd {
     }
     // floats per warp; the odd multiple of 8 puts the tiles two warps apart 16 banks apart (column sums)
     static __host__ __device__ int floats(int ns) { return 16 * (pitch_for(ns) + SeGeo<WB>::sparse_pitch(ns)) + 8; }
+    static __host__ __device__ int pitch16_for(int ns) { return 32 * steps(ns) + 16; }
     // tap of column 16 + p of dS, -1: none
     static __device__ __forceinline__ int tap(const Taps& t, int p) {
         const int j = p <= WB ? WB - p - t.d_lo : t.n_dense + p - WB - 1;
@@ -748,6 +752,9 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
             const float* hi = lo + 8 * sb.pitch;
             const uint32_t a0 = pack_bf16x2(lo[0], lo[1]), a1 = pack_bf16x2(hi[0], hi[1]);
             const uint32_t a2 = pack_bf16x2(lo[8], lo[9]), a3 = pack_bf16x2(hi[8], hi[9]);
+            unsigned char* d16 = sb.ds16 + g * sb.pitch16 + 32 * kk + 4 * tig;
+            *reinterpret_cast<uint32_t*>(d16) = a0; *reinterpret_cast<uint32_t*>(d16 + 16) = a2;
+            *reinterpret_cast<uint32_t*>(d16 + 8 * sb.pitch16) = a1; *reinterpret_cast<uint32_t*>(d16 + 8 * sb.pitch16 + 16) = a3;
 #pragma unroll
             for (int jn = 0; jn < D / 8; ++jn) {
                 const uint2 b = __ldg(sb.seb + (kk * (D / 8) + jn) * 32 + L.lane);
@@ -810,10 +817,10 @@ __global__ void se_prep_kernel(const float* __restrict__ scale_embed, const floa
     }
 }
 
-// [kWarps] dgain terms, then per warp a DsStage or, with scale_embed, a SeBwd tile; then the query rows
+// [kWarps] dgain terms, then per warp a DsStage or, with scale_embed, a SeBwd tile; then the query rows and dS as bf16
 template <int D, int WB>
 inline size_t dq_smem_bytes(int J, int ns, bool se) {
-    return sizeof(float) * kWarps * (size_t)(1 + (se ? SeBwd<WB>::floats(ns) : DsStage<WB>::floats(ns, J))) + (se ? (size_t)kRows * (2 * D + 16) : 0);
+    return sizeof(float) * kWarps * (size_t)(1 + (se ? SeBwd<WB>::floats(ns) : DsStage<WB>::floats(ns, J))) + (se ? (size_t)kRows * (2 * D + 16 + SeBwd<WB>::pitch16_for(ns)) : 0);
 }
 
 template <int D, int WB, int G, int CT, bool SE, int ST>
@@ -839,6 +846,8 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
         sb.tile = stage + kWarps + L.warp * per_se;
         sb.sparse = sb.tile + 16 * sb.pitch;
         sb.q_s = reinterpret_cast<unsigned char*>(stage + kWarps + kWarps * per_se);
+        sb.pitch16 = SeBwd<WB>::pitch16_for(t.n_sparse);
+        sb.ds16 = sb.q_s + kRows * (2 * D + 16) + L.warp * 16 * sb.pitch16;
     }
     __syncthreads();
     const int g0 = blockIdx.x * kRows + L.warp * 16;
@@ -855,6 +864,8 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
         if constexpr (SE)
             for (int e = L.lane; e < 16 * (2 * D + 16) / 16; e += 32)
                 reinterpret_cast<uint4*>(sb.q_s + (size_t)L.warp * 16 * (2 * D + 16))[e] = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (SE)
+            for (int e = L.lane; e < sb.pitch16; e += 32) reinterpret_cast<uint4*>(sb.ds16)[e] = make_uint4(0u, 0u, 0u, 0u);
     } else if (g0 >= WB && g0 + 16 <= N) {
         dgrow = dq_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stage_w, t.n_sparse, bh, h, g0, L, sb);
     } else {
@@ -871,6 +882,7 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
         // CTA partial of dscale_embed = scale * dS^T . Q[64 x D]; warp w takes n-tiles w, w+4, ...
         constexpr int QP = 2 * D + 16;
         const uint32_t q_base = static_cast<uint32_t>(__cvta_generic_to_shared(sb.q_s));
+        const uint32_t ds_base = q_base + kRows * QP + ((L.lane & 7) + (L.lane >> 4) * 8) * sb.pitch16 + ((L.lane >> 3) & 1) * 16;
 #pragma unroll 1
         for (int jn = L.warp; jn < D / 8; jn += kWarps) {
 #pragma unroll 1
@@ -878,13 +890,11 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
                 float c[4];
 #pragma unroll
                 for (int kk = 0; kk < kRows / 16; ++kk) {
-                    const float* r0 = stage + kWarps + kk * per_se + 2 * L.tig * sb.pitch + 16 + 16 * mt + L.g;
-                    const float* r8 = r0 + 8 * sb.pitch;
-                    uint32_t b0, b1;
-                    const uint32_t addr = q_base + (16 * kk + (L.lane & 15)) * QP + 16 * jn;
-                    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
-                    const uint32_t a0 = pack_bf16x2(r0[0], r0[sb.pitch]), a1 = pack_bf16x2(r0[8], r0[sb.pitch + 8]);
-                    const uint32_t a2 = pack_bf16x2(r8[0], r8[sb.pitch]), a3 = pack_bf16x2(r8[8], r8[sb.pitch + 8]);
+                    uint32_t a0, a1, a2, a3, b0, b1;
+                    const uint32_t q_at = q_base + (16 * kk + (L.lane & 15)) * QP + 16 * jn, ds_at = ds_base + 16 * kk * sb.pitch16 + 32 * mt;
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(q_at));
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3) : "r"(ds_at));
                     if (kk == 0) mma16816_z(c, a0, a1, a2, a3, b0, b1); else mma16816(c, a0, a1, a2, a3, b0, b1);
                 }
                 // the tile's partial goes to global memory; dse_group_kernel adds the tiles of a group
