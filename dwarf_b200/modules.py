@@ -53,8 +53,10 @@ def _log_linear_bias(offsets, num_heads):
 def _plain(*mods):
     """True when each of the modules is the stock class with fp32-style parameters and nobody listens in on it (hooks): its
     forward may then be part of a larger native node."""
+    if torch.nn.modules.module._has_any_global_hook():
+        return False
     for m, cls in mods:
-        if type(m) is not cls or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or m.bias is None:
+        if type(m) is not cls or "forward" in m.__dict__ or m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or m.bias is None:
             return False
     return True
 
