@@ -255,6 +255,24 @@ def test_causal_mean_forward_and_backward_vs_float64(shape, dtype):
     assert dwarf_b200.causal_mean(x.half().to("cuda:0")).dtype == torch.float16
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 8), (3, 31, 8), (2, 257, 72), (1, 512, 16), (2, 1025, 40), (1, 2048, 24), (2, 2049, 16), (1, 5000, 8)])
+def test_causal_mean_adds_in_its_stated_order(shape):
+    """32 chunks of ceil(N / 32) rows, row by row, chunk sums one after the other: bit for bit, whatever the launch."""
+    B, N, D = shape
+    x = torch.randn(*shape, generator=torch.Generator().manual_seed(N))
+    n = -(-N // 32)
+    want, before = torch.empty_like(x), torch.zeros(B, D)
+    for first in range(0, N, n):
+        run, chunk = before.clone(), torch.zeros(B, D)
+        for r in range(first, min(first + n, N)):
+            run, chunk = run + x[:, r], chunk + x[:, r]
+            want[:, r] = run * (torch.ones(()) / (r + 1))
+        before = before + chunk
+    assert torch.equal(dwarf_b200.causal_mean(x.to("cuda:0")).cpu(), want)
+    assert torch.equal(dwarf_b200.causal_mean(x.bfloat16().to("cuda:0")).cpu().float(),
+                       dwarf_b200.causal_mean(x.bfloat16().float().to("cuda:0")).bfloat16().cpu().float())
+
+
 def test_interference_injection_feeds_kv_inject_like_the_reference_block():
     """The reference's interference block (train/train_2048_condU.py:283-297) written with PyTorch's
     cumsum against InterferenceInjection + DSQGAttentionQW(kv_inject=...): same output, same gradient."""
