@@ -65,6 +65,7 @@ _SIGNATURES = {
     "dsqg_layer_norm_fwd": (c_int, [c_void_p] * 3 + [c_float] + [c_void_p] * 3 + [ctypes.c_longlong, c_int, c_void_p]),
     "dsqg_layer_norm_bwd_scratch_bytes": (c_size_t, [ctypes.c_longlong, c_int]),
     "dsqg_layer_norm_bwd": (c_int, [c_void_p] * 8 + [c_size_t, ctypes.c_longlong, c_int, c_void_p]),
+    "dsqg_layer_norm_bwd_split": (c_int, [c_void_p] * 9 + [c_size_t, ctypes.c_longlong, c_int, c_void_p]),
     "dsqg_gated_mean": (c_int, [c_void_p] * 4 + [c_int] * 3 + [c_void_p]),
     "dsqg_gated_mean_bwd": (c_int, [c_void_p] * 5 + [c_int] * 3 + [c_void_p]),
     "dsqg_packed_keep_bytes": (c_size_t, [c_int] * 4),

@@ -59,10 +59,10 @@ layer_norm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gam
 }
 
 // ---- layer norm backward with dy = dya (fp32) + dyb (bf16): dx, and per-block partial sums of dgamma / dbeta.
-// One warp per row, each warp walks rows a grid apart; a lane keeps the sums of its columns (at most 32: D <= 1024).
+// mean, rstd: `step` elements from row to row.  One warp per row, each warp walks rows a grid apart; a lane keeps the sums of its columns (at most 32: D <= 1024).
 template <int C4>
 __global__ void __launch_bounds__(kT)
-layer_norm_bwd_kernel(const float* __restrict__ x, const float2* __restrict__ stat, const float* __restrict__ gamma,
+layer_norm_bwd_kernel(const float* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, int step, const float* __restrict__ gamma,
                       const float* __restrict__ dya, const __nv_bfloat16* __restrict__ dyb, float* __restrict__ dx,
                       float* __restrict__ part, long long rows, int D) {
     extern __shared__ float sums[];                            // [2][D]
@@ -71,7 +71,7 @@ layer_norm_bwd_kernel(const float* __restrict__ x, const float2* __restrict__ st
 #pragma unroll
     for (int i = 0; i < C4; ++i) dg[i] = db[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     for (long long row = (long long)blockIdx.x * (kT / 32) + warp; row < rows; row += (long long)gridDim.x * (kT / 32)) {
-        const float2 st = stat[row];
+        const float2 st = make_float2(mean[row * step], rstd[row * step]);
         float4 xh[C4], w[C4];
         float s1 = 0.f, s2 = 0.f;
 #pragma unroll
@@ -252,24 +252,35 @@ size_t dsqg_layer_norm_bwd_scratch_bytes(long long rows, int D) {
     return bad_rows(rows, D) ? 0 : (size_t)norm_blocks(rows) * 2 * D * 4;
 }
 
-int dsqg_layer_norm_bwd(const float* x, const float* stat, const float* gamma, const float* dy, const void* dy_bf16, float* dx,
-                        float* dgamma_dbeta, void* scratch, size_t scratch_bytes, long long rows, int D, void* stream) {
-    if (!x || !stat || !gamma || !dy || !dy_bf16 || !dx || !dgamma_dbeta || !scratch) return DSQG_ERR_NULL_POINTER;
+static int norm_bwd(const float* x, const float* mean, const float* rstd, int step, const float* gamma, const float* dy, const void* dy_bf16, float* dx,
+                    float* dgamma_dbeta, void* scratch, size_t scratch_bytes, long long rows, int D, void* stream) {
+    if (!x || !mean || !rstd || !gamma || !dy || !dy_bf16 || !dx || !dgamma_dbeta || !scratch) return DSQG_ERR_NULL_POINTER;
     if (bad_rows(rows, D)) return DSQG_ERR_BAD_SHAPE;
-    if (bad(x) || bad(stat) || bad(gamma) || bad(dy) || bad(dy_bf16) || bad(dx) || bad(dgamma_dbeta) || bad(scratch)) return DSQG_ERR_MISALIGNED;
+    if (bad(x) || bad(gamma) || bad(dy) || bad(dy_bf16) || bad(dx) || bad(dgamma_dbeta) || bad(scratch)) return DSQG_ERR_MISALIGNED;
     if (scratch_bytes < dsqg_layer_norm_bwd_scratch_bytes(rows, D)) return DSQG_ERR_SCRATCH_TOO_SMALL;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned blocks = norm_blocks(rows);
     const size_t smem = (size_t)2 * D * 4;
     float* part = static_cast<float*>(scratch);
-    const float2* st = reinterpret_cast<const float2*>(stat);
     const __nv_bfloat16* db = static_cast<const __nv_bfloat16*>(dy_bf16);
-    if (D <= 256) layer_norm_bwd_kernel<2><<<blocks, kT, smem, s>>>(x, st, gamma, dy, db, dx, part, rows, D);
-    else if (D <= 512) layer_norm_bwd_kernel<4><<<blocks, kT, smem, s>>>(x, st, gamma, dy, db, dx, part, rows, D);
-    else layer_norm_bwd_kernel<8><<<blocks, kT, smem, s>>>(x, st, gamma, dy, db, dx, part, rows, D);
+    if (D <= 256) layer_norm_bwd_kernel<2><<<blocks, kT, smem, s>>>(x, mean, rstd, step, gamma, dy, db, dx, part, rows, D);
+    else if (D <= 512) layer_norm_bwd_kernel<4><<<blocks, kT, smem, s>>>(x, mean, rstd, step, gamma, dy, db, dx, part, rows, D);
+    else layer_norm_bwd_kernel<8><<<blocks, kT, smem, s>>>(x, mean, rstd, step, gamma, dy, db, dx, part, rows, D);
     if (int rc = status()) return rc;
     sum_rows_kernel<<<(2 * D + 31) / 32, kT, 0, s>>>(part, dgamma_dbeta, (int)blocks, 2 * D);
     return status();
+}
+
+int dsqg_layer_norm_bwd(const float* x, const float* stat, const float* gamma, const float* dy, const void* dy_bf16, float* dx,
+                        float* dgamma_dbeta, void* scratch, size_t scratch_bytes, long long rows, int D, void* stream) {
+    if (!stat) return DSQG_ERR_NULL_POINTER;
+    if (bad(stat)) return DSQG_ERR_MISALIGNED;
+    return norm_bwd(x, stat, stat + 1, 2, gamma, dy, dy_bf16, dx, dgamma_dbeta, scratch, scratch_bytes, rows, D, stream);
+}
+
+int dsqg_layer_norm_bwd_split(const float* x, const float* mean, const float* rstd, const float* gamma, const float* dy, const void* dy_bf16, float* dx,
+                              float* dgamma_dbeta, void* scratch, size_t scratch_bytes, long long rows, int D, void* stream) {
+    return norm_bwd(x, mean, rstd, 1, gamma, dy, dy_bf16, dx, dgamma_dbeta, scratch, scratch_bytes, rows, D, stream);
 }
 
 int dsqg_gated_mean(const float* x, const void* g, float* pool, void* inter, int B, int N, int D, void* stream) {

@@ -27,12 +27,14 @@ constexpr int kChunks = 32, kCols = 32, kScanThreads = 256, kTileRows = 128;
 constexpr int kLanes = kCols / 4, kRowThreads = kScanThreads / kLanes;         // threads beside and above one another in the elementwise parts
 
 // The gate of the interference block around the mean (train/train_2048_condU.py:289-293, fp32 mean of bf16-gated channels), so
-// that its products cost no pass of their own.  Forward: inter = sigmoid(g) * mean.  Backward (REVERSE): the summands are
-// dpool = d * sigmoid(g), and dg = d * pool * s (1 - s) is written on the way (d: gradient of inter).
+// that its products cost no pass of their own.  Forward: inter = sigmoid(g) * mean, the sigmoid rounded to bf16 as the modules
+// have it under autocast (torch.sigmoid of a bf16 projection): the K/V deltas are then theirs bit for bit.  Backward (REVERSE): the
+// summands are dpool = d * sigmoid(g), and dg = d * pool * s (1 - s) is written on the way (d: gradient of inter), both with the sigmoid in fp32.
 struct PoolGate {
     const __nv_bfloat16* g; const __nv_bfloat16* d; const float* pool; __nv_bfloat16* out;       // out: inter / dg
 };
 __device__ __forceinline__ float pool_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+__device__ __forceinline__ float bf16_sigmoid(float x) { return __bfloat162float(__float2bfloat16_rn(1.f / (1.f + expf(-x)))); }
 // Four channels of a row.
 __device__ __forceinline__ void load4(const __nv_bfloat16* p, float (&x)[4]) {
     const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
@@ -188,7 +190,7 @@ causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, i
                 store4(out + o, y);
                 if constexpr (GATED && !REVERSE) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) g[u][c] = pool_sigmoid(g[u][c]) * y[c];
+                    for (int c = 0; c < 4; ++c) g[u][c] = bf16_sigmoid(g[u][c]) * y[c];
                     store4(gate.out + o, g[u]);
                 }
             }

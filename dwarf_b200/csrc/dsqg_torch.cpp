@@ -536,14 +536,13 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         const c10::cuda::CUDAGuard guard(x.device());
         const int64_t B = x.size(0), N = x.size(1), D = x.size(2), M = B * N;
         const Tensor xc = f32c(x), gam = f32c(gamma);
-        const Bf16Pack w = cast_bf16({wg, wk, wv, bg, bk, bv});                   // wk, wv and bk, bv are one matrix and one vector
-        Tensor xi = new_tensor({B, N, D}, at::kFloat, x), xib = new_tensor({M, D}, at::kBFloat16, x), stat = new_tensor({M, 2}, at::kFloat, x);
-        check(dsqg_layer_norm_fwd(fptr(xc), fptr(gam), fptr(f32c(beta)), (float)eps, fptr(xi), ptr(xib), fptr(stat), M, (int)D, stream_of(x)), "dsqg_layer_norm_fwd");
-        const Tensor g = linear(xib, w[0], w[3], M, D, D);
+        const auto [xi, mean, rstd] = at::native_layer_norm(xc, {D}, gam, f32c(beta), eps);
+        const Bf16Pack w = cast_bf16({wg, wk, wv, bg, bk, bv, xi});               // wk, wv and bk, bv are one matrix and one vector
+        const Tensor xib = part(w.buf, {M, D}, w.at[6]), g = linear(xib, w[0], w[3], M, D, D);
         Tensor pool = new_like(xi), inter = new_like(g);
         check(dsqg_gated_mean(fptr(xi), ptr(g), fptr(pool), ptr(inter), (int)B, (int)N, (int)D, stream_of(x)), "dsqg_gated_mean");
         const Tensor kv = linear(inter, w[1], w[4], M, 2 * D, D);
-        ctx->save_for_backward({xc, gam, stat, xib, pool, g, inter, w.buf});
+        ctx->save_for_backward({xc, gam, mean, rstd, xib, pool, g, inter, w.buf});
         ctx->saved_data["x_type"] = (int64_t)x.scalar_type();
         return {heads_view(kv, B, H, N, D / H, 2 * D, 0), heads_view(kv, B, H, N, D / H, 2 * D, D)};
     }
@@ -554,7 +553,7 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
     static variable_list run(AutogradContext* ctx, const variable_list& grads) {
         const NoAutocast no_autocast;
         const variable_list s = ctx->get_saved_variables();
-        const Tensor &x = s[0], &gam = s[1], &stat = s[2], &xib = s[3], &pool = s[4], &g = s[5], &inter = s[6], &w = s[7];
+        const Tensor &x = s[0], &gam = s[1], &mean = s[2], &rstd = s[3], &xib = s[4], &pool = s[5], &g = s[6], &inter = s[7], &w = s[8];
         const c10::cuda::CUDAGuard guard(x.device());
         const int64_t D = x.size(2), M = x.size(0) * x.size(1);
         // [M, 2 D]: the gradients of an attention layer lie like that already
@@ -583,7 +582,8 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         Tensor dx = new_like(x), dgb = new_tensor({2 * D}, at::kFloat, x);
         const size_t bytes = dsqg_layer_norm_bwd_scratch_bytes(M, (int)D);
         const at::DataPtr scratch = scratch_for(bytes);
-        check(dsqg_layer_norm_bwd(fptr(x), fptr(stat), fptr(gam), fptr(dxi), ptr(dxib), fptr(dx), fptr(dgb), scratch.get(), bytes, M, (int)D, stream), "dsqg_layer_norm_bwd");
+        check(dsqg_layer_norm_bwd_split(fptr(x), fptr(mean), fptr(rstd), fptr(gam), fptr(dxi), ptr(dxib), fptr(dx), fptr(dgb), scratch.get(), bytes, M, (int)D, stream),
+              "dsqg_layer_norm_bwd_split");
         return {like_param(dx, (at::ScalarType)ctx->saved_data["x_type"].toInt()), part(dgb, {D}, 0), part(dgb, {D}, D), dwg, part(db, {D}, 0),
                 part(dwkv, {D, D}, 0), part(db, {D}, D), part(dwkv, {D, D}, D * D), part(db, {D}, 2 * D), Tensor(), Tensor()};
     }

@@ -283,8 +283,9 @@ int dsqg_packed_bwd(const dsqg_packed* p, const dsqg_packed_grads* g, void* scra
  * ops around the reference's layer, DWARF train/train_2048_condU.py:171-191 and the interference block :277-295):
  *   dsqg_cast_bf16       fp32 -> bf16 for up to DSQG_CAST_MAX tensors (lengths multiples of 8) in one launch
  *   dsqg_layer_norm_fwd  y = (x - mean) * rstd * gamma + beta in fp32 and bf16; stat [rows,2] = {mean, rstd}
- *   dsqg_layer_norm_bwd  its backward for dy = dy (fp32) + dy_bf16; dgamma_dbeta [2,D]
- *   dsqg_gated_mean      pool = dsqg_causal_mean(x) in fp32 and inter = sigmoid(g) * pool; x, pool, dx fp32, the rest bf16
+ *   dsqg_layer_norm_bwd  its backward for dy = dy (fp32) + dy_bf16; dgamma_dbeta [2,D]; _split: with mean [rows] and rstd [rows]
+ *   dsqg_gated_mean      pool = dsqg_causal_mean(x) in fp32 and inter = sigmoid(g) * pool, the sigmoid rounded to bf16 (as
+ *                        torch.sigmoid gives it for a bf16 g); x, pool, dx fp32, the rest bf16
  *   dsqg_gated_mean_bwd  dg and dx for the gradient dinter of inter
  *   dsqg_inject_kv       columns [D,2D) and [2D,3D) of qkv += k_delta, v_delta (rows qkv_stride / delta_stride elements apart)
  *   dsqg_column_sums     fp32 column sums of up to DSQG_SUM_MAX bf16 matrices of the same number of rows, fixed order
@@ -297,6 +298,8 @@ int dsqg_layer_norm_fwd(const float* x, const float* gamma, const float* beta, f
 size_t dsqg_layer_norm_bwd_scratch_bytes(long long rows, int D);
 int dsqg_layer_norm_bwd(const float* x, const float* stat, const float* gamma, const float* dy, const void* dy_bf16, float* dx,
                         float* dgamma_dbeta, void* scratch, size_t scratch_bytes, long long rows, int D, void* stream);
+int dsqg_layer_norm_bwd_split(const float* x, const float* mean, const float* rstd, const float* gamma, const float* dy, const void* dy_bf16, float* dx,
+                              float* dgamma_dbeta, void* scratch, size_t scratch_bytes, long long rows, int D, void* stream);
 int dsqg_gated_mean(const float* x, const void* g, float* pool, void* inter, int B, int N, int D, void* stream);
 int dsqg_gated_mean_bwd(const void* dinter, const void* g, const float* pool, void* dg, float* dx, int B, int N, int D, void* stream);
 int dsqg_inject_kv(void* qkv, long long qkv_stride, const void* k_delta, const void* v_delta, long long delta_stride, long long rows, int D, void* stream);

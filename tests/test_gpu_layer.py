@@ -90,3 +90,32 @@ def test_layer_under_autocast_vs_fp32(B, N, dim, H, inject):
         assert got.shape == want.shape
         got, want = got.double(), want.double()
         assert (got - want).norm() <= 3e-2 * want.norm() + 1e-2 * got.numel() ** 0.5, (name, (got - want).norm().item(), want.norm().item())
+
+
+@pytest.mark.parametrize("B,N,dim,H", [(1, 1, 64, 2), (3, 701, 256, 8), (2, 97, 96, 3), (1, 300, 1024, 16), (8, 2048, 256, 8)])
+def test_native_layer_gives_what_its_modules_give(B, N, dim, H):
+    """A hook on one projection sends the layer and the interference block through their modules.  The forward rounds at the same places: deltas and output
+    bit for bit.  With them the key gradients agree, and so does even the gradient of the bias on every key, a sum of nothing but their rounding errors;
+    the other gradients are rounded to bf16 at different places on the way (weights: once more in the modules)."""
+    torch.manual_seed(N)
+    attn = dwarf_b200.DSQGAttentionQW(dim, H, dropout=0.0).cuda()
+    block = dwarf_b200.InterferenceInjection(dim, H).cuda()
+    torch.nn.init.normal_(attn.scale_embed, 0, 0.1)
+    x = torch.randn(B, N, dim, device="cuda", requires_grad=True)
+    dy = torch.randn(B, N, dim, device="cuda").bfloat16()
+    named = [("x", x), *attn.named_parameters(), *block.named_parameters()]
+
+    def run(modules):
+        hooks = [m.register_forward_hook(lambda *a: None) for m in (attn.qkv_proj, block.inter_gate)] if modules else []
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            kd, vd = block(x)
+            y = attn(x, kv_inject=(kd, vd))
+        for h in hooks:
+            h.remove()
+        return [kd.detach(), vd.detach(), y.detach()], torch.autograd.grad(y, [p for _, p in named], dy)
+    (fwd, got), (fwd_m, want) = run(False), run(True)
+    for a, b, n in zip(fwd, fwd_m, ("k_delta", "v_delta", "y")):
+        assert torch.equal(a, b), n
+    for (n, _), a, b in zip(named, got, want):
+        a, b = a.double(), b.double()
+        assert (a - b).norm() <= 1e-2 * b.norm(), (n, (a - b).norm().item(), b.norm().item())
