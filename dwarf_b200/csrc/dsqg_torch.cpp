@@ -104,6 +104,10 @@ Tensor f32c(const Tensor& t) {
     if (!t.defined() || (t.scalar_type() == at::kFloat && t.is_contiguous())) return t;
     return t.detach().to(at::kFloat).contiguous();
 }
+// The kernels around the GEMMs and the GEMM plans want 16-byte pointers; a parameter that is a view of a flat buffer, or a caller's
+// activation, may start anywhere and is copied then.
+bool on_16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+Tensor aligned(const Tensor& t) { return !t.defined() || on_16(t.data_ptr()) ? t : t.detach().clone(); }
 Tensor like_param(Tensor g, at::ScalarType dt) { return g.defined() && g.scalar_type() != dt ? g.to(dt) : g; }
 Tensor opt(const std::optional<Tensor>& t) { return t.has_value() ? *t : Tensor(); }
 at::ScalarType type_of(const Tensor& t) { return t.defined() ? t.scalar_type() : at::kFloat; }
@@ -410,6 +414,8 @@ void gemm(void* C, bool f32_out, const void* A, bool ta, const void* B, bool tb,
           int64_t lda = 0) {
     static thread_local std::map<GemmKey, std::unique_ptr<GemmPlan>> plans;
     constexpr size_t kMostPlans = 128;
+    if (!on_16(A) || !on_16(B) || !on_16(C) || !on_16(bias) || lda % 8)                   // what the plans are chosen for
+        throw std::runtime_error("dsqg: GEMM operands must start on 16 bytes");
     cublasLtHandle_t lt = at::cuda::getCurrentCUDABlasLtHandle();
     size_t space = at::cuda::getCUDABlasLtWorkspaceSize();
     const GemmKey key = {on.device().index(), M, N, K, (ta ? 1 : 0) | (tb ? 2 : 0) | (bias ? 4 : 0), f32_out, (int64_t)space, lda};
@@ -480,7 +486,7 @@ Bf16Pack cast_bf16(std::initializer_list<Tensor> src0) {
     Bf16Pack p;
     std::vector<Tensor> src;
     int64_t total = 0;
-    for (const Tensor& t : src0) { src.push_back(f32c(t)); p.at.push_back(total); total += t.numel(); }
+    for (const Tensor& t : src0) { src.push_back(aligned(f32c(t))); p.at.push_back(total); total += t.numel(); }
     p.buf = new_tensor({total}, at::kBFloat16, src[0]);
     const float* sp[DSQG_CAST_MAX]; void* dp[DSQG_CAST_MAX]; long long n[DSQG_CAST_MAX];
     for (size_t k = 0; k < src.size(); ++k) { sp[k] = fptr(src[k]); dp[k] = const_cast<char*>(p[(int)k]); n[k] = src[k].numel(); }
@@ -521,11 +527,11 @@ Tensor heads_view(const Tensor& m, int64_t B, int64_t H, int64_t N, int64_t HD, 
 int64_t heads_stride(const Tensor& t) {
     const int64_t H = t.size(1), N = t.size(2), HD = t.size(3), ld = t.stride(2);
     const bool ok = t.stride(3) == 1 && (H == 1 || t.stride(1) == HD) && ld >= H * HD && ld % 8 == 0 && (t.size(0) == 1 || t.stride(0) == N * ld) &&
-                    (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+                    on_16(t.data_ptr());
     return ok ? ld : 0;
 }
 Tensor rows_of(const Tensor& t) {        // [B,H,N,HD] -> [B*N, H*HD] bf16
-    return t.permute({0, 2, 1, 3}).reshape({t.size(0) * t.size(2), t.size(1) * t.size(3)}).to(at::kBFloat16).contiguous();
+    return aligned(t.permute({0, 2, 1, 3}).reshape({t.size(0) * t.size(2), t.size(1) * t.size(3)}).to(at::kBFloat16).contiguous());
 }
 
 // (k_delta, v_delta) of the interference block (train/train_2048_condU.py:277-295)
@@ -535,8 +541,8 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         const NoAutocast no_autocast;
         const c10::cuda::CUDAGuard guard(x.device());
         const int64_t B = x.size(0), N = x.size(1), D = x.size(2), M = B * N;
-        const Tensor xc = f32c(x), gam = f32c(gamma);
-        const auto [xi, mean, rstd] = at::native_layer_norm(xc, {D}, gam, f32c(beta), eps);
+        const Tensor xc = aligned(f32c(x)), gam = aligned(f32c(gamma));
+        const auto [xi, mean, rstd] = at::native_layer_norm(xc, {D}, gam, aligned(f32c(beta)), eps);
         const Bf16Pack w = cast_bf16({wg, wk, wv, bg, bk, bv, xi});               // wk, wv and bk, bv are one matrix and one vector
         const Tensor xib = part(w.buf, {M, D}, w.at[6]), g = linear(xib, w[0], w[3], M, D, D);
         Tensor pool = new_like(xi), inter = new_like(g);
@@ -600,7 +606,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
         const int64_t B = x.size(0), N = x.size(1), D = x.size(2), M = B * N;
         const bool cast_x = x.scalar_type() == at::kFloat;
         const Bf16Pack w = cast_x ? cast_bf16({wqkv, wg, wo, bqkv, bg, bo, x}) : cast_bf16({wqkv, wg, wo, bqkv, bg, bo});
-        const Tensor xb = cast_x ? part(w.buf, {M, D}, w.at[6]) : x.contiguous();
+        const Tensor xb = cast_x ? part(w.buf, {M, D}, w.at[6]) : aligned(x.contiguous());
         const Tensor proj = linear(xb, w[0], w[3], M, 4 * D, D);
         if (kd.has_value()) {
             Tensor k = *kd, v = *vd;
@@ -628,7 +634,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
         const PackedForward f = {s[2], Tensor(), s[3], s[4], s[5], s[6], s[7], s[8]};
         const int64_t B = f.lse.size(0), H = f.lse.size(1), N = f.lse.size(2), D = f.y.size(2), M = B * N, HD = D / H;
         const c10::cuda::CUDAGuard guard(xb.device());
-        const Tensor dy = bf16c(dy0);
+        const Tensor dy = aligned(bf16c(dy0));
         const char* wb = static_cast<const char*>(ptr(w));
         const Tensor dyo = grad_input(dy, wb + 2 * 4 * D * D, M, D, D, false), dwo = grad_weight(dy, f.y, M, D, D);
         const PackedGrads g = packed_backward(f, dyo, 4 * D, offsets_of(ctx));

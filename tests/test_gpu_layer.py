@@ -119,3 +119,39 @@ def test_native_layer_gives_what_its_modules_give(B, N, dim, H):
     for (n, _), a, b in zip(named, got, want):
         a, b = a.double(), b.double()
         assert (a - b).norm() <= 1e-2 * b.norm(), (n, (a - b).norm().item(), b.norm().item())
+
+
+def _off_by_one(t):
+    """The same values one element off an aligned address (a view of a flat buffer)."""
+    flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    view = flat[1:].view(t.shape)
+    view.copy_(t)
+    assert view.data_ptr() % 16 and view.is_contiguous()
+    return view
+
+
+@pytest.mark.parametrize("x_type", [torch.float32, torch.bfloat16])
+def test_layer_takes_tensors_at_any_address(x_type):
+    """Parameters, inputs, deltas and the upstream gradient that do not start on 16 bytes give what aligned ones give."""
+    B, N, dim, H = 2, 65, 128, 4
+    torch.manual_seed(1)
+    attn = dwarf_b200.DSQGAttentionQW(dim, H, dropout=0.0).cuda()
+    block = dwarf_b200.InterferenceInjection(dim, H).cuda()
+    x0 = torch.randn(B, N, dim, device="cuda", dtype=x_type)
+    dy0 = torch.randn(B, N, dim, device="cuda").bfloat16()
+    d0 = torch.randn(B, N, dim, device="cuda").bfloat16()
+    # scale_embed has to be aligned for the operator itself, with or without a layer around it
+    moved = [(m, n) for mod in (attn, block) for m in mod.modules() for n, _ in m.named_parameters(recurse=False) if n != "scale_embed"]
+    results = []
+    for off in (False, True):
+        place = _off_by_one if off else torch.clone
+        for m, n in moved:
+            setattr(m, n, torch.nn.Parameter(place(getattr(m, n).detach())))
+        x, delta = place(x0).requires_grad_(True), place(d0)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = attn(x, kv_inject=block(x))
+            y2 = attn(x, kv_inject=(delta.view(B, N, H, dim // H).transpose(1, 2),) * 2)
+        wrt = [x, *attn.parameters(), *block.parameters()]
+        results.append([y.detach(), y2.detach(), *torch.autograd.grad(y, wrt, place(dy0))])
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
