@@ -407,7 +407,17 @@ struct GemmPlan {
 void lt_check(cublasStatus_t s, const char* what) {
     if (s != CUBLAS_STATUS_SUCCESS) throw std::runtime_error(std::string("dsqg: ") + what + ": " + cublasGetStatusString(s));
 }
-using GemmKey = std::array<int64_t, 8>;       // device, M, N, K, transposes and bias, output type, workspace, lda
+using GemmKey = std::array<int64_t, 9>;       // device, M, N, K, transposes and bias, output type, workspace, lda, reduction schemes
+
+// The ways a plan may split its contraction, by torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction (as nn.Linear
+// has it): partial sums in the output's 16 bits, in fp32 only, or no split at all.
+uint32_t reduction_schemes() {
+    switch (at::globalContext().allowBF16ReductionCuBLAS()) {
+        case at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK: return CUBLASLT_REDUCTION_SCHEME_MASK;
+        case at::CuBLASReductionOption::DisallowReducedPrecisionAllowSplitK: return CUBLASLT_REDUCTION_SCHEME_COMPUTE_TYPE;
+        default: return CUBLASLT_REDUCTION_SCHEME_NONE;
+    }
+}
 
 // ta: A is stored [K,M]; tb: B is stored [N,K]; lda: elements between A's rows (0: none skipped)
 void gemm(void* C, bool f32_out, const void* A, bool ta, const void* B, bool tb, const void* bias, int64_t M, int64_t N, int64_t K, const Tensor& on,
@@ -418,7 +428,8 @@ void gemm(void* C, bool f32_out, const void* A, bool ta, const void* B, bool tb,
         throw std::runtime_error("dsqg: GEMM operands must start on 16 bytes");
     cublasLtHandle_t lt = at::cuda::getCurrentCUDABlasLtHandle();
     size_t space = at::cuda::getCUDABlasLtWorkspaceSize();
-    const GemmKey key = {on.device().index(), M, N, K, (ta ? 1 : 0) | (tb ? 2 : 0) | (bias ? 4 : 0), f32_out, (int64_t)space, lda};
+    const uint32_t schemes = reduction_schemes();
+    const GemmKey key = {on.device().index(), M, N, K, (ta ? 1 : 0) | (tb ? 2 : 0) | (bias ? 4 : 0), f32_out, (int64_t)space, lda, schemes};
     if (plans.size() >= kMostPlans && !plans.count(key)) plans.clear();
     std::unique_ptr<GemmPlan>& slot = plans[key];
     if (!slot) {
@@ -439,6 +450,7 @@ void gemm(void* C, bool f32_out, const void* A, bool ta, const void* B, bool tb,
         cublasLtMatmulPreference_t pref;
         lt_check(cublasLtMatmulPreferenceCreate(&pref), "cublasLtMatmulPreferenceCreate");
         const uint32_t align = 16;
+        cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_REDUCTION_SCHEME_MASK, &schemes, sizeof schemes);
         cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &space, sizeof space);
         for (auto attr : {CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES,
                           CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_D_BYTES})
@@ -752,6 +764,7 @@ PYBIND11_MODULE(_dsqg_torch, m) {
     m.def("forward_lse", &forward_lse);
     m.def("attention_packed", &attention_packed);
     m.def("layer_applies", &layer_applies);
+    m.def("reduction_schemes", &reduction_schemes);
     m.def("interference", &interference);
     m.def("layer", &layer);
     m.def("causal_mean", &causal_mean);

@@ -138,3 +138,19 @@ def test_odd_head_widths_are_padded_only_when_the_tensor_core_kernels_take_them(
     assert ops._padded_head_dim(q(80, torch.float32), off43, J43, False) == 80
     for D in (32, 64, 96, 128):
         assert ops._padded_head_dim(q(D), off43, J43, False) == D
+
+
+def test_layer_gemms_follow_the_reduced_precision_setting():
+    """The split-K schemes the native layer's GEMM plans may use (cublasLt bits: 1 in place, 2 compute type, 4 output type)."""
+    from dwarf_b200 import _lib
+    n, mm = _lib.native(), torch.backends.cuda.matmul
+    before = mm.allow_bf16_reduced_precision_reduction
+    try:
+        mm.allow_bf16_reduced_precision_reduction = True
+        assert n.reduction_schemes() & 4
+        mm.allow_bf16_reduced_precision_reduction = False
+        assert n.reduction_schemes() == 2
+        mm.allow_bf16_reduced_precision_reduction = (False, False)
+        assert n.reduction_schemes() == 0
+    finally:
+        mm.allow_bf16_reduced_precision_reduction = before
