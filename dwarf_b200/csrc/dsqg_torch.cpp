@@ -515,15 +515,17 @@ Tensor part(const Tensor& buf, at::IntArrayRef sizes, int64_t first) {
 }
 
 struct Columns { const void* p; int64_t ld; int cols; };
-// Column sums of bf16 matrices of `rows` rows, back to back.
+// Column sums of bf16 matrices of `rows` rows, back to back; those without columns are left out.
 Tensor column_sums(std::initializer_list<Columns> ms, int64_t rows, const Tensor& on) {
     int64_t total = 0;
     for (const Columns& m : ms) total += m.cols;
+    if (!total) return Tensor();
     Tensor buf = new_tensor({total}, at::kFloat, on);
     const void* sp[DSQG_SUM_MAX]; long long ld[DSQG_SUM_MAX]; int cols[DSQG_SUM_MAX]; float* dp[DSQG_SUM_MAX];
     int k = 0;
     int64_t o = 0;
     for (const Columns& m : ms) {
+        if (!m.cols) continue;
         sp[k] = m.p; ld[k] = m.ld; cols[k] = m.cols; dp[k] = fptr(buf) + o;
         o += m.cols; ++k;
     }
@@ -574,6 +576,9 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         const Tensor &x = s[0], &gam = s[1], &mean = s[2], &rstd = s[3], &xib = s[4], &pool = s[5], &g = s[6], &inter = s[7], &w = s[8];
         const c10::cuda::CUDAGuard guard(x.device());
         const int64_t D = x.size(2), M = x.size(0) * x.size(1);
+        // what is asked for, of x, gamma, beta, wg, bg, wk, bk, wv, bv
+        const auto need = [&](size_t i) { return ctx->needs_input_grad(i); };
+        const bool n_norm = need(0) || need(1) || need(2), n_in = n_norm || need(3) || need(4), n_wkv = need(5) || need(7), n_bkv = need(6) || need(8);
         // [M, 2 D]: the gradients of an attention layer lie like that already
         Tensor dkv;
         const void* dp = nullptr;
@@ -590,20 +595,31 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         }
         void* stream = stream_of(x);
         const char* wb = static_cast<const char*>(ptr(w));
-        Tensor dinter = new_like(inter), dwkv = new_tensor({2 * D, D}, at::kFloat, x);
-        gemm(ptr(dinter), false, dp, false, wb + 2 * D * D, false, nullptr, M, D, 2 * D, x, ld);
-        gemm(ptr(dwkv), true, dp, true, ptr(inter), false, nullptr, 2 * D, D, M, x, ld);
-        Tensor dg = new_like(g), dxi = new_like(pool);
-        check(dsqg_gated_mean_bwd(ptr(dinter), ptr(g), fptr(pool), ptr(dg), fptr(dxi), (int)x.size(0), (int)x.size(1), (int)D, stream), "dsqg_gated_mean_bwd");
-        const Tensor dxib = grad_input(dg, wb, M, D, D, false), dwg = grad_weight(dg, xib, M, D, D);
-        const Tensor db = column_sums({{ptr(dg), D, (int)D}, {dp, ld, (int)(2 * D)}}, M, x);
-        Tensor dx = new_like(x), dgb = new_tensor({2 * D}, at::kFloat, x);
-        const size_t bytes = dsqg_layer_norm_bwd_scratch_bytes(M, (int)D);
-        const at::DataPtr scratch = scratch_for(bytes);
-        check(dsqg_layer_norm_bwd_split(fptr(x), fptr(mean), fptr(rstd), fptr(gam), fptr(dxi), ptr(dxib), fptr(dx), fptr(dgb), scratch.get(), bytes, M, (int)D, stream),
-              "dsqg_layer_norm_bwd_split");
-        return {like_param(dx, (at::ScalarType)ctx->saved_data["x_type"].toInt()), part(dgb, {D}, 0), part(dgb, {D}, D), dwg, part(db, {D}, 0),
-                part(dwkv, {D, D}, 0), part(db, {D}, D), part(dwkv, {D, D}, D * D), part(db, {D}, 2 * D), Tensor(), Tensor()};
+        Tensor dinter, dwkv, dg, dxi, dwg, dx, dgb;
+        if (n_wkv) {
+            dwkv = new_tensor({2 * D, D}, at::kFloat, x);
+            gemm(ptr(dwkv), true, dp, true, ptr(inter), false, nullptr, 2 * D, D, M, x, ld);
+        }
+        if (n_in) {
+            dinter = new_like(inter); dg = new_like(g); dxi = new_like(pool);
+            gemm(ptr(dinter), false, dp, false, wb + 2 * D * D, false, nullptr, M, D, 2 * D, x, ld);
+            check(dsqg_gated_mean_bwd(ptr(dinter), ptr(g), fptr(pool), ptr(dg), fptr(dxi), (int)x.size(0), (int)x.size(1), (int)D, stream), "dsqg_gated_mean_bwd");
+        }
+        if (need(3)) dwg = grad_weight(dg, xib, M, D, D);
+        const Tensor db = column_sums({{ptr(dg), D, need(4) ? (int)D : 0}, {dp, ld, n_bkv ? (int)(2 * D) : 0}}, M, x);
+        if (n_norm) {
+            const Tensor dxib = grad_input(dg, wb, M, D, D, false);
+            dx = new_like(x); dgb = new_tensor({2 * D}, at::kFloat, x);
+            const size_t bytes = dsqg_layer_norm_bwd_scratch_bytes(M, (int)D);
+            const at::DataPtr scratch = scratch_for(bytes);
+            check(dsqg_layer_norm_bwd_split(fptr(x), fptr(mean), fptr(rstd), fptr(gam), fptr(dxi), ptr(dxib), fptr(dx), fptr(dgb), scratch.get(), bytes, M, (int)D, stream),
+                  "dsqg_layer_norm_bwd_split");
+        }
+        const auto piece = [&](bool wanted, const Tensor& buf, at::IntArrayRef sizes, int64_t first) { return wanted ? part(buf, sizes, first) : Tensor(); };
+        const int64_t kv = need(4) ? D : 0;                    // where the sums of the two biases begin
+        return {need(0) ? like_param(dx, (at::ScalarType)ctx->saved_data["x_type"].toInt()) : Tensor(), piece(need(1), dgb, {D}, 0), piece(need(2), dgb, {D}, D),
+                dwg, piece(need(4), db, {D}, 0), piece(need(5), dwkv, {D, D}, 0), piece(need(6), db, {D}, kv), piece(need(7), dwkv, {D, D}, D * D),
+                piece(need(8), db, {D}, kv + D), Tensor(), Tensor()};
     }
 };
 
@@ -648,22 +664,37 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
         const c10::cuda::CUDAGuard guard(xb.device());
         const Tensor dy = aligned(bf16c(dy0));
         const char* wb = static_cast<const char*>(ptr(w));
-        const Tensor dyo = grad_input(dy, wb + 2 * 4 * D * D, M, D, D, false), dwo = grad_weight(dy, f.y, M, D, D);
-        const PackedGrads g = packed_backward(f, dyo, 4 * D, offsets_of(ctx));
-        const Tensor dw = grad_weight(g.dproj, xb, M, 4 * D, D);
-        const Tensor db = column_sums({{ptr(g.dproj), 4 * D, (int)(4 * D)}, {ptr(dy), D, (int)D}}, M, xb);
+        // what is asked for; edges exist for the tensors that were given
         const auto xt = ctx->saved_data["x_types"].toIntVector();
-        Tensor dx, dk, dv;
-        if (ctx->needs_input_grad(0)) {
+        const bool inject = ctx->saved_data["inject"].toBool();
+        size_t edge = 0;
+        const auto need = [&](bool given = true) { return given && ctx->needs_input_grad(edge++); };
+        const bool n_x = need(), n_k = need(inject), n_v = need(inject), n_wqkv = need(), n_bqkv = need(), n_wg = need(), n_bg = need(), n_wo = need(),
+                   n_bo = need(), n_pb = need(), n_hg = need(f.hg.defined()), n_se = need(f.se.defined());
+        Tensor dx, dk, dv, dw, dwo;
+        PackedGrads g;
+        if (n_wo) dwo = grad_weight(dy, f.y, M, D, D);
+        if (n_x || n_k || n_v || n_wqkv || n_bqkv || n_wg || n_bg || n_pb || n_hg || n_se)
+            g = packed_backward(f, grad_input(dy, wb + 2 * 4 * D * D, M, D, D, false), 4 * D, offsets_of(ctx));
+        // of the columns [qkv | gate], those from `first` on up to `last`
+        const int64_t first = n_wqkv ? 0 : 3 * D, last = n_wg ? 4 * D : 3 * D, sum_first = n_bqkv ? 0 : 3 * D, sum_last = n_bg ? 4 * D : 3 * D;
+        const auto column = [&](int64_t c) { return static_cast<const char*>(ptr(g.dproj)) + 2 * c; };
+        if (last > first) {
+            dw = new_tensor({last - first, D}, at::kFloat, dy);
+            gemm(ptr(dw), true, column(first), true, ptr(xb), false, nullptr, last - first, D, M, dy, 4 * D);
+        }
+        const int sums = (int)std::max<int64_t>(sum_last - sum_first, 0);
+        const Tensor db = column_sums({{sums ? column(sum_first) : nullptr, 4 * D, sums}, {ptr(dy), D, n_bo ? (int)D : 0}}, M, xb);
+        if (n_x) {
             const auto t = (at::ScalarType)xt[0];
             dx = like_param(grad_input(g.dproj, wb, M, 4 * D, D, t == at::kFloat).view({B, N, D}), t);
         }
-        if (ctx->saved_data["inject"].toBool()) {
-            dk = like_param(heads_view(g.dproj, B, H, N, HD, 4 * D, D), (at::ScalarType)xt[1]);
-            dv = like_param(heads_view(g.dproj, B, H, N, HD, 4 * D, 2 * D), (at::ScalarType)xt[2]);
-        }
-        return {dx, dk, dv, part(dw, {3 * D, D}, 0), part(db, {3 * D}, 0), part(dw, {D, D}, 3 * D * D), part(db, {D}, 3 * D), dwo, part(db, {D}, 4 * D),
-                like_param(g.dpb, type_at(ctx, 0)), like_param(g.dhg, type_at(ctx, 1)), like_param(g.dse, type_at(ctx, 2)), Tensor(), Tensor(), Tensor()};
+        if (n_k) dk = like_param(heads_view(g.dproj, B, H, N, HD, 4 * D, D), (at::ScalarType)xt[1]);
+        if (n_v) dv = like_param(heads_view(g.dproj, B, H, N, HD, 4 * D, 2 * D), (at::ScalarType)xt[2]);
+        const auto piece = [&](bool wanted, const Tensor& buf, at::IntArrayRef sizes, int64_t at) { return wanted ? part(buf, sizes, at) : Tensor(); };
+        return {dx, dk, dv, piece(n_wqkv, dw, {3 * D, D}, 0), piece(n_bqkv, db, {3 * D}, 0), piece(n_wg, dw, {D, D}, (3 * D - first) * D), piece(n_bg, db, {D}, 3 * D - sum_first),
+                dwo, piece(n_bo, db, {D}, sums), n_pb ? like_param(g.dpb, type_at(ctx, 0)) : Tensor(), n_hg ? like_param(g.dhg, type_at(ctx, 1)) : Tensor(),
+                n_se ? like_param(g.dse, type_at(ctx, 2)) : Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 

@@ -155,3 +155,39 @@ def test_layer_takes_tensors_at_any_address(x_type):
         results.append([y.detach(), y2.detach(), *torch.autograd.grad(y, wrt, place(dy0))])
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+def test_frozen_parameters_get_no_gradient_and_cost_none():
+    """Each gradient on its own equals its part of the full set, and a backward for the input alone makes no weight gradients."""
+    B, N, dim, H = 1, 65, 1024, 16
+    torch.manual_seed(3)
+    attn = dwarf_b200.DSQGAttentionQW(dim, H, dropout=0.0).cuda()
+    block = dwarf_b200.InterferenceInjection(dim, H).cuda()
+    torch.nn.init.normal_(attn.scale_embed, 0, 0.1)
+    x = torch.randn(B, N, dim, device="cuda", requires_grad=True)
+    dy = torch.randn(B, N, dim, device="cuda").bfloat16()
+    params = [x, *attn.parameters(), *block.parameters()]
+
+    def run():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return attn(x, kv_inject=block(x))
+    want = torch.autograd.grad(run(), params, dy)
+    for i, p in enumerate(params):
+        for q in params:
+            q.requires_grad_(q is p)
+        got = torch.autograd.grad(run(), [p], dy)[0]
+        # one product over fewer columns may be cut up in another way
+        assert got.dtype == want[i].dtype and (got - want[i]).norm() <= 1e-5 * want[i].norm(), i
+        y = run()
+        y.backward(dy)
+        assert all((q.grad is not None) == (q is p) for q in params)
+        p.grad = None
+    for q in params:
+        q.requires_grad_(q is x)
+    y = run()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    torch.autograd.grad(y, [x], dy)
+    # scratch and activations of 65 rows against 32 MB of weight gradients
+    assert torch.cuda.max_memory_allocated() - before < 16 << 20
