@@ -72,6 +72,7 @@ _SIGNATURES = {
     "dsqg_packed_fwd": (c_int, [c_void_p] * 2),
     "dsqg_packed_bwd_scratch_bytes": (c_size_t, [c_void_p]),
     "dsqg_packed_bwd": (c_int, [c_void_p] * 3 + [c_size_t, c_void_p]),
+    "dsqg_packed_bwd_gate": (c_int, [c_void_p] * 2 + [POINTER(Strides), c_void_p, c_size_t, c_void_p]),
     "dsqg_inject_kv": (c_int, [c_void_p, ctypes.c_longlong] + [c_void_p] * 2 + [ctypes.c_longlong] * 2 + [c_int, c_void_p]),
     "dsqg_column_sums": (c_int, [POINTER(c_void_p), POINTER(ctypes.c_longlong), POINTER(c_int), POINTER(c_void_p), c_int,
                                  ctypes.c_longlong, c_void_p]),

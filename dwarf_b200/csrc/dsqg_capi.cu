@@ -339,6 +339,10 @@ size_t dsqg_packed_bwd_scratch_bytes(const dsqg_packed* p) {
 }
 
 int dsqg_packed_bwd(const dsqg_packed* p, const dsqg_packed_grads* g, void* scratch, size_t scratch_bytes, void* stream) {
+    return dsqg_packed_bwd_gate(p, g, nullptr, scratch, scratch_bytes, stream);
+}
+
+int dsqg_packed_bwd_gate(const dsqg_packed* p, const dsqg_packed_grads* g, const dsqg_strides* dgate_strides, void* scratch, size_t scratch_bytes, void* stream) {
     if (!p || !g || !scratch) return DSQG_ERR_NULL_POINTER;
     const int B = p->B, H = p->H, N = p->N, D = p->D;
     int rc = check_op_shape(B, H, N, D, DSQG_DTYPE_BF16);
@@ -350,14 +354,15 @@ int dsqg_packed_bwd(const dsqg_packed* p, const dsqg_packed_grads* g, void* scra
     const float* delta = nullptr;
     if (p->gate) {
         if (!g->dy || !p->out || !g->dgate) return DSQG_ERR_NULL_POINTER;
-        if (bad_strides(&p->out_strides) || bad_strides(&p->gate_strides) || misaligned16(g->dy) || misaligned16(p->out) || misaligned16(p->gate) ||
+        const dsqg_strides dgate_st = dgate_strides ? *dgate_strides : p->gate_strides;
+        if (bad_strides(&p->out_strides) || bad_strides(&p->gate_strides) || bad_strides(&dgate_st) || misaligned16(g->dy) || misaligned16(p->out) || misaligned16(p->gate) ||
             misaligned16(g->dgate) || misaligned16(scratch))
             return DSQG_ERR_MISALIGNED;
         char* mem = static_cast<char*>(scratch) + round256(need);
         float* dl = reinterpret_cast<float*>(mem);
         void* buf = mem + round256((size_t)B * H * N * 4);
         dout_st.batch = (long long)H * N * D; dout_st.head = (long long)N * D; dout_st.row = D;   // head-major: the operator's backward reads whole lines
-        const cudaError_t e = launch_gate_bwd(g->dy, p->out, p->out_strides, p->gate, g->dgate, p->gate_strides, buf, dout_st, dl,
+        const cudaError_t e = launch_gate_bwd(g->dy, p->out, p->out_strides, p->gate, p->gate_strides, g->dgate, dgate_st, buf, dout_st, dl,
                                               B, H, N, D, static_cast<cudaStream_t>(stream));
         if (e != cudaSuccess) return cuda_fail(e);
         dout = buf; delta = dl;
@@ -377,7 +382,7 @@ int dsqg_gate_bwd(const void* dy, const void* y, const void* gate, const dsqg_st
     if (bad_strides(strides) || misaligned16(dy) || misaligned16(y) || misaligned16(gate) || misaligned16(dout) ||
         misaligned16(dgate))
         return DSQG_ERR_MISALIGNED;
-    cudaError_t e = launch_gate_bwd(dy, y, *strides, gate, dgate, *strides, dout, *strides, delta, B, H, N, D, static_cast<cudaStream_t>(stream));
+    cudaError_t e = launch_gate_bwd(dy, y, *strides, gate, *strides, dgate, *strides, dout, *strides, delta, B, H, N, D, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? DSQG_OK : cuda_fail(e);
 }
 

@@ -94,8 +94,8 @@ cudaError_t launch_gated_mean(const float* x, const void* g, float* pool, void* 
 cudaError_t launch_gated_mean_bwd(const void* dinter, const void* g, const float* pool, void* dg, float* dx, int B, int N, int D, cudaStream_t s);
 cudaError_t launch_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, bool reverse, cudaStream_t s);
 // y and dy, gate and dgate, and dout have strides of their own
-cudaError_t launch_gate_bwd(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, void* dgate, const dsqg_strides& gs,
-                            void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s);
+cudaError_t launch_gate_bwd(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, const dsqg_strides& gs, void* dgate,
+                            const dsqg_strides& dgs, void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s);
 cudaError_t launch_fwd_mma(const FwdArgs& a, const Taps& t, cudaStream_t s);
 cudaError_t launch_bwd_mma(const BwdArgs& a, const Taps& t, cudaStream_t s, int stages);
 bool mma_path_supported(int dtype, int D, const Taps& t, bool has_scale_embed);   // backward

@@ -19,17 +19,17 @@ namespace {
 template <int LPR>
 __global__ void __launch_bounds__(256)
 gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ y,
-                const dsqg_strides ys, const __nv_bfloat16* __restrict__ gate, __nv_bfloat16* __restrict__ dgate, const dsqg_strides gs,
+                const dsqg_strides ys, const __nv_bfloat16* __restrict__ gate, const dsqg_strides gs, __nv_bfloat16* __restrict__ dgate, const dsqg_strides dgs,
                 __nv_bfloat16* __restrict__ dout, const dsqg_strides os, float* __restrict__ delta, int B, int H, int N, int D) {
     const unsigned row = (blockIdx.x * 256u + threadIdx.x) / LPR, c = threadIdx.x % LPR * 8;
     if (row >= (unsigned)B * N * H) return;                    // whole lane groups leave
     const unsigned h = row % H, bn = row / H, n = bn % N, b = bn / N;
     auto at = [&](const dsqg_strides& s) { return (size_t)b * s.batch + (size_t)h * s.head + (size_t)n * s.row + c; };
-    const size_t y_at = at(ys), gate_at = at(gs);
+    const size_t y_at = at(ys);
     float acc = 0.f;
     if (c < D) {
         float g[8], d[8], o[8], go[8], gg[8];
-        load8(gate + gate_at, g); load8(dy + y_at, d); load8(y + y_at, o);
+        load8(gate + at(gs), g); load8(dy + y_at, d); load8(y + y_at, o);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const float s = __fdividef(1.f, 1.f + __expf(-g[i]));
@@ -37,7 +37,7 @@ gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
             gg[i] = d[i] * o[i] * (1.f - s);
             acc = fmaf(d[i], o[i], acc);
         }
-        store8(dout + at(os), go); store8(dgate + gate_at, gg);
+        store8(dout + at(os), go); store8(dgate + at(dgs), gg);
     }
     const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1) << ((threadIdx.x & 31) / LPR * LPR);
 #pragma unroll
@@ -46,24 +46,24 @@ gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
 }
 
 template <int LPR>
-cudaError_t gate_launch(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, void* dgate, const dsqg_strides& gs,
-                        void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s) {
+cudaError_t gate_launch(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, const dsqg_strides& gs, void* dgate,
+                        const dsqg_strides& dgs, void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s) {
     const long long threads = (long long)B * N * H * LPR;
     gate_bwd_kernel<LPR><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
-        static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(y), ys, static_cast<const __nv_bfloat16*>(gate),
-        static_cast<__nv_bfloat16*>(dgate), gs, static_cast<__nv_bfloat16*>(dout), os, delta, B, H, N, D);
+        static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(y), ys, static_cast<const __nv_bfloat16*>(gate), gs,
+        static_cast<__nv_bfloat16*>(dgate), dgs, static_cast<__nv_bfloat16*>(dout), os, delta, B, H, N, D);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_gate_bwd(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, void* dgate, const dsqg_strides& gs,
-                            void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s) {
-    if (D <= 8) return gate_launch<1>(dy, y, ys, gate, dgate, gs, dout, os, delta, B, H, N, D, s);
-    if (D <= 16) return gate_launch<2>(dy, y, ys, gate, dgate, gs, dout, os, delta, B, H, N, D, s);
-    if (D <= 32) return gate_launch<4>(dy, y, ys, gate, dgate, gs, dout, os, delta, B, H, N, D, s);
-    if (D <= 64) return gate_launch<8>(dy, y, ys, gate, dgate, gs, dout, os, delta, B, H, N, D, s);
-    return gate_launch<16>(dy, y, ys, gate, dgate, gs, dout, os, delta, B, H, N, D, s);
+cudaError_t launch_gate_bwd(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, const dsqg_strides& gs, void* dgate,
+                            const dsqg_strides& dgs, void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s) {
+    if (D <= 8) return gate_launch<1>(dy, y, ys, gate, gs, dgate, dgs, dout, os, delta, B, H, N, D, s);
+    if (D <= 16) return gate_launch<2>(dy, y, ys, gate, gs, dgate, dgs, dout, os, delta, B, H, N, D, s);
+    if (D <= 32) return gate_launch<4>(dy, y, ys, gate, gs, dgate, dgs, dout, os, delta, B, H, N, D, s);
+    if (D <= 64) return gate_launch<8>(dy, y, ys, gate, gs, dgate, dgs, dout, os, delta, B, H, N, D, s);
+    return gate_launch<16>(dy, y, ys, gate, gs, dgate, dgs, dout, os, delta, B, H, N, D, s);
 }
 
 }  // namespace dsqg

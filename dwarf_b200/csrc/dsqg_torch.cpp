@@ -247,8 +247,8 @@ std::tuple<Tensor, Tensor> forward_lse(const Tensor& q0, const Tensor& k0, const
 }
 
 // ------------------------------------------------------------------------------------ packed projection output
-// What a packed forward leaves for its backward.  proj: the projection output [B*N, cols] (row-major) that q, k, v and, in a layer,
-// the gate are read from in place; keep: the copies of q, k, v that stand in for it (dsqg_packed_keep_bytes).
+// What a packed forward leaves for its backward.  proj: the projection output [B*N, cols] (row-major) that q, k, v and, without a tensor of
+// its own, the gate are read from in place; keep: the copies of q, k, v that stand in for it (dsqg_packed_keep_bytes).
 struct PackedForward { Tensor proj, gate, pb, hg, se, y, lse, keep; };
 
 // q, k, v at columns 0, H*D, 2*H*D of rows of `cols` elements; the gate at column 3*H*D of the same rows or in a tensor laid out like y.
@@ -291,12 +291,14 @@ PackedForward packed_forward(const Tensor& proj, int64_t B, int64_t N, int64_t H
 
 struct PackedGrads { Tensor dproj, dgate, dpb, dhg, dse; };
 
-// dproj [B*N, cols]; proj may be undefined where keep stands in for it and the gate has a tensor of its own.
+// dproj [B*N, cols], the gate's gradient in the last quarter of 4*H*D columns or in a tensor of its own; proj may be undefined where
+// keep stands in for it and the gate has a tensor of its own.
 PackedGrads packed_backward(const PackedForward& f, const Tensor& dy, int64_t cols, const Offsets& off) {
     const int64_t B = f.lse.size(0), N = f.lse.size(2);
     PackedGrads g;
     g.dproj = new_tensor({B * N, cols}, at::kBFloat16, dy);
-    g.dgate = new_like(f.gate); g.dpb = new_like(f.pb); g.dhg = new_like(f.hg); g.dse = new_like(f.se);
+    if (cols == 3 * f.y.size(2)) g.dgate = new_like(f.gate);
+    g.dpb = new_like(f.pb); g.dhg = new_like(f.hg); g.dse = new_like(f.se);
     const dsqg_packed p = describe(f, f.proj.defined() ? ptr(f.proj) : ptr(f.keep), cols, off);
     const int64_t third = (int64_t)p.H * p.D * 2;
     char* at = static_cast<char*>(ptr(g.dproj));
@@ -306,7 +308,7 @@ PackedGrads packed_backward(const PackedForward& f, const Tensor& dy, int64_t co
     d.dpos_bias = fptr(g.dpb); d.dscale_embed = fptr(g.dse); d.dhead_gain = fptr(g.dhg);
     const size_t bytes = dsqg_packed_bwd_scratch_bytes(&p);
     const at::DataPtr scratch = scratch_for(bytes);
-    check(dsqg_packed_bwd(&p, &d, scratch.get(), bytes, stream_of(dy)), "dsqg_packed_bwd");
+    check(dsqg_packed_bwd_gate(&p, &d, g.dgate.defined() ? &p.gate_strides : &p.qkv_strides, scratch.get(), bytes, stream_of(dy)), "dsqg_packed_bwd");
     return g;
 }
 
@@ -624,7 +626,9 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
 };
 
 // qkv projection -> (K/V injection) -> operator -> gate -> output projection (train/train_2048_condU.py:171-191).  The gate's
-// projection is part of the qkv product (one GEMM over [q | k | v | gate] columns, one weight gradient, one input gradient).
+// projection is part of the qkv product (one GEMM over [q | k | v | gate] columns, one weight gradient, one input gradient).  Where the
+// operator leaves copies of q, k, v for its backward, the forward's product is two GEMMs instead, so that only the gate's output is kept
+// beside the copies (B32 N2048 dim 256: 100 MB less per layer than keeping all of it).
 struct LayerNode : torch::autograd::Function<LayerNode> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, const std::optional<Tensor>& kd, const std::optional<Tensor>& vd, const Tensor& wqkv,
                           const Tensor& bqkv, const Tensor& wg, const Tensor& bg, const Tensor& wo, const Tensor& bo, const Tensor& pos_bias,
@@ -635,16 +639,19 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
         const bool cast_x = x.scalar_type() == at::kFloat;
         const Bf16Pack w = cast_x ? cast_bf16({wqkv, wg, wo, bqkv, bg, bo, x}) : cast_bf16({wqkv, wg, wo, bqkv, bg, bo});
         const Tensor xb = cast_x ? part(w.buf, {M, D}, w.at[6]) : aligned(x.contiguous());
-        const Tensor proj = linear(xb, w[0], w[3], M, 4 * D, D);
+        const bool split = with_grad && dsqg_packed_keep_bytes((int)B, (int)H, (int)N, (int)(D / H));
+        const int64_t cols = split ? 3 * D : 4 * D;
+        const Tensor proj = linear(xb, w[0], w[3], M, cols, D);                   // bqkv and bg are one vector
+        const Tensor gate = split ? linear(xb, w[1], w[4], M, D, D).view({B, N, D}) : Tensor();
         if (kd.has_value()) {
             Tensor k = *kd, v = *vd;
             int64_t ld = k.scalar_type() == at::kBFloat16 && v.scalar_type() == at::kBFloat16 ? heads_stride(k) : 0;
             if (!ld || heads_stride(v) != ld) { k = rows_of(k); v = rows_of(v); ld = D; }
-            check(dsqg_inject_kv(ptr(proj), 4 * D, ptr(k), ptr(v), ld, M, (int)D, stream_of(x)), "dsqg_inject_kv");
+            check(dsqg_inject_kv(ptr(proj), cols, ptr(k), ptr(v), ld, M, (int)D, stream_of(x)), "dsqg_inject_kv");
         }
-        const PackedForward f = packed_forward(proj, B, N, H, D / H, 4 * D, Tensor(), pos_bias, opt(hg), opt(se), *off, with_grad);
+        const PackedForward f = packed_forward(proj, B, N, H, D / H, cols, gate, pos_bias, opt(hg), opt(se), *off, with_grad);
         const Tensor out = linear(f.y, w[2], w[5], M, D, D).view({B, N, D});
-        ctx->save_for_backward({xb, w.buf, proj, f.pb, f.hg, f.se, f.y, f.lse, f.keep});
+        ctx->save_for_backward({xb, w.buf, f.keep.defined() ? Tensor() : proj, f.gate, f.pb, f.hg, f.se, f.y, f.lse, f.keep});
         ctx->saved_data["offsets"] = (int64_t)(intptr_t)off;
         ctx->saved_data["types"] = types_of(pos_bias, opt(hg), opt(se));
         ctx->saved_data["x_types"] = std::vector<int64_t>{(int64_t)x.scalar_type(), (int64_t)type_of(opt(kd)), (int64_t)type_of(opt(vd))};
@@ -659,7 +666,7 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
         const NoAutocast no_autocast;
         const variable_list s = ctx->get_saved_variables();
         const Tensor &xb = s[0], &w = s[1];
-        const PackedForward f = {s[2], Tensor(), s[3], s[4], s[5], s[6], s[7], s[8]};
+        const PackedForward f = {s[2], s[3], s[4], s[5], s[6], s[7], s[8], s[9]};
         const int64_t B = f.lse.size(0), H = f.lse.size(1), N = f.lse.size(2), D = f.y.size(2), M = B * N, HD = D / H;
         const c10::cuda::CUDAGuard guard(xb.device());
         const Tensor dy = aligned(bf16c(dy0));

@@ -259,8 +259,9 @@ int dsqg_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, i
  * bf16; every pointer is a DEVICE pointer except offsets.  gate has strides of its own, so that it may lie in the output
  * of the same projection as q, k, v; the gradients are laid out like what they belong to.
  * keep (nullable, with a gate only; dsqg_packed_keep_bytes, which is 0 where it would not pay): the forward leaves copies of
- * q, k and v there that the backward reads faster than the strided rows; a backward given keep does not read q, k, v.  The same
- * keep (or none) has to be given to both.  scratch: dsqg_packed_bwd_scratch_bytes. */
+ * q, k and v there that the backward reads faster than the strided rows; a backward given keep does not read q, k, v, so that
+ * qkv_strides then describe their gradients only.  The same keep (or none) has to be given to both.  dsqg_packed_bwd_gate: dgate laid out
+ * in its own way (dgate_strides; NULL: like gate).  scratch: dsqg_packed_bwd_scratch_bytes. */
 typedef struct dsqg_packed {
     const void* q; const void* k; const void* v; dsqg_strides qkv_strides;
     const void* gate; dsqg_strides gate_strides;                              /* nullable */
@@ -278,6 +279,8 @@ size_t dsqg_packed_keep_bytes(int B, int H, int N, int D);
 int dsqg_packed_fwd(const dsqg_packed* p, void* stream);
 size_t dsqg_packed_bwd_scratch_bytes(const dsqg_packed* p);
 int dsqg_packed_bwd(const dsqg_packed* p, const dsqg_packed_grads* g, void* scratch, size_t scratch_bytes, void* stream);
+int dsqg_packed_bwd_gate(const dsqg_packed* p, const dsqg_packed_grads* g, const dsqg_strides* dgate_strides, void* scratch, size_t scratch_bytes,
+                         void* stream);
 
 /* What an attention layer under bf16 autocast does between its GEMMs and the operator, one pass each (the PyTorch
  * ops around the reference's layer, DWARF train/train_2048_condU.py:171-191 and the interference block :277-295):

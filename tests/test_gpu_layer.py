@@ -191,3 +191,24 @@ def test_frozen_parameters_get_no_gradient_and_cost_none():
     torch.autograd.grad(y, [x], dy)
     # scratch and activations of 65 rows against 32 MB of weight gradients
     assert torch.cuda.max_memory_allocated() - before < 16 << 20
+
+
+@pytest.mark.parametrize("dim,H", [(256, 8), (256, 4)])
+def test_what_a_layer_keeps_for_its_backward(dim, H):
+    """Between forward and backward: x and the result of the operator in bf16, and once q, k, v and the gate (head width 32: as copies
+    that stand in for the projection's output), row statistics, weights in bf16; the layer's output besides."""
+    B, N = 4, 2048
+    attn = dwarf_b200.DSQGAttentionQW(dim, H, dropout=0.0).cuda()
+    x = torch.randn(B, N, dim, device="cuda", requires_grad=True)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        attn(x).sum().backward()                          # workspaces of the first call
+        x.grad = None
+        attn.zero_grad(set_to_none=True)
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        y = attn(x)
+    torch.cuda.synchronize()
+    unit = B * N * dim * 2
+    most = (1 + 1 + 4 + 1) * unit + B * H * N * 4 + (5 * dim * dim + 5 * dim) * 2
+    assert torch.cuda.memory_allocated() - before <= most + (1 << 20), (torch.cuda.memory_allocated() - before) / unit
+    y.float().sum().backward()
