@@ -74,15 +74,19 @@ fwd_generic_kernel(const FwdArgs a, const Taps t) {
         q[r] = active && n0 + r < N ? load4(qb + (size_t)(n0 + r) * D) : zero;
         acc[r] = zero; m[r] = -INFINITY; l[r] = 0.f;
     }
-    // Taps j0 .. j0 + 7.  RUN: consecutive offsets.  INSIDE: every partner row of the warp exists; otherwise any row of the
-    // sequence stands in for one that does not (its score is -inf, its weight 0).
+    // Taps j0 .. j0 + 7.  RUN: consecutive offsets.  INSIDE: every partner row of the warp exists; otherwise any key row of the
+    // sequence stands in for one that does not (its score is -inf), and a value of zero (a weight of 0 would not hold off an infinity or NaN there).
     auto chunk = [&](auto RUNC, auto INSIDEC, int j0) {
         constexpr bool RUN = decltype(RUNC)::value, INSIDE = decltype(INSIDEC)::value;
         auto at = [&](const T* p, int n, int i) {
             if constexpr (INSIDE) return load4(p + (ptrdiff_t)n * D + i * D);
             else return load4(p + (ptrdiff_t)min(max(n + i, 0), N - 1) * D);
         };
-        const int first = n0 - off_s[j0] - 7;                     // RUN: the eleven rows start here
+        auto value = [&](int n, int i) {
+            const float4 v = at(vb, n, i);
+            return INSIDE || (n + i >= 0 && n + i < N) ? v : zero;
+        };
+        const int first = n0 - off_s[j0] - 7;                     // RUN: the R + 7 rows start here
         float s[R];
         {
             float part[R][8];
@@ -149,7 +153,7 @@ fwd_generic_kernel(const FwdArgs a, const Taps t) {
         if constexpr (RUN) {
 #pragma unroll
             for (int i = 0; i < R + 7; ++i) {
-                const float4 v = at(vb, first, i);
+                const float4 v = value(first, i);
 #pragma unroll
                 for (int r = 0; r < R; ++r)
                     if (7 + r - i >= 0 && 7 + r - i < 8) fold(r, 7 + r - i, v);
@@ -159,7 +163,7 @@ fwd_generic_kernel(const FwdArgs a, const Taps t) {
             for (int c = 0; c < 8; ++c) {
                 const int dc = off_s[min(j0 + c, J - 1)];
 #pragma unroll
-                for (int r = 0; r < R; ++r) fold(r, c, at(vb, n0 - dc, r));
+                for (int r = 0; r < R; ++r) fold(r, c, value(n0 - dc, r));
             }
         }
     };
