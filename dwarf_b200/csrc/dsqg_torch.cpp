@@ -129,12 +129,14 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
     if (hg.defined() && !shape_is(hg, {H})) want("head_gain", H, 0, hg);
 }
 
-// Head dimension the kernels are called with: ops._padded_head_dim has the reasons for padding; the widths 48 and 80 have
+// Head dimension the kernels are called with.  The bf16 tensor-core kernels exist for multiples of 32 up to 128; another bf16 width
+// is zero-padded up to the next of those where they take the padded problem, with the scale 1/sqrt(D) of the true width:
+// several times faster than the CUDA-core kernels on the odd width (the reference pads to a power of two inside its kernels,
+// kernels/dsqg_attention_v2.py:344).  The widths 48 and 80 (the reference's 85M condM model, train/train_2048_85m_condM.py:67-69) have
 // kernels of their own for the usual dense window without scale_embed (B8 H8 N2048 HD80 forward + backward: the copies into
-// 96 columns and back took 232 us of 454).
-int64_t padded_head_dim(const Tensor& q, const Offsets& off, bool has_se) {
-    const int64_t D = q.size(3);
-    if (q.scalar_type() != at::kBFloat16 || D % 32 == 0 || D > 128 || D % 8 != 0) return D;
+// 96 columns and back took 232 us of 454).  fp32 is never padded.
+int64_t padded_head_dim(int64_t D, bool bf16, const Offsets& off, bool has_se) {
+    if (!bf16 || D % 32 == 0 || D > 128 || D % 8 != 0) return D;
     const int64_t Dp = (D + 31) / 32 * 32;
     const bool own = (D == 48 || D == 80) && !has_se;
     if (own && dsqg_tensor_core_path(DSQG_DTYPE_BF16, 96, off.v.data(), off.J(), 0)) return D;
@@ -157,7 +159,7 @@ Forward attention_forward(const Tensor& q0, const Tensor& k0, const Tensor& v0, 
     Forward f;
     f.pb = f32c(pos_bias); f.hg = f32c(head_gain); f.se = f32c(scale_embed);
     f.D = q0.size(3);
-    const int64_t Dp = padded_head_dim(q0, off, scale_embed.defined());
+    const int64_t Dp = padded_head_dim(f.D, dt == DSQG_DTYPE_BF16, off, scale_embed.defined());
     f.q = q0; f.k = k0; f.v = v0;
     if (Dp != f.D) {                                    // zero columns change no score and give zero outputs
         f.q = pad_to(f.q, Dp); f.k = pad_to(f.k, Dp); f.v = pad_to(f.v, Dp); f.se = pad_to(f.se, Dp);
@@ -798,6 +800,7 @@ std::tuple<Tensor, Tensor> ring_advance(const Tensor& head0, const Tensor& fill0
 PYBIND11_MODULE(_dsqg_torch, m) {
     py::class_<Offsets, std::unique_ptr<Offsets, py::nodelete>>(m, "Offsets").def_property_readonly("J", &Offsets::J);
     m.def("offsets", &intern_offsets, py::return_value_policy::reference);
+    m.def("padded_head_dim", [](int64_t D, bool bf16, const Offsets* off, bool has_se) { return padded_head_dim(D, bf16, *off, has_se); });
     m.def("attention", &attention);
     m.def("forward_lse", &forward_lse);
     m.def("attention_packed", &attention_packed);

@@ -32,22 +32,6 @@ def _dtype_code(t: torch.Tensor) -> int:
     raise TypeError(f"dsqg: q/k/v must be bfloat16 or float32, got {t.dtype}")
 
 
-def _padded_head_dim(q, off, J, has_scale_embed):
-    """Head dimension the kernels are called with.  The bf16 tensor-core kernels exist for
-    D in {32, 64, 96, 128}; another bf16 head dimension (80 in the reference's 85M condM model,
-    train/train_2048_85m_condM.py:67-69; 48) is zero-padded up to the next of those when the
-    tensor-core kernels take the padded problem, with the scale 1/sqrt(D) of the true width passed
-    explicitly: several times faster than the CUDA-core kernels on the odd width.  The reference
-    pads to a power of two inside its kernels (kernels/dsqg_attention_v2.py:344).  fp32 tensors
-    are never padded."""
-    D = q.shape[-1]
-    if q.dtype != torch.bfloat16 or D % 32 == 0 or D > 128 or D % 8 != 0:
-        return D
-    Dp = (D + 31) // 32 * 32
-    lib = _lib.load()
-    return Dp if lib.dsqg_tensor_core_path(_lib.DSQG_DTYPE_BF16, Dp, off, J, int(has_scale_embed)) else D
-
-
 class DSQGFunction:
     """out = DSQG(q, k, v; pos_bias, head_gain, scale_embed, offsets) with autograd (an autograd node in native code,
     csrc/dsqg_torch.cpp).

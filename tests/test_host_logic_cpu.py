@@ -126,18 +126,17 @@ def test_two_rank_gloo_sharding_and_timing_reduction():
 def test_odd_head_widths_are_padded_only_when_the_tensor_core_kernels_take_them():
     """Host-side choice of the head dimension the kernels are called with (no device access)."""
     from dwarf_b200 import _lib, ops
-    off43, J43 = _lib.offsets_array(ops.OFFSETS_43)
-    wide = tuple(range(41)) + (128, 384, 1536)
-    offw, Jw = _lib.offsets_array(wide)
-    q = lambda D, dt=torch.bfloat16: torch.zeros(1, 1, 4, D, dtype=dt)
-    assert ops._padded_head_dim(q(80), off43, J43, False) == 96
-    assert ops._padded_head_dim(q(48), off43, J43, False) == 64
-    assert ops._padded_head_dim(q(48), off43, J43, True) == 64       # scale_embed runs on the 64-wide kernels
-    assert ops._padded_head_dim(q(80), off43, J43, True) == 80       # but not on the 96-wide ones
-    assert ops._padded_head_dim(q(80), offw, Jw, False) == 80        # dense window wider than 32
-    assert ops._padded_head_dim(q(80, torch.float32), off43, J43, False) == 80
+    off43, offw = _lib.offsets_handle(ops.OFFSETS_43), _lib.offsets_handle(tuple(range(41)) + (128, 384, 1536))
+    width = lambda D, off=off43, se=False, bf16=True: _lib.native().padded_head_dim(D, bf16, off, se)
+    assert width(80) == 80 and width(48) == 48             # kernels of their own
+    assert width(72) == 96 and width(40) == 64 and width(112) == 128
+    assert width(48, se=True) == 64                        # scale_embed runs on the 64-wide kernels
+    assert width(80, se=True) == 80                        # but not on the 96-wide ones
+    assert width(80, offw) == 80                           # dense window wider than 32
+    assert width(72, offw) == 72
+    assert width(80, bf16=False) == 80 and width(72, bf16=False) == 72
     for D in (32, 64, 96, 128):
-        assert ops._padded_head_dim(q(D), off43, J43, False) == D
+        assert width(D) == D
 
 
 def test_layer_gemms_follow_the_reduced_precision_setting():
