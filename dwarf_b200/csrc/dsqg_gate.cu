@@ -15,8 +15,8 @@ namespace {
 
 // LPR lanes per (batch, row, head), eight elements each.  Five tensors pass through once, so memory is the bound: with
 // one thread per row (the row's 16-byte pieces 64 bytes or more apart from lane to lane) a warp's load touched 16 lines
-// for 512 bytes; B32 H8 N2048 D32 (168 MB) 46.7 us then, 28.8 us now.
-template <int LPR>
+// for 512 bytes; B32 H8 N2048 D32 (168 MB) 46.7 us then, 28.8 us now.  SAME: dgate is laid out like gate (one address less to form).
+template <int LPR, bool SAME>
 __global__ void __launch_bounds__(256)
 gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ y,
                 const dsqg_strides ys, const __nv_bfloat16* __restrict__ gate, const dsqg_strides gs, __nv_bfloat16* __restrict__ dgate, const dsqg_strides dgs,
@@ -25,11 +25,11 @@ gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
     if (row >= (unsigned)B * N * H) return;                    // whole lane groups leave
     const unsigned h = row % H, bn = row / H, n = bn % N, b = bn / N;
     auto at = [&](const dsqg_strides& s) { return (size_t)b * s.batch + (size_t)h * s.head + (size_t)n * s.row + c; };
-    const size_t y_at = at(ys);
+    const size_t y_at = at(ys), gate_at = at(gs), dgate_at = SAME ? gate_at : at(dgs);
     float acc = 0.f;
     if (c < D) {
         float g[8], d[8], o[8], go[8], gg[8];
-        load8(gate + at(gs), g); load8(dy + y_at, d); load8(y + y_at, o);
+        load8(gate + gate_at, g); load8(dy + y_at, d); load8(y + y_at, o);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const float s = __fdividef(1.f, 1.f + __expf(-g[i]));
@@ -37,7 +37,7 @@ gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
             gg[i] = d[i] * o[i] * (1.f - s);
             acc = fmaf(d[i], o[i], acc);
         }
-        store8(dout + at(os), go); store8(dgate + at(dgs), gg);
+        store8(dout + at(os), go); store8(dgate + dgate_at, gg);
     }
     const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1) << ((threadIdx.x & 31) / LPR * LPR);
 #pragma unroll
@@ -49,7 +49,8 @@ template <int LPR>
 cudaError_t gate_launch(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, const dsqg_strides& gs, void* dgate,
                         const dsqg_strides& dgs, void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s) {
     const long long threads = (long long)B * N * H * LPR;
-    gate_bwd_kernel<LPR><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+    const bool same = gs.batch == dgs.batch && gs.head == dgs.head && gs.row == dgs.row;
+    (same ? gate_bwd_kernel<LPR, true> : gate_bwd_kernel<LPR, false>)<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
         static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(y), ys, static_cast<const __nv_bfloat16*>(gate), gs,
         static_cast<__nv_bfloat16*>(dgate), dgs, static_cast<__nv_bfloat16*>(dout), os, delta, B, H, N, D);
     return cudaGetLastError();
