@@ -410,7 +410,7 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
 // Tuning per head dimension (measured on B200): warps per CTA, sparse taps folded together,
 // resident CTAs per SM the register budget is set for.
 template <int D> struct FwdTune {
-    static constexpr int warps = 4, group = D == 64 || D > 80 ? 1 : 2, ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));   // D = 64: 104.8 us (107.8 with group 2)
+    static constexpr int warps = 4, group = D == 64 || D > 80 ? 1 : 2, ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));   // D = 64: 92.8 us at 16x12x2048 (88.7 with group 2, which was behind, 107.8 to 104.8, before rows came in 32-byte pieces)
     // With scale_embed a CTA first lays out the table, about a quarter of a tile's time, so a warp does up to three tiles with it.
     // The count is the one for which (waves of CTAs) x (tiles + 1/4) is least: one where the grid is a single wave (2x8x777x32 11.6 us,
     // 12.5 with two), two or three where that saves a wave or its table (4x8x2048x32 19.5 -> 18.7, 32x8x2048x32 101.4 -> 97.3,
@@ -463,7 +463,7 @@ fwd_mma_kernel(const FwdArgs a, const Taps t, const int tiles_se) {
 // resident CTAs per SM the register budget is set for (spills against warps in flight).
 template <int D> struct BwdTune {
     static constexpr int dq_group = D <= 80 ? 2 : 1, dq_ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D == 80 ? 3 : 2));   // D = 32: 98.5 us (108.8 with 4 CTAs, 103.3 with group 1); D = 80: 69.0 us (80 with 2 CTAs)
-    static constexpr int dq_group_se = D == 32 ? 2 : 1, dq_ctas_se = 4;    // with scale_embed: D = 32 172 us (180 with group 1 and 5 CTAs), D = 64 231 us (242 with group 2)
+    static constexpr int dq_group_se = D == 32 ? 2 : 1, dq_ctas_se = 4;    // with scale_embed: 32x8x2048x32 164.8 us (166.8 with group 1 and 5 CTAs), 16x12x2048x64 216.9 us (224.7 with group 2)
     static constexpr int dkdv_group_se = D <= 64 ? 2 : 1, dkdv_ctas_se = D == 32 ? 4 : 3;
     static constexpr int dkdv_group = D <= 80 ? 2 : 1, dkdv_ctas = D == 32 ? 4 : (D <= 64 ? 3 : 2);   // D = 80: 78.1 us (83 with group 1, 96-109 with 3 CTAs)
 };

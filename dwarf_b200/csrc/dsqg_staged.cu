@@ -1,6 +1,6 @@
 // Forward with TMA-staged V (bf16 storage, fp32 accumulate; D in {32, 64}; dense offsets within
 // 0..32; up to 16 sparse taps).  Opt-in (kernel path 3): on B200 it measures slower than the
-// register-fed kernels of dsqg_mma.cu (cfg1 forward 102 us against 75 us), so the automatic choice
+// register-fed kernels of dsqg_mma.cu (cfg1 forward 102 us against 75 us when it was written and 66 us now), so the automatic choice
 // never takes it; it stays as the measured alternative and as the home of the copy-engine code.
 //
 // Math: DWARF reference kernels/dsqg_attention_v3.py:60-163, with the per-head output gain of
