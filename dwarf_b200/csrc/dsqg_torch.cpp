@@ -386,9 +386,10 @@ Tensor causal_mean(const Tensor& x0) {
 // step (1.9 ms of host time for 0.95 ms of GPU work at B8 N2048 dim 256) is their GEMMs (cuBLAS through ATen), the operator
 // and the kernels of csrc/dsqg_layer.cu.  Weight gradients leave the GEMM in fp32 instead of being rounded to bf16 and cast.
 
-// Autocast is done by hand inside the nodes.
+// Autocast and autograd are done by hand inside the nodes.
 struct NoAutocast {
     c10::impl::ExcludeDispatchKeyGuard guard{c10::autocast_dispatch_keyset};
+    at::AutoDispatchBelowADInplaceOrView below;
 };
 
 // Row-major C[M,N] = op(A) . op(B) (+ bias[N]) on bf16 operands, C in bf16 or fp32, through cuBLASLt with plans kept per thread and
@@ -560,6 +561,7 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         const c10::cuda::CUDAGuard guard(x.device());
         const int64_t B = x.size(0), N = x.size(1), D = x.size(2), M = B * N;
         const Tensor xc = aligned(f32c(x)), gam = aligned(f32c(gamma));
+        // the modules' own kernel, and so their bits: the deltas round as theirs do, and with them the gradients that nearly cancel
         const auto [xi, mean, rstd] = at::native_layer_norm(xc, {D}, gam, aligned(f32c(beta)), eps);
         const Bf16Pack w = cast_bf16({wg, wk, wv, bg, bk, bv, xi});               // wk, wv and bk, bv are one matrix and one vector
         const Tensor xib = part(w.buf, {M, D}, w.at[6]), g = linear(xib, w[0], w[3], M, D, D);
