@@ -16,8 +16,13 @@ namespace {
 // LPR lanes per (batch, row, head), eight elements each.  Five tensors pass through once, so memory is the bound: with
 // one thread per row (the row's 16-byte pieces 64 bytes or more apart from lane to lane) a warp's load touched 16 lines
 // for 512 bytes; B32 H8 N2048 D32 (168 MB) 46.7 us then, 28.8 us now.  SAME: dgate is laid out like gate (one address less to form).
+//
+// Up to D = 32 delta is summed element by element, lane after lane, as one thread would: ds = P (dP - delta) is rounded to bf16, and another order
+// moves single roundings, which a gradient that nearly cancels (a bias on every key) shows.  At 40 registers (six CTAs per SM)
+// the chain hides behind the loads: 28.9 us with it and without (31.0 with five CTAs).  At D = 64 and 128 it would not: 24.7 against 22.8 us
+// (B8 H12 N2048) and 35.6 against 28.8 (B8 H8); there the lanes' sums are added in pairs.
 template <int LPR, bool SAME>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)
 gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ y,
                 const dsqg_strides ys, const __nv_bfloat16* __restrict__ gate, const dsqg_strides gs, __nv_bfloat16* __restrict__ dgate, const dsqg_strides dgs,
                 __nv_bfloat16* __restrict__ dout, const dsqg_strides os, float* __restrict__ delta, int B, int H, int N, int D) {
@@ -26,23 +31,35 @@ gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __res
     const unsigned h = row % H, bn = row / H, n = bn % N, b = bn / N;
     auto at = [&](const dsqg_strides& s) { return (size_t)b * s.batch + (size_t)h * s.head + (size_t)n * s.row + c; };
     const size_t y_at = at(ys), gate_at = at(gs), dgate_at = SAME ? gate_at : at(dgs);
-    float acc = 0.f;
+    float d[8] = {}, o[8] = {};
     if (c < D) {
-        float g[8], d[8], o[8], go[8], gg[8];
+        float g[8], go[8], gg[8];
         load8(gate + gate_at, g); load8(dy + y_at, d); load8(y + y_at, o);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const float s = __fdividef(1.f, 1.f + __expf(-g[i]));
             go[i] = d[i] * s;
             gg[i] = d[i] * o[i] * (1.f - s);
-            acc = fmaf(d[i], o[i], acc);
         }
         store8(dout + at(os), go); store8(dgate + dgate_at, gg);
     }
     const unsigned group = LPR == 32 ? 0xffffffffu : ((1u << LPR) - 1) << ((threadIdx.x & 31) / LPR * LPR);
+    float acc = 0.f;
+    if constexpr (LPR <= 4) {
 #pragma unroll
-    for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(group, acc, o);
-    if (c == 0) delta[((size_t)b * H + h) * N + n] = acc;
+        for (int l = 0; l < LPR; ++l) {                        // every lane adds its products to what the lane before has; the l-th lane's count
+            float t = l ? __shfl_sync(group, acc, l - 1, LPR) : 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) t = fmaf(d[i], o[i], t);
+            acc = t;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc = fmaf(d[i], o[i], acc);
+#pragma unroll
+        for (int l = LPR / 2; l > 0; l >>= 1) acc += __shfl_xor_sync(group, acc, l);
+    }
+    if (threadIdx.x % LPR == LPR - 1) delta[((size_t)b * H + h) * N + n] = acc;
 }
 
 template <int LPR>
