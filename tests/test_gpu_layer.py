@@ -223,3 +223,22 @@ def test_what_a_layer_keeps_for_its_backward(dim, H):
     most = (1 + 1 + 4 + 1) * unit + B * H * N * 4 + (5 * dim * dim + 5 * dim) * 2
     assert torch.cuda.memory_allocated() - before <= most + (1 << 20), (torch.cuda.memory_allocated() - before) / unit
     y.float().sum().backward()
+
+
+def test_results_may_be_changed_in_place():
+    """As those of the modules: the layer's output and the deltas are tensors of their own to autograd."""
+    torch.manual_seed(4)
+    attn = dwarf_b200.DSQGAttentionQW(64, 2, dropout=0.0).cuda()
+    block = dwarf_b200.InterferenceInjection(64, 2).cuda()
+    x = torch.randn(2, 40, 64, device="cuda", requires_grad=True)
+    params = [x, *attn.parameters(), *block.parameters()]
+
+    def run(in_place):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            kd, vd = block(x)
+            kd = kd.mul_(2) if in_place else kd * 2
+            y = attn(x, kv_inject=(kd, vd))
+        y = y.mul_(4) if in_place else y * 4
+        return torch.autograd.grad(y, params, torch.ones_like(y))
+    for a, b in zip(run(True), run(False)):
+        assert torch.equal(a, b)
