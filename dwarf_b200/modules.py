@@ -148,7 +148,7 @@ class _DSQGAttentionBase(nn.Module):
         """The whole layer as one autograd node (csrc/dsqg_torch.cpp) under bf16 autocast, or None where that does not apply."""
         qkv, gate, out = self.qkv_proj, self.gate_proj, self.out_proj
         if not x.is_cuda or not _plain((qkv, nn.Linear), (gate, nn.Linear), (out, nn.Linear)) or x.dim() != 3 or x.shape[-1] != self.embedding_dim \
-                or self.embedding_dim % 8:
+                or self.embedding_dim % 8 or type(self).attend is not _DSQGAttentionBase.attend or "attend" in self.__dict__:
             return None
         n = _lib.native()
         if not n.layer_applies(x, [qkv.weight, qkv.bias, gate.weight, gate.bias, out.weight, out.bias]):

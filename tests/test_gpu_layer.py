@@ -242,3 +242,16 @@ def test_results_may_be_changed_in_place():
         return torch.autograd.grad(y, params, torch.ones_like(y))
     for a, b in zip(run(True), run(False)):
         assert torch.equal(a, b)
+
+
+def test_a_subclass_may_bring_its_own_attend():
+    class Scaled(dwarf_b200.DSQGAttentionQW):
+        def attend(self, x, kv_inject=None):
+            y, k, v = super().attend(x, kv_inject)
+            return y * 2, k, v
+    torch.manual_seed(0)
+    a, b = dwarf_b200.DSQGAttentionQW(64, 2, dropout=0.0).cuda(), Scaled(64, 2, dropout=0.0).cuda()
+    b.load_state_dict(a.state_dict())
+    x = torch.randn(2, 20, 64, device="cuda")
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        assert torch.equal(b(x), a(x) * 2)
