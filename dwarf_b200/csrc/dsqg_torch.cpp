@@ -114,6 +114,12 @@ at::ScalarType type_of(const Tensor& t) { return t.defined() ? t.scalar_type() :
 
 bool shape_is(const Tensor& t, std::initializer_list<int64_t> s) { return t.sizes() == at::IntArrayRef(s); }
 
+// The kernels get plain pointers: a tensor on the host or on another GPU would be read as if it were on this one.
+void check_device(const char* who, const Tensor& on, std::initializer_list<const Tensor*> ts) {
+    for (const Tensor* t : ts)
+        if (t->defined() && t->device() != on.device()) throw py::value_error(std::string(who) + ": all tensors must be on " + on.device().str() + ", got one on " + t->device().str());
+}
+
 void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& pb, const Tensor& hg, const Tensor& se, int J) {
     if (!q.is_cuda()) throw std::runtime_error("dsqg: tensors must live on a CUDA device (there is no CPU path)");
     if (q.dim() != 4) throw py::value_error("dsqg: q must be [B,H,N,HD], got " + shape_of(q));
@@ -127,6 +133,7 @@ void check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
     if (!shape_is(pb, {J, H})) want("pos_bias", J, H, pb);
     if (se.defined() && !shape_is(se, {J, D})) want("scale_embed", J, D, se);
     if (hg.defined() && !shape_is(hg, {H})) want("head_gain", H, 0, hg);
+    check_device("dsqg", q, {&pb, &se, &hg});
 }
 
 // Head dimension the kernels are called with.  The bf16 tensor-core kernels exist for multiples of 32 up to 128; another bf16 width
@@ -274,6 +281,7 @@ dsqg_packed describe(const PackedForward& f, void* proj, int64_t cols, const Off
 PackedForward packed_forward(const Tensor& proj, int64_t B, int64_t N, int64_t H, int64_t D, int64_t cols, const Tensor& gate, const Tensor& pos_bias,
                              const Tensor& head_gain, const Tensor& scale_embed, const Offsets& off, bool with_grad) {
     const int64_t J = off.J();
+    check_device("dsqg", proj, {&gate, &pos_bias, &head_gain, &scale_embed});
     PackedForward f;
     f.proj = proj;
     f.gate = gate.defined() ? gate.contiguous() : gate;
@@ -735,7 +743,8 @@ Tensor layer(const Tensor& x, const std::optional<Tensor>& kd, const std::option
 struct StepParams { Tensor pb, hg, se; };
 
 void check_step(const char* who, const Tensor& q, const Tensor& k, const Tensor& v, at::ScalarType dt, int64_t S, int64_t H, int64_t D,
-                const Tensor& head, const Tensor& fill, const Tensor& pb, int J) {
+                const Tensor& ring, const Tensor& head, const Tensor& fill, const Tensor& pb, const Tensor& hg, const Tensor& se, int J) {
+    check_device(who, q, {&k, &v, &ring, &head, &fill, &pb, &hg, &se});
     const char* names[3] = {"q", "k_new", "v_new"};
     const Tensor* ts[3] = {&q, &k, &v};
     for (int i = 0; i < 3; ++i)
@@ -753,7 +762,8 @@ Tensor decode_step(const Tensor& q, const Tensor& k, const Tensor& v, const Tens
     if (k_ring.dim() != 4) throw py::value_error("dsqg_decode: k_ring and v_ring must be contiguous [S,H,R,D]");
     const int64_t S = k_ring.size(0), H = k_ring.size(1), R = k_ring.size(2), D = k_ring.size(3);
     const Tensor fill = opt(fill0);
-    check_step("dsqg_decode", q, k, v, k_ring.scalar_type(), S, H, D, head, fill, pos_bias, off->J());
+    check_step("dsqg_decode", q, k, v, k_ring.scalar_type(), S, H, D, k_ring, head, fill, pos_bias, opt(hg), opt(se), off->J());
+    check_device("dsqg_decode", q, {&v_ring});
     if (v_ring.sizes() != k_ring.sizes() || !k_ring.is_contiguous() || !v_ring.is_contiguous())
         throw py::value_error("dsqg_decode: k_ring and v_ring must be contiguous [S,H,R,D]");
     const StepParams p = {f32c(pos_bias), f32c(opt(hg)), f32c(opt(se))};
@@ -776,7 +786,7 @@ Tensor decode_step_kv(const Tensor& q, const Tensor& k, const Tensor& v, const T
     if (lead && (layer < 0 || layer >= kv.size(0))) throw py::index_error("dsqg_decode_kv: no such layer");
     const int64_t S = kv.size(lead), H = kv.size(1 + lead), R = kv.size(2 + lead), D = kv.size(4 + lead);
     const Tensor fill = opt(fill0);
-    check_step("dsqg_decode_kv", q, k, v, kv.scalar_type(), S, H, D, head, fill, pos_bias, off->J());
+    check_step("dsqg_decode_kv", q, k, v, kv.scalar_type(), S, H, D, kv, head, fill, pos_bias, opt(hg), opt(se), off->J());
     const StepParams p = {f32c(pos_bias), f32c(opt(hg)), f32c(opt(se))};
     const c10::cuda::CUDAGuard guard(q.device());
     Tensor out = out0.has_value() ? *out0 : new_like(q);

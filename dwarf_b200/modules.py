@@ -158,7 +158,7 @@ class _DSQGAttentionBase(nn.Module):
         if not self._packed:
             return None
         kd, vd = (None, None) if kv_inject is None else kv_inject
-        if kd is not None and (kd.shape != (x.shape[0], self.num_heads, x.shape[1], self.head_dim) or vd.shape != kd.shape or not kd.is_cuda or not vd.is_cuda):
+        if kd is not None and (kd.shape != (x.shape[0], self.num_heads, x.shape[1], self.head_dim) or vd.shape != kd.shape or kd.device != x.device or vd.device != x.device):
             return None
         return n.layer(x, kd, vd, qkv.weight, qkv.bias, gate.weight, gate.bias, out.weight, out.bias, self.pos_bias, getattr(self, "if_gain", None),
                        getattr(self, "scale_embed", None), _lib.offsets_handle(self._offsets), self.num_heads)

@@ -255,3 +255,23 @@ def test_a_subclass_may_bring_its_own_attend():
     x = torch.randn(2, 20, 64, device="cuda")
     with torch.autocast("cuda", dtype=torch.bfloat16):
         assert torch.equal(b(x), a(x) * 2)
+
+
+def test_tensors_elsewhere_are_refused_on_the_host():
+    """A parameter or delta on the CPU raises before anything is launched."""
+    q = torch.randn(1, 2, 40, 32, device="cuda").bfloat16()
+    offsets = dwarf_b200.OFFSETS_43
+    pb, gain = torch.zeros(len(offsets), 2), torch.ones(2)
+    for p, g in ((pb, None), (pb.cuda(), gain)):
+        with pytest.raises(ValueError, match="cuda:0"):
+            dwarf_b200.dsqg_attention(q, q, q, p, g, None, offsets)
+        with pytest.raises(ValueError, match="cuda:0"):
+            dwarf_b200.dsqg_attention_packed(torch.randn(1, 40, 3, 2, 32, device="cuda").bfloat16(), p, g, None, offsets)
+        cache = dwarf_b200.DSQGRingCache(1, 3, 2, 32)
+        cache.advance()
+        with pytest.raises(ValueError, match="cuda:0"):
+            cache.step(0, *(torch.zeros(3, 2, 32, device="cuda", dtype=torch.bfloat16) for _ in range(3)), p, g)
+    attn = dwarf_b200.DSQGAttentionQW(64, 2, dropout=0.0).cuda()
+    delta = torch.zeros(1, 2, 40, 32)
+    with torch.autocast("cuda", dtype=torch.bfloat16), pytest.raises(RuntimeError):
+        attn(torch.randn(1, 40, 64, device="cuda"), kv_inject=(delta, delta))
