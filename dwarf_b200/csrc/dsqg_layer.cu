@@ -26,7 +26,8 @@ __global__ void __launch_bounds__(kT) cast_kernel(const CastArgs a) {
     }
 }
 
-// ---- layer norm forward: one warp per row.  y in fp32 (for the running mean) and bf16 (for the GEMM)
+// ---- layer norm forward: one warp per row.  y in fp32 (for the running mean) and bf16 (for the GEMM).  For callers of the C interface (29 us at
+// 65,536 x 256); the autograd node of the interference block takes PyTorch's kernel (112 us, and a cast), whose last bits its deltas follow.
 __global__ void __launch_bounds__(kT)
 layer_norm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
                       float* __restrict__ y, __nv_bfloat16* __restrict__ yb, float2* __restrict__ stat, long long rows, int D) {
