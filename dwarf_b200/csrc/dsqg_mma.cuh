@@ -76,7 +76,14 @@ __device__ __forceinline__ void load_row_at(RowFrag<D>& f, const __nv_bfloat16* 
     }
 }
 
-// One row; zero-filled when !valid (the pointer is not dereferenced then).
+// This thread's pieces from p on, zero when !valid (the pointer is not dereferenced then).
+template <int D, bool A32 = true>
+__device__ __forceinline__ void load_piece(RowFrag<D>& f, const __nv_bfloat16* p, bool valid) {
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j) f.r[j] = 0u;
+    if (valid) load_row_at<D, A32>(f, p);
+}
+// One row; zero-filled when !valid.
 template <int D, bool A32 = true>
 __device__ __forceinline__ void load_row(RowFrag<D>& f, const __nv_bfloat16* row_ptr, int tig, bool valid) {
 #pragma unroll
@@ -236,7 +243,7 @@ struct Lane {
     bool owner;          // holds the diagonal entries of rows g and g+8
     int owner_lane;      // lane of this quad's owner
     __device__ Lane() {
-        warp = threadIdx.x >> 5; lane = threadIdx.x & 31; g = lane >> 2; tig = lane & 3;
+        warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); lane = threadIdx.x & 31; g = lane >> 2; tig = lane & 3;
         owner = tig == (g >> 1);
         owner_lane = (lane & ~3) | (g >> 1);
     }

@@ -36,6 +36,40 @@ constexpr int kRows = 16 * kWarps; // rows per CTA
 // gradients, everything that is read contiguous.
 constexpr int kContiguous = 0, kStrided = 1, kStridedAny = 2, kKept = 3;
 
+// Where this thread's piece of row `tile row + g + rows` of a tensor lies: a pointer that is the same for the whole warp, plus a lane part (32 bits where
+// rows follow one another, CI).  A tap's address is then formed once per warp by the uniform datapath, and K and V share the lane part;
+// a pointer per lane and tensor cost four more registers and four vector instructions per tap and tensor, which these kernels, held to the
+// registers of four to six CTAs per SM, paid for in spills.  The product is opaque, or the compiler adds the lane part first.
+template <int D, bool CI> struct Rows {
+    const __nv_bfloat16* tile;
+    long long rs;                                        // row stride in bytes (strided tensors)
+    std::conditional_t<CI, unsigned, long long> lane;
+    // p: row 0 of the sequence; row0: first row of the tile; stride: elements from row to row
+    __device__ __forceinline__ Rows(const void* p, size_t base, int row0, ptrdiff_t stride, const Lane& L) {
+        tile = static_cast<const __nv_bfloat16*>(p) + base + (ptrdiff_t)row0 * stride;
+        rs = 2 * (long long)stride;
+        if constexpr (CI) lane = 2u * (unsigned)(L.g * D + kLane<D> * L.tig);
+        else lane = L.g * rs + 2 * kLane<D> * L.tig;
+    }
+    __device__ __forceinline__ const __nv_bfloat16* at(int rows) const {
+        unsigned long long x;
+        if constexpr (CI) asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(x) : "r"(rows), "n"(2 * D), "l"(tile));
+        else asm("mad.lo.s64 %0, %1, %2, %3;" : "=l"(x) : "l"((long long)rows), "l"(rs), "l"(tile));
+        return reinterpret_cast<const __nv_bfloat16*>(x + lane);
+    }
+    // rows r and r + 8
+    template <bool AL> __device__ __forceinline__ void load2(RowFrag<D>& lo, RowFrag<D>& hi, int rows) const {
+        const __nv_bfloat16* x = at(rows);
+        load_row_at<D, AL>(lo, x);
+        load_row_at<D, AL>(hi, CI ? x + 8 * D : at(rows + 8));
+    }
+    template <bool AL> __device__ __forceinline__ void load2(RowFrag<D>& lo, RowFrag<D>& hi, int rows, bool v_lo, bool v_hi) const {
+        const __nv_bfloat16* x = at(rows);
+        load_piece<D, AL>(lo, x, v_lo);
+        load_piece<D, AL>(hi, CI ? x + 8 * D : at(rows + 8), v_hi);
+    }
+};
+
 // ------------------------------------------------------------------------------ forward
 // Online softmax over the dense window, then over the sparse taps, with the per-element
 // bookkeeping moved out of the tile loop:
@@ -194,7 +228,7 @@ template <int WB> struct StartTable {
 };
 
 template <int D, int WB, bool INTERIOR, int kTapGroup, bool SE, int ST>
-__device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, const int2* tap_s, int ns,
+__device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, const int2* tap_s, const Taps& t, int ns,
                                          int bh, int h, int g0, const Lane& L, const SeRows& se, float* se_tile) {
     // scale_embed: the warp's tile, dense part first; qs0 / qs1: sparse entries of rows g / g + 8
     const int sp = SE ? SeGeo<WB>::sparse_pitch(ns) : 0;
@@ -209,16 +243,12 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
     const ptrdiff_t RS = ST ? (ptrdiff_t)a.in_sn : D, OS = ST ? (ptrdiff_t)a.out_sn : D;   // row strides of q/k/v and of out
     const size_t base = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : (size_t)bh * N * D;
     const size_t obase = ST ? (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh : base;
-    const __nv_bfloat16* qp = static_cast<const __nv_bfloat16*>(a.q) + base;
-    // per-thread pointers to this thread's chunk of row row_lo of K and V
-    const __nv_bfloat16* kl = static_cast<const __nv_bfloat16*>(a.k) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
-    const __nv_bfloat16* vl = static_cast<const __nv_bfloat16*>(a.v) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
+    const Rows<D, !ST> qr(a.q, base, g0, RS, L), kr(a.k, base, g0, RS, L), vr(a.v, base, g0, RS, L);
     const float c2 = a.scale * kLog2e;
     const int kb0 = g0 - WB;
 
     RowFrag<D> qa, qb;
-    load_row<D, AL>(qa, qp + (size_t)row_lo * RS, tig, ok_lo);
-    load_row<D, AL>(qb, qp + (size_t)row_hi * RS, tig, ok_hi);
+    qr.template load2<AL>(qa, qb, 0, ok_lo, ok_hi);
     // Copies for the backward: tensor x (0: q, 1: k, 2: v), rows g / g + 8
     auto keep = [&](int x, const RowFrag<D>& f, int row, bool ok) {
         if (ST && a.keep && ok)
@@ -229,6 +259,7 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
     const float* se_lane = se_tile + g * (SeGeo<WB>::kPitch - 1) + 16 + 2 * tig;
 
     // ---- dense window: key row of n-tile nt for this thread is kb0 + 8 nt + g = row_lo - WB + 8 nt
+    const __nv_bfloat16* k_band = kr.at(-WB);
     float S[NT][4];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
@@ -238,12 +269,9 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             StartTable<WB>::get(S[nt], start, nt);
         }
         RowFrag<D> kf;
-        if (INTERIOR) {
-            load_row_at<D, AL>(kf, kl + (8 * nt - WB) * RS);
-        } else {
-            const int kr = kb0 + 8 * nt + g;
-            load_row<D, AL>(kf, kl + (ptrdiff_t)(8 * nt - WB) * RS - kLane<D> * tig, tig, kr >= 0 && kr < N);
-        }
+        const __nv_bfloat16* kp = ST ? kr.at(8 * nt - WB) : k_band + 8 * nt * D;
+        if (INTERIOR) load_row_at<D, AL>(kf, kp);
+        else load_piece<D, AL>(kf, kp, kb0 + 8 * nt + g >= 0 && kb0 + 8 * nt + g < N);
         if (nt >= WB / 8) keep(1, kf, nt == WB / 8 ? row_lo : row_hi, nt == WB / 8 ? ok_lo : ok_hi);
         mma_rows(S[nt], qa, qb, kf);
     }
@@ -269,16 +297,19 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
         l_lo += S[nt][0] + S[nt][1]; l_hi += S[nt][2] + S[nt][3];
     }
     float O[D / 8][4];
+    const __nv_bfloat16* v_band = vr.at(-WB);
 #pragma unroll
     for (int c = 0; c < NT / 2; ++c) {
         RowFrag<D> vf0, vf1, vt0, vt1;
+        const __nv_bfloat16* vp0 = ST ? vr.at(16 * c - WB) : v_band + 16 * c * D;
+        const __nv_bfloat16* vp1 = ST ? vr.at(16 * c + 8 - WB) : vp0 + 8 * D;
         if (INTERIOR) {
-            load_row_at<D, AL>(vf0, vl + (16 * c - WB) * RS);
-            load_row_at<D, AL>(vf1, vl + (16 * c + 8 - WB) * RS);
+            load_row_at<D, AL>(vf0, vp0);
+            load_row_at<D, AL>(vf1, vp1);
         } else {
-            const int kr = kb0 + 16 * c + g;
-            load_row<D, AL>(vf0, vl + (ptrdiff_t)(16 * c - WB) * RS - kLane<D> * tig, tig, kr >= 0 && kr < N);
-            load_row<D, AL>(vf1, vl + (ptrdiff_t)(16 * c + 8 - WB) * RS - kLane<D> * tig, tig, kr + 8 >= 0 && kr + 8 < N);
+            const int r = kb0 + 16 * c + g;
+            load_piece<D, AL>(vf0, vp0, r >= 0 && r < N);
+            load_piece<D, AL>(vf1, vp1, r + 8 >= 0 && r + 8 < N);
         }
         if (c == WB / 16) { keep(2, vf0, row_lo, ok_lo); keep(2, vf1, row_hi, ok_hi); }
         transpose_frag(vt0, vf0); transpose_frag(vt1, vf1);
@@ -327,13 +358,10 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
         float pbv[G];
 #pragma unroll
         for (int i = 0; i < G; ++i) {
-            const int2 tp = tap_s[si + i];
-            const ptrdiff_t off = (ptrdiff_t)tp.x * RS;
+            const int2 tp = make_int2(t.sparse[si + i], tap_s[si + i].y);
             pbv[i] = __int_as_float(tp.y);
-            load_row_at<D, AL>(kf0[i], kl - off);
-            load_row_at<D, AL>(kf1[i], kl - off + 8 * RS);
-            load_row_at<D, AL>(vf0[i], vl - off);
-            load_row_at<D, AL>(vf1[i], vl - off + 8 * RS);
+            kr.template load2<AL>(kf0[i], kf1[i], -tp.x);
+            vr.template load2<AL>(vf0[i], vf1[i], -tp.x);
         }
         float x0[G], x1[G];
 #pragma unroll
@@ -361,11 +389,11 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
     // usual tap sets do not reach from, and the last partial tile).
     int si = 0;
     if constexpr (INTERIOR)
-        for (; si + kTapGroup <= ns && g0 >= tap_s[si + kTapGroup - 1].x; si += kTapGroup)
+        for (; si + kTapGroup <= ns && g0 >= t.sparse[si + kTapGroup - 1]; si += kTapGroup)
             full_taps(std::integral_constant<int, kTapGroup>(), si);
 #pragma unroll 1
     for (; si < ns; ++si) {
-        const int delta = tap_s[si].x;
+        const int delta = t.sparse[si];
         if (g0 + 15 < delta) break;                       // taps ascend: no row of the tile reaches back that far
         if (INTERIOR && g0 >= delta) {
             full_taps(std::integral_constant<int, 1>(), si);
@@ -373,12 +401,9 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
             const float pbv = __int_as_float(tap_s[si].y);
             const int kr0 = row_lo - delta, kr1 = row_hi - delta;
             const bool v0 = kr0 >= 0 && kr0 < N, v1 = kr1 >= 0 && kr1 < N;
-            const ptrdiff_t off = (ptrdiff_t)delta * RS + kLane<D> * tig;
             RowFrag<D> kf0, kf1, vf0[1], vf1[1];
-            load_row<D, AL>(kf0, kl - off, tig, v0);
-            load_row<D, AL>(kf1, kl - off + 8 * RS, tig, v1);
-            load_row<D, AL>(vf0[0], vl - off, tig, v0);
-            load_row<D, AL>(vf1[0], vl - off + 8 * RS, tig, v1);
+            kr.template load2<AL>(kf0, kf1, -delta, v0, v1);
+            vr.template load2<AL>(vf0[0], vf1[0], -delta, v0, v1);
             float s0[4], s1[4];
             mma_rows_z(s0, qa, qb, kf0);
             mma_rows_z(s1, qa, qb, kf1);
@@ -410,7 +435,9 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
 // Tuning per head dimension (measured on B200): warps per CTA, sparse taps folded together,
 // resident CTAs per SM the register budget is set for.
 template <int D> struct FwdTune {
-    static constexpr int warps = 4, group = D == 64 || D > 80 ? 1 : 2, ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));   // D = 64: 92.8 us at 16x12x2048 (88.7 with group 2, which was behind, 107.8 to 104.8, before rows came in 32-byte pieces)
+    // Since a tap's address is one uniform product (Rows), registers allow more CTAs: D = 32 two taps, 7 CTAs (72 registers) 60.4 us at 32x8x2048,
+    // 6 CTAs 64.1, 5 CTAs 66.8 (65.5 before); D = 64 79.7 us at 16x12x2048 (one tap 87.8, 5 CTAs 86.2; 92.4 before).
+    static constexpr int warps = 4, group = D > 96 ? 1 : 2, ctas = D == 32 ? 7 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));
     // With scale_embed a CTA first lays out the table, about a quarter of a tile's time, so a warp does up to three tiles with it.
     // The count is the one for which (waves of CTAs) x (tiles + 1/4) is least: one where the grid is a single wave (2x8x777x32 11.6 us,
     // 12.5 with two), two or three where that saves a wave or its table (4x8x2048x32 19.5 -> 18.7, 32x8x2048x32 101.4 -> 97.3,
@@ -453,8 +480,8 @@ fwd_mma_kernel(const FwdArgs a, const Taps t, const int tiles_se) {
     for (int i = 0; i < tiles; ++i) {
         const int g0 = (blockIdx.x * tiles + i) * (16 * W) + L.warp * 16;
         if (g0 >= N) return;
-        if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
-        else fwd_tile<D, WB, false, G, SE, ST>(a, start, tap_s, t.n_sparse, bh, h, g0, L, se, se_tile);
+        if (g0 >= WB && g0 + 16 <= N) fwd_tile<D, WB, true, G, SE, ST>(a, start, tap_s, t, t.n_sparse, bh, h, g0, L, se, se_tile);
+        else fwd_tile<D, WB, false, G, SE, ST>(a, start, tap_s, t, t.n_sparse, bh, h, g0, L, se, se_tile);
         if (SE) __syncwarp();
     }
 }
@@ -462,10 +489,16 @@ fwd_mma_kernel(const FwdArgs a, const Taps t, const int tiles_se) {
 // Tuning per head dimension (measured on B200): sparse taps whose loads are issued together and
 // resident CTAs per SM the register budget is set for (spills against warps in flight).
 template <int D> struct BwdTune {
-    static constexpr int dq_group = D <= 80 ? 2 : 1, dq_ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D == 80 ? 3 : 2));   // D = 32: 98.5 us (108.8 with 4 CTAs, 103.3 with group 1); D = 80: 69.0 us (80 with 2 CTAs)
-    static constexpr int dq_group_se = D == 32 ? 2 : 1, dq_ctas_se = 4;    // with scale_embed: 32x8x2048x32 164.8 us (166.8 with group 1 and 5 CTAs), 16x12x2048x64 216.9 us (224.7 with group 2)
-    static constexpr int dkdv_group_se = D <= 64 ? 2 : 1, dkdv_ctas_se = D == 32 ? 4 : 3;
-    static constexpr int dkdv_group = D <= 80 ? 2 : 1, dkdv_ctas = D == 32 ? 4 : (D <= 64 ? 3 : 2);   // D = 80: 78.1 us (83 with group 1, 96-109 with 3 CTAs)
+    // 8x8x2048 unless said otherwise, us: D = 32 at 32x8x2048 89.7 (6 CTAs 90.6, one tap and 6 CTAs 91.0, 4 CTAs 96.7), D = 64 at 16x12x2048
+    // 114.9 (two taps 119.7), D = 80 59.8 (one tap 60.3), D = 96 66.0 (two taps 69.6, 2 CTAs 71.7-78.0), D = 128 84.5 (one tap 89.9)
+    static constexpr int dq_group = D == 64 || D == 96 ? 1 : 2, dq_ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));
+    // scale_embed: 32x8x2048x32 154.9 (5 CTAs 155.1, one tap 158-164), 16x12x2048x64 202.6 (one tap 208.6, 3 CTAs 205-212)
+    static constexpr int dq_group_se = 2, dq_ctas_se = 4;
+    // D = 32 at 32x8x2048 94.2 (4 CTAs 98.1, 6 CTAs 110-115), D = 64 at 16x12x2048 132.4 (two taps 134.9), D = 48 44.3, D = 80 69.0 (one tap 73.8,
+    // 3 CTAs 82), D = 96 78.8 (one tap 82.1), D = 128 116.0 (two taps 125.2)
+    static constexpr int dkdv_group = D == 64 ? 3 : (D > 96 ? 1 : 2), dkdv_ctas = D == 32 ? 5 : (D <= 64 ? 3 : 2);
+    // scale_embed: 32x8x2048x32 129.1 (one tap 128.9, 4 CTAs 133.3), 16x12x2048x64 185.0 (two taps 187.1, 4 CTAs 238)
+    static constexpr int dkdv_group_se = D == 32 ? 2 : 1, dkdv_ctas_se = D == 32 ? 5 : 3;
 };
 // Where a warp of the plain dQ kernel puts its ds values for dpos_bias.  Element (g + 8 half, 8 nt + 2 tig + c) of a
 // tile belongs to offset g - 2 tig - c + 8 k with k = WB / 8 + half - nt, so elements of neighbouring n-tiles share
@@ -535,7 +568,7 @@ template <int WB> struct SeBwd {
 
 template <int D, int WB, bool INTERIOR, int G, bool SE, int ST>
 __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, const int2* tap_s,
-                                         float* stage_w, int ns, int bh, int h, int g0, const Lane& L, const SeBwd<WB>& sb) {
+                                         float* stage_w, const Taps& t, int ns, int bh, int h, int g0, const Lane& L, const SeBwd<WB>& sb) {
     constexpr int NT = (WB + 16) / 8;
     using Stage = DsStage<WB>;
     const int N = a.N, g = L.g, tig = L.tig;
@@ -545,11 +578,8 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     const ptrdiff_t GS = ST ? (ptrdiff_t)a.in_sn : D, RS = CI ? D : GS, OS = CI ? D : (ptrdiff_t)a.out_sn;   // row strides of dq, q/k/v, out/dout
     const size_t cbase = (size_t)bh * N * D, gbase = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : cbase, base = CI ? cbase : gbase;
     const size_t obase = CI ? cbase : (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh;
-    const __nv_bfloat16* qp = static_cast<const __nv_bfloat16*>(a.q) + base;
-    const __nv_bfloat16* op = static_cast<const __nv_bfloat16*>(a.out) + obase;
-    const __nv_bfloat16* dop = static_cast<const __nv_bfloat16*>(a.dout) + obase;
-    const __nv_bfloat16* kl = static_cast<const __nv_bfloat16*>(a.k) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
-    const __nv_bfloat16* vl = static_cast<const __nv_bfloat16*>(a.v) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
+    const Rows<D, CI> qr(a.q, base, g0, RS, L), kr(a.k, base, g0, RS, L), vr(a.v, base, g0, RS, L);
+    const Rows<D, CI> orow(a.out, obase, g0, OS, L), dr(a.dout, obase, g0, OS, L);
     const float c2 = a.scale * kLog2e;
     const float gain = a.head_gain ? a.head_gain[h] : 1.f;
     const int kb0 = g0 - WB;
@@ -557,10 +587,8 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     f32x2 dgrow2 = 0ull;
 
     RowFrag<D> qa, qb, da, db;
-    load_row<D, AL>(qa, qp + (size_t)row_lo * RS, tig, ok_lo);
-    load_row<D, AL>(qb, qp + (size_t)row_hi * RS, tig, ok_hi);
-    load_row<D, AL>(da, dop + (size_t)row_lo * OS, tig, ok_lo);
-    load_row<D, AL>(db, dop + (size_t)row_hi * OS, tig, ok_hi);
+    qr.template load2<AL>(qa, qb, 0, ok_lo, ok_hi);
+    dr.template load2<AL>(da, db, 0, ok_lo, ok_hi);
     if constexpr (SE) {
         // the sparse part also goes to global memory for the dK/dV kernel (a row of ns8 floats per query)
         const int ns8 = (ns + 7) / 8 * 8;
@@ -582,8 +610,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
         delta_hi = ok_hi ? a.delta_pre[(size_t)bh * N + row_hi] : 0.f;
     } else {
         RowFrag<D> oa, ob;
-        load_row<D, AL>(oa, op + (size_t)row_lo * OS, tig, ok_lo);
-        load_row<D, AL>(ob, op + (size_t)row_hi * OS, tig, ok_hi);
+        orow.template load2<AL>(oa, ob, 0, ok_lo, ok_hi);
         delta_lo = quad_sum(frag_dot(da, oa));
         delta_hi = quad_sum(frag_dot(db, ob));
     }
@@ -600,6 +627,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     float* se_lane = SE ? sb.tile + g * (sb.pitch - 1) + 16 + 2 * tig : nullptr;
 
     // ---- dense window
+    const __nv_bfloat16 *k_band = kr.at(-WB), *v_band = vr.at(-WB);
 #pragma unroll
     for (int c = 0; c < NT / 2; ++c) {
         RowFrag<D> kf[2];
@@ -614,14 +642,16 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
                 StartTable<WB>::get(s, start, nt);
             }
             RowFrag<D> vf;
+            const __nv_bfloat16* kp = CI ? k_band + 8 * nt * D : kr.at(8 * nt - WB);
+            const __nv_bfloat16* vp = CI ? v_band + 8 * nt * D : vr.at(8 * nt - WB);
             if (INTERIOR) {
-                load_row_at<D, AL>(kf[hf], kl + (8 * nt - WB) * RS);
-                load_row_at<D, AL>(vf, vl + (8 * nt - WB) * RS);
+                load_row_at<D, AL>(kf[hf], kp);
+                load_row_at<D, AL>(vf, vp);
             } else {
-                const int kr = kb0 + 8 * nt + g;
-                const bool kv = kr >= 0 && kr < N;
-                load_row<D, AL>(kf[hf], kl + (ptrdiff_t)(8 * nt - WB) * RS - kLane<D> * tig, tig, kv);
-                load_row<D, AL>(vf, vl + (ptrdiff_t)(8 * nt - WB) * RS - kLane<D> * tig, tig, kv);
+                const int r = kb0 + 8 * nt + g;
+                const bool valid = r >= 0 && r < N;
+                load_piece<D, AL>(kf[hf], kp, valid);
+                load_piece<D, AL>(vf, vp, valid);
             }
             mma_rows(s, qa, qb, kf[hf]);
             mma_rows_z(dp, da, db, vf);
@@ -695,13 +725,10 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
         float pbv[GG];
 #pragma unroll
         for (int i = 0; i < GG; ++i) {
-            const int2 tp = tap_s[si + i];
-            const ptrdiff_t off = (ptrdiff_t)tp.x * RS;
+            const int2 tp = make_int2(t.sparse[si + i], tap_s[si + i].y);
             pbv[i] = __int_as_float(tp.y);
-            load_row_at<D, AL>(kf0[i], kl - off);
-            load_row_at<D, AL>(kf1[i], kl - off + 8 * RS);
-            load_row_at<D, AL>(vf0[i], vl - off);
-            load_row_at<D, AL>(vf1[i], vl - off + 8 * RS);
+            kr.template load2<AL>(kf0[i], kf1[i], -tp.x);
+            vr.template load2<AL>(vf0[i], vf1[i], -tp.x);
         }
 #pragma unroll
         for (int i = 0; i < GG; ++i) {
@@ -715,22 +742,19 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     // as in the forward: only interior tiles load taps unpredicated, so no key row past the end is read
     int si = 0;
     if constexpr (INTERIOR)
-        for (; si + G <= ns && g0 >= tap_s[si + G - 1].x; si += G) full_taps(std::integral_constant<int, G>(), si);
+        for (; si + G <= ns && g0 >= t.sparse[si + G - 1]; si += G) full_taps(std::integral_constant<int, G>(), si);
 #pragma unroll 1
     for (; si < ns; ++si) {
-        const int delta = tap_s[si].x;
+        const int delta = t.sparse[si];
         if (g0 + 15 < delta) break;
         if (INTERIOR && g0 >= delta) {
             full_taps(std::integral_constant<int, 1>(), si);
         } else {
             const float pbv = __int_as_float(tap_s[si].y);
             const bool v0 = row_lo >= delta && row_lo - delta < N, v1 = row_hi >= delta && row_hi - delta < N;
-            const ptrdiff_t off = (ptrdiff_t)delta * RS + kLane<D> * tig;
             RowFrag<D> kf0, kf1, vf0, vf1;
-            load_row<D, AL>(kf0, kl - off, tig, v0);
-            load_row<D, AL>(kf1, kl - off + 8 * RS, tig, v1);
-            load_row<D, AL>(vf0, vl - off, tig, v0);
-            load_row<D, AL>(vf1, vl - off + 8 * RS, tig, v1);
+            kr.template load2<AL>(kf0, kf1, -delta, v0, v1);
+            vr.template load2<AL>(vf0, vf1, -delta, v0, v1);
             float s0[4], s1[4], e0[4], e1[4];
             mma_rows_z(s0, qa, qb, kf0); mma_rows_z(s1, qa, qb, kf1);
             mma_rows_z(e0, da, db, vf0); mma_rows_z(e1, da, db, vf1);
@@ -867,9 +891,9 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
         if constexpr (SE)
             for (int e = L.lane; e < sb.pitch16; e += 32) reinterpret_cast<uint4*>(sb.ds16)[e] = make_uint4(0u, 0u, 0u, 0u);
     } else if (g0 >= WB && g0 + 16 <= N) {
-        dgrow = dq_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stage_w, t.n_sparse, bh, h, g0, L, sb);
+        dgrow = dq_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stage_w, t, t.n_sparse, bh, h, g0, L, sb);
     } else {
-        dgrow = dq_tile<D, WB, false, G, SE, ST>(a, start, tap_s, stage_w, t.n_sparse, bh, h, g0, L, sb);
+        dgrow = dq_tile<D, WB, false, G, SE, ST>(a, start, tap_s, stage_w, t, t.n_sparse, bh, h, g0, L, sb);
     }
     if constexpr (!SE)
         if (g0 < N) Stage::sum(stage_w, t, L.lane);
@@ -963,7 +987,7 @@ dse_group_kernel(const float* __restrict__ tmp, float* __restrict__ part, int ti
 // sparse tap adds the entry of its query row, which the dQ kernel left in qs_rows.
 template <int D, int WB, bool INTERIOR, int G, bool SE, int ST>
 __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, const int2* tap_s, const float* stat_w,
-                                          int ns, int bh, int h, int m0, const Lane& L, const float* se_tile) {
+                                          const Taps& t, int ns, int bh, int h, int m0, const Lane& L, const float* se_tile) {
     constexpr int NT = (WB + 16) / 8, kStat = kRows + WB;
     const int N = a.N, g = L.g, tig = L.tig;
     const int row_lo = m0 + g, row_hi = row_lo + 8;
@@ -972,23 +996,24 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
     const ptrdiff_t GS = ST ? (ptrdiff_t)a.in_sn : D, RS = CI ? D : GS, OS = CI ? D : (ptrdiff_t)a.out_sn;   // row strides of dk/dv, q/k/v, dout
     const size_t cbase = (size_t)bh * N * D, gbase = ST ? (size_t)(bh / a.H) * a.in_sb + (size_t)h * a.in_sh : cbase, base = CI ? cbase : gbase;
     const size_t obase = CI ? cbase : (size_t)(bh / a.H) * a.out_sb + (size_t)h * a.out_sh;
-    const __nv_bfloat16* kp = static_cast<const __nv_bfloat16*>(a.k) + base;
-    const __nv_bfloat16* vp = static_cast<const __nv_bfloat16*>(a.v) + base;
-    const __nv_bfloat16* ql = static_cast<const __nv_bfloat16*>(a.q) + base + (ptrdiff_t)row_lo * RS + kLane<D> * tig;
-    const __nv_bfloat16* dl = static_cast<const __nv_bfloat16*>(a.dout) + obase + (ptrdiff_t)row_lo * OS + kLane<D> * tig;
-    const float2* rs = reinterpret_cast<const float2*>(a.delta) + (size_t)bh * N + row_lo;
+    const Rows<D, CI> kr(a.k, base, m0, RS, L), vr(a.v, base, m0, RS, L), qr(a.q, base, m0, RS, L), dr(a.dout, obase, m0, OS, L);
+    const float2* rs = reinterpret_cast<const float2*>(a.delta) + (size_t)bh * N + m0;
+    auto stat_at = [&](int rows) {                       // of query row row_lo + rows
+        unsigned long long x;
+        asm("mad.wide.s32 %0, %1, 8, %2;" : "=l"(x) : "r"(rows), "l"(rs));
+        return reinterpret_cast<const float2*>(x + 8u * (unsigned)g);
+    };
     const float c2 = a.scale * kLog2e;
     const float gain = a.head_gain ? a.head_gain[h] : 1.f;
 
     RowFrag<D> ka, kb, va, vb;
-    load_row<D, AL>(ka, kp + (size_t)row_lo * RS, tig, ok_lo);
-    load_row<D, AL>(kb, kp + (size_t)row_hi * RS, tig, ok_hi);
-    load_row<D, AL>(va, vp + (size_t)row_lo * RS, tig, ok_lo);
-    load_row<D, AL>(vb, vp + (size_t)row_hi * RS, tig, ok_hi);
+    kr.template load2<AL>(ka, kb, 0, ok_lo, ok_hi);
+    vr.template load2<AL>(va, vb, 0, ok_lo, ok_hi);
     float dK[D / 8][4], dV[D / 8][4];
     const float* se_lane = SE ? se_tile + 2 * tig * (kSeKeyPitch<WB> - 1) + WB + 16 + g : nullptr;
 
     // ---- dense window: query row of n-tile nt for this thread is m0 + 8 nt + g
+    const __nv_bfloat16 *q_band = qr.at(0), *d_band = dr.at(0);
 #pragma unroll
     for (int c = 0; c < NT / 2; ++c) {
         if (!INTERIOR && c > 0 && m0 + 16 * c >= N) break;   // warp-uniform: no query rows left
@@ -1003,13 +1028,15 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
             } else {
                 StartTable<WB>::get(s, start, nt);
             }
+            const __nv_bfloat16* qp = CI ? q_band + 8 * nt * D : qr.at(8 * nt);
+            const __nv_bfloat16* dp_ = CI ? d_band + 8 * nt * D : dr.at(8 * nt);
             if (INTERIOR) {
-                load_row_at<D, AL>(qf[hf], ql + 8 * nt * RS);
-                load_row_at<D, AL>(df[hf], dl + 8 * nt * OS);
+                load_row_at<D, AL>(qf[hf], qp);
+                load_row_at<D, AL>(df[hf], dp_);
             } else {
                 const bool qv = m0 + 8 * nt + g < N;
-                load_row<D, AL>(qf[hf], ql + (ptrdiff_t)8 * nt * RS - kLane<D> * tig, tig, qv);
-                load_row<D, AL>(df[hf], dl + (ptrdiff_t)8 * nt * OS - kLane<D> * tig, tig, qv);
+                load_piece<D, AL>(qf[hf], qp, qv);
+                load_piece<D, AL>(df[hf], dp_, qv);
             }
             mma_rows(s, ka, kb, qf[hf]);
             mma_rows_z(dp, va, vb, df[hf]);
@@ -1065,20 +1092,18 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
         float b0[GG], b1[GG];
 #pragma unroll
         for (int i = 0; i < GG; ++i) {
-            const int2 tp = tap_s[si + i];
-            const ptrdiff_t off = (ptrdiff_t)tp.x * RS, offd = (ptrdiff_t)tp.x * OS;
+            const int2 tp = make_int2(t.sparse[si + i], tap_s[si + i].y);
             if constexpr (SE) {
                 b0[i] = __ldg(qs_r + (size_t)tp.x * ns8 + si + i);
                 b1[i] = __ldg(qs_r + (size_t)(tp.x + 8) * ns8 + si + i);
             } else {
                 b0[i] = b1[i] = __int_as_float(tp.y);
             }
-            load_row_at<D, AL>(qf0[i], ql + off);
-            load_row_at<D, AL>(qf1[i], ql + off + 8 * RS);
-            load_row_at<D, AL>(df0[i], dl + offd);
-            load_row_at<D, AL>(df1[i], dl + offd + 8 * OS);
-            st0[i] = __ldg(rs + tp.x);
-            st1[i] = __ldg(rs + tp.x + 8);
+            qr.template load2<AL>(qf0[i], qf1[i], tp.x);
+            dr.template load2<AL>(df0[i], df1[i], tp.x);
+            const float2* st = stat_at(tp.x);
+            st0[i] = __ldg(st);
+            st1[i] = __ldg(st + 8);
         }
 #pragma unroll
         for (int i = 0; i < GG; ++i) {
@@ -1090,10 +1115,10 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
         }
     };
     int si = 0;
-    for (; si + G <= ns && m0 + 16 + tap_s[si + G - 1].x <= N; si += G) full_taps(std::integral_constant<int, G>(), si);
+    for (; si + G <= ns && m0 + 16 + t.sparse[si + G - 1] <= N; si += G) full_taps(std::integral_constant<int, G>(), si);
 #pragma unroll 1
     for (; si < ns; ++si) {
-        const int delta = tap_s[si].x;
+        const int delta = t.sparse[si];
         if (m0 + delta >= N) break;                     // taps ascend: no query row reads these keys any more
         if (m0 + 16 + delta <= N) {
             full_taps(std::integral_constant<int, 1>(), si);
@@ -1104,14 +1129,12 @@ __device__ __forceinline__ void dkdv_tile(const BwdArgs& a, const float* start, 
                 b0 = v0 ? __ldg(qs_r + (size_t)delta * ns8 + si) : 0.f;
                 b1 = v1 ? __ldg(qs_r + (size_t)(delta + 8) * ns8 + si) : 0.f;
             }
-            const ptrdiff_t off = (ptrdiff_t)delta * RS - kLane<D> * tig, offd = (ptrdiff_t)delta * OS - kLane<D> * tig;
             RowFrag<D> qf0, qf1, df0, df1;
-            load_row<D, AL>(qf0, ql + off, tig, v0);
-            load_row<D, AL>(qf1, ql + off + 8 * RS, tig, v1);
-            load_row<D, AL>(df0, dl + offd, tig, v0);
-            load_row<D, AL>(df1, dl + offd + 8 * OS, tig, v1);
-            const float2 st0 = v0 ? __ldg(rs + delta) : make_float2(0.f, 0.f);
-            const float2 st1 = v1 ? __ldg(rs + delta + 8) : make_float2(0.f, 0.f);
+            qr.template load2<AL>(qf0, qf1, delta, v0, v1);
+            dr.template load2<AL>(df0, df1, delta, v0, v1);
+            const float2* st = stat_at(delta);
+            const float2 st0 = v0 ? __ldg(st) : make_float2(0.f, 0.f);
+            const float2 st1 = v1 ? __ldg(st + 8) : make_float2(0.f, 0.f);
             float s0[4], s1[4], e0[4], e1[4];
             mma_rows_z(s0, ka, kb, qf0); mma_rows_z(s1, ka, kb, qf1);
             mma_rows_z(e0, va, vb, df0); mma_rows_z(e1, va, vb, df1);
@@ -1178,9 +1201,9 @@ bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int
     const float* se_w = SE ? se_tile + L.warp * 16 * kSeKeyPitch<WB> : nullptr;
     const float* start = StartTable<WB>::lane(start_s, L);
     if (m0 + 16 + WB <= N)
-        dkdv_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, se_w);
+        dkdv_tile<D, WB, true, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t, t.n_sparse, bh, h, m0, L, se_w);
     else
-        dkdv_tile<D, WB, false, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t.n_sparse, bh, h, m0, L, se_w);
+        dkdv_tile<D, WB, false, G, SE, ST>(a, start, tap_s, stat_s + L.warp * 16, t, t.n_sparse, bh, h, m0, L, se_w);
 }
 
 // Raises a kernel's dynamic shared-memory limit to what this launch needs.  The attribute is set
