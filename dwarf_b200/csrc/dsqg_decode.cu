@@ -103,6 +103,7 @@ __device__ __forceinline__ void merge_and_store(TapState& st, const DecodeArgs& 
 template <typename T, int TPR, int ROUNDS>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 decode_kernel(const DecodeArgs a, const Taps t) {
+    stream_wait();
     constexpr int GROUPS = 32 / TPR;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int sh = blockIdx.x * kWarpsPerBlock + warp;      // (sequence, head) pair
@@ -184,6 +185,7 @@ template <int TPR, int ROUNDS, int VSM, int CTAS, bool PDL>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, CTAS)
 decode_1pass_kernel(const DecodeArgs a, const Taps t) {
     if constexpr (PDL) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    else stream_wait();
     using T = __nv_bfloat16;
     constexpr int GROUPS = 32 / TPR;
     constexpr int VREG = ROUNDS - VSM;
@@ -314,24 +316,14 @@ template <int TPR, int ROUNDS, int VSM, int CTAS>
 cudaError_t decode_launch_1pass(const DecodeArgs& a, const Taps& t, cudaStream_t s, bool overlap) {
     const int pairs = a.S * a.H;
     const unsigned blocks = (pairs + kWarpsPerBlock - 1) / kWarpsPerBlock;
-    if (!overlap) {
-        decode_1pass_kernel<TPR, ROUNDS, VSM, CTAS, false><<<blocks, kWarpsPerBlock * 32, 0, s>>>(a, t);
-        return cudaGetLastError();
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks); cfg.blockDim = dim3(kWarpsPerBlock * 32); cfg.dynamicSmemBytes = 0; cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, decode_1pass_kernel<TPR, ROUNDS, VSM, CTAS, true>, a, t);
+    return launch_after(overlap ? decode_1pass_kernel<TPR, ROUNDS, VSM, CTAS, true> : decode_1pass_kernel<TPR, ROUNDS, VSM, CTAS, false>, blocks,
+                        kWarpsPerBlock * 32, 0, s, a, t);
 }
 
 template <typename T, int TPR, int ROUNDS>
 cudaError_t decode_launch_r(const DecodeArgs& a, const Taps& t, cudaStream_t s) {
     const int pairs = a.S * a.H;
-    decode_kernel<T, TPR, ROUNDS><<<(pairs + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, s>>>(a, t);
-    return cudaGetLastError();
+    return launch_after(decode_kernel<T, TPR, ROUNDS>, (pairs + kWarpsPerBlock - 1) / kWarpsPerBlock, kWarpsPerBlock * 32, 0, s, a, t);
 }
 
 template <typename T, int TPR>
@@ -369,6 +361,7 @@ cudaError_t decode_launch(const DecodeArgs& a, const Taps& t, cudaStream_t s, bo
 __global__ void ring_prefill_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, uint4* k_ring, uint4* v_ring,
                                     int32_t* head, int32_t* fill, int SH, int H, int N, int R, int chunks_per_row,
                                     int ring_chunks) {
+    stream_wait();
     const int keep = N < R ? N : R;
     const long long total = (long long)SH * keep * chunks_per_row;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -394,13 +387,12 @@ cudaError_t launch_ring_prefill(const void* k, const void* v, void* k_ring, void
     long long blocks = (total + 255) / 256;
     if (blocks < (S + 255) / 256) blocks = (S + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    ring_prefill_kernel<<<(int)blocks, 256, 0, s>>>(static_cast<const uint4*>(k), static_cast<const uint4*>(v),
-                                                  static_cast<uint4*>(k_ring), static_cast<uint4*>(v_ring), head, fill,
-                                                  S * H, H, N, R, chunks, interleaved ? 2 * chunks : chunks);
-    return cudaGetLastError();
+    return launch_after(ring_prefill_kernel, (unsigned)blocks, 256, 0, s, static_cast<const uint4*>(k), static_cast<const uint4*>(v),
+                        static_cast<uint4*>(k_ring), static_cast<uint4*>(v_ring), head, fill, S * H, H, N, R, chunks, interleaved ? 2 * chunks : chunks);
 }
 
 __global__ void __launch_bounds__(256) ring_advance_kernel(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R) {
+    stream_wait();
     const int s = blockIdx.x * 256 + threadIdx.x;
     if (s >= S) return;
     const int h = (head[s] + 1) % R;
@@ -409,8 +401,7 @@ __global__ void __launch_bounds__(256) ring_advance_kernel(const int32_t* head, 
 }
 
 cudaError_t launch_ring_advance(const int32_t* head, const int32_t* fill, int32_t* head_out, int32_t* fill_out, int S, int R, cudaStream_t s) {
-    ring_advance_kernel<<<(S + 255) / 256, 256, 0, s>>>(head, fill, head_out, fill_out, S, R);
-    return cudaGetLastError();
+    return launch_after(ring_advance_kernel, (S + 255) / 256, 256, 0, s, head, fill, head_out, fill_out, S, R);
 }
 
 cudaError_t launch_decode(const DecodeArgs& a, const Taps& t, int dtype, cudaStream_t s, bool overlap) {

@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256, 6)
 gate_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ y,
                 const dsqg_strides ys, const __nv_bfloat16* __restrict__ gate, const dsqg_strides gs, __nv_bfloat16* __restrict__ dgate, const dsqg_strides dgs,
                 __nv_bfloat16* __restrict__ dout, const dsqg_strides os, float* __restrict__ delta, int B, int H, int N, int D) {
+    stream_wait();
     const unsigned row = (blockIdx.x * 256u + threadIdx.x) / LPR, c = threadIdx.x % LPR * 8;
     if (row >= (unsigned)B * N * H) return;                    // whole lane groups leave
     const unsigned h = row % H, bn = row / H, n = bn % N, b = bn / N;
@@ -67,10 +68,9 @@ cudaError_t gate_launch(const void* dy, const void* y, const dsqg_strides& ys, c
                         const dsqg_strides& dgs, void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s) {
     const long long threads = (long long)B * N * H * LPR;
     const bool same = gs.batch == dgs.batch && gs.head == dgs.head && gs.row == dgs.row;
-    (same ? gate_bwd_kernel<LPR, true> : gate_bwd_kernel<LPR, false>)<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+    return launch_after(same ? gate_bwd_kernel<LPR, true> : gate_bwd_kernel<LPR, false>, (unsigned)((threads + 255) / 256), 256, 0, s,
         static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(y), ys, static_cast<const __nv_bfloat16*>(gate), gs,
         static_cast<__nv_bfloat16*>(dgate), dgs, static_cast<__nv_bfloat16*>(dout), os, delta, B, H, N, D);
-    return cudaGetLastError();
 }
 
 }  // namespace

@@ -56,6 +56,7 @@ fwd_generic_kernel(const FwdArgs a, const Taps t) {
     constexpr int R = kFwdRows, GPB = kFwdThreads / LPR;
     __shared__ float pb_s[DSQG_MAX_TAPS];
     __shared__ int off_s[DSQG_MAX_TAPS];
+    stream_wait();
     const int bh = blockIdx.y, h = bh % a.H, N = a.N, D = EXACT ? 4 * LPR : a.D, J = t.J;
     const int g = threadIdx.x / LPR, li = threadIdx.x % LPR, d0 = 4 * li, tap_lane = li & 7;
     const bool active = d0 < D;
@@ -197,6 +198,7 @@ fwd_generic_kernel(const FwdArgs a, const Taps t) {
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kThreads)
 bwd_dq_generic_kernel(const BwdArgs a, const Taps t) {
+    stream_wait();
     constexpr int RPB = kThreads / TPR;
     extern __shared__ float smem[];
     __shared__ float pb_s[DSQG_MAX_TAPS];
@@ -316,6 +318,7 @@ bwd_dq_generic_kernel(const BwdArgs a, const Taps t) {
 template <typename T, int TPR>
 __global__ void __launch_bounds__(kThreads)
 bwd_dkdv_generic_kernel(const BwdArgs a, const Taps t) {
+    stream_wait();
     constexpr int RPB = kThreads / TPR;
     __shared__ float pb_s[DSQG_MAX_TAPS];
     const int J = t.J, D = a.D;
@@ -386,14 +389,14 @@ bwd_dkdv_generic_kernel(const BwdArgs a, const Taps t) {
 // partial sums, then a fixed shared-memory tree), so the result is bitwise reproducible.
 __global__ void __launch_bounds__(kReduceThreads)
 bwd_reduce_params_kernel(const BwdArgs a, const int J) {
+    stream_wait();
     __shared__ float red[kReduceThreads];
     reduce_one_param(a, J, blockIdx.x, red);
 }
 
 cudaError_t launch_reduce_params(const BwdArgs& a, int J, cudaStream_t s) {
     const int total = J * a.H + a.H + ((a.dscale_embed && a.scale_embed) ? J * a.D : 0);
-    bwd_reduce_params_kernel<<<total, kReduceThreads, 0, s>>>(a, J);
-    return cudaGetLastError();
+    return launch_after(bwd_reduce_params_kernel, total, kReduceThreads, 0, s, a, J);
 }
 
 namespace {
@@ -401,9 +404,7 @@ template <typename T, int LPR>
 cudaError_t fwd_launch(const FwdArgs& a, const Taps& t, cudaStream_t s) {
     constexpr int RPB = kFwdThreads / LPR * kFwdRows;
     dim3 grid((a.N + RPB - 1) / RPB, a.B * a.H);
-    if (a.D == 4 * LPR) fwd_generic_kernel<T, LPR, true><<<grid, kFwdThreads, 0, s>>>(a, t);
-    else fwd_generic_kernel<T, LPR, false><<<grid, kFwdThreads, 0, s>>>(a, t);
-    return cudaGetLastError();
+    return launch_after(a.D == 4 * LPR ? fwd_generic_kernel<T, LPR, true> : fwd_generic_kernel<T, LPR, false>, grid, kFwdThreads, 0, s, a, t);
 }
 template <typename T>
 cudaError_t fwd_launch_width(const FwdArgs& a, const Taps& t, cudaStream_t s) {
@@ -425,13 +426,11 @@ cudaError_t bwd_launch(BwdArgs a, const Taps& t, cudaStream_t s, int stages) {
     cudaError_t e = cudaSuccess;
     if (stages & DSQG_BWD_STAGE_DQ) {
         dim3 grid_q(a.tiles_per_bh, a.B * a.H);
-        bwd_dq_generic_kernel<T, TPR><<<grid_q, kThreads, smem, s>>>(a, t);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if ((e = launch_after(bwd_dq_generic_kernel<T, TPR>, grid_q, kThreads, smem, s, a, t)) != cudaSuccess) return e;
     }
     if (stages & DSQG_BWD_STAGE_DKDV) {
         dim3 grid_k((a.N + RPB - 1) / RPB, a.B * a.H);
-        bwd_dkdv_generic_kernel<T, TPR><<<grid_k, kThreads, 0, s>>>(a, t);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if ((e = launch_after(bwd_dkdv_generic_kernel<T, TPR>, grid_k, kThreads, 0, s, a, t)) != cudaSuccess) return e;
     }
     if (stages & DSQG_BWD_STAGE_REDUCE) e = launch_reduce_params(a, t.J, s);
     return e;

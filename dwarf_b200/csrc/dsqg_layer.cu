@@ -15,6 +15,7 @@ constexpr int kT = 256;
 struct CastArgs { const float* src[DSQG_CAST_MAX]; __nv_bfloat16* dst[DSQG_CAST_MAX]; long long end[DSQG_CAST_MAX]; int count; };   // end: running sum of the lengths
 
 __global__ void __launch_bounds__(kT) cast_kernel(const CastArgs a) {
+    stream_wait();
     const long long total = a.end[a.count - 1];
     for (long long i = ((long long)blockIdx.x * kT + threadIdx.x) * 8; i < total; i += (long long)gridDim.x * kT * 8) {
         int k = 0;
@@ -31,6 +32,7 @@ __global__ void __launch_bounds__(kT) cast_kernel(const CastArgs a) {
 __global__ void __launch_bounds__(kT)
 layer_norm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta, float eps,
                       float* __restrict__ y, __nv_bfloat16* __restrict__ yb, float2* __restrict__ stat, long long rows, int D) {
+    stream_wait();
     const long long row = (long long)blockIdx.x * (kT / 32) + (threadIdx.x >> 5);
     if (row >= rows) return;
     const int lane = threadIdx.x & 31;
@@ -66,6 +68,7 @@ __global__ void __launch_bounds__(kT)
 layer_norm_bwd_kernel(const float* __restrict__ x, const float* __restrict__ mean, const float* __restrict__ rstd, int step, const float* __restrict__ gamma,
                       const float* __restrict__ dya, const __nv_bfloat16* __restrict__ dyb, float* __restrict__ dx,
                       float* __restrict__ part, long long rows, int D) {
+    stream_wait();
     extern __shared__ float sums[];                            // [2][D]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float4 dg[C4], db[C4];
@@ -124,6 +127,7 @@ layer_norm_bwd_kernel(const float* __restrict__ x, const float* __restrict__ mea
 
 // out[c] = sum_b part[b][c], one warp per 32 columns, rows of the table split over the warps of a block
 __global__ void __launch_bounds__(kT) sum_rows_kernel(const float* __restrict__ part, float* __restrict__ out, int n, int C) {
+    stream_wait();
     __shared__ float red[kT / 32][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
     float s = 0.f;
@@ -142,6 +146,7 @@ __global__ void __launch_bounds__(kT) sum_rows_kernel(const float* __restrict__ 
 // ---- k += k_delta, v += v_delta on columns D .. 3 D of qkv; rows lq / ld elements apart
 __global__ void __launch_bounds__(kT) inject_kernel(__nv_bfloat16* __restrict__ qkv, long long lq, const __nv_bfloat16* __restrict__ kd,
                                                     const __nv_bfloat16* __restrict__ vd, long long ld, long long rows, int D) {
+    stream_wait();
     const long long i = (long long)blockIdx.x * kT + threadIdx.x;
     const int per = D / 8;                                     // 16-byte pieces of a delta row
     if (i >= rows * 2 * per) return;
@@ -161,6 +166,7 @@ struct SumArgs { const __nv_bfloat16* src[DSQG_SUM_MAX]; float* dst[DSQG_SUM_MAX
 constexpr int kSumThreads = 512, kSumCols = 64, kSumRows = kSumThreads / (kSumCols / 8);
 
 __global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(kSumThreads) column_sum_kernel(const SumArgs a) {
+    stream_wait();
     __shared__ float red[kSumRows][kSumCols + 1];
     __shared__ float total[8][kSumCols];
     asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");      // block 0 may be written to once it has started
@@ -212,7 +218,7 @@ inline unsigned blocks_for(long long n) { return (unsigned)((n + kT - 1) / kT); 
 constexpr int kNormBlocks = 148 * 2;
 inline unsigned norm_blocks(long long rows) { const long long b = (rows + kT / 32 - 1) / (kT / 32); return (unsigned)(b < kNormBlocks ? b : kNormBlocks); }
 inline bool bad(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) != 0; }
-inline int status() { return cudaGetLastError() == cudaSuccess ? DSQG_OK : DSQG_ERR_CUDA; }
+inline int status(cudaError_t e) { return e == cudaSuccess ? DSQG_OK : DSQG_ERR_CUDA; }
 inline bool bad_rows(long long rows, int D) { return rows < 1 || D < 8 || D % 8 || D > 1024 || rows * D > 0x7fffffffffLL; }
 
 }  // namespace
@@ -235,8 +241,7 @@ int dsqg_cast_bf16(const float* const* src, void* const* dst, const long long* n
         a.src[k] = src[k]; a.dst[k] = static_cast<__nv_bfloat16*>(dst[k]); a.end[k] = total += n[k];
     }
     const unsigned blocks = blocks_for(total / 8);
-    cast_kernel<<<blocks < 148 * 16 ? blocks : 148 * 16, kT, 0, static_cast<cudaStream_t>(stream)>>>(a);
-    return status();
+    return status(launch_after(cast_kernel, blocks < 148 * 16 ? blocks : 148 * 16, kT, 0, static_cast<cudaStream_t>(stream), a));
 }
 
 int dsqg_layer_norm_fwd(const float* x, const float* gamma, const float* beta, float eps, float* y, void* y_bf16, float* stat,
@@ -244,9 +249,8 @@ int dsqg_layer_norm_fwd(const float* x, const float* gamma, const float* beta, f
     if (!x || !gamma || !beta || !y || !y_bf16 || !stat) return DSQG_ERR_NULL_POINTER;
     if (bad_rows(rows, D)) return DSQG_ERR_BAD_SHAPE;
     if (bad(x) || bad(gamma) || bad(beta) || bad(y) || bad(y_bf16) || bad(stat)) return DSQG_ERR_MISALIGNED;
-    layer_norm_fwd_kernel<<<(unsigned)((rows + kT / 32 - 1) / (kT / 32)), kT, 0, static_cast<cudaStream_t>(stream)>>>(
-        x, gamma, beta, eps, y, static_cast<__nv_bfloat16*>(y_bf16), reinterpret_cast<float2*>(stat), rows, D);
-    return status();
+    return status(launch_after(layer_norm_fwd_kernel, (unsigned)((rows + kT / 32 - 1) / (kT / 32)), kT, 0, static_cast<cudaStream_t>(stream),
+        x, gamma, beta, eps, y, static_cast<__nv_bfloat16*>(y_bf16), reinterpret_cast<float2*>(stat), rows, D));
 }
 
 size_t dsqg_layer_norm_bwd_scratch_bytes(long long rows, int D) {
@@ -264,12 +268,9 @@ static int norm_bwd(const float* x, const float* mean, const float* rstd, int st
     const size_t smem = (size_t)2 * D * 4;
     float* part = static_cast<float*>(scratch);
     const __nv_bfloat16* db = static_cast<const __nv_bfloat16*>(dy_bf16);
-    if (D <= 256) layer_norm_bwd_kernel<2><<<blocks, kT, smem, s>>>(x, mean, rstd, step, gamma, dy, db, dx, part, rows, D);
-    else if (D <= 512) layer_norm_bwd_kernel<4><<<blocks, kT, smem, s>>>(x, mean, rstd, step, gamma, dy, db, dx, part, rows, D);
-    else layer_norm_bwd_kernel<8><<<blocks, kT, smem, s>>>(x, mean, rstd, step, gamma, dy, db, dx, part, rows, D);
-    if (int rc = status()) return rc;
-    sum_rows_kernel<<<(2 * D + 31) / 32, kT, 0, s>>>(part, dgamma_dbeta, (int)blocks, 2 * D);
-    return status();
+    auto kern = D <= 256 ? layer_norm_bwd_kernel<2> : (D <= 512 ? layer_norm_bwd_kernel<4> : layer_norm_bwd_kernel<8>);
+    if (int rc = status(launch_after(kern, blocks, kT, smem, s, x, mean, rstd, step, gamma, dy, db, dx, part, rows, D))) return rc;
+    return status(launch_after(sum_rows_kernel, (2 * D + 31) / 32, kT, 0, s, part, dgamma_dbeta, (int)blocks, 2 * D));
 }
 
 int dsqg_layer_norm_bwd(const float* x, const float* stat, const float* gamma, const float* dy, const void* dy_bf16, float* dx,
@@ -302,9 +303,8 @@ int dsqg_inject_kv(void* qkv, long long qkv_stride, const void* k_delta, const v
     if (!qkv || !k_delta || !v_delta) return DSQG_ERR_NULL_POINTER;
     if (rows < 1 || D < 8 || D % 8) return DSQG_ERR_BAD_SHAPE;
     if (bad(qkv) || bad(k_delta) || bad(v_delta) || delta_stride < D || delta_stride % 8 || qkv_stride < 3 * D || qkv_stride % 8) return DSQG_ERR_MISALIGNED;
-    inject_kernel<<<blocks_for(rows * (D / 4)), kT, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<__nv_bfloat16*>(qkv), qkv_stride, static_cast<const __nv_bfloat16*>(k_delta), static_cast<const __nv_bfloat16*>(v_delta), delta_stride, rows, D);
-    return status();
+    return status(launch_after(inject_kernel, blocks_for(rows * (D / 4)), kT, 0, static_cast<cudaStream_t>(stream),
+        static_cast<__nv_bfloat16*>(qkv), qkv_stride, static_cast<const __nv_bfloat16*>(k_delta), static_cast<const __nv_bfloat16*>(v_delta), delta_stride, rows, D));
 }
 
 int dsqg_column_sums(const void* const* src, const long long* row_stride, const int* cols, float* const* dst, int count, long long rows, void* stream) {
@@ -321,8 +321,7 @@ int dsqg_column_sums(const void* const* src, const long long* row_stride, const 
         a.slice_end[k] = slices += (cols[k] + kSumCols - 1) / kSumCols;
     }
     if (slices > 65535) return DSQG_ERR_BAD_SHAPE;
-    column_sum_kernel<<<dim3(8, slices), kSumThreads, 0, static_cast<cudaStream_t>(stream)>>>(a);
-    return status();
+    return status(launch_after(column_sum_kernel, dim3(8, slices), kSumThreads, 0, static_cast<cudaStream_t>(stream), a));
 }
 
 }  // extern "C"

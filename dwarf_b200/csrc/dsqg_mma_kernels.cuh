@@ -458,6 +458,7 @@ template <int D> struct FwdTune {
 template <int D, int WB, bool SE, int ST>
 __global__ void __launch_bounds__(FwdTune<D>::warps * 32, SE ? FwdTune<D>::ctas_se : FwdTune<D>::ctas)
 fwd_mma_kernel(const FwdArgs a, const Taps t, const int tiles_se) {
+    stream_wait();
     constexpr int W = FwdTune<D>::warps, G = SE ? FwdTune<D>::group_se : FwdTune<D>::group;
     extern __shared__ __align__(16) float se_smem[];      // scale_embed: the table, then a tile per warp
     __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
@@ -811,6 +812,7 @@ __host__ __device__ inline SePre se_pre_layout(const void* base, int ns, int D) 
 }
 template <int D, int WB>
 __global__ void se_prep_kernel(const float* __restrict__ scale_embed, const float* __restrict__ pos_bias, float scale, const Taps t, int H, void* out) {
+    stream_wait();
     const SePre P = se_pre_layout<WB>(out, t.n_sparse, D);
     const int R = SeGeo<WB>::rows(t.n_sparse);
     __nv_bfloat162* hi = reinterpret_cast<__nv_bfloat162*>(const_cast<__nv_bfloat16*>(P.hi));
@@ -850,6 +852,7 @@ inline size_t dq_smem_bytes(int J, int ns, bool se) {
 template <int D, int WB, int G, int CT, bool SE, int ST>
 __global__ void __launch_bounds__(kWarps * 32, CT)
 bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
+    stream_wait();
     using Stage = DsStage<WB>;
     extern __shared__ __align__(16) float stage[];     // see dq_smem_bytes
     __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
@@ -962,6 +965,7 @@ bwd_dq_mma_kernel(const BwdArgs a, const Taps t) {
 // the tiles' partials (written by the dQ kernel) in tile order.
 __global__ void __launch_bounds__(256)
 dse_group_kernel(const float* __restrict__ tmp, float* __restrict__ part, int tiles_per_bh, int groups_bh, int JD) {
+    stream_wait();
     const int bh = blockIdx.y, grp = blockIdx.x, first = grp * kSeGroup;
     const int members = tiles_per_bh - first < kSeGroup ? tiles_per_bh - first : kSeGroup;
     const float* src = tmp + ((size_t)bh * tiles_per_bh + first) * JD;
@@ -1153,6 +1157,7 @@ template <int WB> inline size_t dkdv_smem_bytes(bool se) { return se ? (size_t)(
 template <int D, int WB, int G, int CT, bool SE, int ST>
 __global__ void __launch_bounds__(kWarps * 32, CT)
 bwd_dkdv_mma_kernel(const BwdArgs a, const Taps t, const int n_reduce, const int reduce_stride) {
+    stream_wait();
     constexpr int kStat = kRows + WB;                  // query rows the CTA's dense windows touch
     extern __shared__ __align__(16) float se_tile[];   // scale_embed: [kStat][kSeKeyPitch]
     __shared__ __align__(16) float start_s[SE ? 4 : StartTable<WB>::kSize];
@@ -1242,8 +1247,7 @@ cudaError_t fwd_launch_mode(const FwdArgs& a, const Taps& t, cudaStream_t s) {
         const cudaError_t e = ensure_dynamic_smem(fwd_mma_kernel<D, WB, SE, ST>, smem, seen);
         if (e != cudaSuccess) return e;
     }
-    fwd_mma_kernel<D, WB, SE, ST><<<grid, W * 32, smem, s>>>(a, t, tiles_se);
-    return cudaGetLastError();
+    return launch_after(fwd_mma_kernel<D, WB, SE, ST>, grid, W * 32, smem, s, a, t, tiles_se);
 }
 
 template <int D, int WB, bool SE>
@@ -1277,19 +1281,16 @@ cudaError_t bwd_launch_mode(BwdArgs a, const Taps& t, cudaStream_t s, int stages
     cudaError_t e = cudaSuccess;
     if (stages & DSQG_BWD_STAGE_DQ) {
         if constexpr (SE) {
-            se_prep_kernel<D, WB><<<1, 1024, 0, s>>>(a.scale_embed, a.pos_bias, a.scale, t, a.H, a.se_pre);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            if ((e = launch_after(se_prep_kernel<D, WB>, 1, 1024, 0, s, a.scale_embed, a.pos_bias, a.scale, t, a.H, a.se_pre)) != cudaSuccess) return e;
         }
         auto kern = bwd_dq_mma_kernel<D, WB, SE ? T::dq_group_se : T::dq_group, SE ? T::dq_ctas_se : T::dq_ctas, SE, ST>;
         const size_t smem = dq_smem_bytes<D, WB>(t.J, t.n_sparse, SE);
         static int seen[64] = {0};
         if ((e = ensure_dynamic_smem(kern, smem, seen)) != cudaSuccess) return e;
-        kern<<<grid, kWarps * 32, smem, s>>>(a, t);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if ((e = launch_after(kern, grid, kWarps * 32, smem, s, a, t)) != cudaSuccess) return e;
         if constexpr (SE) {
             const int groups_bh = (a.tiles_per_bh + kSeGroup - 1) / kSeGroup;
-            dse_group_kernel<<<dim3(groups_bh, a.B * a.H), 256, 0, s>>>(a.dse_tmp, a.dse_part, a.tiles_per_bh, groups_bh, t.J * a.D);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            if ((e = launch_after(dse_group_kernel, dim3(groups_bh, a.B * a.H), 256, 0, s, a.dse_tmp, a.dse_part, a.tiles_per_bh, groups_bh, t.J * a.D)) != cudaSuccess) return e;
         }
     }
     // With both stages in one call the reduction rides on CTAs of the dK/dV kernel (same code,
@@ -1303,8 +1304,8 @@ cudaError_t bwd_launch_mode(BwdArgs a, const Taps& t, cudaStream_t s, int stages
         const size_t smem = dkdv_smem_bytes<WB>(SE);
         static int seen[64] = {0};
         if ((e = ensure_dynamic_smem(kern, smem, seen)) != cudaSuccess) return e;
-        kern<<<grid, kWarps * 32, smem, s>>>(a, t, fuse ? n_out : 0, fuse && (long long)grid.x * grid.y >= n_out ? (int)((long long)grid.x * grid.y / n_out) : 1);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        e = launch_after(kern, grid, kWarps * 32, smem, s, a, t, fuse ? n_out : 0, fuse && (long long)grid.x * grid.y >= n_out ? (int)((long long)grid.x * grid.y / n_out) : 1);
+        if (e != cudaSuccess) return e;
     }
     if ((stages & DSQG_BWD_STAGE_REDUCE) && !fuse) e = launch_reduce_params(a, t.J, s);
     return e;

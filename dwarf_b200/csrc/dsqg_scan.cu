@@ -55,6 +55,7 @@ __device__ __forceinline__ void store4(float* p, const float (&x)[4]) { *reinter
 template <typename T, bool REVERSE, int CB, bool GATED = false>
 __global__ void __launch_bounds__(kScanThreads, 4)
 causal_mean_kernel(const T* __restrict__ x, T* __restrict__ out, int N, int D, int len, int tile, const PoolGate gate) {
+    stream_wait();
     constexpr int kRanks = kChunks / CB, kItems = CB * kCols, K = (kItems + kScanThreads - 1) / kScanThreads, U = GATED && REVERSE ? 2 : 4;
     extern __shared__ __align__(16) float vals[];
     __shared__ float part[kChunks][kCols];
@@ -208,10 +209,12 @@ cudaError_t launch_scan(const T* x, T* out, int B, int N, int D, const PoolGate&
         if (cudaError_t e = cudaFuncSetAttribute(causal_mean_kernel<T, REVERSE, CB, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kChunks / CB, (D + kCols - 1) / kCols, B); cfg.blockDim = dim3(kScanThreads); cfg.dynamicSmemBytes = smem; cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kChunks / CB; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // as launch_after
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, causal_mean_kernel<T, REVERSE, CB, GATED>, x, out, N, D, len, tile, gate);
 }
 
