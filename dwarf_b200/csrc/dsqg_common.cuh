@@ -194,6 +194,13 @@ inline void carve_bwd_scratch(BwdArgs& a, int rows_per_tile, int J, bool has_se)
     a.dse_tmp = nullptr;
 }
 
+// Packed fp32 pairs (sm_100): one instruction for two elements, each rounded as by the scalar form.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpair(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+
 // ---------------------------------------------------------------------------------
 // Device helpers: 8-element row slices in fp32 registers, from bf16 or fp32 storage.
 // ---------------------------------------------------------------------------------

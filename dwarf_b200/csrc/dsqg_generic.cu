@@ -37,16 +37,18 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
 __device__ __forceinline__ float dot4(float4 a, float4 b, float c) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, c)))); }
 
 // Forward.  LPR lanes hold a row, four elements each; a lane group owns kFwdRows consecutive query rows and
-// takes the taps eight at a time (online softmax over the chunks).  What bounds it is the L1 data path and the
-// shuffles, not the multiply-adds, hence
+// takes the taps eight at a time (online softmax over the chunks).  What bounds it is the L1 data path, the
+// shuffles and issue slots, not the multiply-adds, hence
 //   * one 16-byte load of four lanes covers whole 128-byte lines (eight elements per lane, two loads 32 bytes
 //     apart, moved the same rows in twice as many passes);
 //   * eight consecutive offsets of two consecutive rows touch only nine key rows, loaded once;
 //   * the partial dot products of eight taps are summed over the lanes by halving (seven shuffles per row
 //     instead of 3 x 8), which leaves one tap's score per lane: its exponential is computed once and handed
-//     back with one shuffle.
-// B2 H8 N2048 D32 fp32, 43 taps: 19.5 us against 31.8 us with one row per group and one tap at a time (a
-// quarter of its instructions are now the multiply-adds; four rows per group or 256 threads: 24 us and more).
+//     back with one shuffle;
+//   * four taps or less at the end are a chunk of four, and the multiply-adds work on packed pairs.
+// fp32, 43 taps, us: B2 H8 N2048 D32 17.5 (19.3 with scalar multiply-adds and chunks of eight only, 31.8 with one row per group and one tap at a
+// time; four rows per group or 256 threads 24 and more), B14 97.9 (107.2), B8 H8 N2048 D64 115.0 (122.9), B2 H8 N1500 D128 44.1 (47.0), B1 H8 N300
+// D32 5.8 (5.9).  Scores first and values after, the scores waiting in shared memory: 17.6 with 7 CTAs per SM, but 7.4 at B1 H8 N300.
 constexpr int kFwdRows = 2, kFwdThreads = 128;
 
 // EXACT: D == 4 LPR, so that the rows of a run are compile-time offsets apart.
@@ -58,125 +60,150 @@ fwd_generic_kernel(const FwdArgs a, const Taps t) {
     __shared__ int off_s[DSQG_MAX_TAPS];
     stream_wait();
     const int bh = blockIdx.y, h = bh % a.H, N = a.N, D = EXACT ? 4 * LPR : a.D, J = t.J;
-    const int g = threadIdx.x / LPR, li = threadIdx.x % LPR, d0 = 4 * li, tap_lane = li & 7;
+    const int g = threadIdx.x / LPR, li = threadIdx.x % LPR, d0 = 4 * li;
     const bool active = d0 < D;
     for (int j = threadIdx.x; j < J; j += kFwdThreads) { pb_s[j] = a.pos_bias[j * a.H + h]; off_s[j] = t.delta(j); }
     __syncthreads();
     const int n0 = (blockIdx.x * GPB + g) * R;
     const size_t base = (size_t)bh * N * D + (active ? d0 : 0);
-    const T* qb = static_cast<const T*>(a.q) + base;
     const T* kb = static_cast<const T*>(a.k) + base;
     const T* vb = static_cast<const T*>(a.v) + base;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 q[R], acc[R];
-    float m[R], l[R];                       // l: this lane's taps only
+    float4 q[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        q[r] = active && n0 + r < N ? load4(qb + (size_t)(n0 + r) * D) : zero;
-        acc[r] = zero; m[r] = -INFINITY; l[r] = 0.f;
-    }
-    // Taps j0 .. j0 + 7.  RUN: consecutive offsets.  INSIDE: every partner row of the warp exists; otherwise any key row of the
+    for (int r = 0; r < R; ++r) q[r] = active && n0 + r < N ? load4(static_cast<const T*>(a.q) + base + (size_t)(n0 + r) * D) : zero;
+    auto dot = [](const float4& x, const float4& y) {
+        const f32x2 s = fma2(pair(x.z, x.w), pair(y.z, y.w), mul2(pair(x.x, x.y), pair(y.x, y.y)));
+        float lo, hi;
+        unpair(s, lo, hi);
+        return lo + hi;
+    };
+    // Taps j0 .. j0 + C - 1.  RUN: consecutive offsets.  INSIDE: every partner row of the warp exists; otherwise any key row of the
     // sequence stands in for one that does not (its score is -inf), and a value of zero (a weight of 0 would not hold off an infinity or NaN there).
-    auto chunk = [&](auto RUNC, auto INSIDEC, int j0) {
-        constexpr bool RUN = decltype(RUNC)::value, INSIDE = decltype(INSIDEC)::value;
-        auto at = [&](const T* p, int n, int i) {
-            if constexpr (INSIDE) return load4(p + (ptrdiff_t)n * D + i * D);
-            else return load4(p + (ptrdiff_t)min(max(n + i, 0), N - 1) * D);
-        };
-        auto value = [&](int n, int i) {
-            const float4 v = at(vb, n, i);
-            return INSIDE || (n + i >= 0 && n + i < N) ? v : zero;
-        };
-        const int first = n0 - off_s[j0] - 7;                     // RUN: the R + 7 rows start here
-        float s[R];
-        {
-            float part[R][8];
-            if constexpr (RUN) {
-#pragma unroll
-                for (int i = 0; i < R + 7; ++i) {
-                    const float4 k = at(kb, first, i);
-#pragma unroll
-                    for (int r = 0; r < R; ++r)
-                        if (7 + r - i >= 0 && 7 + r - i < 8) part[r][7 + r - i] = dot4(q[r], k, 0.f);
-                }
-            } else {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const int dl = off_s[min(j0 + c, J - 1)];
-#pragma unroll
-                    for (int r = 0; r < R; ++r) part[r][c] = dot4(q[r], at(kb, n0 - dl, r), 0.f);
-                }
-            }
-            if (a.scale_embed != nullptr && active) {
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const float4 e = load4(a.scale_embed + (size_t)min(j0 + c, J - 1) * D + d0);
-#pragma unroll
-                    for (int r = 0; r < R; ++r) part[r][c] = dot4(q[r], e, part[r][c]);
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-#pragma unroll
-                for (int half = 4; half > 0; half >>= 1) {
-                    const bool up = li & half;
-#pragma unroll
-                    for (int c = 0; c < half; ++c) {
-                        const float keep = up ? part[r][c + half] : part[r][c], send = up ? part[r][c] : part[r][c + half];
-                        part[r][c] = keep + __shfl_xor_sync(0xffffffffu, send, half);
-                    }
-                }
-                s[r] = part[r][0];
-#pragma unroll
-                for (int o = 8; o < LPR; o <<= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
-            }
-        }
-        const int j = j0 + tap_lane, dl = off_s[min(j, J - 1)];
-        float p[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const float x = j < J && n0 + r >= dl ? fmaf(s[r], a.scale, pb_s[min(j, J - 1)]) : -INFINITY;
-            float mx = x;
-#pragma unroll
-            for (int o = 4; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-            const float mn = fmaxf(m[r], mx), ms = mn == -INFINITY ? 0.f : mn;
-            const float cor = Exp<T>::f(m[r] - ms);
-            p[r] = Exp<T>::f(x - ms);
-            m[r] = mn;
-            l[r] = fmaf(l[r], cor, p[r]);
-            acc[r].x *= cor; acc[r].y *= cor; acc[r].z *= cor; acc[r].w *= cor;
-        }
-        auto fold = [&](int r, int c, const float4& v) {
-            const float w = __shfl_sync(0xffffffffu, p[r], c, 8);
-            acc[r].x = fmaf(w, v.x, acc[r].x); acc[r].y = fmaf(w, v.y, acc[r].y);
-            acc[r].z = fmaf(w, v.z, acc[r].z); acc[r].w = fmaf(w, v.w, acc[r].w);
-        };
+    auto row_at = [&](auto INSIDEC, const T* p, int n, int i) {
+        if constexpr (decltype(INSIDEC)::value) return load4(p + (ptrdiff_t)n * D + i * D);
+        else return load4(p + (ptrdiff_t)min(max(n + i, 0), N - 1) * D);
+    };
+    auto scores = [&](auto CC, auto RUNC, auto INSIDEC, int j0, float (&x)[R]) {
+        constexpr int C = decltype(CC)::value;
+        constexpr bool RUN = decltype(RUNC)::value;
+        float part[R][C];
         if constexpr (RUN) {
+            const int first = n0 - off_s[j0] - (C - 1);                     // the R + C - 1 rows start here
 #pragma unroll
-            for (int i = 0; i < R + 7; ++i) {
-                const float4 v = value(first, i);
+            for (int i = 0; i < R + C - 1; ++i) {
+                const float4 k = row_at(INSIDEC, kb, first, i);
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    if (7 + r - i >= 0 && 7 + r - i < 8) fold(r, 7 + r - i, v);
+                    if (C - 1 + r - i >= 0 && C - 1 + r - i < C) part[r][C - 1 + r - i] = dot(q[r], k);
             }
         } else {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < C; ++c) {
+                const int dl = off_s[min(j0 + c, J - 1)];
+#pragma unroll
+                for (int r = 0; r < R; ++r) part[r][c] = dot(q[r], row_at(INSIDEC, kb, n0 - dl, r));
+            }
+        }
+        if (a.scale_embed != nullptr && active) {
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                const float4 e = load4(a.scale_embed + (size_t)min(j0 + c, J - 1) * D + d0);
+#pragma unroll
+                for (int r = 0; r < R; ++r) part[r][c] += dot(q[r], e);
+            }
+        }
+        const int j = j0 + (li & (C - 1)), dl = off_s[min(j, J - 1)];
+        const bool mine = j < J && (C == 8 || (li & 7) < C);                // every tap counts on one lane of eight
+        const float pb = pb_s[min(j, J - 1)];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+#pragma unroll
+            for (int half = C / 2; half > 0; half >>= 1) {
+                const bool up = li & half;
+#pragma unroll
+                for (int c = 0; c < half; ++c) {
+                    const float keep = up ? part[r][c + half] : part[r][c], send = up ? part[r][c] : part[r][c + half];
+                    part[r][c] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+                }
+            }
+            float s = part[r][0];
+#pragma unroll
+            for (int o = C; o < LPR; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            x[r] = mine && n0 + r >= dl ? fmaf(s, a.scale, pb) : -INFINITY;
+        }
+    };
+    f32x2 acc[R][2];
+    float m[R], l[R];                       // maximum; sum over this lane's taps only
+#pragma unroll
+    for (int r = 0; r < R; ++r) { m[r] = -INFINITY; l[r] = 0.f; acc[r][0] = acc[r][1] = 0ull; }
+    auto group_max = [](float x) {
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+        return x;
+    };
+    auto finite = [](float x) { return x == -INFINITY ? 0.f : x; };
+    auto values = [&](auto CC, auto RUNC, auto INSIDEC, int j0, const float (&x)[R]) {
+        constexpr int C = decltype(CC)::value;
+        constexpr bool RUN = decltype(RUNC)::value, INSIDE = decltype(INSIDEC)::value;
+        float p[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            p[r] = Exp<T>::f(x[r] - finite(m[r]));
+            l[r] += p[r];
+        }
+        auto fold = [&](int r, int c, int n, int i, float4 v) {
+            if (!INSIDE && (n + i < 0 || n + i >= N)) v = zero;
+            const float w = __shfl_sync(0xffffffffu, p[r], c, 8);
+            acc[r][0] = fma2(pair(w, w), pair(v.x, v.y), acc[r][0]);
+            acc[r][1] = fma2(pair(w, w), pair(v.z, v.w), acc[r][1]);
+        };
+        if constexpr (RUN) {
+            const int first = n0 - off_s[j0] - (C - 1);
+#pragma unroll
+            for (int i = 0; i < R + C - 1; ++i) {
+                const float4 v = row_at(INSIDEC, vb, first, i);
+#pragma unroll
+                for (int r = 0; r < R; ++r)
+                    if (C - 1 + r - i >= 0 && C - 1 + r - i < C) fold(r, C - 1 + r - i, first, i, v);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
                 const int dc = off_s[min(j0 + c, J - 1)];
 #pragma unroll
-                for (int r = 0; r < R; ++r) fold(r, c, value(n0 - dc, r));
+                for (int r = 0; r < R; ++r) fold(r, c, n0 - dc, r, row_at(INSIDEC, vb, n0 - dc, r));
             }
         }
     };
+    auto chunk = [&](auto C, auto run, auto inside, int j0) {
+        float x[R];
+        scores(C, run, inside, j0, x);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float mn = fmaxf(m[r], group_max(x[r])), cor = Exp<T>::f(m[r] - finite(mn));
+            m[r] = mn;
+            l[r] *= cor;
+            acc[r][0] = mul2(acc[r][0], pair(cor, cor)); acc[r][1] = mul2(acc[r][1], pair(cor, cor));
+        }
+        values(C, run, inside, j0, x);
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    std::integral_constant<int, 8> eight;
+    std::integral_constant<int, 4> four;
 #pragma unroll 1
     for (int j0 = 0; j0 < J; j0 += 8) {
         if (!__any_sync(0xffffffffu, n0 + R - 1 >= off_s[j0])) break;                                // offsets ascend
         const bool run = j0 + 8 <= t.n_dense;
         const bool inside = __all_sync(0xffffffffu, n0 >= off_s[min(j0 + 7, J - 1)] && n0 + R <= N);
-        if (run && inside) chunk(std::true_type(), std::true_type(), j0);
-        else if (run) chunk(std::true_type(), std::false_type(), j0);
-        else if (inside) chunk(std::false_type(), std::true_type(), j0);
-        else chunk(std::false_type(), std::false_type(), j0);
+        if (j0 + 4 >= J) {
+            if (inside) chunk(four, No(), Yes(), j0); else chunk(four, No(), No(), j0);
+        } else if (run) {
+            if (inside) chunk(eight, Yes(), Yes(), j0); else chunk(eight, Yes(), No(), j0);
+        } else {
+            if (inside) chunk(eight, No(), Yes(), j0); else chunk(eight, No(), No(), j0);
+        }
     }
     const float gain = a.head_gain ? a.head_gain[h] : 1.f;
 #pragma unroll
@@ -186,8 +213,10 @@ fwd_generic_kernel(const FwdArgs a, const Taps t) {
         for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         if (n0 + r >= N) continue;
         const float inv = sum > 0.f ? gain / sum : 0.f;
+        float4 o;
+        unpair(acc[r][0], o.x, o.y); unpair(acc[r][1], o.z, o.w);
         if (active)
-            store4(static_cast<T*>(a.out) + base + (size_t)(n0 + r) * D, make_float4(acc[r].x * inv, acc[r].y * inv, acc[r].z * inv, acc[r].w * inv));
+            store4(static_cast<T*>(a.out) + base + (size_t)(n0 + r) * D, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv));
         if (li == 0) a.lse[(size_t)bh * N + n0 + r] = sum > 0.f ? m[r] + logf(sum) : -INFINITY;
     }
 }

@@ -275,13 +275,6 @@ __device__ __forceinline__ void diag_fma(float (&acc)[D / 8][4], float x_lo, flo
     }
 }
 
-// Packed fp32 pairs (sm_100): one instruction for two elements, each rounded as by the scalar form.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ void unpair(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-
 // The running maximum of the online softmax only moves when a score exceeds it by more than this
 // (log2 units): probabilities stay below 2^kSlack, which fp32 sums and bf16 values absorb.
 constexpr float kSlack = 16.f;
