@@ -190,6 +190,9 @@ int dsqg_bwd(const void* q, const void* k, const void* v,
                            B, H, N, D, dtype, stream, DSQG_BWD_STAGE_ALL);
 }
 
+// What the backward of a gated forward starts from: BwdArgs::gate.
+struct GateBwd { const void* dy; const void* y; const void* gate; void* dgate; dsqg_strides y_st, gate_st, dgate_st; };
+
 static int bwd_impl(const void* q, const void* k, const void* v,
                     const float* pos_bias, const float* scale_embed, const float* head_gain,
                     const int32_t* offsets, int J,
@@ -199,7 +202,7 @@ static int bwd_impl(const void* q, const void* k, const void* v,
                     void* scratch, size_t scratch_bytes,
                     int B, int H, int N, int D, int dtype, void* stream, int stages, float scale,
                     const dsqg_strides* in_st = nullptr, const dsqg_strides* out_st = nullptr,
-                    const float* delta_pre = nullptr, bool kept = false);
+                    const float* delta_pre = nullptr, bool kept = false, const GateBwd* gate = nullptr);
 
 int dsqg_bwd_stages(const void* q, const void* k, const void* v,
                     const float* pos_bias, const float* scale_embed, const float* head_gain,
@@ -235,7 +238,7 @@ static int bwd_impl(const void* q, const void* k, const void* v,
                     float* dpos_bias, float* dscale_embed, float* dhead_gain,
                     void* scratch, size_t scratch_bytes,
                     int B, int H, int N, int D, int dtype, void* stream, int stages, float scale,
-                    const dsqg_strides* in_st, const dsqg_strides* out_st, const float* delta_pre, bool kept) {
+                    const dsqg_strides* in_st, const dsqg_strides* out_st, const float* delta_pre, bool kept, const GateBwd* gate) {
     if (stages < 1 || stages > DSQG_BWD_STAGE_ALL) return DSQG_ERR_UNSUPPORTED;
     if (!q || !k || !v || !pos_bias || !out || !lse || !dout || !dq || !dk || !dv || !dpos_bias || !scratch)
         return DSQG_ERR_NULL_POINTER;
@@ -263,13 +266,18 @@ static int bwd_impl(const void* q, const void* k, const void* v,
     a.B = B; a.H = H; a.N = N; a.D = D;
     a.scale = scale > 0.f ? scale : 1.0f / sqrtf((float)D);
     a.strided = 0; a.delta_pre = nullptr; a.kept = 0;
+    a.dy = a.y = a.gate = nullptr; a.dgate = nullptr; a.y_st = a.gate_st = a.dgate_st = dsqg_strides{};
     a.in_sb = a.in_sh = a.in_sn = a.out_sb = a.out_sh = a.out_sn = 0;
     NvtxRange range(in_st ? "dsqg_bwd_strided" : "dsqg_bwd");
     if (in_st) {
         if (!out_st) return DSQG_ERR_NULL_POINTER;
         if (bad_strides(in_st) || bad_strides(out_st)) return DSQG_ERR_MISALIGNED;
         if (!mma_path_supported(dtype, D, t, scale_embed != nullptr)) return DSQG_ERR_UNSUPPORTED;
-        if (kept && (!kept_pays(D) || !delta_pre)) return DSQG_ERR_UNSUPPORTED;
+        if (kept && (!kept_pays(D) || !gate)) return DSQG_ERR_UNSUPPORTED;
+        if (gate) {
+            a.dy = gate->dy; a.y = gate->y; a.gate = gate->gate; a.dgate = gate->dgate;
+            a.y_st = gate->y_st; a.gate_st = gate->gate_st; a.dgate_st = gate->dgate_st;
+        }
         a.strided = 1; a.delta_pre = delta_pre; a.kept = kept;
         a.in_sb = in_st->batch; a.in_sh = in_st->head; a.in_sn = in_st->row;
         a.out_sb = out_st->batch; a.out_sh = out_st->head; a.out_sn = out_st->row;
@@ -335,7 +343,7 @@ size_t dsqg_packed_bwd_scratch_bytes(const dsqg_packed* p) {
     const size_t need = dsqg_bwd_scratch_bytes(p->J, p->B, p->H, p->N, p->D, p->scale_embed != nullptr);
     if (!need || !p->gate) return need;
     const size_t rows = (size_t)p->B * p->H * p->N;
-    return round256(need) + round256(rows * 4) + rows * p->D * 2;          // delta and dout of the gate's backward
+    return round256(need) + rows * p->D * 2;                               // dout of the gate's backward
 }
 
 int dsqg_packed_bwd(const dsqg_packed* p, const dsqg_packed_grads* g, void* scratch, size_t scratch_bytes, void* stream) {
@@ -351,27 +359,22 @@ int dsqg_packed_bwd_gate(const dsqg_packed* p, const dsqg_packed_grads* g, const
     const size_t need = dsqg_bwd_scratch_bytes(p->J, B, H, N, D, p->scale_embed != nullptr);
     const void* dout = g->dy;
     dsqg_strides dout_st = p->out_strides;
-    const float* delta = nullptr;
+    GateBwd gate = {};
     if (p->gate) {
         if (!g->dy || !p->out || !g->dgate) return DSQG_ERR_NULL_POINTER;
         const dsqg_strides dgate_st = dgate_strides ? *dgate_strides : p->gate_strides;
         if (bad_strides(&p->out_strides) || bad_strides(&p->gate_strides) || bad_strides(&dgate_st) || misaligned16(g->dy) || misaligned16(p->out) || misaligned16(p->gate) ||
             misaligned16(g->dgate) || misaligned16(scratch))
             return DSQG_ERR_MISALIGNED;
-        char* mem = static_cast<char*>(scratch) + round256(need);
-        float* dl = reinterpret_cast<float*>(mem);
-        void* buf = mem + round256((size_t)B * H * N * 4);
         dout_st.batch = (long long)H * N * D; dout_st.head = (long long)N * D; dout_st.row = D;   // head-major: the operator's backward reads whole lines
-        const cudaError_t e = launch_gate_bwd(g->dy, p->out, p->out_strides, p->gate, p->gate_strides, g->dgate, dgate_st, buf, dout_st, dl,
-                                              B, H, N, D, static_cast<cudaStream_t>(stream));
-        if (e != cudaSuccess) return cuda_fail(e);
-        dout = buf; delta = dl;
+        dout = static_cast<char*>(scratch) + round256(need);
+        gate = {g->dy, p->out, p->gate, g->dgate, p->out_strides, p->gate_strides, dgate_st};
     }
     const size_t part = (size_t)B * H * N * D;
     const __nv_bfloat16* kept = static_cast<const __nv_bfloat16*>(p->keep);
     return bwd_impl(kept ? kept : p->q, kept ? kept + part : p->k, kept ? kept + 2 * part : p->v, p->pos_bias, p->scale_embed, p->head_gain,
                     p->offsets, p->J, p->out, p->lse, dout, g->dq, g->dk, g->dv, g->dpos_bias, g->dscale_embed, g->dhead_gain, scratch, need,
-                    B, H, N, D, DSQG_DTYPE_BF16, stream, DSQG_BWD_STAGE_ALL, 0.f, &p->qkv_strides, &dout_st, delta, kept != nullptr);
+                    B, H, N, D, DSQG_DTYPE_BF16, stream, DSQG_BWD_STAGE_ALL, 0.f, &p->qkv_strides, &dout_st, nullptr, kept != nullptr, p->gate ? &gate : nullptr);
 }
 
 int dsqg_gate_bwd(const void* dy, const void* y, const void* gate, const dsqg_strides* strides,
@@ -382,7 +385,7 @@ int dsqg_gate_bwd(const void* dy, const void* y, const void* gate, const dsqg_st
     if (bad_strides(strides) || misaligned16(dy) || misaligned16(y) || misaligned16(gate) || misaligned16(dout) ||
         misaligned16(dgate))
         return DSQG_ERR_MISALIGNED;
-    cudaError_t e = launch_gate_bwd(dy, y, *strides, gate, *strides, dgate, *strides, dout, *strides, delta, B, H, N, D, static_cast<cudaStream_t>(stream));
+    cudaError_t e = launch_gate_bwd(dy, y, gate, dgate, dout, *strides, delta, B, H, N, D, static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? DSQG_OK : cuda_fail(e);
 }
 

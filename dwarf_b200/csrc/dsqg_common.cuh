@@ -64,6 +64,10 @@ struct BwdArgs {
     int strided;
     long long in_sb, in_sh, in_sn, out_sb, out_sh, out_sn;
     const float* delta_pre;
+    // Strided only, gate nullable: dout does not exist yet.  The dQ kernel forms dout = dy * sigmoid(gate), dgate = dy * y * (1 - sigmoid(gate)) and delta for its
+    // rows and writes dout (out_* strides) for the dK/dV kernel; y is out, the gated result, laid out like dy.
+    const void* dy; const void* y; const void* gate; void* dgate;
+    dsqg_strides y_st, gate_st, dgate_st;
     // Strided only: q, k, v and dout are contiguous [B,H,N,D] all the same (in_* then addresses dq, dk, dv only; needs delta_pre).
     int kept;
 };
@@ -115,9 +119,9 @@ cudaError_t launch_ring_advance(const int32_t* head, const int32_t* fill, int32_
 cudaError_t launch_gated_mean(const float* x, const void* g, float* pool, void* inter, int B, int N, int D, cudaStream_t s);
 cudaError_t launch_gated_mean_bwd(const void* dinter, const void* g, const float* pool, void* dg, float* dx, int B, int N, int D, cudaStream_t s);
 cudaError_t launch_causal_mean(const void* x, void* out, int B, int N, int D, int dtype, bool reverse, cudaStream_t s);
-// y and dy, gate and dgate, and dout have strides of their own
-cudaError_t launch_gate_bwd(const void* dy, const void* y, const dsqg_strides& ys, const void* gate, const dsqg_strides& gs, void* dgate,
-                            const dsqg_strides& dgs, void* dout, const dsqg_strides& os, float* delta, int B, int H, int N, int D, cudaStream_t s);
+// all five tensors laid out alike
+cudaError_t launch_gate_bwd(const void* dy, const void* y, const void* gate, void* dgate, void* dout, const dsqg_strides& st, float* delta, int B, int H, int N, int D,
+                            cudaStream_t s);
 cudaError_t launch_fwd_mma(const FwdArgs& a, const Taps& t, cudaStream_t s);
 cudaError_t launch_bwd_mma(const BwdArgs& a, const Taps& t, cudaStream_t s, int stages);
 bool mma_path_supported(int dtype, int D, const Taps& t, bool has_scale_embed);   // backward

@@ -225,6 +225,24 @@ __device__ __forceinline__ void store_acc_rows_gated(const float (&acc)[D / 8][4
     if (ok_hi) half(std::integral_constant<int, 1>(), gate_hi, row_hi, s_hi);
 }
 
+// One row of the sigmoid gate's backward (this thread's elements): d is dy and becomes dout = dy * s, y becomes dgate = dy * y * (1 - s), s = sigmoid(gate).
+template <int D>
+__device__ __forceinline__ void gate_row(RowFrag<D>& d, RowFrag<D>& y, const RowFrag<D>& gate) {
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j) {
+        float out[2], dg[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            auto f = [&](uint32_t u) { return __uint_as_float(i ? u & 0xffff0000u : u << 16); };
+            const float s = __fdividef(1.f, 1.f + __expf(-f(gate.r[j]))), dy = f(d.r[j]);
+            out[i] = dy * s;
+            dg[i] = dy * f(y.r[j]) * (1.f - s);
+        }
+        d.r[j] = pack_bf16x2(out[0], out[1]);
+        y.r[j] = pack_bf16x2(dg[0], dg[1]);
+    }
+}
+
 // Partial dot product of two row fragments over this thread's elements (fp32).
 template <int D>
 __device__ __forceinline__ float frag_dot(const RowFrag<D>& a, const RowFrag<D>& b) {
@@ -235,6 +253,28 @@ __device__ __forceinline__ float frag_dot(const RowFrag<D>& a, const RowFrag<D>&
         s = fmaf(__uint_as_float(a.r[j] & 0xffff0000u), __uint_as_float(b.r[j] & 0xffff0000u), s);
     }
     return s;
+}
+
+// The whole row's dot product on all four lanes.  At D = 32 its elements are added one after the other, as one thread would: ds = P (dP - delta) is
+// rounded to bf16, and another order moves single roundings, which a gradient that nearly cancels (a bias on every key) shows.
+template <int D>
+__device__ __forceinline__ float row_dot(const RowFrag<D>& a, const RowFrag<D>& b) {
+    if constexpr (D == 32) {
+        float acc = 0.f;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {                        // every lane adds its products to what the lane before has; the l-th lane's count
+            float s = l ? __shfl_sync(0xffffffffu, acc, l - 1, 4) : 0.f;
+#pragma unroll
+            for (int j = 0; j < D / 8; ++j) {
+                s = fmaf(__uint_as_float(a.r[j] << 16), __uint_as_float(b.r[j] << 16), s);
+                s = fmaf(__uint_as_float(a.r[j] & 0xffff0000u), __uint_as_float(b.r[j] & 0xffff0000u), s);
+            }
+            acc = s;
+        }
+        return __shfl_sync(0xffffffffu, acc, 3, 4);
+    } else {
+        return quad_sum(frag_dot(a, b));
+    }
 }
 
 // Lane roles inside a 16-row tile held as MMA fragments (rows g and g+8 per lane).

@@ -588,8 +588,31 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
     f32x2 dgrow2 = 0ull;
 
     RowFrag<D> qa, qb, da, db;
+    float delta_lo, delta_hi;
+    bool have_dout = ST != kKept;
+    if constexpr (ST != kContiguous) have_dout = have_dout && !a.gate;
+    if constexpr (ST != kContiguous) if (!have_dout) {       // the gate's backward for these rows first
+        auto rows = [&](const void* p, const dsqg_strides& st) {
+            return Rows<D, false>(p, (size_t)(bh / a.H) * st.batch + (size_t)h * st.head, g0, (ptrdiff_t)st.row, L);
+        };
+        RowFrag<D> ya, yb, ga, gb;
+        rows(a.dy, a.y_st).template load2<AL>(da, db, 0, ok_lo, ok_hi);
+        rows(a.y, a.y_st).template load2<AL>(ya, yb, 0, ok_lo, ok_hi);
+        rows(a.gate, a.gate_st).template load2<AL>(ga, gb, 0, ok_lo, ok_hi);
+        delta_lo = row_dot(da, ya); delta_hi = row_dot(db, yb);
+        gate_row(da, ya, ga); gate_row(db, yb, gb);
+        const Rows<D, false> dg = rows(a.dgate, a.dgate_st);
+        if (ok_lo) {
+            store_row_at<D, AL>(ya.r, const_cast<__nv_bfloat16*>(dg.at(0)));
+            store_row_at<D, AL>(da.r, const_cast<__nv_bfloat16*>(dr.at(0)));
+        }
+        if (ok_hi) {
+            store_row_at<D, AL>(yb.r, const_cast<__nv_bfloat16*>(dg.at(8)));
+            store_row_at<D, AL>(db.r, const_cast<__nv_bfloat16*>(dr.at(8)));
+        }
+    }
     qr.template load2<AL>(qa, qb, 0, ok_lo, ok_hi);
-    dr.template load2<AL>(da, db, 0, ok_lo, ok_hi);
+    if (have_dout) dr.template load2<AL>(da, db, 0, ok_lo, ok_hi);
     if constexpr (SE) {
         // the sparse part also goes to global memory for the dK/dV kernel (a row of ns8 floats per query)
         const int ns8 = (ns + 7) / 8 * 8;
@@ -605,11 +628,10 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
             *reinterpret_cast<uint4*>(qrow + 8 * (2 * D + 16) + o) = make_uint4(qb.r[4 * c], qb.r[4 * c + 1], qb.r[4 * c + 2], qb.r[4 * c + 3]);
         }
     }
-    float delta_lo, delta_hi;
-    if (ST && a.delta_pre) {       // sum_d dout*out was formed by an earlier kernel (gate backward)
+    if (ST && ST != kKept && have_dout && a.delta_pre) {       // sum_d dout*out was formed by an earlier kernel (gate backward)
         delta_lo = ok_lo ? a.delta_pre[(size_t)bh * N + row_lo] : 0.f;
         delta_hi = ok_hi ? a.delta_pre[(size_t)bh * N + row_hi] : 0.f;
-    } else {
+    } else if (have_dout) {
         RowFrag<D> oa, ob;
         orow.template load2<AL>(oa, ob, 0, ok_lo, ok_hi);
         delta_lo = quad_sum(frag_dot(da, oa));
@@ -1314,7 +1336,8 @@ cudaError_t bwd_launch_mode(BwdArgs a, const Taps& t, cudaStream_t s, int stages
 template <int D, int WB, bool SE>
 cudaError_t bwd_launch_se(BwdArgs a, const Taps& t, cudaStream_t s, int stages) {
     if constexpr (kLane<D> == 16) {       // 32-byte pieces
-        if (!aligned_to(32, {a.q, a.k, a.v, a.out, a.dout, a.dq, a.dk, a.dv}, {a.in_sb, a.in_sh, a.in_sn, a.out_sb, a.out_sh, a.out_sn})) {
+        if (!aligned_to(32, {a.q, a.k, a.v, a.out, a.dout, a.dq, a.dk, a.dv, a.dy, a.y, a.gate, a.dgate}, {a.in_sb, a.in_sh, a.in_sn, a.out_sb, a.out_sh, a.out_sn}) ||
+            (a.gate && !aligned_to(32, {}, {a.y_st.batch, a.y_st.head, a.y_st.row, a.gate_st.batch, a.gate_st.head, a.gate_st.row, a.dgate_st.batch, a.dgate_st.head, a.dgate_st.row}))) {
             if (!a.strided) {
                 a.in_sn = a.out_sn = D; a.in_sh = a.out_sh = (long long)a.N * D; a.in_sb = a.out_sb = (long long)a.H * a.N * D;
             }

@@ -330,3 +330,43 @@ def test_strided_entries_take_any_row_layouts_not_only_the_packed_one():
     for got, want in ((dq, qc.grad), (dk, kc.grad), (dv, vc.grad)):
         assert torch.equal(got, want.permute(0, 2, 1, 3))
     assert torch.equal(dpb, pb2.grad)
+
+
+@pytest.mark.parametrize("N", [1, 15, 16, 17, 63, 65, 150])
+@pytest.mark.parametrize("D,offset_of_gate", [(32, 0), (32, 8), (64, 0), (64, 8), (128, 0)])
+def test_gate_backward_inside_the_dq_kernel_is_the_standalone_kernels(N, D, offset_of_gate):
+    """dgate, and through dout and delta the other gradients, at the edges of a tile and with a gate that starts on 16 bytes only: against
+    dsqg_gate_bwd followed by the strided backward.  dgate is one formula per element: equal; the rest is too up to D = 32, where delta is
+    added in the same order, and within a bf16 rounding step of its inputs elsewhere."""
+    from dwarf_b200 import _lib
+    lib, B, H, offsets = _lib.load(), 2, 3, O.OFFSETS_43
+    qkv, gate, dy, pb, gain = (t.cuda() for t in _case(B, N, H, D, offsets, N + D))
+    flat = torch.zeros(gate.numel() + 16, dtype=torch.bfloat16, device="cuda")
+    gate = flat[offset_of_gate:offset_of_gate + gate.numel()].view_as(gate).copy_(gate).detach()
+    a = [t.detach().requires_grad_(True) for t in (qkv, gate, pb, gain)]
+    y = dwarf_b200.dsqg_attention_packed(a[0], a[2], a[3], a[1], offsets)
+    got = torch.autograd.grad(y, a, dy)
+    st = _lib.Strides(N * H * D, D, H * D)
+    dout, dgate, delta = torch.empty_like(dy), torch.empty_like(dy), torch.empty(B, H, N, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.dsqg_gate_bwd(dy.data_ptr(), y.data_ptr(), gate.contiguous().data_ptr(), st, dout.data_ptr(), dgate.data_ptr(), delta.data_ptr(), B, H, N, D, stream),
+               "gate")
+    assert torch.equal(got[1], dgate)
+    b = [t.detach().requires_grad_(True) for t in (qkv, pb, gain)]
+    z = dwarf_b200.dsqg_attention_packed(b[0], b[1], b[2], None, offsets)
+    off, J = _lib.offsets_array(offsets)
+    lse = torch.empty(B, H, N, device="cuda")
+    in_st = _lib.Strides(N * 3 * H * D, D, 3 * H * D)
+    at = [qkv.data_ptr() + i * H * D * 2 for i in range(3)]
+    _lib.check(lib.dsqg_fwd_strided(*at, in_st, pb.data_ptr(), gain.data_ptr(), off, J, torch.empty_like(z).data_ptr(), st, None, lse.data_ptr(), B, H, N, D, 0, stream, 0.0),
+               "fwd")
+    dqkv, dpb, dg = torch.empty_like(qkv), torch.empty_like(pb), torch.empty_like(gain)
+    scratch = torch.empty(lib.dsqg_bwd_scratch_bytes(J, B, H, N, D, 0), dtype=torch.uint8, device="cuda")
+    to = [dqkv.data_ptr() + i * H * D * 2 for i in range(3)]
+    _lib.check(lib.dsqg_bwd_strided(*at, in_st, pb.data_ptr(), gain.data_ptr(), off, J, z.data_ptr(), lse.data_ptr(), dout.data_ptr(), st, delta.data_ptr(), *to,
+                                    dpb.data_ptr(), dg.data_ptr(), scratch.data_ptr(), scratch.numel(), B, H, N, D, 0, stream, 0.0), "bwd")
+    for x, r in ((got[0], dqkv), (got[2], dpb), (got[3], dg)):
+        if D == 32:
+            assert torch.equal(x, r)
+        else:
+            assert ((x.float() - r.float()).abs() <= 2 ** -8 * r.float().abs() + 2 ** -8 * r.float().abs().max()).all()
