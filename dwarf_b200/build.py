@@ -13,7 +13,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 INCLUDE = os.path.join(os.path.dirname(PKG_DIR), "include")
 LIB_PATH = os.path.join(PKG_DIR, "libdsqg_b200.so")
 EXT_PATH = os.path.join(PKG_DIR, "_dsqg_torch.so")
-SOURCES = ["dsqg_capi.cu", "dsqg_dispatch.cu", "dsqg_generic.cu", "dsqg_decode.cu", "dsqg_mma.cu", "dsqg_mma_d64.cu", "dsqg_mma_window.cu", "dsqg_mma_widths.cu", "dsqg_staged.cu", "dsqg_umma.cu", "dsqg_static.cu", "dsqg_gate.cu", "dsqg_scan.cu", "dsqg_layer.cu"]
+SOURCES = ["dsqg_capi.cu", "dsqg_dispatch.cu", "dsqg_generic.cu", "dsqg_decode.cu", "dsqg_mma.cu", "dsqg_mma_d64.cu", "dsqg_mma_window.cu", "dsqg_mma_widths.cu", "dsqg_staged.cu", "dsqg_umma.cu", "dsqg_static.cu", "dsqg_gate.cu", "dsqg_scan.cu", "dsqg_layer.cu", "dsqg_wgrad.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]
 

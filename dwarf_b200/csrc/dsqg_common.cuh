@@ -100,6 +100,20 @@ inline cudaError_t launch_after(void (*kern)(Params...), dim3 grid, dim3 block, 
     if (e != cudaSuccess) cudaGetLastError();            // reported here and not again by the next check
     return e;
 }
+// The same with blocks of `cluster` consecutive x indices as thread-block clusters.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_clusters_after(unsigned cluster, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = s; c.attrs = at; c.numAttrs = 2;
+    const cudaError_t e = cudaLaunchKernelEx(&c, kern, static_cast<Params>(args)...);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
 __device__ __forceinline__ void stream_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -136,6 +150,7 @@ cudaError_t launch_wait_timeout(long long limit_cycles, int site, cudaStream_t s
 bool umma_supported(int dtype, int D, const Taps& t, bool has_scale_embed);
 cudaError_t launch_fwd_umma(const FwdArgs& a, const Taps& t, cudaStream_t s);
 cudaError_t read_umma_error(int* value, bool reset);
+cudaError_t read_wgrad_error(int* value, bool reset);
 
 // Whether the backward of strided tensors gains from contiguous copies of q, k, v that the forward leaves (FwdArgs::keep): rows shorter
 // than a 128-byte line cost as much L1 time as whole lines unless the next row follows (B32 H8 N2048 D32: dQ 126 -> 104, dK/dV

@@ -50,10 +50,11 @@ extern "C" int dsqg_set_kernel_path(int path) {
 }
 
 extern "C" int dsqg_device_error(int reset) {
-    int v = 0, w = 0;
+    int v = 0, w = 0, g = 0;
     if (dsqg::read_stage_error(&v, reset != 0) != cudaSuccess) return -1;
     if (dsqg::read_umma_error(&w, reset != 0) != cudaSuccess) return -1;
-    return v ? v : w;
+    if (dsqg::read_wgrad_error(&g, reset != 0) != cudaSuccess) return -1;
+    return v ? v : w ? w : g;
 }
 
 extern "C" int dsqg_test_wait_timeout(long long limit_cycles, void* stream) {

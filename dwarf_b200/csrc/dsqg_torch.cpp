@@ -501,6 +501,23 @@ Tensor grad_weight(const Tensor& dY, const Tensor& X, int64_t M, int64_t N, int6
     return C;
 }
 
+// Weight and bias gradients of two projections over the same M rows in one launch (csrc/dsqg_wgrad.cu) instead of a GEMM each and their
+// column sums.  Both sides of the line, us (M rows, two products [4 D, D] and [D, D]): D 256: M 1,024 7.6 against 9.8, 16,384 23.3 : 49.5,
+// 65,536 73 : 110; D 128: 6.4 : 9.5, 18.4 : 39.9, 55.5 : 83.  Its error against 64 bits is a half to a sixth of the GEMMs' there.  At D 512
+// 16,384 rows it still wins (51 : 73), but not at 384 (125 : 121 with [2 D, D]), and above 512 it loses: more tiles than clusters that run at
+// once.  The sums are split, so a caller who rules splits out (reduction_schemes) gets the GEMMs.
+bool one_launch_weight_grads(int64_t M, int64_t D) {
+    return D >= 128 && D <= 256 && D % 64 == 0 && M <= 65536 && reduction_schemes() != CUBLASLT_REDUCTION_SCHEME_NONE;
+}
+struct WeightGrad { const void* dy; int64_t ld; int64_t cols; const void* x; float* dw; float* sums; };
+void weight_grads(const std::array<WeightGrad, 2>& jobs, int count, int64_t M, int64_t D, const Tensor& on) {
+    const void *dy[2], *x[2]; long long ld[2]; int cols[2]; float *dw[2], *sums[2];
+    for (int k = 0; k < count; ++k) {
+        dy[k] = jobs[k].dy; x[k] = jobs[k].x; ld[k] = jobs[k].ld; cols[k] = (int)jobs[k].cols; dw[k] = jobs[k].dw; sums[k] = jobs[k].sums;
+    }
+    check(dsqg_weight_grads(dy, ld, cols, x, dw, sums, count, M, (int)D, stream_of(on)), "dsqg_weight_grads");
+}
+
 // fp32 tensors as bf16 back to back in one buffer, in one launch; at[k]: where the k-th begins (elements).
 struct Bf16Pack {
     Tensor buf;
@@ -610,8 +627,9 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
         void* stream = stream_of(x);
         const char* wb = static_cast<const char*>(ptr(w));
         Tensor dinter, dwkv, dg, dxi, dwg, dx, dgb;
-        if (n_wkv) {
-            dwkv = new_tensor({2 * D, D}, at::kFloat, x);
+        const bool one_launch = n_wkv && need(3) && one_launch_weight_grads(M, D);
+        if (n_wkv) dwkv = new_tensor({2 * D, D}, at::kFloat, x);
+        if (n_wkv && !one_launch) {
             gemm(ptr(dwkv), true, dp, true, ptr(inter), false, nullptr, 2 * D, D, M, x, ld);
         }
         if (n_in) {
@@ -619,8 +637,17 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
             gemm(ptr(dinter), false, dp, false, wb + 2 * D * D, false, nullptr, M, D, 2 * D, x, ld);
             check(dsqg_gated_mean_bwd(ptr(dinter), ptr(g), fptr(pool), ptr(dg), fptr(dxi), (int)x.size(0), (int)x.size(1), (int)D, stream), "dsqg_gated_mean_bwd");
         }
-        if (need(3)) dwg = grad_weight(dg, xib, M, D, D);
-        const Tensor db = column_sums({{ptr(dg), D, need(4) ? (int)D : 0}, {dp, ld, n_bkv ? (int)(2 * D) : 0}}, M, x);
+        const int64_t kv = need(4) ? D : 0;                    // where the sums of the two biases begin
+        Tensor db;
+        if (one_launch) {
+            dwg = new_tensor({D, D}, at::kFloat, x);
+            if (kv || n_bkv) db = new_tensor({kv + (n_bkv ? 2 * D : 0)}, at::kFloat, x);
+            weight_grads({{{dp, ld, 2 * D, ptr(inter), fptr(dwkv), n_bkv ? fptr(db) + kv : nullptr}, {ptr(dg), D, D, ptr(xib), fptr(dwg), kv ? fptr(db) : nullptr}}},
+                         2, M, D, x);
+        } else {
+            if (need(3)) dwg = grad_weight(dg, xib, M, D, D);
+            db = column_sums({{ptr(dg), D, need(4) ? (int)D : 0}, {dp, ld, n_bkv ? (int)(2 * D) : 0}}, M, x);
+        }
         if (n_norm) {
             const Tensor dxib = grad_input(dg, wb, M, D, D, false);
             dx = new_like(x); dgb = new_tensor({2 * D}, at::kFloat, x);
@@ -630,7 +657,6 @@ struct InterferenceNode : torch::autograd::Function<InterferenceNode> {
                   "dsqg_layer_norm_bwd_split");
         }
         const auto piece = [&](bool wanted, const Tensor& buf, at::IntArrayRef sizes, int64_t first) { return wanted ? part(buf, sizes, first) : Tensor(); };
-        const int64_t kv = need(4) ? D : 0;                    // where the sums of the two biases begin
         return {need(0) ? like_param(dx, (at::ScalarType)ctx->saved_data["x_type"].toInt()) : Tensor(), piece(need(1), dgb, {D}, 0), piece(need(2), dgb, {D}, D),
                 dwg, piece(need(4), db, {D}, 0), piece(need(5), dwkv, {D, D}, 0), piece(need(6), db, {D}, kv), piece(need(7), dwkv, {D, D}, D * D),
                 piece(need(8), db, {D}, kv + D), Tensor(), Tensor()};
@@ -692,18 +718,25 @@ struct LayerNode : torch::autograd::Function<LayerNode> {
                    n_bo = need(), n_pb = need(), n_hg = need(f.hg.defined()), n_se = need(f.se.defined());
         Tensor dx, dk, dv, dw, dwo;
         PackedGrads g;
-        if (n_wo) dwo = grad_weight(dy, f.y, M, D, D);
-        if (n_x || n_k || n_v || n_wqkv || n_bqkv || n_wg || n_bg || n_pb || n_hg || n_se)
-            g = packed_backward(f, grad_input(dy, wb + 2 * 4 * D * D, M, D, D, false), 4 * D, offsets_of(ctx));
         // of the columns [qkv | gate], those from `first` on up to `last`
         const int64_t first = n_wqkv ? 0 : 3 * D, last = n_wg ? 4 * D : 3 * D, sum_first = n_bqkv ? 0 : 3 * D, sum_last = n_bg ? 4 * D : 3 * D;
+        const int sums = (int)std::max<int64_t>(sum_last - sum_first, 0);
+        const bool one_launch = last > first && n_wo && (!sums || (sum_first == first && sum_last == last)) && one_launch_weight_grads(M, D);
+        if (n_wo && !one_launch) dwo = grad_weight(dy, f.y, M, D, D);
+        if (n_x || n_k || n_v || n_wqkv || n_bqkv || n_wg || n_bg || n_pb || n_hg || n_se)
+            g = packed_backward(f, grad_input(dy, wb + 2 * 4 * D * D, M, D, D, false), 4 * D, offsets_of(ctx));
         const auto column = [&](int64_t c) { return static_cast<const char*>(ptr(g.dproj)) + 2 * c; };
-        if (last > first) {
-            dw = new_tensor({last - first, D}, at::kFloat, dy);
+        if (last > first) dw = new_tensor({last - first, D}, at::kFloat, dy);
+        if (last > first && !one_launch) {
             gemm(ptr(dw), true, column(first), true, ptr(xb), false, nullptr, last - first, D, M, dy, 4 * D);
         }
-        const int sums = (int)std::max<int64_t>(sum_last - sum_first, 0);
-        const Tensor db = column_sums({{sums ? column(sum_first) : nullptr, 4 * D, sums}, {ptr(dy), D, n_bo ? (int)D : 0}}, M, xb);
+        Tensor db;
+        if (one_launch) {
+            dwo = new_tensor({D, D}, at::kFloat, dy);
+            if (sums || n_bo) db = new_tensor({sums + (n_bo ? D : 0)}, at::kFloat, dy);
+            weight_grads({{{column(first), 4 * D, last - first, ptr(xb), fptr(dw), sums ? fptr(db) : nullptr},
+                           {ptr(dy), D, D, ptr(f.y), fptr(dwo), n_bo ? fptr(db) + sums : nullptr}}}, 2, M, D, dy);
+        } else db = column_sums({{sums ? column(sum_first) : nullptr, 4 * D, sums}, {ptr(dy), D, n_bo ? (int)D : 0}}, M, xb);
         if (n_x) {
             const auto t = (at::ScalarType)xt[0];
             dx = like_param(grad_input(g.dproj, wb, M, 4 * D, D, t == at::kFloat).view({B, N, D}), t);

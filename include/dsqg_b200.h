@@ -292,9 +292,13 @@ int dsqg_packed_bwd_gate(const dsqg_packed* p, const dsqg_packed_grads* g, const
  *   dsqg_gated_mean_bwd  dg and dx for the gradient dinter of inter
  *   dsqg_inject_kv       columns [D,2D) and [2D,3D) of qkv += k_delta, v_delta (rows qkv_stride / delta_stride elements apart)
  *   dsqg_column_sums     fp32 column sums of up to DSQG_SUM_MAX bf16 matrices of the same number of rows, fixed order
+ *   dsqg_weight_grads    dw[k] [cols[k], D] = dy[k]^T . x[k] in fp32 and sums[k] [cols[k]] = column sums of dy[k] (null: left out) for
+ *                        up to DSQG_WGRAD_MAX pairs of `rows` rows in one launch; dy rows dy_stride elements apart, x rows of D; D and
+ *                        cols multiples of 64; fixed order of the sums
  * D a multiple of 8 (layer norm: at most 1024); all pointers 16-byte aligned; src, dst, n, row_stride, cols: HOST arrays. */
 #define DSQG_CAST_MAX 8
 #define DSQG_SUM_MAX 4
+#define DSQG_WGRAD_MAX 2
 int dsqg_cast_bf16(const float* const* src, void* const* dst, const long long* n, int count, void* stream);
 int dsqg_layer_norm_fwd(const float* x, const float* gamma, const float* beta, float eps, float* y, void* y_bf16, float* stat,
                         long long rows, int D, void* stream);
@@ -308,6 +312,8 @@ int dsqg_gated_mean_bwd(const void* dinter, const void* g, const float* pool, vo
 int dsqg_inject_kv(void* qkv, long long qkv_stride, const void* k_delta, const void* v_delta, long long delta_stride, long long rows, int D, void* stream);
 int dsqg_column_sums(const void* const* src, const long long* row_stride, const int* cols, float* const* dst, int count, long long rows,
                      void* stream);
+int dsqg_weight_grads(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
+                      int count, long long rows, int D, void* stream);
 
 /* Single-token decode over a circular K/V ring buffer.
  * Replaces: nothing executable -- the reference only describes the O(1) cache in prose

@@ -275,3 +275,61 @@ def test_tensors_elsewhere_are_refused_on_the_host():
     delta = torch.zeros(1, 2, 40, 32)
     with torch.autocast("cuda", dtype=torch.bfloat16), pytest.raises(RuntimeError):
         attn(torch.randn(1, 40, 64, device="cuda"), kv_inject=(delta, delta))
+
+
+# rows: less than a stage, its edges, more blocks than steps, all eight blocks of a cluster with a ragged end; cols and D: tiles half empty,
+# two widths, several across.  dy is a block of columns of a wider matrix; the second job may lack its sums.
+@pytest.mark.parametrize("rows,D,cols", [(1, 64, (64,)), (63, 64, (128, 64)), (65, 128, (192, 128)), (511, 192, (576, 192)), (513, 256, (1024, 256)),
+                                         (300, 512, (2048, 512)), (4099, 256, (512, 256)), (777, 320, (64, 704))])
+def test_weight_grads(rows, D, cols):
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(rows + D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    wide = [rnd(rows, c + 24) for c in cols]
+    dy, x = [w[:, 8:8 + c] for w, c in zip(wide, cols)], [rnd(rows, D) for _ in cols]
+    dw = [torch.full((c + 1, D), 7.0, device="cuda") for c in cols]
+    sums = [torch.full((c + 1,), 7.0, device="cuda") for c in cols]
+    arr = lambda t, v: (t * len(v))(*v)  # noqa: E731
+    ptrs = lambda ts: arr(ctypes.c_void_p, [t.data_ptr() for t in ts])  # noqa: E731
+
+    def call(sum_ptrs, D=D, cols=cols, rows=rows):
+        return lib.dsqg_weight_grads(ptrs(dy), arr(ctypes.c_longlong, [w.stride(0) for w in wide]), arr(ctypes.c_int, list(cols)), ptrs(x), ptrs(dw), sum_ptrs,
+                                     len(cols), rows, D, _stream())
+    _lib.check(call(ptrs(sums)), "weight_grads")
+    first = [w.clone() for w in dw]
+    # one tensor-core step takes 16 products and rounds once: at most rows / 16 roundings of 2^-23 of the running sum
+    rel = 2.0 ** -23 * max(8, rows / 16)
+    for d, xx, w, s, c in zip(dy, x, dw, sums, cols):
+        _close(w[:c], d.double().t() @ xx.double(), rel, "dw")
+        _close(s[:c], d.double().sum(0), rel, "sums")
+        assert (w[c] == 7).all() and s[c] == 7                       # nothing past the end
+    for w in dw:
+        w.zero_()
+    _lib.check(call(arr(ctypes.c_void_p, [0] * len(cols))), "weight_grads without sums")
+    assert all(torch.equal(a[:c], b[:c]) for a, b, c in zip(first, dw, cols))      # the same bits on every call
+    assert all(s[c] == 7 for s, c in zip(sums, cols))
+    assert call(ptrs(sums), D=D + 8) == call(ptrs(sums), cols=[c + 8 for c in cols]) == call(ptrs(sums), rows=0) == -2
+
+
+@pytest.mark.parametrize("dim,N", [(128, 97), (256, 300)])
+def test_weight_gradients_of_a_layer_with_and_without_split_sums(dim, N):
+    """A caller who allows no split of a sum gets one GEMM per weight; the gradients are those of the one launch."""
+    torch.manual_seed(dim)
+    with torch.device("cuda"):
+        attn, inject = dwarf_b200.DSQGAttentionQW(dim, dim // 32, seq_len=N, dropout=0.0), dwarf_b200.InterferenceInjection(dim, dim // 32)
+    x, dy = torch.randn(2, N, dim, device="cuda"), torch.randn(2, N, dim, device="cuda").bfloat16()
+    wrt = [*attn.parameters(), *inject.parameters()]
+
+    def grads():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = attn(x, kv_inject=inject(x))
+        return torch.autograd.grad(y, wrt, dy)
+    was = torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction
+    one = grads()
+    try:
+        torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = (False, False)
+        many = grads()
+    finally:
+        torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = was
+    for a, b in zip(one, many):
+        _close(a, b, 2e-3, "gradient")        # the projections' GEMMs may round other bf16 values when they may not split
