@@ -114,10 +114,9 @@ inline cudaError_t launch_clusters_after(unsigned cluster, void (*kern)(Params..
     if (e != cudaSuccess) cudaGetLastError();
     return e;
 }
-__device__ __forceinline__ void stream_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+__device__ __forceinline__ void wait_ahead() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void stream_wait() { wait_ahead(); let_next_in(); }
 
 // Launchers (defined in the .cu files; return a cudaError_t from the launch).
 cudaError_t launch_fwd(const FwdArgs& a, const Taps& t, int dtype, cudaStream_t s);   // dispatcher

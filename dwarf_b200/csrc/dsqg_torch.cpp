@@ -502,10 +502,11 @@ Tensor grad_weight(const Tensor& dY, const Tensor& X, int64_t M, int64_t N, int6
 }
 
 // Weight and bias gradients of two projections over the same M rows in one launch (csrc/dsqg_wgrad.cu) instead of a GEMM each and their
-// column sums.  Both sides of the line, us (M rows, two products [4 D, D] and [D, D]): D 256: M 1,024 7.6 against 9.8, 16,384 23.3 : 49.5,
-// 65,536 73 : 110; D 128: 6.4 : 9.5, 18.4 : 39.9, 55.5 : 83.  Its error against 64 bits is a half to a sixth of the GEMMs' there.  At D 512
-// 16,384 rows it still wins (51 : 73), but not at 384 (125 : 121 with [2 D, D]), and above 512 it loses: more tiles than clusters that run at
-// once.  The sums are split, so a caller who rules splits out (reduction_schemes) gets the GEMMs.
+// column sums.  Both sides of the line, us (M rows, two products [4 D, D] and [D, D]): D 256: M 1,024 7.6 against 9.8, 16,384 23.1 : 49.5,
+// 65,536 70 : 107; D 128: 6.4 : 9.5, 18.4 : 39.9, 55.5 : 83.  Its error against 64 bits is at most the GEMMs', mostly a half to a sixth of it.  At D 512
+// 16,384 rows it still wins (51 : 73), but not at 384 (125 : 121 with [2 D, D] and 65,536 rows), and above 512 it loses: more tiles than clusters that
+// run at once.  Beyond 65,536 rows its sums are longer than the GEMMs' and their error larger.  The sums are split, so a caller who rules splits
+// out (reduction_schemes) gets the GEMMs.
 bool one_launch_weight_grads(int64_t M, int64_t D) {
     return D >= 128 && D <= 256 && D % 64 == 0 && M <= 65536 && reduction_schemes() != CUBLASLT_REDUCTION_SCHEME_NONE;
 }

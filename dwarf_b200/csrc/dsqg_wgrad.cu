@@ -14,9 +14,10 @@
 // Every wait is bounded (stg::mbar_wait); a block that gives up writes NaN and sets the device error word.
 //
 // Bound by what an SM can fetch (90 GB/s a block measured, from L2 or HBM; all 148 together would outrun HBM): [1024, 256] + [256, 256]
-// gradients with their sums, against two library GEMMs and a pass for the sums: 4,096 rows 11.0 us : 18.5, 16,384 23.3 : 49.5, 65,536
-// 73 : 110 (HBM's floor there 36).  A tile of 128 x 256 with eight blocks a cluster took 25 and 72 us for the first two products, but
-// 24 and 70 instead of 18.7 and 56 for [512, 256] + [256, 256], whose six tiles leave most of the chip idle: hence two widths.
+// gradients with their sums, against two library GEMMs and a pass for the sums: 4,096 rows 11.0 us : 18.5, 16,384 23.1 : 49.5, 65,536
+// 70 : 107 (HBM's floor there 36).  A tile of 128 x 256 with eight blocks a cluster took 25 and 72 us for the first two products, but
+// 24 and 70 instead of 18.7 and 54 for [512, 256] + [256, 256], whose six tiles leave most of the chip idle: hence two widths.  The sums cost 6 of
+// the 70 us (shared-memory reads beside the tensor cores'); added by one tile in two instead of half by each they cost 10.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -36,16 +37,16 @@ constexpr int kTM = 128;                       // columns of dY of a tile
 constexpr int kBox = 64;                       // rows and columns of a staged box
 constexpr int kBoxBytes = kBox * 128;
 constexpr int kThreads = 192, kCopyWarp = 4, kMmaWarp = 5;
-constexpr int kSumRows = 8;                    // rows of a stage added side by side
 constexpr int kMostSplit = 8;
+constexpr long long kLimit = 4000000000LL;      // cycles before a wait gives up: two seconds, far above any time slice of a shared GPU
 // TN: columns of X of a tile
 template <int TN>
 struct Layout {
     static constexpr int a_bytes = kTM / kBox * kBoxBytes, stage_bytes = a_bytes + TN / kBox * kBoxBytes;      // 48 / 32 KB
     static constexpr int stages = 192 * 1024 / stage_bytes;
     static constexpr int pitch = TN + 4;                           // floats per row of the partial tile (16-byte stores of neighbouring rows: other banks)
-    static constexpr int sum0 = stages * stage_bytes;              // column sums [kSumRows][kTM], then their total [kTM]
-    static constexpr int bars0 = sum0 + (kSumRows + 1) * kTM * 4;
+    static constexpr int sum0 = stages * stage_bytes;              // column sums of 8 row classes x kTM columns or 16 x 64, then their total [kTM]
+    static constexpr int bars0 = sum0 + (8 + 1) * kTM * 4;
     static constexpr int full = 0, empty = stages, done = 2 * stages, bars = done + 1;
     static constexpr int total = bars0 + 256 + 1024;               // 1,024: alignment of the swizzle atoms
     static_assert(kTM * pitch * 4 <= sum0, "the partial tile lies over the stages");
@@ -97,10 +98,15 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
     const Job job = j ? a.job[1] : a.job[0];
     const int across = (a.D + TN - 1) / TN, in_job = tile - (j ? a.job[0].tiles_end : 0);
     const int c0 = in_job / across * kTM, k0 = in_job % across * TN;
-    const bool sums = job.sum && k0 == 0;
+    // dY's columns are added by the tiles of the first columns of X: all 128 by one, or 64 each by two
+    const bool halves = across > 1, sums = job.sum && k0 < (halves ? 2 * TN : TN);
+    const int sum_cols = halves ? 64 : kTM, sum_c = halves ? k0 / TN * 64 : 0;
     const int blocks = (a.rows + kBox - 1) / kBox;
     const int first = (int)((long long)blocks * rank / a.split), count = (int)((long long)blocks * (rank + 1) / a.split) - first;
 
+    // tensor memory is asked for when nothing of the kernel ahead holds or still wants any, and before the next kernel may: two kernels
+    // that wait for each other's columns would wait for good
+    wait_ahead();
     if (tid == 0) {
         *abort_flag = 0;
         for (int i = 0; i < kStages; ++i) { mbar_init(bars + 8 * (kFull + i), 1); mbar_init(bars + 8 * (kEmpty + i), sums ? 5 : 1); }
@@ -115,7 +121,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    stream_wait();
+    let_next_in();
 
     if (warp == kCopyWarp) {
         if (lane == 0) {
@@ -123,7 +129,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             int i = 0;
             for (; i < count; ++i) {
                 const int st = i % kStages;
-                if (i >= kStages && !mbar_wait(bars + 8 * (kEmpty + st), (i / kStages - 1) & 1, abort_flag, 0x501)) break;
+                if (i >= kStages && !mbar_wait(bars + 8 * (kEmpty + st), (i / kStages - 1) & 1, abort_flag, 0x501, kLimit)) break;
                 const uint32_t bar = bars + 8 * (kFull + st), dst = sb + st * kStageBytes;
                 const int row = (first + i) * kBox;
                 mbar_arrive_expect_tx(bar, kStageBytes);               // boxes outside a matrix arrive as zeros
@@ -135,7 +141,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             // after an abort: no copy of this block may be in flight when its shared memory is released
             if (*abort_flag) {
                 volatile int keep_waiting = 0;
-                for (int k = i > kStages ? i - kStages : 0; k < i; ++k) mbar_wait(bars + 8 * (kFull + k % kStages), (k / kStages) & 1, &keep_waiting, 0x504);
+                for (int k = i > kStages ? i - kStages : 0; k < i; ++k) mbar_wait(bars + 8 * (kFull + k % kStages), (k / kStages) & 1, &keep_waiting, 0x504, kLimit);
             }
         }
         __syncwarp();
@@ -144,7 +150,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             const uint64_t desc0 = mn_desc(sb);
             for (int i = 0; i < count; ++i) {
                 const int st = i % kStages;
-                if (!mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x502)) break;
+                if (!mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x502, kLimit)) break;
                 tc_fence_after();
                 const uint64_t da = desc0 + (uint32_t)(st * kStageBytes >> 4), db = da + (uint32_t)(kABytes >> 4);
 #pragma unroll
@@ -158,35 +164,37 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
     } else {
         float* csum = reinterpret_cast<float*>(smem + kSum0);
         if (sums) {
-            // thread: eight columns (one 16-byte chunk) of the rows r, r + 8, ... of each stage; the chunk index is XORed with row & 7
-            const int chunk = tid & 7, half = tid >> 3 & 1, r = tid >> 4;
-            const unsigned char* src = smem + half * kBoxBytes + r * 128 + ((chunk ^ r) << 4);
+            // thread: eight columns (one 16-byte chunk) of every 8th or 16th row of a stage; the chunk index is XORed with row & 7
+            const int chunk = tid & 7, half = halves ? sum_c / 64 : tid >> 3 & 1, r = tid >> (halves ? 3 : 4), apart = halves ? 16 : 8;
+            const unsigned char* src = smem + half * kBoxBytes + r * 128 + ((chunk ^ (r & 7)) << 4);
             float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int i = 0; i < count; ++i) {
                 const int st = i % kStages;
-                if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x503))) break;
-                uint4 u[kBox / kSumRows];
+                if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x503, kLimit))) break;
+                uint4 u[8];
 #pragma unroll
-                for (int k = 0; k < kBox / kSumRows; ++k) u[k] = *reinterpret_cast<const uint4*>(src + st * kStageBytes + k * kSumRows * 128);
+                for (int k = 0; k < 8; ++k)
+                    u[k] = k < 4 || !halves ? *reinterpret_cast<const uint4*>(src + st * kStageBytes + k * apart * 128) : make_uint4(0u, 0u, 0u, 0u);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bars + 8 * (kEmpty + st));
 #pragma unroll
-                for (int k = 0; k < kBox / kSumRows; ++k) {
+                for (int k = 0; k < 8; ++k) {
+                    if (k >= 4 && halves) break;
                     const uint32_t w[4] = {u[k].x, u[k].y, u[k].z, u[k].w};
 #pragma unroll
                     for (int e = 0; e < 4; ++e) { s[2 * e] += __uint_as_float(w[e] << 16); s[2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u); }
                 }
             }
 #pragma unroll
-            for (int e = 0; e < 8; ++e) csum[r * kTM + half * 64 + chunk * 8 + e] = s[e];
+            for (int e = 0; e < 8; ++e) csum[r * sum_cols + (halves ? 0 : half * 64) + chunk * 8 + e] = s[e];
             asm volatile("bar.sync 1, 128;" ::: "memory");
             float t = 0.f;
-#pragma unroll
-            for (int k = 0; k < kSumRows; ++k) t += csum[k * kTM + tid];
-            csum[kSumRows * kTM + tid] = t;
+            if (tid < sum_cols)
+                for (int k = 0; k < apart; ++k) t += csum[k * sum_cols + tid];
+            csum[8 * kTM + tid] = t;
         }
         // accumulator row = tensor-memory lane = tid; the stages are free once every product has completed
-        const bool ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * kDone, 0, abort_flag, 0x505)) && !*abort_flag;
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * kDone, 0, abort_flag, 0x505, kLimit) && !*abort_flag);
         tc_fence_after();
         float* part = reinterpret_cast<float*>(smem) + tid * kPitch;
         const uint32_t acc = tmem + ((uint32_t)(32 * warp) << 16);
@@ -226,10 +234,10 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             for (int b = 1; b < 8; ++b) if (b < a.split) { t.x += v[b].x; t.y += v[b].y; t.z += v[b].z; t.w += v[b].w; }
             *reinterpret_cast<float4*>(job.dw + (size_t)(c0 + r) * a.D + k0 + c) = t;
         }
-        if (sums && rank == 0 && tid < min(kTM, job.cols - c0)) {
+        if (sums && rank == 0 && tid < min(sum_cols, job.cols - c0 - sum_c)) {
             float t = 0.f;
-            for (int b = 0; b < a.split; ++b) t += cluster_load(cluster_addr(sb + kSum0 + (kSumRows * kTM + tid) * 4, b));
-            job.sum[c0 + tid] = t;
+            for (int b = 0; b < a.split; ++b) t += cluster_load(cluster_addr(sb + kSum0 + (8 * kTM + tid) * 4, b));
+            job.sum[c0 + sum_c + tid] = t;
         }
     }
     cluster_sync();                                                    // nobody's shared memory goes while others read it
