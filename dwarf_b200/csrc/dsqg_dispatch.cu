@@ -15,10 +15,10 @@ namespace dsqg {
 static std::atomic<int> g_path{0};
 
 // Where the tcgen05 forward is taken instead of the register-fed one: 128-byte rows (D = 64), no sparse taps, at least two
-// 128-row tiles for each SM's persistent block.  Offsets 0..31, L2 cold, tcgen05 / register-fed: 6,144 tiles (16x12x4096) 84.0 / 90.1 us,
-// 3,072 tiles 49.2 / 51.2, 1,536 tiles 30.7 / 31.7, 768 tiles 22.5 / 20.5, 576 tiles 18.4 / 16.4, 320 tiles 14.3 / 14.4, 288 tiles 14.3 / 12.3.
-// So it pays from about ten tiles per SM; the line at two was drawn when the register-fed kernel took 56.1 us at 3,072 tiles, and
-// callers know it (dsqg_b200.h).
+// 128-row tiles for each SM's persistent block.  The line was drawn when the register-fed kernel took 56.1 us at 3,072 tiles (tcgen05 49).  It is
+// ahead at every size now (offsets 0..31, L2 cold, tcgen05 / register-fed: 6,144 tiles (16x12x4096) 85.0 / 78.8 us, 3,072 tiles 50.2 / 46.1,
+// 1,536 tiles 31.7 / 27.6, 768 tiles 21.5 / 19.5, 320 tiles 15.4 / 13.3); the line stays because which kernel's bits a call returns is stated to
+// callers (dsqg_b200.h).
 static bool umma_pays(const FwdArgs& a, const Taps& t, int dtype) {
     return a.D == 64 && t.n_sparse == 0 && !a.strided &&
            (long long)a.B * a.H * ((a.N + 127) / 128) >= 2 * 148 && umma_supported(dtype, a.D, t, a.scale_embed != nullptr);
