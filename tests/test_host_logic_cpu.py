@@ -153,3 +153,20 @@ def test_layer_gemms_follow_the_reduced_precision_setting():
         assert n.reduction_schemes() == 0
     finally:
         mm.allow_bf16_reduced_precision_reduction = before
+
+
+def test_ring_cache_offsets_survive_copies_pickles_and_assignment():
+    """The native form of the offsets that a cache keeps follows its offsets and never leaves the process."""
+    import copy
+    import pickle
+
+    from dwarf_b200 import DSQGRingCache, _lib
+    cache = DSQGRingCache(1, 2, 1, 32, offsets=[0, 1, 5], device="cpu")
+    cache._handle = _lib.offsets_handle(cache.offsets)
+    for other in (copy.copy(cache), copy.deepcopy(cache), pickle.loads(pickle.dumps(cache))):
+        assert other.offsets == (0, 1, 5) and other._handle is None and other.R == 6 and torch.equal(other.kv, cache.kv)
+    old = DSQGRingCache.__new__(DSQGRingCache)
+    old.__setstate__({"offsets": (0, 1), "R": 2})               # what a cache was pickled as before it kept the handle
+    assert old.offsets == (0, 1) and old._handle is None
+    cache.offsets = [0, 2]
+    assert cache.offsets == (0, 2) and cache._handle is None
