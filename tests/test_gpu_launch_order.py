@@ -63,3 +63,45 @@ def test_decode_after_calls_that_write_its_rings():
     for _ in range(5):
         for a, b in zip(apart, run(lambda: None)):
             assert torch.equal(a, b)
+
+
+def test_two_streams_that_join_eager_and_captured():
+    """A call behind two streams' calls reads both results: events and graph edges hold for kernels that may start early."""
+    B, H, N, D, J = 4, 8, 1000, 32, len(dwarf_b200.OFFSETS_43)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(B, H, N, D, generator=g, device="cuda").bfloat16() for _ in range(3))
+    pb = torch.randn(J, H, generator=g, device="cuda") * 0.1
+    op = lambda a, b, c: dwarf_b200.dsqg_attention(a, b, c, pb, None, None, dwarf_b200.OFFSETS_43)  # noqa: E731
+    want = [op(q, k, v), op(v, q, k)]
+    want.append(op(want[0], want[1], want[0]))
+    want.append(op(want[2], want[1], want[0]))
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def work():
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            two = op(v, q, k)
+        one = op(q, k, v)
+        main.wait_stream(side)
+        three = op(one, two, one)
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            four = op(three, two, one)
+        main.wait_stream(side)
+        return [one, two, three, four]
+
+    with torch.cuda.stream(main):
+        for _ in range(5):
+            got = work()
+            torch.cuda.synchronize()                    # before a tensor of one stream is given back while the other may read it
+            assert all(torch.equal(a, b) for a, b in zip(want, got))
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=main):
+            got = work()
+        for _ in range(5):
+            for t in got:
+                t.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(want, got))
