@@ -86,7 +86,8 @@ struct DecodeArgs {
 // Programmatic dependent launch, for every kernel of the library: its blocks are scheduled as the last blocks of the kernel ahead of it in the stream leave,
 // instead of after that kernel's completion has been noticed.  stream_wait comes first in the kernel, so nothing of it runs before the results of
 // what is ahead are visible: order and results are those of a plain launch.  It lets the next kernel's blocks come only once it has waited
-// itself: a decode step that reads ahead of its own wait (dsqg_decode_overlapped) then finds everything but the kernel ahead of it finished.
+// itself: a decode step that reads ahead of its own wait (dsqg_decode_overlapped) then finds everything but the kernel ahead of it finished.  That
+// step keeps to it too: it reads early, but hands over after its wait like the others.
 // Worth 1.5 to 2 us a launch, passes of one kind in a row, us: 2x8x777x32 forward and backward 28.8 -> 23.4, 8x8x1000x32 44.3 -> 39.4, 8x8x2048x80
 // 168.2 -> 164.5, 32x8x2048x32 243.2 -> 236.8, fp32 forward 2x8x2048x32 20.6 -> 19.2, 1x8x300x32 8.3 -> 6.0.
 template <typename... Params, typename... Args>

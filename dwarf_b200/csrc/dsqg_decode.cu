@@ -176,16 +176,18 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 //
-// PDL = true is the overlapped form (programmatic dependent launch): the kernel lets the next
-// kernel of the stream start at once, and itself reads only head, fill and the ring rows of taps
-// with delta > 0 before it waits for the kernels ahead of it; q, k_new, v_new are read and the
-// ring and out are written after that wait.  The ring gather of one layer then overlaps the tail
-// of whatever runs before it.
+// PDL = true is the overlapped form (programmatic dependent launch): the kernel reads only head,
+// fill and the ring rows of taps with delta > 0 before it waits for the kernels ahead of it; q,
+// k_new, v_new are read and the ring and out are written after that wait.  The ring gather of one
+// layer then overlaps the tail of whatever runs before it.  The next kernel is let in after the wait
+// and not before it: a step that is two behind a writer would read beside it otherwise, since the
+// step between them has not waited for the writer either when it starts.
+// (At the kernel's top instead: ten layers of the benchmark shape 85.8 us a step against 87.7, five
+// layers of 4 sequences 30.9 against 31.5.)
 template <int TPR, int ROUNDS, int VSM, int CTAS, bool PDL>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32, CTAS)
 decode_1pass_kernel(const DecodeArgs a, const Taps t) {
-    if constexpr (PDL) asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-    else stream_wait();
+    if constexpr (!PDL) stream_wait();
     using T = __nv_bfloat16;
     constexpr int GROUPS = 32 / TPR;
     constexpr int VREG = ROUNDS - VSM;
@@ -232,7 +234,7 @@ decode_1pass_kernel(const DecodeArgs a, const Taps t) {
         }
     }
     if constexpr (PDL) {
-        asm volatile("griddepcontrol.wait;\n" ::: "memory");
+        stream_wait();
         if (g == 0 && t.delta(0) == 0) {                 // offsets ascend: only tap 0 can be delta 0
             const bool on = fill > 0 && active;
             if (on) cp_async16(&k_sm[warp][0][lane], kn + d0); else k_sm[warp][0][lane] = zero4;
@@ -332,8 +334,8 @@ cudaError_t decode_launch(const DecodeArgs& a, const Taps& t, cudaStream_t s, bo
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
         // bf16 rings, up to 12 rounds: single-pass kernel.  K rows and seven rounds of V rows in shared memory leave 80
         // registers, six CTAs per SM: every warp of the benchmark shape (256 sequences, 12 heads of 64, 43 taps) is resident at once.
-        // Ten overlapped layers of it: 86 us (88 with five rounds of V, 97 with one round more than 43 taps need; 116 with
-        // five CTAs; 115 with the online softmax, one tap after the other, that this kernel had before).
+        // Ten overlapped layers of it: 88 us; measured when it took 86: 88 with five rounds of V, 97 with one round more than 43 taps need, 116 with
+        // five CTAs, 115 with the online softmax, one tap after the other, that this kernel had before.
         if (rounds <= 6) return decode_launch_1pass<TPR, 6, 0, 24 / kWarpsPerBlock>(a, t, s, overlap);
         if (rounds <= 11) return decode_launch_1pass<TPR, 11, 7, 24 / kWarpsPerBlock>(a, t, s, overlap);
         if (rounds <= 12) return decode_launch_1pass<TPR, 12, 6, 24 / kWarpsPerBlock>(a, t, s, overlap);

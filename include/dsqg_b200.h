@@ -357,10 +357,14 @@ int dsqg_ring_prefill_kv(const void* k, const void* v, void* kv_ring,
  * v_new are read, and the rings and out written, only after the wait.  The caller therefore
  * promises that the kernel launched just before this call on the same stream writes none of
  * head, fill, k_ring, v_ring of THIS call (true for a stack of layers that each own their rings
- * and share one write head advanced once per token, after some other kernel).  It also lets the
- * kernel launched after it start early if that kernel was launched in the same way; an ordinary
- * kernel after it waits as usual.  bf16 rings with at most 12 taps per lane group (J <= 48 at
- * D = 64, J <= 96 at D = 32) take this form; other cases run exactly as dsqg_decode. */
+ * and share one write head advanced once per token, after some other kernel).  What was launched
+ * before that kernel has finished by then: every kernel of this library lets the next one start only
+ * after it has waited for what is ahead of it.  (A kernel of the caller's own that is launched with
+ * programmatic stream serialisation and lets the next one start before its own wait gives no such
+ * assurance: directly ahead of this call, it extends the promise to the kernel before it.)  A kernel
+ * launched after this call in the same way starts early in its turn; an ordinary one waits as usual.
+ * bf16 rings with at most 12 taps per lane group (J <= 48 at D = 64, J <= 96 at D = 32) take this
+ * form; other cases run exactly as dsqg_decode. */
 int dsqg_decode_overlapped(const void* q, const void* k_new, const void* v_new,
                            void* k_ring, void* v_ring, const int32_t* head, const int32_t* fill,
                            const float* pos_bias, const float* scale_embed, const float* head_gain,

@@ -105,3 +105,56 @@ def test_two_streams_that_join_eager_and_captured():
             graph.replay()
             torch.cuda.synchronize()
             assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+@pytest.mark.parametrize("D", [32, 64])
+@pytest.mark.parametrize("writer", ["step", "prefill"])
+def test_overlapped_steps_two_behind_a_kernel_that_writes_their_ring(writer, D):
+    """A writes a ring, an overlapped step on other rings follows, then an overlapped step on the ring that A wrote, its write heads known ahead:
+    the promise (the kernel just ahead writes none of them) is kept, so that step sees everything A wrote."""
+    S, H, N = 64, 8, 1800
+    offsets = dwarf_b200.OFFSETS_43
+    R = max(offsets) + 1
+    g = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").to(torch.bfloat16)  # noqa: E731
+    bias = torch.randn(len(offsets), H, generator=g, device="cuda") * 0.1
+    prefix, toks = (rnd(S, H, N, D), rnd(S, H, N, D)), [[rnd(S, H, D) for _ in range(3)] for _ in range(3)]
+    small = [t[:2].contiguous() for t in toks[1]]                    # the step in between: few blocks, over at once
+    heads = [torch.full((S,), (N + i) % R, dtype=torch.int32, device="cuda") for i in range(2)]
+    old = [rnd(S, H, R, 2, D), rnd(2, H, R, 2, D)]
+    caches = [dwarf_b200.DSQGRingCache(1, S, H, D), dwarf_b200.DSQGRingCache(1, 2, H, D)]
+    out = [torch.empty_like(toks[0][0]), torch.empty_like(small[0]), torch.empty_like(toks[2][0])]
+
+    def work(wait):
+        rings = [c.kv[0] for c in caches]
+        for ring, x in zip(rings, old):
+            ring.copy_(x)
+        wait()
+        step = lambda t, ring, head, o, overlap: dwarf_b200.dsqg_decode_step_kv(*t, ring, head, bias, offsets=offsets, out=o, overlap=overlap)  # noqa: E731
+        if writer == "step":
+            step(toks[0], rings[0], heads[0], out[0], False)
+        else:
+            caches[0].prefill(0, *prefix)
+        wait()
+        step(small, rings[1], heads[0][:2], out[1], True)
+        wait()
+        step(toks[2], rings[0], heads[1 if writer == "step" else 0], out[2], True)
+        wait()
+        return [*out[1:], *rings]
+
+    apart = [t.clone() for t in work(torch.cuda.synchronize)]
+    same = lambda got: all(torch.equal(a, b) for a, b in zip(apart, got))  # noqa: E731
+    for _ in range(20):
+        assert same(work(lambda: None))
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = work(lambda: None)
+        for _ in range(20):
+            for t in got:
+                t.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert same(got)
