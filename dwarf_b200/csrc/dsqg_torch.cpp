@@ -516,7 +516,16 @@ void weight_grads(const std::array<WeightGrad, 2>& jobs, int count, int64_t M, i
     for (int k = 0; k < count; ++k) {
         dy[k] = jobs[k].dy; x[k] = jobs[k].x; ld[k] = jobs[k].ld; cols[k] = (int)jobs[k].cols; dw[k] = jobs[k].dw; sums[k] = jobs[k].sums;
     }
-    check(dsqg_weight_grads(dy, ld, cols, x, dw, sums, count, M, (int)D, stream_of(on)), "dsqg_weight_grads");
+    const int status = dsqg_weight_grads(dy, ld, cols, x, dw, sums, count, M, (int)D, stream_of(on));
+    if (status != DSQG_ERR_UNSUPPORTED) return check(status, "dsqg_weight_grads");
+    // a driver that makes no tensor maps: GEMMs and column sums into the same places
+    const void* sp[2]; long long sld[2]; int sc[2]; float* to[2];
+    int n = 0;
+    for (int k = 0; k < count; ++k) {
+        gemm(dw[k], true, dy[k], true, x[k], false, nullptr, cols[k], D, M, on, ld[k] == cols[k] ? 0 : ld[k]);
+        if (sums[k]) { sp[n] = dy[k]; sld[n] = ld[k]; sc[n] = cols[k]; to[n] = sums[k]; ++n; }
+    }
+    if (n) check(dsqg_column_sums(sp, sld, sc, to, n, M, stream_of(on)), "dsqg_column_sums");
 }
 
 // fp32 tensors as bf16 back to back in one buffer, in one launch; at[k]: where the k-th begins (elements).

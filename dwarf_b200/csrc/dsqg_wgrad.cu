@@ -334,7 +334,7 @@ extern "C" int dsqg_weight_grads(const void* const* dy, const long long* dy_stri
         // 64-column blocks of a row-major matrix as the "heads" of a tensor of 64-wide rows
         if (!stg::make_map(&maps[2 * k], &a.job[k].a_hf, dy[k], 1, cols[k] / kBox, (int)rows, kBox, rows * dy_stride[k], kBox, dy_stride[k], kBox) ||
             !stg::make_map(&maps[2 * k + 1], &a.job[k].b_hf, x[k], 1, D / kBox, (int)rows, kBox, rows * D, kBox, D, kBox))
-            return DSQG_ERR_CUDA;
+            return DSQG_ERR_UNSUPPORTED;
     }
     if (count == 1) { maps[2] = maps[0]; maps[3] = maps[1]; }
     const Share p = choose(*fit, a, count);

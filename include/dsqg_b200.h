@@ -294,7 +294,7 @@ int dsqg_packed_bwd_gate(const dsqg_packed* p, const dsqg_packed_grads* g, const
  *   dsqg_column_sums     fp32 column sums of up to DSQG_SUM_MAX bf16 matrices of the same number of rows, fixed order
  *   dsqg_weight_grads    dw[k] [cols[k], D] = dy[k]^T . x[k] in fp32 and sums[k] [cols[k]] = column sums of dy[k] (null: left out) for
  *                        up to DSQG_WGRAD_MAX pairs of `rows` rows in one launch; dy rows dy_stride elements apart, x rows of D; D and
- *                        cols multiples of 64; fixed order of the sums
+ *                        cols multiples of 64; fixed order of the sums; DSQG_ERR_UNSUPPORTED where the driver makes no tensor map for them
  * D a multiple of 8 (layer norm: at most 1024); all pointers 16-byte aligned; src, dst, n, row_stride, cols: HOST arrays. */
 #define DSQG_CAST_MAX 8
 #define DSQG_SUM_MAX 4

@@ -333,3 +333,37 @@ def test_weight_gradients_of_a_layer_with_and_without_split_sums(dim, N):
         torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = was
     for a, b in zip(one, many):
         _close(a, b, 2e-3, "gradient")        # the projections' GEMMs may round other bf16 values when they may not split
+
+
+_NO_TENSOR_MAPS = """
+import ctypes, sys
+fake = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)         # ahead of the library's own symbol
+import torch
+from tests.test_gpu_layer import _layer_gradients
+torch.save([t.cpu() for t in _layer_gradients(128, 97)], sys.argv[2])
+assert fake.fake_calls() == 2
+"""
+
+
+def _layer_gradients(dim, N):
+    torch.manual_seed(dim)
+    with torch.device("cuda"):
+        attn, inject = dwarf_b200.DSQGAttentionQW(dim, dim // 32, seq_len=N, dropout=0.0), dwarf_b200.InterferenceInjection(dim, dim // 32)
+        x, dy = torch.randn(2, N, dim, requires_grad=True), torch.randn(2, N, dim).bfloat16()
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = attn(x, kv_inject=inject(x))
+    return torch.autograd.grad(y, [x, *attn.parameters(), *inject.parameters()], dy)
+
+
+def test_a_layer_without_tensor_maps_takes_its_gemms(tmp_path):
+    """Where the driver makes no tensor maps dsqg_weight_grads is refused, and the backward has GEMMs for the same gradients.  The refusal comes
+    from a stand-in for the entry that a child process loads first."""
+    import subprocess
+    import sys
+    from tests.conftest import ROOT
+    src, lib, out = tmp_path / "fake.c", tmp_path / "fake.so", tmp_path / "grads.pt"
+    src.write_text("static int calls; int dsqg_weight_grads(void) { ++calls; return -8; } int fake_calls(void) { return calls; }")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", str(lib), str(src)], check=True)
+    subprocess.run([sys.executable, "-c", _NO_TENSOR_MAPS, str(lib), str(out)], check=True, cwd=ROOT, timeout=300)
+    for a, b in zip(torch.load(out), _layer_gradients(128, 97)):
+        _close(a.cuda(), b, 2e-3, "gradient")         # the sums are formed in another order; one of them nearly cancels
