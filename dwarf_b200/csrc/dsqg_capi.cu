@@ -80,6 +80,8 @@ const char* dsqg_status_str(int status) {
         case DSQG_ERR_STATIC_SCRATCH_EXCEEDED:
             return "dsqg_bwd_static: this problem needs more scratch than the built-in DSQG_STATIC_SCRATCH_BYTES; "
                    "use dsqg_bwd with a caller-allocated buffer";
+        case DSQG_ERR_WAIT:
+            return "a bounded wait inside a kernel of an earlier call gave up: that call's results are NaN (dsqg_device_error(1) says where and clears this)";
         default: return "unknown status";
     }
 }

@@ -146,6 +146,10 @@ bool staged_supported(int dtype, int D, const Taps& t, bool has_scale_embed);
 cudaError_t launch_fwd_staged(const FwdArgs& a, const Taps& t, cudaStream_t s);
 cudaError_t read_stage_error(int* value, bool reset);
 cudaError_t launch_wait_timeout(long long limit_cycles, int site, cudaStream_t s);
+// The current device's word in host memory (dsqg_dispatch.cu), where a bounded wait that gives up can be seen without a synchronisation:
+// for kernels (null where there is none), and what it holds.
+int* wait_error_word();
+int wait_error_seen();
 // forward with the dense window on tcgen05 tensor cores and tensor memory (dsqg_umma.cu)
 bool umma_supported(int dtype, int D, const Taps& t, bool has_scale_embed);
 cudaError_t launch_fwd_umma(const FwdArgs& a, const Taps& t, cudaStream_t s);

@@ -3,6 +3,7 @@
 // other head sizes, dense windows wider than the tensor-core kernels are built for).  One
 // decision per call, made on the host from the shape alone.
 #include <atomic>
+#include <mutex>
 
 #include "dsqg_common.cuh"
 
@@ -13,6 +14,7 @@ namespace dsqg {
 // (dsqg_staged.cu; not chosen automatically: it measures slower on B200), 4 = the forward with the
 // dense window on tcgen05 / tensor memory wherever it applies (dsqg_umma.cu; not chosen automatically).
 static std::atomic<int> g_path{0};
+constexpr int kErrorDevices = 64;
 
 // Where the tcgen05 forward is taken instead of the register-fed one: 128-byte rows (D = 64), no sparse taps, at least two
 // 128-row tiles for each SM's persistent block.  The line was drawn when the register-fed kernel took 56.1 us at 3,072 tiles (tcgen05 49).  It is
@@ -41,6 +43,44 @@ cudaError_t launch_bwd(const BwdArgs& a, const Taps& t, int dtype, cudaStream_t 
     return launch_bwd_generic(a, t, dtype, s, stages);
 }
 
+// One page of page-locked host memory, asked for once (also while a stream is being captured: no stream takes part in it).
+static int* error_words() {
+    static std::mutex mu;
+    static int* words = nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!words) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, kErrorDevices * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            words = static_cast<int*>(p);
+            for (int i = 0; i < kErrorDevices; ++i) words[i] = 0;
+        } else {
+            cudaGetLastError();
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    return words;
+}
+static int* host_word() {
+    int dev = 0;
+    int* words = error_words();
+    return words && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kErrorDevices ? words + dev : nullptr;
+}
+int* wait_error_word() {
+    void* p = nullptr;
+    int* w = host_word();
+    return w && cudaHostGetDevicePointer(&p, w, 0) == cudaSuccess ? static_cast<int*>(p) : nullptr;
+}
+int wait_error_seen() {
+    const volatile int* w = host_word();
+    return w ? *w : 0;
+}
+static void clear_wait_error() {
+    volatile int* w = host_word();
+    if (w) *w = 0;
+}
+
 }  // namespace dsqg
 
 extern "C" int dsqg_set_kernel_path(int path) {
@@ -51,9 +91,11 @@ extern "C" int dsqg_set_kernel_path(int path) {
 
 extern "C" int dsqg_device_error(int reset) {
     int v = 0, w = 0, g = 0;
+    if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return -1; }
     if (dsqg::read_stage_error(&v, reset != 0) != cudaSuccess) return -1;
     if (dsqg::read_umma_error(&w, reset != 0) != cudaSuccess) return -1;
     if (dsqg::read_wgrad_error(&g, reset != 0) != cudaSuccess) return -1;
+    if (reset) dsqg::clear_wait_error();
     return v ? v : w ? w : g;
 }
 

@@ -147,9 +147,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 static __device__ int g_stage_error = 0;
 
 // Bounded wait.  `abort_flag` lives in shared memory; once set, every wait of the block returns
-// at once, so the kernel ends instead of hanging.  Returns false when the wait gave up.
+// at once, so the kernel ends instead of hanging.  Returns false when the wait gave up; `report`
+// (nullable) is a word in host memory that is told as well (wait_error_word).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int site,
-                                          long long limit = kWaitCycleLimit) {
+                                          long long limit = kWaitCycleLimit, int* report = nullptr) {
     if (mbar_try_wait(bar, parity)) return true;
     const long long t0 = clock64();
     for (uint32_t it = 0;; ++it) {
@@ -162,6 +163,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
     *abort_flag = 1;
     atomicCAS(&g_stage_error, 0, site);
+    if (report) {
+        *reinterpret_cast<volatile int*>(report) = site;
+        __threadfence_system();
+    }
     return false;
 }
 

@@ -334,16 +334,16 @@ fwd_staged_kernel(const FwdArgs a, const Taps t, const Plan pl, const Maps mf,
 }
 
 // One thread waits on a barrier that nothing ever signals, with the given cycle limit: the wait
-// gives up, records `site` in the error word and the kernel returns.  Used by the test of the
+// gives up, records `site` in the error words and the kernel returns.  Used by the test of the
 // bounded-wait path; no copy is in flight, nothing can hang.
-__global__ void wait_timeout_kernel(long long limit_cycles, int site) {
+__global__ void wait_timeout_kernel(long long limit_cycles, int site, int* report) {
     __shared__ __align__(8) unsigned long long bar;
     __shared__ int abort_flag;
     const uint32_t b = smem_u32(&bar);
     mbar_init(b, 1);
     abort_flag = 0;
     fence_mbar_init();
-    mbar_wait(b, 0, &abort_flag, site, limit_cycles);
+    mbar_wait(b, 0, &abort_flag, site, limit_cycles, report);
 }
 
 // ------------------------------------------------------------------------------ host side
@@ -440,7 +440,7 @@ cudaError_t launch_fwd_staged(const FwdArgs& a, const Taps& t, cudaStream_t s) {
 }
 
 cudaError_t launch_wait_timeout(long long limit_cycles, int site, cudaStream_t s) {
-    stg::wait_timeout_kernel<<<1, 1, 0, s>>>(limit_cycles, site);
+    stg::wait_timeout_kernel<<<1, 1, 0, s>>>(limit_cycles, site, wait_error_word());
     return cudaGetLastError();
 }
 

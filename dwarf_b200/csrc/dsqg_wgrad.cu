@@ -11,7 +11,8 @@
 // tile while the tensor cores work on it, which costs no second pass over dY.
 //   warp 4 (one lane): copies (cp.async.bulk.tensor, four or six stages of 64 rows)    warp 5 (one lane): tcgen05.mma, M 128, N 128 or 256
 //   warps 0-3: column sums, then accumulators -> shared memory (over the stages)    all: a share of the cluster's sum -> dW
-// Every wait is bounded (stg::mbar_wait); a block that gives up writes NaN and sets the device error word.
+// Every wait is bounded (stg::mbar_wait); a block that gives up writes NaN and sets the device error word and the one in host memory, which
+// the next call looks at.
 //
 // Bound by what an SM can fetch (90 GB/s a block measured, from L2 or HBM; all 148 together would outrun HBM): [1024, 256] + [256, 256]
 // gradients with their sums, against two library GEMMs and a pass for the sums: 4,096 rows 11.0 us : 18.5, 16,384 23.1 : 49.5, 65,536
@@ -56,7 +57,7 @@ struct Layout {
 
 static_assert(DSQG_WGRAD_MAX == 2, "two jobs, four tensor maps");
 struct Job { int cols, tiles_end; float* dw; float* sum; bool a_hf, b_hf; };
-struct Args { Job job[DSQG_WGRAD_MAX]; int rows, D, split; };
+struct Args { Job job[DSQG_WGRAD_MAX]; int rows, D, split; int* report; };
 
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
     uint32_t there;
@@ -129,7 +130,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             int i = 0;
             for (; i < count; ++i) {
                 const int st = i % kStages;
-                if (i >= kStages && !mbar_wait(bars + 8 * (kEmpty + st), (i / kStages - 1) & 1, abort_flag, 0x501, kLimit)) break;
+                if (i >= kStages && !mbar_wait(bars + 8 * (kEmpty + st), (i / kStages - 1) & 1, abort_flag, 0x501, kLimit, a.report)) break;
                 const uint32_t bar = bars + 8 * (kFull + st), dst = sb + st * kStageBytes;
                 const int row = (first + i) * kBox;
                 mbar_arrive_expect_tx(bar, kStageBytes);               // boxes outside a matrix arrive as zeros
@@ -141,7 +142,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             // after an abort: no copy of this block may be in flight when its shared memory is released
             if (*abort_flag) {
                 volatile int keep_waiting = 0;
-                for (int k = i > kStages ? i - kStages : 0; k < i; ++k) mbar_wait(bars + 8 * (kFull + k % kStages), (k / kStages) & 1, &keep_waiting, 0x504, kLimit);
+                for (int k = i > kStages ? i - kStages : 0; k < i; ++k) mbar_wait(bars + 8 * (kFull + k % kStages), (k / kStages) & 1, &keep_waiting, 0x504, kLimit, a.report);
             }
         }
         __syncwarp();
@@ -150,7 +151,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             const uint64_t desc0 = mn_desc(sb);
             for (int i = 0; i < count; ++i) {
                 const int st = i % kStages;
-                if (!mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x502, kLimit)) break;
+                if (!mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x502, kLimit, a.report)) break;
                 tc_fence_after();
                 const uint64_t da = desc0 + (uint32_t)(st * kStageBytes >> 4), db = da + (uint32_t)(kABytes >> 4);
 #pragma unroll
@@ -170,7 +171,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int i = 0; i < count; ++i) {
                 const int st = i % kStages;
-                if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x503, kLimit))) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x503, kLimit, a.report))) break;
                 uint4 u[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
@@ -194,7 +195,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             csum[8 * kTM + tid] = t;
         }
         // accumulator row = tensor-memory lane = tid; the stages are free once every product has completed
-        const bool ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * kDone, 0, abort_flag, 0x505, kLimit) && !*abort_flag);
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * kDone, 0, abort_flag, 0x505, kLimit, a.report) && !*abort_flag);
         tc_fence_after();
         float* part = reinterpret_cast<float*>(smem) + tid * kPitch;
         const uint32_t acc = tmem + ((uint32_t)(32 * warp) << 16);
@@ -337,6 +338,8 @@ extern "C" int dsqg_weight_grads(const void* const* dy, const long long* dy_stri
             return DSQG_ERR_UNSUPPORTED;
     }
     if (count == 1) { maps[2] = maps[0]; maps[3] = maps[1]; }
+    if (wait_error_seen()) return DSQG_ERR_WAIT;
+    a.report = wait_error_word();
     const Share p = choose(*fit, a, count);
     a.split = p.split;
     int tiles = 0;

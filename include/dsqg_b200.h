@@ -16,9 +16,10 @@
  *   - offsets: HOST pointer to J int32 values, strictly ascending, >= 0.  The leading run
  *     of consecutive integers is treated as the dense window, the rest as sparse taps.
  *   - stream: a cudaStream_t passed as void* (NULL = legacy default stream).
- *   - The caller owns every buffer; the library allocates nothing.  The only state it keeps
- *     between calls is named where it is declared: the kernel-path knob
- *     (dsqg_set_kernel_path), the device error word (dsqg_device_error), the built-in scratch
+ *   - The caller owns every buffer; the library allocates no device memory.  The only state it
+ *     keeps between calls is named where it is declared: the kernel-path knob
+ *     (dsqg_set_kernel_path), the error words (dsqg_device_error; one page of page-locked host
+ *     memory, asked for by the first dsqg_weight_grads), the built-in scratch
  *     of dsqg_bwd_static with its per-device address cache, and per-kernel "attribute set"
  *     flags.  The caller makes the device current (cudaSetDevice) before calling.
  *   - Every function returns DSQG_OK (0) or a negative dsqg_status; nothing throws, traps
@@ -47,7 +48,8 @@ typedef enum {
     DSQG_ERR_SCRATCH_TOO_SMALL = -6,
     DSQG_ERR_CUDA = -7,           /* a CUDA runtime/driver call failed (see dsqg_last_cuda_error) */
     DSQG_ERR_UNSUPPORTED = -8,    /* valid request that this build has no kernel for */
-    DSQG_ERR_STATIC_SCRATCH_EXCEEDED = -9  /* dsqg_bwd_static: problem needs more than DSQG_STATIC_SCRATCH_BYTES */
+    DSQG_ERR_STATIC_SCRATCH_EXCEEDED = -9,  /* dsqg_bwd_static: problem needs more than DSQG_STATIC_SCRATCH_BYTES */
+    DSQG_ERR_WAIT = -10           /* dsqg_weight_grads: a wait in an earlier call on this device gave up (see dsqg_device_error) */
 } dsqg_status;
 
 enum { DSQG_DTYPE_BF16 = 0, DSQG_DTYPE_F32 = 1 };
@@ -72,16 +74,18 @@ int dsqg_version(void);
 int dsqg_set_kernel_path(int path);
 
 /* Device-side error word of the current device (no counterpart in the reference).  The
- * kernels that wait on shared-memory barriers for the copy engine or the tensor cores (kernel paths 3 and 4) bound every
- * such wait; a wait that runs out records its site id here and the kernel returns with
- * unspecified output instead of hanging.  0 = no error, -1 = the word could not be read.
- * Synchronises the device.  reset != 0 clears the word after reading. */
+ * kernels that wait on shared-memory barriers for the copy engine or the tensor cores (kernel paths 3
+ * and 4, dsqg_weight_grads) bound every such wait; a wait that runs out records its site id here and
+ * the kernel returns with unspecified output (dsqg_weight_grads: NaN) instead of hanging.  0 = no
+ * error, -1 = the word could not be read.  Synchronises the device.  reset != 0 clears the word after reading.
+ * dsqg_weight_grads also sees it without being asked: once a wait of its kernel has given up on the
+ * current device, later calls launch nothing and return DSQG_ERR_WAIT until the word is cleared. */
 int dsqg_device_error(int reset);
 
 /* Test hook for the bounded wait (no counterpart in the reference): launches one thread that
  * waits, for at most limit_cycles SM cycles (1 .. 2e9), on a barrier nothing signals.  The wait
- * gives up, dsqg_device_error() then reports site 0x7e57, and the kernel returns: nothing is
- * in flight, nothing hangs or faults. */
+ * gives up, dsqg_device_error() then reports site 0x7e57 (and dsqg_weight_grads DSQG_ERR_WAIT), and
+ * the kernel returns: nothing is in flight, nothing hangs or faults. */
 int dsqg_test_wait_timeout(long long limit_cycles, void* stream);
 
 /* Forward.

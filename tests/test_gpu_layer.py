@@ -367,3 +367,17 @@ def test_a_layer_without_tensor_maps_takes_its_gemms(tmp_path):
     subprocess.run([sys.executable, "-c", _NO_TENSOR_MAPS, str(lib), str(out)], check=True, cwd=ROOT, timeout=300)
     for a, b in zip(torch.load(out), _layer_gradients(128, 97)):
         _close(a.cuda(), b, 2e-3, "gradient")         # the sums are formed in another order; one of them nearly cancels
+
+
+def test_a_wait_that_gave_up_is_reported_by_the_next_backward():
+    """Gradients of a kernel whose wait ran out are NaN; whoever goes on training on them hears of it, and can go on once the word is cleared."""
+    lib = _lib.load()
+    want = _layer_gradients(128, 97)
+    assert lib.dsqg_device_error(1) == 0
+    _lib.check(lib.dsqg_test_wait_timeout(20000, _stream()), "wait")
+    torch.cuda.synchronize()
+    for _ in range(2):                                               # until it is cleared
+        with pytest.raises(_lib.DSQGError, match="status -10: .* gave up"):
+            _layer_gradients(128, 97)
+    assert lib.dsqg_device_error(1) == 0x7e57 and lib.dsqg_device_error(0) == 0
+    assert all(torch.equal(a, b) for a, b in zip(want, _layer_gradients(128, 97)))
