@@ -68,7 +68,7 @@ struct BwdArgs {
     // rows and writes dout (out_* strides) for the dK/dV kernel; y is out, the gated result, laid out like dy.
     const void* dy; const void* y; const void* gate; void* dgate;
     dsqg_strides y_st, gate_st, dgate_st;
-    // Strided only: q, k, v and dout are contiguous [B,H,N,D] all the same (in_* then addresses dq, dk, dv only; needs delta_pre).
+    // Strided only, with a gate: q, k, v and dout are contiguous [B,H,N,D] all the same (in_* then addresses dq, dk, dv only).
     int kept;
 };
 
@@ -83,13 +83,14 @@ struct DecodeArgs {
     int ring_stride;   // elements between two slots of a ring: D for separate K and V rings [S,H,R,D], 2 D for one ring [S,H,R,2,D]
 };
 
-// Programmatic dependent launch, for every kernel of the library: its blocks are scheduled as the last blocks of the kernel ahead of it in the stream leave,
+// Programmatic dependent launch, for every kernel of the library but the forwards with copy-engine staging (dsqg_staged.cu, dsqg_umma.cu: plain launches): its blocks are scheduled as the last blocks of the kernel ahead of it in the stream leave,
 // instead of after that kernel's completion has been noticed.  stream_wait comes first in the kernel, so nothing of it runs before the results of
 // what is ahead are visible: order and results are those of a plain launch.  It lets the next kernel's blocks come only once it has waited
 // itself: a decode step that reads ahead of its own wait (dsqg_decode_overlapped) then finds everything but the kernel ahead of it finished.  That
 // step keeps to it too: it reads early, but hands over after its wait like the others.
-// Worth 1.5 to 2 us a launch, passes of one kind in a row, us: 2x8x777x32 forward and backward 28.8 -> 23.4, 8x8x1000x32 44.3 -> 39.4, 8x8x2048x80
-// 168.2 -> 164.5, 32x8x2048x32 243.2 -> 236.8, fp32 forward 2x8x2048x32 20.6 -> 19.2, 1x8x300x32 8.3 -> 6.0.
+// Worth 1.5 to 2 us a launch where kernels follow one another without a gap; us, passes of one kind in a row: 2x8x777x32 forward and backward on the GPU
+// 28.8 -> 23.4, 8x8x1000x32 44.3 -> 39.4, 8x8x2048x80 168.2 -> 164.5, 32x8x2048x32 243.2 -> 236.8, fp32 forward 2x8x2048x32 20.5 -> 18.9.  Behind a gap, on
+// inputs that have just been made for instance, there is nothing to gain.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_after(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
     cudaLaunchAttribute at;

@@ -12,15 +12,15 @@ namespace dsqg {
 // 0 = automatic, 1 = always the generic kernels, 2 = the register-fed tensor-core kernels (what the
 // automatic choice uses where they apply, except for the one case in umma_pays()), 3 = the forward with TMA-staged V wherever it applies
 // (dsqg_staged.cu; not chosen automatically: it measures slower on B200), 4 = the forward with the
-// dense window on tcgen05 / tensor memory wherever it applies (dsqg_umma.cu; not chosen automatically).
+// dense window on tcgen05 / tensor memory wherever it applies (dsqg_umma.cu; chosen automatically in the case of umma_pays() only).
 static std::atomic<int> g_path{0};
 constexpr int kErrorDevices = 64;
 
 // Where the tcgen05 forward is taken instead of the register-fed one: 128-byte rows (D = 64), no sparse taps, at least two
-// 128-row tiles for each SM's persistent block.  The line was drawn when the register-fed kernel took 56.1 us at 3,072 tiles (tcgen05 49).  It is
-// ahead at every size now (offsets 0..31, L2 cold, tcgen05 / register-fed: 6,144 tiles (16x12x4096) 85.0 / 78.8 us, 3,072 tiles 50.2 / 46.1,
-// 1,536 tiles 31.7 / 27.6, 768 tiles 21.5 / 19.5, 320 tiles 15.4 / 13.3); the line stays because which kernel's bits a call returns is stated to
-// callers (dsqg_b200.h).
+// 128-row tiles for each SM's persistent block.  The line was drawn when the register-fed kernel took 56.1 us at 3,072 tiles (tcgen05 49).  It no longer
+// stands for speed: the register-fed kernel is 8 to 15 % ahead at every size now (offsets 0..31, L2 cold, tcgen05 / register-fed: 6,144 tiles (16x12x4096)
+// 85.0 / 78.8 us, 3,072 tiles 50.2 / 46.1, 1,536 tiles 31.7 / 27.6, 768 tiles 21.5 / 19.5, 320 tiles 15.4 / 13.3).  Moving it changes which kernel's bits
+// these calls return (dsqg_b200.h says which), and that is all that keeps it.
 static bool umma_pays(const FwdArgs& a, const Taps& t, int dtype) {
     return a.D == 64 && t.n_sparse == 0 && !a.strided &&
            (long long)a.B * a.H * ((a.N + 127) / 128) >= 2 * 148 && umma_supported(dtype, a.D, t, a.scale_embed != nullptr);

@@ -34,7 +34,6 @@ __device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<f
 __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
     *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
 }
-__device__ __forceinline__ float dot4(float4 a, float4 b, float c) { return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, c)))); }
 
 // Forward.  LPR lanes hold a row, four elements each; a lane group owns kFwdRows consecutive query rows and
 // takes the taps eight at a time (online softmax over the chunks).  What bounds it is the L1 data path, the

@@ -437,6 +437,9 @@ __device__ __forceinline__ void fwd_tile(const FwdArgs& a, const float* start, c
 template <int D> struct FwdTune {
     // Since a tap's address is one uniform product (Rows), registers allow more CTAs: D = 32 two taps, 7 CTAs (72 registers) 60.4 us at 32x8x2048,
     // 6 CTAs 64.1, 5 CTAs 66.8 (65.5 before); D = 64 79.7 us at 16x12x2048 (one tap 87.8, 5 CTAs 86.2; 92.4 before).
+    // Swept on contiguous tensors only.  The strided and 16-byte instantiations take the same constants, although their 64-bit lane parts (Rows) need more
+    // registers; bytes spilled (stores / loads), contiguous, strided, 16-byte: D = 32 32/32, 60/64, -; D = 64 0/0, 16/16, 48/48; with scale_embed D = 32
+    // 0/0, 20/28, -; D = 64 12/20, 8/8, 24/28.  Packed forward with gate 32x8x2048x32 107 us.
     static constexpr int warps = 4, group = D > 96 ? 1 : 2, ctas = D == 32 ? 7 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));
     // With scale_embed a CTA first lays out the table, about a quarter of a tile's time, so a warp does up to three tiles with it.
     // The count is the one for which (waves of CTAs) x (tiles + 1/4) is least: one where the grid is a single wave (2x8x777x32 11.6 us,
@@ -491,12 +494,16 @@ fwd_mma_kernel(const FwdArgs a, const Taps t, const int tiles_se) {
 // resident CTAs per SM the register budget is set for (spills against warps in flight).
 template <int D> struct BwdTune {
     // 8x8x2048 unless said otherwise, us: D = 32 at 32x8x2048 89.7 (6 CTAs 90.6, one tap and 6 CTAs 91.0, 4 CTAs 96.7), D = 64 at 16x12x2048
-    // 114.9 (two taps 119.7), D = 80 59.8 (one tap 60.3), D = 96 66.0 (two taps 69.6, 2 CTAs 71.7-78.0), D = 128 84.5 (one tap 89.9)
+    // 114.9 (two taps 119.7), D = 80 59.8 (one tap 60.3), D = 96 66.0 (two taps 69.6, 2 CTAs 71.7-78.0), D = 128 84.5 (one tap 89.9).
+    // All figures here are of contiguous tensors; the other instantiations take the same constants unswept (see FwdTune).  Bytes spilled (stores / loads),
+    // contiguous, strided, 16-byte: dQ D = 32 48/52, 28/48, - (kept 48/52); D = 64 60/60, 100/124, 96/128; D = 96 12/12, 60/68, 68/76; with scale_embed
+    // D = 64 28/40, 160/176, 104/124; dK/dV D = 64 16/16, 48/48, 20/20.  Packed backward with gate, us: 32x8x2048x32 191, 16x12x2048x64 297, 8x8x2048x128 248.5.
     static constexpr int dq_group = D == 64 || D == 96 ? 1 : 2, dq_ctas = D == 32 ? 5 : (D <= 64 ? 4 : (D <= 96 ? 3 : 2));
     // scale_embed: 32x8x2048x32 154.9 (5 CTAs 155.1, one tap 158-164), 16x12x2048x64 202.6 (one tap 208.6, 3 CTAs 205-212)
     static constexpr int dq_group_se = 2, dq_ctas_se = 4;
     // D = 32 at 32x8x2048 94.2 (4 CTAs 98.1, 6 CTAs 110-115), D = 64 at 16x12x2048 132.4 (two taps 134.9), D = 48 44.3, D = 80 69.0 (one tap 73.8,
-    // 3 CTAs 82), D = 96 78.8 (one tap 82.1), D = 128 116.0 (two taps 125.2)
+    // 3 CTAs 82), D = 96 78.8 (one tap 82.1), D = 128 116.0 (two taps 125.2; two 16 x 128 accumulators and four row fragments do not fit 255
+    // registers: 900 bytes spilled and 896 read back a thread, strided 1,144 / 1,152)
     static constexpr int dkdv_group = D == 64 ? 3 : (D > 96 ? 1 : 2), dkdv_ctas = D == 32 ? 5 : (D <= 64 ? 3 : 2);
     // scale_embed: 32x8x2048x32 129.1 (one tap 128.9, 4 CTAs 133.3), 16x12x2048x64 185.0 (two taps 187.1, 4 CTAs 238)
     static constexpr int dkdv_group_se = D == 32 ? 2 : 1, dkdv_ctas_se = D == 32 ? 5 : 3;
@@ -1297,7 +1304,6 @@ cudaError_t fwd_launch_mma(const FwdArgs& a, const Taps& t, cudaStream_t s) {
 template <int D, int WB, bool SE, int ST>
 cudaError_t bwd_launch_mode(BwdArgs a, const Taps& t, cudaStream_t s, int stages) {
     using T = BwdTune<D>;
-    constexpr int NT = (WB + 16) / 8;
     if constexpr (SE) carve_bwd_scratch_mma_se(a, t.J); else carve_bwd_scratch(a, kRows, t.J, false);
     dim3 grid((a.N + kRows - 1) / kRows, a.B * a.H);
     cudaError_t e = cudaSuccess;
@@ -1335,6 +1341,8 @@ cudaError_t bwd_launch_mode(BwdArgs a, const Taps& t, cudaStream_t s, int stages
 
 template <int D, int WB, bool SE>
 cudaError_t bwd_launch_se(BwdArgs a, const Taps& t, cudaStream_t s, int stages) {
+    // A gate that starts on 16 bytes only takes both kernels along: packed backward 16x12x2048x64 326.5 us against 297.0 (337.6 wherever it started when it
+    // had a kernel of its own ahead of these), 8x8x2048x128 267.7 against 248.5 (267.4).
     if constexpr (kLane<D> == 16) {       // 32-byte pieces
         if (!aligned_to(32, {a.q, a.k, a.v, a.out, a.dout, a.dq, a.dk, a.dv, a.dy, a.y, a.gate, a.dgate}, {a.in_sb, a.in_sh, a.in_sn, a.out_sb, a.out_sh, a.out_sn}) ||
             (a.gate && !aligned_to(32, {}, {a.y_st.batch, a.y_st.head, a.y_st.row, a.gate_st.batch, a.gate_st.head, a.gate_st.row, a.dgate_st.batch, a.dgate_st.head, a.dgate_st.row}))) {

@@ -505,7 +505,9 @@ Tensor grad_weight(const Tensor& dY, const Tensor& X, int64_t M, int64_t N, int6
 // column sums.  Both sides of the line, us (M rows, two products [4 D, D] and [D, D]): D 256: M 1,024 7.6 against 9.8, 16,384 23.1 : 49.5,
 // 65,536 70 : 107; D 128: 6.4 : 9.5, 18.4 : 39.9, 55.5 : 83.  Its error against 64 bits is at most the GEMMs', mostly a half to a sixth of it.  At D 512
 // 16,384 rows it still wins (51 : 73), but not at 384 (125 : 121 with [2 D, D] and 65,536 rows), and above 512 it loses: more tiles than clusters that
-// run at once.  Beyond 65,536 rows its sums are longer than the GEMMs' and their error larger.  The sums are split, so a caller who rules splits
+// run at once.  The limit of 65,536 rows is one of precision: a block's chain of running sums grows with the rows.  Relative error against 64 bits, this
+// kernel : GEMMs, D 256: 65,536 rows 1.2e-5 : 1.9e-5, 131,072 2.5e-5 : 1.8e-5, 262,144 5.0e-5 : 3.6e-5 (D 128 9.1e-6 : 1.7e-5, 1.9e-5 : 1.8e-5, 3.8e-5 : 3.1e-5; D 192
+// 1.2e-5 : 1.2e-5, 2.5e-5 : 2.2e-5, 5.0e-5 : 3.2e-5), although it would be faster there too: 131,072 rows 132 us : 94 + 90 for the sums, 262,144 273 : 177 + 200.  The sums are split, so a caller who rules splits
 // out (reduction_schemes) gets the GEMMs.
 bool one_launch_weight_grads(int64_t M, int64_t D) {
     return D >= 128 && D <= 256 && D % 64 == 0 && M <= 65536 && reduction_schemes() != CUBLASLT_REDUCTION_SCHEME_NONE;

@@ -148,7 +148,7 @@ def test_what_the_path_does_not_take_falls_through_to_the_default_kernels():
         assert torch.equal(out4, out0) and torch.equal(lse4, lse0)
 
 
-def test_the_automatic_choice_takes_the_tcgen05_forward_where_it_measures_faster():
+def test_the_automatic_choice_takes_the_tcgen05_forward_from_296_tiles_on():
     """D = 64, no sparse taps, at least 296 tiles of 128 rows: the bits of kernel path 4, not of the
     register-fed kernel; a smaller problem of the same kind stays on the register-fed kernel."""
     dev = torch.device("cuda", 0)
