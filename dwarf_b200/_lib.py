@@ -78,6 +78,8 @@ _SIGNATURES = {
                                  ctypes.c_longlong, c_void_p]),
     "dsqg_weight_grads": (c_int, [POINTER(c_void_p), POINTER(ctypes.c_longlong), POINTER(c_int)] + [POINTER(c_void_p)] * 3
                           + [c_int, ctypes.c_longlong, c_int, c_void_p]),
+    "dsqg_test_weight_grads_timeout": (c_int, [POINTER(c_void_p), POINTER(ctypes.c_longlong), POINTER(c_int)] + [POINTER(c_void_p)] * 3
+                                       + [c_int, ctypes.c_longlong, c_int, ctypes.c_longlong, c_void_p]),
     "dsqg_causal_mean": (c_int, [c_void_p, c_void_p] + [c_int] * 5 + [c_void_p]),
     "dsqg_decode_kv": (c_int, [c_void_p] * 3 + [c_void_p] + [c_void_p] * 2 + [c_void_p] * 3
                        + [POINTER(c_int32), c_int, c_int] + [c_void_p] + [c_int] * 4 + [c_void_p, c_int]),

@@ -4,15 +4,15 @@
 // Reference math: nn.Linear's backward for the projections of DWARF train/train_2048_condU.py:171-191, :277-295.
 //
 // The outputs are small (256 x 256 to 1024 x 256) and the contraction is long (batch x sequence), so the contraction is what
-// is split: a cluster of up to eight blocks shares one 128 x 256 tile of dW, each block takes a range of rows of dY and X and
+// is split: a cluster of up to eight blocks shares one 128 x 128 or 128 x 256 tile of dW, each block takes a range of rows of dY and X and
 // the fp32 partial tiles are added over distributed shared memory, block 0's first: fixed order, no scratch, no second pass.
 // Both operands lie with the contraction as their slow dimension; they are staged as 64-row boxes of 64 columns (128 bytes, one
 // swizzle atom) and enter tcgen05.mma as MN-major tiles, so nothing is transposed.  Warps 0-3 add dY's columns from the staged
 // tile while the tensor cores work on it, which costs no second pass over dY.
 //   warp 4 (one lane): copies (cp.async.bulk.tensor, four or six stages of 64 rows)    warp 5 (one lane): tcgen05.mma, M 128, N 128 or 256
 //   warps 0-3: column sums, then accumulators -> shared memory (over the stages)    all: a share of the cluster's sum -> dW
-// Every wait is bounded (stg::mbar_wait); a block that gives up writes NaN and sets the device error word and the one in host memory, which
-// the next call looks at.
+// Every wait is bounded (stg::mbar_wait).  A block that gives up sets the device error word and the one in host memory, which the next call
+// looks at, and its cluster writes NaN to its part of dW and of the sums; copies and products in flight are waited for all the same.
 //
 // Bound by what an SM can fetch (90 GB/s a block measured, from L2 or HBM; all 148 together would outrun HBM): [1024, 256] + [256, 256]
 // gradients with their sums, against two library GEMMs and a pass for the sums: 4,096 rows 11.0 us : 18.5, 16,384 23.1 : 49.5, 65,536
@@ -57,7 +57,7 @@ struct Layout {
 
 static_assert(DSQG_WGRAD_MAX == 2, "two jobs, four tensor maps");
 struct Job { int cols, tiles_end; float* dw; float* sum; bool a_hf, b_hf; };
-struct Args { Job job[DSQG_WGRAD_MAX]; int rows, D, split; int* report; };
+struct Args { Job job[DSQG_WGRAD_MAX]; int rows, D, split; int* report; long long limit; };       // limit: cycles before a wait gives up
 
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
     uint32_t there;
@@ -74,6 +74,11 @@ __device__ __forceinline__ float cluster_load(uint32_t addr) {
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
     return v;
 }
+__device__ __forceinline__ int cluster_load_int(uint32_t addr) {
+    int v;
+    asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -81,7 +86,8 @@ __device__ __forceinline__ void cluster_sync() {
 __device__ __forceinline__ uint64_t mn_desc(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(kBoxBytes >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-template <int TN>
+// STALL: the last block of every cluster never asks for the second half of its rows, so that waits run out (dsqg_test_weight_grads_timeout).
+template <int TN, bool STALL = false>
 __global__ void __launch_bounds__(kThreads, 1)
 weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CUtensorMap map_b0,
                    const __grid_constant__ CUtensorMap map_a1, const __grid_constant__ CUtensorMap map_b1) {
@@ -127,10 +133,11 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
     if (warp == kCopyWarp) {
         if (lane == 0) {
             const Tma ta = {j ? &map_a1 : &map_a0, job.a_hf}, tb = {j ? &map_b1 : &map_b0, job.b_hf};
+            const int copies = STALL && rank == a.split - 1 ? count / 2 : count;
             int i = 0;
-            for (; i < count; ++i) {
+            for (; i < copies; ++i) {
                 const int st = i % kStages;
-                if (i >= kStages && !mbar_wait(bars + 8 * (kEmpty + st), (i / kStages - 1) & 1, abort_flag, 0x501, kLimit, a.report)) break;
+                if (i >= kStages && !mbar_wait(bars + 8 * (kEmpty + st), (i / kStages - 1) & 1, abort_flag, 0x501, a.limit, a.report)) break;
                 const uint32_t bar = bars + 8 * (kFull + st), dst = sb + st * kStageBytes;
                 const int row = (first + i) * kBox;
                 mbar_arrive_expect_tx(bar, kStageBytes);               // boxes outside a matrix arrive as zeros
@@ -139,11 +146,9 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
 #pragma unroll
                 for (int b = 0; b < TN / kBox; ++b) tb.load(dst + kABytes + b * kBoxBytes, bar, row, k0 / kBox + b, 0);
             }
-            // after an abort: no copy of this block may be in flight when its shared memory is released
-            if (*abort_flag) {
-                volatile int keep_waiting = 0;
-                for (int k = i > kStages ? i - kStages : 0; k < i; ++k) mbar_wait(bars + 8 * (kFull + k % kStages), (k / kStages) & 1, &keep_waiting, 0x504, kLimit, a.report);
-            }
+            // no copy may be in flight when the shared memory is released, whoever gave up and when: a flag of its own
+            volatile int keep_waiting = 0;
+            for (int k = i > kStages ? i - kStages : 0; k < i; ++k) mbar_wait(bars + 8 * (kFull + k % kStages), (k / kStages) & 1, &keep_waiting, 0x504, kLimit, a.report);
         }
         __syncwarp();
     } else if (warp == kMmaWarp) {
@@ -151,7 +156,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             const uint64_t desc0 = mn_desc(sb);
             for (int i = 0; i < count; ++i) {
                 const int st = i % kStages;
-                if (!mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x502, kLimit, a.report)) break;
+                if (!mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x502, a.limit, a.report)) break;
                 tc_fence_after();
                 const uint64_t da = desc0 + (uint32_t)(st * kStageBytes >> 4), db = da + (uint32_t)(kABytes >> 4);
 #pragma unroll
@@ -160,6 +165,8 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
                 umma_commit(bars + 8 * (kEmpty + st));
             }
             umma_commit(bars + 8 * kDone);
+            volatile int keep_waiting = 0;                             // as above: no product when the tensor memory is released
+            mbar_wait(bars + 8 * kDone, 0, &keep_waiting, 0x506, kLimit, a.report);
         }
         __syncwarp();
     } else {
@@ -171,7 +178,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int i = 0; i < count; ++i) {
                 const int st = i % kStages;
-                if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x503, kLimit, a.report))) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(bars + 8 * (kFull + st), (i / kStages) & 1, abort_flag, 0x503, a.limit, a.report))) break;
                 uint4 u[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
@@ -195,7 +202,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             csum[8 * kTM + tid] = t;
         }
         // accumulator row = tensor-memory lane = tid; the stages are free once every product has completed
-        const bool ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * kDone, 0, abort_flag, 0x505, kLimit, a.report) && !*abort_flag);
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(bars + 8 * kDone, 0, abort_flag, 0x505, a.limit, a.report) && !*abort_flag);
         tc_fence_after();
         float* part = reinterpret_cast<float*>(smem) + tid * kPitch;
         const uint32_t acc = tmem + ((uint32_t)(32 * warp) << 16);
@@ -209,9 +216,6 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
 #pragma unroll
                 for (int e = 0; e < 8; ++e) *reinterpret_cast<float4*>(part + c + 4 * e) = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
             }
-        } else {
-            const float nan = __int_as_float(0x7fffffff);
-            for (int c = 0; c < TN; ++c) part[c] = nan;
         }
         tc_fence_before();
     }
@@ -224,6 +228,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
         uint32_t base[8];
 #pragma unroll
         for (int b = 0; b < 8; ++b) base[b] = cluster_addr(sb, b < a.split ? b : 0);
+        const int gave_up = lane < a.split ? cluster_load_int(cluster_addr(sb + kBars0 + 8 * kNumBars + 8, lane)) : 0;      // the blocks' abort_flag
         for (int e = tid; e < rows * wide; e += kThreads) {
             const int r = r0 + e / wide, c = e % wide * 4;
             const uint32_t off = (uint32_t)(r * kPitch + c) * 4;
@@ -239,6 +244,12 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
             float t = 0.f;
             for (int b = 0; b < a.split; ++b) t += cluster_load(cluster_addr(sb + kSum0 + (8 * kTM + tid) * 4, b));
             job.sum[c0 + sum_c + tid] = t;
+        }
+        if (__any_sync(0xffffffffu, gave_up)) {                        // each thread over what it wrote itself
+            const float nan = __int_as_float(0x7fffffff);
+            for (int e = tid; e < rows * wide; e += kThreads)
+                *reinterpret_cast<float4*>(job.dw + (size_t)(c0 + r0 + e / wide) * a.D + k0 + e % wide * 4) = make_float4(nan, nan, nan, nan);
+            if (sums && rank == 0 && tid < min(sum_cols, job.cols - c0 - sum_c)) job.sum[c0 + sum_c + tid] = nan;
         }
     }
     cluster_sync();                                                    // nobody's shared memory goes while others read it
@@ -310,12 +321,18 @@ cudaError_t read_wgrad_error(int* value, bool reset) {
     return e;
 }
 
-}  // namespace dsqg
+namespace wgrad {
 
-extern "C" int dsqg_weight_grads(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
-                                 int count, long long rows, int D, void* stream) {
-    using namespace dsqg;
-    using namespace dsqg::wgrad;
+template <int TN, bool STALL>
+cudaError_t launch(const Args& a, int tiles, const CUtensorMap* maps, cudaStream_t s) {
+    if (STALL)
+        if (cudaError_t e = cudaFuncSetAttribute(weight_grad_kernel<TN, STALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<TN>::total)) return e;
+    return launch_clusters_after(a.split, weight_grad_kernel<TN, STALL>, tiles * a.split, kThreads, Layout<TN>::total, s, a, maps[0], maps[1], maps[2], maps[3]);
+}
+
+template <bool STALL>
+int weight_grads(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
+                 int count, long long rows, int D, long long limit, void* stream) {
     if (!dy || !dy_stride || !cols || !x || !dw || !sums) return DSQG_ERR_NULL_POINTER;
     if (count < 1 || count > DSQG_WGRAD_MAX || rows < 1 || rows > (1LL << 30) || D < kBox || D % kBox || D > (1 << 20)) return DSQG_ERR_BAD_SHAPE;
     if (!stg::tensor_map_encoder_available()) return DSQG_ERR_UNSUPPORTED;
@@ -326,7 +343,7 @@ extern "C" int dsqg_weight_grads(const void* const* dy, const long long* dy_stri
     if (device_fit(dev, &fit) != cudaSuccess) { cudaGetLastError(); return DSQG_ERR_CUDA; }
     Args a = {};
     CUtensorMap maps[2 * DSQG_WGRAD_MAX] = {};
-    a.rows = (int)rows; a.D = D;
+    a.rows = (int)rows; a.D = D; a.limit = limit;
     for (int k = 0; k < count; ++k) {
         if (!dy[k] || !x[k] || !dw[k]) return DSQG_ERR_NULL_POINTER;
         if (cols[k] < kBox || cols[k] % kBox || cols[k] > (1 << 20)) return DSQG_ERR_BAD_SHAPE;
@@ -345,7 +362,24 @@ extern "C" int dsqg_weight_grads(const void* const* dy, const long long* dy_stri
     int tiles = 0;
     for (int k = 0; k < count; ++k) a.job[k].tiles_end = tiles += tiles_of(a.job[k].cols, D, p.wide ? 256 : 128);
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const cudaError_t e = p.wide ? launch_clusters_after(p.split, weight_grad_kernel<256>, tiles * p.split, kThreads, Layout<256>::total, s, a, maps[0], maps[1], maps[2], maps[3])
-                                 : launch_clusters_after(p.split, weight_grad_kernel<128>, tiles * p.split, kThreads, Layout<128>::total, s, a, maps[0], maps[1], maps[2], maps[3]);
+    const cudaError_t e = p.wide ? launch<256, STALL>(a, tiles, maps, s) : launch<128, STALL>(a, tiles, maps, s);
     return e == cudaSuccess ? DSQG_OK : DSQG_ERR_CUDA;
 }
+
+}  // namespace wgrad
+}  // namespace dsqg
+
+extern "C" {
+
+int dsqg_weight_grads(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
+                      int count, long long rows, int D, void* stream) {
+    return dsqg::wgrad::weight_grads<false>(dy, dy_stride, cols, x, dw, sums, count, rows, D, dsqg::wgrad::kLimit, stream);
+}
+
+int dsqg_test_weight_grads_timeout(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
+                                   int count, long long rows, int D, long long limit_cycles, void* stream) {
+    if (limit_cycles < 1 || limit_cycles > 2000000000LL) return DSQG_ERR_UNSUPPORTED;
+    return dsqg::wgrad::weight_grads<true>(dy, dy_stride, cols, x, dw, sums, count, rows, D, limit_cycles, stream);
+}
+
+}  // extern "C"

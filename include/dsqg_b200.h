@@ -318,6 +318,11 @@ int dsqg_column_sums(const void* const* src, const long long* row_stride, const 
                      void* stream);
 int dsqg_weight_grads(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
                       int count, long long rows, int D, void* stream);
+/* Test hook for its bounded waits (no counterpart in the reference): the last thread block of every cluster asks for half of its rows only, so that
+ * the waits for the others run out after limit_cycles (1 .. 2e9) SM cycles.  dw and sums are then NaN, dsqg_device_error() reports where, and
+ * nothing is left in flight. */
+int dsqg_test_weight_grads_timeout(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
+                                   int count, long long rows, int D, long long limit_cycles, void* stream);
 
 /* Single-token decode over a circular K/V ring buffer.
  * Replaces: nothing executable -- the reference only describes the O(1) cache in prose

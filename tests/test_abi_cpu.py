@@ -206,3 +206,4 @@ def test_strided_gate_scan_and_interleaved_ring_argument_errors(lib):
                                                 2, 2, kw.get("N", 8), kw.get("D", 64), kw.get("R", 16), 0, None)
     assert pre(k=None) == -1 and pre(kv=None) == -1 and pre(N=0) == -2 and pre(R=0) == -2 and pre(kv=_fake(3) + 4) == -5
     assert lib.dsqg_test_wait_timeout(0, None) == -8 and lib.dsqg_test_wait_timeout(3 * 10 ** 9, None) == -8
+    assert lib.dsqg_test_weight_grads_timeout(*[None] * 6, 1, 64, 64, 0, None) == -8 and lib.dsqg_test_weight_grads_timeout(*[None] * 6, 1, 64, 64, 1000, None) == -1

@@ -381,3 +381,28 @@ def test_a_wait_that_gave_up_is_reported_by_the_next_backward():
             _layer_gradients(128, 97)
     assert lib.dsqg_device_error(1) == 0x7e57 and lib.dsqg_device_error(0) == 0
     assert all(torch.equal(a, b) for a, b in zip(want, _layer_gradients(128, 97)))
+
+
+@pytest.mark.parametrize("rows,D,cols", [(64, 128, (128,)), (700, 192, (320, 64)), (4099, 256, (1024, 256))])
+def test_weight_grads_whose_waits_run_out_are_nan_throughout(rows, D, cols):
+    """A block that never gets the second half of its rows: every weight gradient and every column sum is NaN, the words say so, and the next call is as before."""
+    lib = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    dy, x = ([torch.randn(rows, c, generator=g, device="cuda").bfloat16() for c in cs] for cs in (cols, [D] * len(cols)))
+    dw, sums = [torch.empty(c + 1, D, device="cuda") for c in cols], [torch.empty(c + 1, device="cuda") for c in cols]
+    arr = lambda t, v: (t * len(v))(*v)  # noqa: E731
+    ptrs = lambda ts: arr(ctypes.c_void_p, [t.data_ptr() for t in ts])  # noqa: E731
+    args = (ptrs(dy), arr(ctypes.c_longlong, cols), arr(ctypes.c_int, cols), ptrs(x), ptrs(dw), ptrs(sums), len(cols), rows, D)
+
+    def call(timeout):
+        for t in (*dw, *sums):
+            t.fill_(7.0)
+        _lib.check(lib.dsqg_test_weight_grads_timeout(*args, 1000000, _stream()) if timeout else lib.dsqg_weight_grads(*args, _stream()), "weight_grads")
+        torch.cuda.synchronize()
+        return [t.clone() for t in (*dw, *sums)]
+    want = call(False)
+    for t in call(True):
+        assert t[:-1].isnan().all() and (t[-1] == 7).all()               # and nothing past the end
+    assert lib.dsqg_weight_grads(*args, _stream()) == -10
+    assert lib.dsqg_device_error(1) & ~0xf == 0x500 and lib.dsqg_device_error(0) == 0
+    assert all(torch.equal(a, b) for a, b in zip(want, call(False)))
