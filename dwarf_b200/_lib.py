@@ -78,6 +78,7 @@ _SIGNATURES = {
                                  ctypes.c_longlong, c_void_p]),
     "dsqg_weight_grads": (c_int, [POINTER(c_void_p), POINTER(ctypes.c_longlong), POINTER(c_int)] + [POINTER(c_void_p)] * 3
                           + [c_int, ctypes.c_longlong, c_int, c_void_p]),
+    "dsqg_weight_grads_split": (c_int, [POINTER(c_int), c_int, ctypes.c_longlong, c_int, POINTER(c_int)]),
     "dsqg_test_weight_grads_timeout": (c_int, [POINTER(c_void_p), POINTER(ctypes.c_longlong), POINTER(c_int)] + [POINTER(c_void_p)] * 3
                                        + [c_int, ctypes.c_longlong, c_int, ctypes.c_longlong, c_void_p]),
     "dsqg_causal_mean": (c_int, [c_void_p, c_void_p] + [c_int] * 5 + [c_void_p]),

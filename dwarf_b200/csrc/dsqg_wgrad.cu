@@ -257,7 +257,7 @@ weight_grad_kernel(const Args a, const __grid_constant__ CUtensorMap map_a0, con
     if (warp == kMmaWarp) tmem_dealloc(tmem, TN);
 }
 
-// Clusters of 1 .. kMostSplit blocks that run at once on the device (GPCs hold different numbers of SMs), asked once.
+// Clusters of 1 .. kMostSplit blocks that run at once on the device, asked once; only whether any does is of interest (choose).
 struct Fit { int clusters[2][kMostSplit + 1]; };
 template <int TN>
 cudaError_t fill_fit(int (&clusters)[kMostSplit + 1]) {
@@ -290,18 +290,20 @@ cudaError_t device_fit(int dev, const Fit** out) {
 int tiles_of(int cols, int D, int TN) { return (cols + kTM - 1) / kTM * ((D + TN - 1) / TN); }
 
 // What bounds a block is what its SM can fetch (90 GB/s measured; the tensor cores would take twice that), so the tile width and the split
-// are those with the least to fetch per block, rounds of clusters counted.
+// are those with the least to fetch per block, rounds of clusters counted.  How many clusters run at once differs from one B200 to the next (148 SMs in
+// GPCs of different sizes), but the split is the order of the sums, and a call has to return the same bits on every one: so the figures are
+// those of one GPU (cudaOccupancyMaxActiveClusters for both widths), wherever this runs.
+constexpr int kAtOnce[kMostSplit + 1] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
 struct Share { bool wide; int split; };
-Share choose(const Fit& fit, const Args& a, int count) {
+Share choose(const int* cols, int count, long long rows, int D) {
     Share best = {true, 1};
     long long least = -1;
-    const int blocks = (a.rows + kBox - 1) / kBox;
+    const long long blocks = (rows + kBox - 1) / kBox;
     for (int w = 1; w >= 0; --w) {
         int tiles = 0;
-        for (int k = 0; k < count; ++k) tiles += tiles_of(a.job[k].cols, a.D, w ? 256 : 128);
+        for (int k = 0; k < count; ++k) tiles += tiles_of(cols[k], D, w ? 256 : 128);
         for (int s = 1; s <= kMostSplit && s <= blocks; ++s) {
-            const int at_once = fit.clusters[w][s];
-            if (at_once < 1) continue;
+            const int at_once = kAtOnce[s];
             // steps of 64 rows, and about five steps' worth of time to start and to add the tiles
             const long long cost = (long long)((tiles + at_once - 1) / at_once) * ((blocks + s - 1) / s + 5) * (w ? 3 : 2);
             if (least < 0 || cost < least) { least = cost; best = {w != 0, s}; }
@@ -330,11 +332,18 @@ cudaError_t launch(const Args& a, int tiles, const CUtensorMap* maps, cudaStream
     return launch_clusters_after(a.split, weight_grad_kernel<TN, STALL>, tiles * a.split, kThreads, Layout<TN>::total, s, a, maps[0], maps[1], maps[2], maps[3]);
 }
 
+bool bad_sizes(const int* cols, int count, long long rows, int D) {
+    if (count < 1 || count > DSQG_WGRAD_MAX || rows < 1 || rows > (1LL << 30) || D < kBox || D % kBox || D > (1 << 20)) return true;
+    for (int k = 0; k < count; ++k)
+        if (cols[k] < kBox || cols[k] % kBox || cols[k] > (1 << 20)) return true;
+    return false;
+}
+
 template <bool STALL>
 int weight_grads(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
                  int count, long long rows, int D, long long limit, void* stream) {
     if (!dy || !dy_stride || !cols || !x || !dw || !sums) return DSQG_ERR_NULL_POINTER;
-    if (count < 1 || count > DSQG_WGRAD_MAX || rows < 1 || rows > (1LL << 30) || D < kBox || D % kBox || D > (1 << 20)) return DSQG_ERR_BAD_SHAPE;
+    if (bad_sizes(cols, count, rows, D)) return DSQG_ERR_BAD_SHAPE;
     if (!stg::tensor_map_encoder_available()) return DSQG_ERR_UNSUPPORTED;
     int dev = 0;
     const auto off16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; };
@@ -346,7 +355,6 @@ int weight_grads(const void* const* dy, const long long* dy_stride, const int* c
     a.rows = (int)rows; a.D = D; a.limit = limit;
     for (int k = 0; k < count; ++k) {
         if (!dy[k] || !x[k] || !dw[k]) return DSQG_ERR_NULL_POINTER;
-        if (cols[k] < kBox || cols[k] % kBox || cols[k] > (1 << 20)) return DSQG_ERR_BAD_SHAPE;
         if (off16(dy[k]) || off16(x[k]) || off16(dw[k]) || dy_stride[k] < cols[k] || dy_stride[k] % 8 || dy_stride[k] > (1 << 24)) return DSQG_ERR_MISALIGNED;
         a.job[k].cols = cols[k]; a.job[k].dw = dw[k]; a.job[k].sum = sums[k];
         // 64-column blocks of a row-major matrix as the "heads" of a tensor of 64-wide rows
@@ -357,7 +365,8 @@ int weight_grads(const void* const* dy, const long long* dy_stride, const int* c
     if (count == 1) { maps[2] = maps[0]; maps[3] = maps[1]; }
     if (wait_error_seen()) return DSQG_ERR_WAIT;
     a.report = wait_error_word();
-    const Share p = choose(*fit, a, count);
+    const Share p = choose(cols, count, rows, D);
+    if (fit->clusters[p.wide][p.split] < 1) return DSQG_ERR_UNSUPPORTED;       // part of a GPU that is too small for such a cluster
     a.split = p.split;
     int tiles = 0;
     for (int k = 0; k < count; ++k) a.job[k].tiles_end = tiles += tiles_of(a.job[k].cols, D, p.wide ? 256 : 128);
@@ -370,6 +379,15 @@ int weight_grads(const void* const* dy, const long long* dy_stride, const int* c
 }  // namespace dsqg
 
 extern "C" {
+
+int dsqg_weight_grads_split(const int* cols, int count, long long rows, int D, int* tile_cols) {
+    using namespace dsqg::wgrad;
+    if (!cols || !tile_cols) return DSQG_ERR_NULL_POINTER;
+    if (bad_sizes(cols, count, rows, D)) return DSQG_ERR_BAD_SHAPE;
+    const Share p = choose(cols, count, rows, D);
+    *tile_cols = p.wide ? 256 : 128;
+    return p.split;
+}
 
 int dsqg_weight_grads(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
                       int count, long long rows, int D, void* stream) {

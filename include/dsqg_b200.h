@@ -298,7 +298,10 @@ int dsqg_packed_bwd_gate(const dsqg_packed* p, const dsqg_packed_grads* g, const
  *   dsqg_column_sums     fp32 column sums of up to DSQG_SUM_MAX bf16 matrices of the same number of rows, fixed order
  *   dsqg_weight_grads    dw[k] [cols[k], D] = dy[k]^T . x[k] in fp32 and sums[k] [cols[k]] = column sums of dy[k] (null: left out) for
  *                        up to DSQG_WGRAD_MAX pairs of `rows` rows in one launch; dy rows dy_stride elements apart, x rows of D; D and
- *                        cols multiples of 64; fixed order of the sums; DSQG_ERR_UNSUPPORTED where the driver makes no tensor map for them
+ *                        cols multiples of 64; the order of the sums depends on the sizes alone; DSQG_ERR_UNSUPPORTED where the driver makes no tensor
+ *                        map for them or the device (a part of a GPU) is too small for the clusters
+ *   dsqg_weight_grads_split  that order: returns s, the number of ranges of rows whose fp32 sums are added first to last (range r begins at row
+ *                        64 floor(r ceil(rows / 64) / s)), or a negative status; *tile_cols: columns of dw a thread block forms.  Needs no device
  * D a multiple of 8 (layer norm: at most 1024); all pointers 16-byte aligned; src, dst, n, row_stride, cols: HOST arrays. */
 #define DSQG_CAST_MAX 8
 #define DSQG_SUM_MAX 4
@@ -318,6 +321,7 @@ int dsqg_column_sums(const void* const* src, const long long* row_stride, const 
                      void* stream);
 int dsqg_weight_grads(const void* const* dy, const long long* dy_stride, const int* cols, const void* const* x, float* const* dw, float* const* sums,
                       int count, long long rows, int D, void* stream);
+int dsqg_weight_grads_split(const int* cols, int count, long long rows, int D, int* tile_cols);
 /* Test hook for its bounded waits (no counterpart in the reference): the last thread block of every cluster asks for half of its rows only, so that
  * the waits for the others run out after limit_cycles (1 .. 2e9) SM cycles.  dw and sums are then NaN, dsqg_device_error() reports where, and
  * nothing is left in flight. */

@@ -207,3 +207,16 @@ def test_strided_gate_scan_and_interleaved_ring_argument_errors(lib):
     assert pre(k=None) == -1 and pre(kv=None) == -1 and pre(N=0) == -2 and pre(R=0) == -2 and pre(kv=_fake(3) + 4) == -5
     assert lib.dsqg_test_wait_timeout(0, None) == -8 and lib.dsqg_test_wait_timeout(3 * 10 ** 9, None) == -8
     assert lib.dsqg_test_weight_grads_timeout(*[None] * 6, 1, 64, 64, 0, None) == -8 and lib.dsqg_test_weight_grads_timeout(*[None] * 6, 1, 64, 64, 1000, None) == -1
+
+
+def test_split_of_the_weight_gradients_follows_from_the_sizes_alone():
+    """The order of dsqg_weight_grads' sums is the same on every GPU: it is known without one.  (ranges of rows, columns of a tile)"""
+    def split(cols, rows, D):
+        tile = ctypes.c_int(0)
+        return lib.dsqg_weight_grads_split((ctypes.c_int * len(cols))(*cols), len(cols), rows, D, ctypes.byref(tile)), tile.value
+    lib = _lib.load()
+    want = {((1024, 256), 1, 256): (1, 128), ((1024, 256), 1024, 256): (6, 128), ((1024, 256), 65536, 256): (6, 128), ((512, 256), 16384, 256): (8, 128),
+            ((512, 128), 1024, 128): (8, 128), ((768, 192), 16384, 192): (6, 128), ((2048, 512), 16384, 512): (3, 256)}
+    assert {k: split(*k) for k in want} == want
+    assert split((1024,), 0, 256)[0] == split((1000,), 64, 256)[0] == split((64,), 64, 100)[0] == -2
+    assert lib.dsqg_weight_grads_split(None, 1, 64, 64, None) == -1
