@@ -60,7 +60,7 @@ struct BwdArgs {
     int B, H, N, D;
     float scale;
     // Strided addressing as in FwdArgs: in_* for q, k, v, dq, dk, dv; out_* for out and dout.
-    // delta_pre (nullable, [B,H,N] fp32): sum_d dout*out per row when an earlier kernel formed it.
+    // delta_pre (nullable, [B,H,N] fp32): sum_d dout*out per row when the caller of a strided entry formed it (dsqg_gate_bwd does); an operator call leaves it null.
     int strided;
     long long in_sb, in_sh, in_sn, out_sb, out_sh, out_sn;
     const float* delta_pre;

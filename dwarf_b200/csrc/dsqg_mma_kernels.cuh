@@ -635,7 +635,7 @@ __device__ __forceinline__ float dq_tile(const BwdArgs& a, const float* start, c
             *reinterpret_cast<uint4*>(qrow + 8 * (2 * D + 16) + o) = make_uint4(qb.r[4 * c], qb.r[4 * c + 1], qb.r[4 * c + 2], qb.r[4 * c + 3]);
         }
     }
-    if (ST && ST != kKept && have_dout && a.delta_pre) {       // sum_d dout*out was formed by an earlier kernel (gate backward)
+    if (ST && ST != kKept && have_dout && a.delta_pre) {       // sum_d dout*out was handed in by a caller of the strided entries
         delta_lo = ok_lo ? a.delta_pre[(size_t)bh * N + row_lo] : 0.f;
         delta_hi = ok_hi ? a.delta_pre[(size_t)bh * N + row_hi] : 0.f;
     } else if (have_dout) {
